@@ -121,6 +121,22 @@ class SelectArgs(C.Structure):
     ]
 
 
+class DescentArgs(C.Structure):
+    _fields_ = [
+        ("V", C.c_int), ("T", C.c_int), ("K", C.c_int), ("P", C.c_int), ("n_designs", C.c_int), ("ld", C.c_int),
+        ("p0", C.c_int), ("n_a", C.c_int), ("n_b", C.c_int), ("za", C.c_int), ("zb", C.c_int), ("ltop", C.c_int),
+        ("n_groups", C.c_int), ("n_list", C.c_int), ("n_rounds", C.c_int), ("n_cell_groups", C.c_int),
+        ("n_chunks", C.c_int), ("rows", C.c_void_p), ("yr_hi", C.c_void_p), ("yr_lo", C.c_void_p),
+        ("yexp", C.c_void_p), ("u_hi", C.c_void_p), ("u_lo", C.c_void_p), ("uexp", C.c_void_p),
+        ("coef", C.c_void_p), ("logdet_R", C.c_void_p), ("logdet_XtX", C.c_void_p),
+        ("chunk_start", C.c_void_p), ("chunk_pairs", C.c_void_p), ("slots", C.c_void_p), ("list", C.c_void_p),
+        ("lat_slot", C.c_void_p), ("lattice", C.c_void_p), ("cell_slots", C.c_void_p),
+        ("cell_group", C.c_void_p), ("cell_pairs", C.c_void_p), ("cell_list", C.c_void_p),
+        ("tile_design", C.c_void_p), ("best", C.c_void_p), ("best_crit", C.c_void_p), ("flag", C.c_void_p),
+        ("work", C.c_void_p), ("work_bytes", C.c_size_t),
+    ]
+
+
 class GlsArgs(C.Structure):
     _fields_ = [
         ("V", C.c_int), ("T", C.c_int), ("K", C.c_int), ("dof", C.c_int), ("center", C.c_int),
@@ -157,6 +173,8 @@ SIGNATURES = {
     "ffs_reml_project_simt": ([C.POINTER(ProjectArgs), C.c_void_p], C.c_int),
     "ffs_reml_surface": ([C.POINTER(SurfaceArgs), C.c_void_p], C.c_int),
     "ffs_reml_select": ([C.POINTER(SelectArgs), C.c_void_p], C.c_int),
+    "ffs_reml_descent_work_bytes": ([C.POINTER(DescentArgs)], C.c_size_t),
+    "ffs_reml_descent": ([C.POINTER(DescentArgs), C.c_void_p], C.c_int),
     "ffs_reml_gls": ([C.POINTER(GlsArgs), C.c_void_p], C.c_int),
     "ffs_reml_set_stats": ([C.POINTER(SetStatsArgs), C.c_void_p], C.c_int),
     "ffs_reml_gls_dsort": ([C.POINTER(DsortArgs), C.c_void_p], C.c_int),

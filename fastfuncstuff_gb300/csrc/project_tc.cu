@@ -19,12 +19,18 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
+#include "project_tc.cuh"
 
 namespace ffsk {
 namespace {
+
+// GRID: every voxel against every pair, in order. LIST: the caller's work
+// items. PAIRS: row tiles against lists of pairs (PairProject).
+enum Mode { GRID, LIST, PAIRS };
 
 constexpr int BM = 128;         // voxels per tile (TMEM lanes)
 constexpr int BK = 64;          // k elements per stage (one 128-byte swizzle row)
@@ -46,18 +52,49 @@ struct TcParams {
   float* proj;
   int* flag;
   const int* v_dev;    // grid mode: device count of the operand rows to project (or NULL: V)
+  // pairs mode (PairProject): nblk blocks of at most g pairs per row tile, a
+  // pair's K columns of B at every kp = K rounded up to 8 (the 1024-byte
+  // repeat of the 128-byte swizzle, so that each pair's box lands in phase)
+  const int* list;
+  int n_list, kp, nblk, Pd;
+  const int* tile_design;
+  const int4* tiles;
+  const int* n_tiles;
 };
 
 // One work item: BM operand rows from v0 (nv of them real) against the np
 // pairs whose U rows start at row_b.
 struct Item {
   int v0, nv, row_b, np, out0, slot0, N;
+  const int* list;  // pairs mode: the np entries; row_b is then the design's first pair
 };
 
-template <bool LIST>
+template <Mode MODE>
 __device__ __forceinline__ Item item_at(const TcParams& prm, int item, int Vd) {
   Item it;
-  if (LIST) {
+  if (MODE == PAIRS) {
+    const int t = item / prm.nblk, first = (item % prm.nblk) * prm.g;
+    int dsg = 0, n = prm.n_list;
+    it.list = prm.list;
+    if (prm.tiles) {
+      const int4 w = prm.tiles[t];
+      it.v0 = w.x;
+      it.nv = w.y;
+      dsg = w.z / prm.Pd;
+      it.list += (size_t)(w.z % prm.Pd) * PAIR_SLOTS;
+      for (n = 0; n < PAIR_SLOTS && it.list[n] >= 0;) ++n;
+    } else {
+      it.v0 = t * BM;
+      it.nv = min(BM, prm.V - it.v0);
+      if (prm.tile_design) dsg = prm.tile_design[it.v0 >> 8];
+    }
+    it.row_b = dsg * prm.Pd;
+    it.list += first;
+    it.np = max(0, min(prm.g, n - first));
+    it.out0 = it.v0;
+    it.slot0 = 0;
+    it.N = (it.np * prm.kp + 15) / 16 * 16;
+  } else if (MODE == LIST) {
     const ffs_tc_item w = prm.items[item];
     it.v0 = w.v0;
     it.nv = w.nv;
@@ -149,7 +186,7 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 // run together share voxel tiles in L2). The TMA ring of STAGES k-blocks runs
 // across items; TMEM holds two 256-column accumulators so the epilogue warps
 // drain item i while the MMA warp accumulates item i + 1.
-template <bool LIST>
+template <Mode MODE>
 __global__ void __launch_bounds__(192, 1)
     project_tc_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
                       const __grid_constant__ CUtensorMap tb_hi, const __grid_constant__ CUtensorMap tb_lo,
@@ -168,8 +205,10 @@ __global__ void __launch_bounds__(192, 1)
   if (*reinterpret_cast<volatile int*>(prm.flag) != 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // grid mode: the rows to project (a device count when given)
-  const int Vd = (!LIST && prm.v_dev) ? min(prm.V, max(0, *prm.v_dev)) : prm.V;
-  const int n_items = LIST ? *prm.n_items : prm.n_col_tiles * ((Vd + BM - 1) / BM);
+  const int Vd = (MODE == GRID && prm.v_dev) ? min(prm.V, max(0, *prm.v_dev)) : prm.V;
+  const int n_items = MODE == LIST    ? *prm.n_items
+                      : MODE == PAIRS ? prm.nblk * (prm.tiles ? *prm.n_tiles : (prm.V + BM - 1) / BM)
+                                      : prm.n_col_tiles * ((Vd + BM - 1) / BM);
   const int nk = prm.ld / BK;
 
   if (threadIdx.x == 0) {
@@ -198,8 +237,9 @@ __global__ void __launch_bounds__(192, 1)
     int kc = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-      const Item it = item_at<LIST>(prm, item, Vd);
+      const Item it = item_at<MODE>(prm, item, Vd);
       const int v0 = it.v0, row_b = it.row_b;
+      if (MODE == PAIRS && it.np == 0) continue;  // a block past the end of the cell's list
       for (int kb = 0; kb < nk; ++kb, ++kc) {
         const int s = kc % STAGES;
         if (kc >= STAGES && !mbar_wait(empty + s, ((kc / STAGES) - 1) & 1)) {
@@ -208,20 +248,31 @@ __global__ void __launch_bounds__(192, 1)
           break;
         }
         uint8_t* st = smem + s * stage_bytes;
-        mbar_expect_tx(full + s, (uint32_t)stage_bytes);
+        mbar_expect_tx(full + s, MODE == PAIRS ? (uint32_t)(2 * A_TILE + it.np * prm.K * BK * 4) : (uint32_t)stage_bytes);
         const int k0 = kb * BK;
         tma_load_2d(st, &ta_hi, full + s, k0, v0);
         tma_load_2d(st + A_TILE, &ta_lo, full + s, k0, v0);
-        tma_load_2d(st + 2 * A_TILE, &tb_hi, full + s, k0, row_b);
-        tma_load_2d(st + 2 * A_TILE + b_tile, &tb_lo, full + s, k0, row_b);
+        if (MODE == PAIRS) {
+          uint8_t* b = st + 2 * A_TILE;
+          for (int i = 0; i < it.np; ++i, b += prm.kp * BK * 2) {
+            const int r = (row_b + (it.list[i] & 0xffffff)) * prm.K;
+            tma_load_2d(b, &tb_hi, full + s, k0, r);
+            tma_load_2d(b + b_tile, &tb_lo, full + s, k0, r);
+          }
+        } else {
+          tma_load_2d(st + 2 * A_TILE, &tb_hi, full + s, k0, row_b);
+          tma_load_2d(st + 2 * A_TILE + b_tile, &tb_lo, full + s, k0, row_b);
+        }
       }
     }
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer
     int kc = 0, local = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++local) {
-      const uint32_t idesc = idesc_f16(BM, item_at<LIST>(prm, item, Vd).N);
+    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+      const Item it = item_at<MODE>(prm, item, Vd);
+      if (MODE == PAIRS && it.np == 0) continue;
+      const uint32_t idesc = idesc_f16(BM, it.N);
       const int buf = local & 1;
       const uint32_t acc = tmem + (uint32_t)(buf * 256);
       if (local >= 2 && !mbar_wait(acc_empty + buf, ((local >> 1) - 1) & 1)) {
@@ -255,13 +306,19 @@ __global__ void __launch_bounds__(192, 1)
         mma_commit(empty + s);
       }
       mma_commit(acc_full + buf);
+      ++local;
     }
   } else if (warp >= 2) {
     // ---- epilogue: square and sum each pair's K columns from TMEM
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     const int row = q * 32 + lane;
     int local = 0;
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++local) {
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+      Item pit;
+      if (MODE == PAIRS) {
+        pit = item_at<MODE>(prm, item, Vd);
+        if (pit.np == 0) continue;
+      }
       const int buf = local & 1;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full + buf, (local >> 1) & 1));
       if (!ok) {
@@ -272,8 +329,14 @@ __global__ void __launch_bounds__(192, 1)
       // grid mode keeps the exact form whose timing was measured best; the
       // work-list mode differs in where the result goes
       int v, p_first, ncols, nmax, out_row, out_slot = 0;
-      if (LIST) {
-        const Item it = item_at<LIST>(prm, item, Vd);
+      if (MODE == PAIRS) {
+        v = row < pit.nv ? pit.v0 + row : prm.V;
+        p_first = pit.row_b;
+        ncols = pit.np * prm.kp;
+        nmax = pit.N;
+        out_row = 0;
+      } else if (MODE == LIST) {
+        const Item it = item_at<MODE>(prm, item, Vd);
         v = row < it.nv ? it.v0 + row : prm.V;
         p_first = it.row_b / prm.K;
         ncols = it.np * prm.K;
@@ -303,16 +366,28 @@ __global__ void __launch_bounds__(192, 1)
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          if (c0 + i < ncols) {
+          if (MODE == PAIRS && c0 + i < ncols) {
+            const float x = __uint_as_float(r[i]);
+            if (j < prm.K) run = fmaf(x, x, run);  // columns K .. kp of a pair hold nothing
+            if (++j == prm.kp) {
+              const int e = pit.list[pl], p = p_first + (e & 0xffffff), slot = e >> 24;
+              if (v < prm.V)
+                prm.proj[prm.tiles ? (size_t)v * PAIR_SLOTS + slot : (size_t)slot * prm.V + v] =
+                    ldexpf(run, -2 * (ey + prm.uexp[p]));
+              run = 0.f;
+              j = 0;
+              ++pl;
+            }
+          } else if (MODE != PAIRS && c0 + i < ncols) {
             const float x = __uint_as_float(r[i]);
             run = fmaf(x, x, run);
             if (++j == prm.K) {
               const int p = p_first + pl;
               if (p < prm.P && v < prm.V) {
                 const float val = ldexpf(run, -2 * (ey + prm.uexp[p]));
-                if (LIST && prm.s_vox > 0)
+                if (MODE == LIST && prm.s_vox > 0)
                   prm.proj[(size_t)out_row + pl] = val;
-                else if (LIST)
+                else if (MODE == LIST)
                   prm.proj[(size_t)(out_slot + pl) * prm.V + out_row] = val;
                 else
                   prm.proj[(size_t)p * prm.V + v] = val;
@@ -327,6 +402,7 @@ __global__ void __launch_bounds__(192, 1)
       // this accumulator may be overwritten now
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty + buf)) : "memory");
+      ++local;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -381,7 +457,7 @@ int launch_tc(const ffs_project_args* a, const TcParams& prm, int max_items, voi
   const int stage_bytes = 2 * A_TILE + 2 * prm.NB * BK * 2;
   const size_t smem = (size_t)STAGES * stage_bytes + 1024 + 128;
   FFS_REQUIRE(smem <= 227 * 1024, "project_tc: tile needs %zu bytes of shared memory", smem);
-  auto kern = prm.items ? project_tc_kernel<true> : project_tc_kernel<false>;
+  auto kern = prm.items ? project_tc_kernel<LIST> : project_tc_kernel<GRID>;
   FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), smem));
   int n_sm = 0;
   FFS_CUDA(sm_count(&n_sm));
@@ -406,6 +482,47 @@ int tc_pairs_for(int K, int P) {
 }
 
 }  // namespace
+
+int project_pairs(const PairProject& a, cudaStream_t stream) {
+  TcParams prm{};
+  prm.V = a.V;
+  prm.K = a.K;
+  prm.P = a.P;
+  prm.ld = a.ld;
+  prm.T = a.T;
+  prm.kp = (a.K + 7) & ~7;
+  const int most = a.tiles ? PAIR_SLOTS : a.n_list;  // pairs of one row tile
+  prm.g = std::min(most, 256 / prm.kp);
+  prm.nblk = ceil_div(most, prm.g);
+  prm.N = (prm.g * prm.kp + 15) / 16 * 16;
+  prm.NB = prm.N;
+  prm.n_col_tiles = 1;
+  prm.yexp = a.yexp;
+  prm.uexp = a.uexp;
+  prm.proj = a.proj;
+  prm.flag = a.flag;
+  prm.list = a.list;
+  prm.n_list = a.n_list;
+  prm.Pd = a.P;
+  prm.tile_design = a.tile_design;
+  prm.tiles = a.tiles;
+  prm.n_tiles = a.n_tiles;
+  CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
+  int st;
+  if ((st = make_map(&ta_hi, a.hi, a.ld, a.V, BM))) return st;
+  if ((st = make_map(&ta_lo, a.lo, a.ld, a.V, BM))) return st;
+  if ((st = make_map(&tb_hi, a.u_hi, a.ld, a.n_designs * a.P * a.K, a.K))) return st;
+  if ((st = make_map(&tb_lo, a.u_lo, a.ld, a.n_designs * a.P * a.K, a.K))) return st;
+  const size_t smem = (size_t)STAGES * (2 * A_TILE + 2 * prm.NB * BK * 2) + 1024 + 128;
+  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(project_tc_kernel<PAIRS>), smem));
+  int n_sm = 0;
+  FFS_CUDA(sm_count(&n_sm));
+  const long long items = (long long)prm.nblk * (a.tiles ? a.max_tiles : ceil_div(a.V, BM));
+  project_tc_kernel<PAIRS><<<(int)std::min<long long>(items, n_sm), 192, smem, stream>>>(ta_hi, ta_lo, tb_hi, tb_lo,
+                                                                                        prm);
+  return check_launch("project_tc_kernel (pairs)");
+}
+
 }  // namespace ffsk
 
 using namespace ffsk;
@@ -432,7 +549,7 @@ extern "C" int ffs_reml_project_tc(const ffs_project_args* a, void* stream) {
   }
   for (const void* ptr : {(const void*)a->yr_hi, (const void*)a->yr_lo, (const void*)a->u_hi, (const void*)a->u_lo})
     FFS_REQUIRE(((uintptr_t)ptr & 15) == 0, "ffs_reml_project_tc: operands must be 16-byte aligned");
-  TcParams prm;
+  TcParams prm{};
   prm.V = a->V;
   prm.K = a->K;
   prm.P = a->P;
@@ -467,7 +584,7 @@ extern "C" int ffs_reml_project_tc_list(const ffs_project_args* a, const ffs_tc_
               "ffs_reml_project_tc_list: max_pairs=%d x K=%d must fit one 256-column tile", max_pairs, a->K);
   for (const void* ptr : {(const void*)a->yr_hi, (const void*)a->yr_lo, (const void*)a->u_hi, (const void*)a->u_lo})
     FFS_REQUIRE(((uintptr_t)ptr & 15) == 0, "ffs_reml_project_tc_list: operands must be 16-byte aligned");
-  TcParams prm;
+  TcParams prm{};
   prm.V = a->V;
   prm.K = a->K;
   prm.P = a->P;

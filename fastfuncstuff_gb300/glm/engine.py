@@ -26,7 +26,7 @@ import numpy as np
 import torch
 
 from .. import _lib
-from .grid import RemlGrid, RunLayout
+from .grid import RemlGrid, RunLayout, descent_plan
 
 LD_ALIGN = 64  # k extent of one tcgen05 pipeline stage
 
@@ -649,6 +649,66 @@ def prep(Y: torch.Tensor, f: GridFactors, *, do_scale: bool = True, tensor_core:
     return out
 
 
+def _descent_plan(f: GridFactors, V: int):
+    """The device arrays of the grid's descent plan when ``V`` voxels are
+    better searched by it than over the full surface, else None."""
+    if f.U_hi is None or f.band_coef is not None or V * f.P * f.T < DESCENT_MIN_WORK:
+        return None
+    g, dev = f.grid, f.coef.device
+    cached = g.__dict__.setdefault("_descent", {})
+    if "plan" not in cached:
+        cached["plan"] = descent_plan(g)
+    plan = cached["plan"]
+    if plan is None or DESCENT_SHARE * plan.evaluated > g.P:
+        return None
+    if str(dev) not in cached:
+        cached[str(dev)] = {k: torch.from_numpy(np.ascontiguousarray(getattr(plan, k))).to(dev)
+                            for k in ("slots", "list", "lat_slot", "cell_slots", "cell_group", "cell_pairs", "cell_list")}
+    return plan, cached[str(dev)]
+
+
+# The descent takes about twenty launches where the full surface takes three:
+# below this many voxels x pairs x samples the surface is no slower (search of
+# V voxels, us, descent / surface: 117 pairs, T = 400: V = 8,000 213 / 192,
+# 16,000 328 / 339; 561 pairs, T = 400: 2,000 267 / 208, 4,000 275 / 329,
+# 200,000 2656 / 12052; T = 200: 4,000 211 / 194, 8,000 220 / 317). A grid of
+# which the descent could read more than half takes the surface too.
+DESCENT_MIN_WORK = 600_000_000
+DESCENT_SHARE = 2
+
+
+def descent(pr: PrepOut, f: GridFactors, plan, *, tile_design: torch.Tensor | None = None):
+    """(best [V], best_crit [V], flag) of the prepared rows (``rows``,
+    ``yr_hi``, ``yr_lo``, ``yexp``) by the hierarchical descent, which forms
+    only the pairs it reads (``ffs_reml_descent``); ``plan`` from
+    ``_descent_plan``. The answers are the full surface's bit for bit."""
+    lib = _lib.load()
+    dev = f.coef.device
+    p, d = plan
+    g = f.grid
+    V, T = pr.rows.shape
+    best = torch.empty(V, dtype=torch.int32, device=dev)
+    best_crit = torch.empty(V, dtype=torch.float32, device=dev)
+    flag = torch.zeros(1, dtype=torch.int32, device=dev)
+    a = _lib.DescentArgs(V=V, T=T, K=f.K, P=f.P, n_designs=f.n_designs, ld=f.ld, p0=g.p0, n_a=len(g.a_axis),
+                         n_b=len(g.b_axis), za=g.za, zb=g.zb, ltop=g.ltop, n_groups=p.n_groups, n_list=p.list.size,
+                         n_rounds=p.n_rounds, n_cell_groups=p.cell_slots.shape[0], n_chunks=f.chunk_start.numel() - 1,
+                         rows=_p(pr.rows), yr_hi=_p(pr.yr_hi), yr_lo=_p(pr.yr_lo), yexp=_p(pr.yexp), u_hi=_p(f.U_hi),
+                         u_lo=_p(f.U_lo), uexp=_p(f.uexp), coef=_p(f.coef), logdet_R=_p(f.logdet_R),
+                         logdet_XtX=_p(f.logdet_XtX), chunk_start=_p(f.chunk_start), chunk_pairs=_p(f.chunk_pairs),
+                         slots=_p(d["slots"]), list=_p(d["list"]), lat_slot=_p(d["lat_slot"]), lattice=_p(f.lattice),
+                         cell_slots=_p(d["cell_slots"]), cell_group=_p(d["cell_group"]),
+                         cell_pairs=_p(d["cell_pairs"]), cell_list=_p(d["cell_list"]), tile_design=_p(tile_design),
+                         best=_p(best), best_crit=_p(best_crit), flag=_p(flag))
+    n = int(lib.ffs_reml_descent_work_bytes(C.byref(a)))
+    if n == 0:
+        raise ValueError("ffs_reml_descent: " + lib.ffs_last_error().decode())
+    work = torch.empty(n, dtype=torch.uint8, device=dev)
+    a.work, a.work_bytes = _p(work), n
+    _run("ffs_reml_descent", lib.ffs_reml_descent, C.byref(a), _stream(), launches=5 + 9 * p.n_rounds)
+    return best, best_crit, flag
+
+
 def search(Y: torch.Tensor, f: GridFactors, *, hierarchical: bool = True, projector: str = "tc",
            do_scale: bool = True, keep_surface: bool = False, keep_yr: bool = False,
            q0: torch.Tensor | None = None, join=None) -> SearchOut:
@@ -667,9 +727,15 @@ def search(Y: torch.Tensor, f: GridFactors, *, hierarchical: bool = True, projec
         raise ValueError("the factors were built without the tensor-core operands")
     if projector not in ("tc", "simt"):
         raise ValueError(f"unknown projector {projector!r}")
-    pr = prep(Y, f, do_scale=do_scale, tensor_core=use_tc, q0=q0)
+    plan = _descent_plan(f, V) if hierarchical and use_tc and not (keep_surface or keep_yr) else None
+    pr = prep(Y, f, do_scale=do_scale, tensor_core=use_tc, q0=q0, want_yr_t=plan is None, want_rows=plan is not None)
     if join is not None:  # the factors may still be in flight on another stream
         join()
+    if plan is not None:
+        best, best_crit, flag = descent(pr, f, plan)
+        out = SearchOut(best=best, best_crit=best_crit, scale=pr.scale)
+        out._flag = flag
+        return out
 
     proj = torch.empty(P, V, dtype=torch.float32, device=dev)
     flag = torch.zeros(1, dtype=torch.int32, device=dev)
@@ -781,15 +847,25 @@ def search_designs(Y: torch.Tensor, f: GridFactors, slots: DesignSlots, *, hiera
     Y = Y.to(dtype=torch.float32).contiguous()
     q0 = f.U.view(D, P, K, -1)[:, f.grid.p0].contiguous()  # [D][K][ld_t]: U of (0, 0) per design
     scale = torch.empty(V, dtype=torch.float32, device=dev)
-    yr_t = torch.empty(T, Vp, dtype=torch.float32, device=dev)
+    plan = _descent_plan(f, V) if hierarchical else None
+    yr_t = torch.empty(T, Vp, dtype=torch.float32, device=dev) if plan is None else None
+    rows = torch.empty(Vp, T, dtype=torch.float32, device=dev) if plan is not None else None
     yr_hi = torch.empty(Vp, ld, dtype=torch.int16, device=dev)
     yr_lo = torch.empty(Vp, ld, dtype=torch.int16, device=dev)
     yexp = torch.empty(Vp, dtype=torch.int32, device=dev)
     pa = _lib.PrepArgs(V=Vp, T=T, K=K, Y=_p(Y), Q0=_p(q0), do_scale=int(do_scale), center=0, ld_y=ld,
                        scale=_p(scale), yr_t=_p(yr_t), yr_hi=_p(yr_hi), yr_lo=_p(yr_lo), yexp=_p(yexp),
-                       idx=_p(slots.idx), feats=None, n_runs=0, run_start=None, yr_rows=None,
+                       idx=_p(slots.idx), feats=None, n_runs=0, run_start=None, yr_rows=_p(rows),
                        center_dev=_p(f.center_flag), tile_design=_p(slots.tile32))
     _run("ffs_reml_prep", lib.ffs_reml_prep, C.byref(pa), st)
+    if plan is not None:
+        pr = PrepOut(scale, None, yr_hi, yr_lo, yexp)
+        pr.rows = rows
+        best, best_crit, flag = descent(pr, f, plan, tile_design=slots.tile256)
+        out = SearchOut(best=best[slots.real], best_crit=best_crit[slots.real], scale=scale)
+        out._flag = flag
+        out._keep = (q0, pr)
+        return out
 
     proj = torch.empty(P, Vp, dtype=torch.float32, device=dev)
     flag = torch.zeros(1, dtype=torch.int32, device=dev)

@@ -235,6 +235,116 @@ def hierarchical_ltop(n_a: int, n_b: int, afni_faithful: bool) -> int:
     return max(0, min(n_a, n_b).bit_length() - 2)
 
 
+DESCENT_SLOTS = 8    # pair slots per group, and neighbours per cell (csrc/descent.cu D_SLOTS)
+DESCENT_GROUPS = 8   # most groups of the levels every voxel evaluates (TOP_GROUPS)
+
+
+@dataclass
+class DescentPlan:
+    """Where the hierarchical descent's pairs sit (ffs_descent_args), from the lattice alone."""
+
+    slots: np.ndarray       # (n_groups * 8,) pairs of the levels every voxel evaluates
+    list: np.ndarray        # pair | slot << 24, (0, 0) last
+    lat_slot: np.ndarray    # (n_a * n_b,)
+    cell_slots: np.ndarray  # (n_cell_groups, 8)
+    cell_group: np.ndarray  # (n_rounds, P)
+    cell_pairs: np.ndarray  # (n_rounds, P, 8)
+    cell_list: np.ndarray   # (n_rounds, P, 8)
+
+    @property
+    def n_groups(self) -> int:
+        return self.slots.size // DESCENT_SLOTS
+
+    @property
+    def n_rounds(self) -> int:
+        return self.cell_group.shape[0]
+
+    @property
+    def evaluated(self) -> int:
+        """Most pairs a voxel is evaluated at."""
+        return self.list.size - 1 + DESCENT_SLOTS * self.n_rounds
+
+
+def descent_plan(g: RemlGrid) -> DescentPlan | None:
+    """The plan of the grid's hierarchical descent (fastfuncstuff/glm/arma.py:2224-2322);
+    None when its first level alone has more pairs than the top kernel takes.
+
+    The pairs that some voxel can read at each level follow from the lattice:
+    level ltop reads a fixed sub-lattice, each later one the neighbours (clamped
+    to the lattice) of the cells reachable so far. The levels join the first
+    evaluation while its pairs fit the top kernel; each level after them is a
+    round over the reachable cells."""
+    n_a, n_b = g.lattice.shape
+    ident = lambda_is_zero(g.a, g.b)
+
+    def neighbours(ai, bi, step):
+        """The <= 8 other lattice points a level reads around (ai, bi), in its order."""
+        seen, out = {(ai, bi)}, []
+        for ob in (-1, 0, 1):
+            for oa in (-1, 0, 1):
+                at = (min(max(ai + oa * step, 0), n_a - 1), min(max(bi + ob * step, 0), n_b - 1))
+                if at not in seen:
+                    seen.add(at)
+                    out.append(at)
+        return out
+
+    top = 1 << g.ltop
+    cells = {(g.za, g.zb)} | {(i, j) for j in range(0, n_b, top) for i in range(0, n_a, top)}
+    cells = {c for c in cells if g.lattice[c] >= 0}
+
+    def slots_of(points):
+        p = np.array(sorted(int(g.lattice[c]) for c in points), np.int64)
+        p = p[~ident[p]]
+        if p.size == 0:
+            return np.full(DESCENT_SLOTS, -1, np.int32)
+        _, rank = coefficient_chunks(g.a[p], g.b[p])
+        out = np.where(rank >= 0, p[np.maximum(rank, 0)], -1).astype(np.int32)
+        return np.concatenate([out, np.full(-out.size % DESCENT_SLOTS, -1, np.int32)])
+
+    slots, level = slots_of(cells), g.ltop
+    if slots.size > DESCENT_SLOTS * DESCENT_GROUPS:
+        return None
+    while level > 0:
+        more = cells | {q for c in cells for q in neighbours(*c, 1 << (level - 1)) if g.lattice[q] >= 0}
+        s = slots_of(more)
+        if s.size > DESCENT_SLOTS * DESCENT_GROUPS:
+            break
+        cells, slots, level = more, s, level - 1
+    filled = np.nonzero(slots >= 0)[0]
+    pair_list = np.concatenate([slots[filled] | (filled << 24), [g.p0 | (slots.size << 24)]]).astype(np.int32)
+    lat_slot = np.full((n_a, n_b), -1, np.int32)
+    at = {int(slots[i]): int(i) for i in filled}
+    for c in cells:
+        p = int(g.lattice[c])
+        lat_slot[c] = -2 if ident[p] else at[p]
+    n_rounds, S = level, DESCENT_SLOTS
+    cell_group = np.zeros((n_rounds, g.P), np.int32)
+    cell_pairs = np.full((n_rounds, g.P, S), -1, np.int32)
+    cell_list = np.full((n_rounds, g.P, S), -1, np.int32)
+    cell_slots: list = []
+    for r in range(n_rounds):
+        reach = set()
+        for c in sorted(cells):
+            p, own, lst = int(g.lattice[c]), [-1] * S, []
+            for s_, q in enumerate(neighbours(*c, 1 << (n_rounds - 1 - r))):
+                pq = int(g.lattice[q])
+                if pq < 0:
+                    continue
+                reach.add(q)
+                if ident[pq]:
+                    cell_pairs[r, p, s_] = -2 - pq
+                else:
+                    cell_pairs[r, p, s_] = own[s_] = pq
+                    lst.append(pq | (s_ << 24))
+            cell_list[r, p, : len(lst)] = lst
+            cell_group[r, p] = len(cell_slots)
+            cell_slots.append(own)
+        cells = cells | reach
+    return DescentPlan(slots=slots, list=pair_list, lat_slot=lat_slot.reshape(-1),
+                       cell_slots=np.array(cell_slots, np.int32).reshape(-1, S), cell_group=cell_group,
+                       cell_pairs=cell_pairs, cell_list=cell_list)
+
+
 def make_grid(a_grid, b_grid, use_double: bool = False) -> RemlGrid:
     """Valid pairs of the grids, in the reference's order.
 

@@ -378,6 +378,58 @@ typedef struct {
 
 int ffs_reml_select(const ffs_select_args* a, void* stream);
 
+/* ------------------------------------------------------------- hierarchical descent
+ * The hierarchical selector of ffs_reml_select without the full surface: the
+ * pairs that AFNI's descent reads are formed and no others (projection,
+ * recurrence and criterion as ffs_reml_project_tc and ffs_reml_surface form
+ * them, bit for bit, so best and best_crit are theirs). The first levels are
+ * evaluated for every row at the pairs of `slots`; each of the n_rounds levels
+ * left sorts the rows by their pair (the cell) and evaluates the cell's <= 8
+ * neighbours. The plan (which pair sits where) depends on the lattice only:
+ *   slots       [n_groups * 8] pairs of the first levels that are not identity
+ *               pairs (lambda == 0), quarters of 4 slots sharing one a, -1 empty
+ *   list        [n_list] pair | slot << 24 of the filled slots, then p0 at slot
+ *               n_groups * 8
+ *   lat_slot    [n_a * n_b] slot of each lattice point, -1 no pair (or a pair
+ *               these levels do not read), -2 an identity pair
+ *   cell_slots  [n_cell_groups * 8] the pairs of each cell's neighbours
+ *   cell_group  [n_rounds][P] row of cell_slots of the cell (any where none)
+ *   cell_pairs  [n_rounds][P][8] the neighbours at step 2^(n_rounds - 1 - r) in
+ *               the selector's order (b outer, a inner, clamped to the lattice,
+ *               repeats and the cell itself left out): a pair p, -1 none, or
+ *               -2 - p an identity pair. Slot s of the cell's group is
+ *               neighbour s.
+ *   cell_list   [n_rounds][P][8] pair | s << 24 of the neighbours that are
+ *               neither, then -1
+ * chunk_start / chunk_pairs: the grid's surface chunks (ffs_surface_args): they
+ * decide how each pair's sums are blocked. Rows of several designs come in
+ * tiles of 256 of one design (tile_design), as ffs_reml_prep lays them out;
+ * U and logdet_XtX are then [n_designs][P]. flag as in ffs_project_args. */
+typedef struct {
+  int V, T, K, P, n_designs, ld;
+  int p0, n_a, n_b, za, zb, ltop;
+  int n_groups, n_list, n_rounds, n_cell_groups, n_chunks;
+  const float* rows;           /* [V][T] residualised rows (yr_rows), 16-byte aligned */
+  const uint16_t* yr_hi; const uint16_t* yr_lo; const int* yexp;   /* [V][ld], [V]    */
+  const uint16_t* u_hi; const uint16_t* u_lo; const int* uexp;
+  const float* coef;
+  const double* logdet_R; const double* logdet_XtX;
+  const int* chunk_start; const int* chunk_pairs;
+  const int* slots; const int* list; const int* lat_slot; const int* lattice;
+  const int* cell_slots; const int* cell_group; const int* cell_pairs; const int* cell_list;
+  const int* tile_design;      /* [V / 256] or NULL                                   */
+  int* best;                   /* [V] pair                                            */
+  float* best_crit;            /* [V]                                                 */
+  int* flag;
+  void* work;                  /* ffs_reml_descent_work_bytes(), 256-byte aligned     */
+  size_t work_bytes;
+} ffs_descent_args;
+
+/* Bytes of workspace (0 and a message for arguments ffs_reml_descent refuses);
+ * only the sizes are read. */
+size_t ffs_reml_descent_work_bytes(const ffs_descent_args* a);
+int ffs_reml_descent(const ffs_descent_args* a, void* stream);
+
 /* ---------------------------------------------------------------------- GLS
  * The GLS refit at each voxel's chosen pair (fastfuncstuff/glm/arma.py:4784-5590):
  * betas by G' y with one refinement step on the unwhitened residual, sigma2 from

@@ -87,3 +87,141 @@ def test_ljung_box_lags_against_direct_binning(T, K, runs, censor):
     e = (-(-T // 32) + 12) * 2.0**-24
     tol = 2 * e * slope + e * e * T * (T + 2.0) * plan[2].sum() + 4e-7 * want
     assert (np.abs(got.ljung_box.numpy() - want) <= tol).all()
+
+
+# ------------------------------------------------------------------ the hierarchical descent
+
+
+def grid_for(n):
+    a, b = G.get_default_arma_grids() if n is None else (torch.linspace(-0.8, 0.8, n),) * 2
+    return G.make_grid(a, b)
+
+
+def full_descent(surf, g):
+    """(pair, value) of the selector over a whole surface, read as the reference reads it."""
+    n_a, n_b = g.lattice.shape
+    value = lambda c: np.inf if g.lattice[c] < 0 else surf[g.lattice[c]]
+    cell = (g.za, g.zb)
+    low = value(cell)
+    for lev in range(g.ltop, -1, -1):
+        s = 1 << lev
+        if lev == g.ltop:
+            cand = [(i, j) for j in range(0, n_b, s) for i in range(0, n_a, s)]
+        else:
+            cand = [(min(max(cell[0] + i * s, 0), n_a - 1), min(max(cell[1] + j * s, 0), n_b - 1))
+                    for j in (-1, 0, 1) for i in (-1, 0, 1)]
+        best = cand[0]
+        for c in cand[1:]:
+            if value(c) < value(best):
+                best = c
+        if value(best) < low:
+            cell, low = best, value(best)
+    return int(g.lattice[cell]), low
+
+
+@pytest.mark.parametrize("n", [None, 5, 9, 17, 18, 21, 33])
+@pytest.mark.parametrize("afni", [False, True])
+def test_descent_plan_reads_what_the_selector_reads(n, afni):
+    """The plan walked on the host over random and smooth surfaces gives the
+    whole surface's selection, for lattices of every divisibility (identity
+    pairs share one value, as they do in the criterion)."""
+    G.set_afni_mode(afni)
+    try:
+        g = grid_for(n)
+    finally:
+        G.set_afni_mode(False)
+    p = G.descent_plan(g)
+    ident = G.lambda_is_zero(g.a, g.b)
+    rng = np.random.default_rng(n or 1)
+    n_b = g.lattice.shape[1]
+    for k in range(60):
+        if k % 2:
+            surf = rng.standard_normal(g.P)
+        else:
+            surf = (g.a - rng.uniform(-0.8, 0.8)) ** 2 + (g.b - rng.uniform(-0.8, 0.8)) ** 2 + rng.uniform(-1, 1) * g.a * g.b
+        surf[ident] = surf[g.p0]
+        seen = np.full(g.P, np.inf)  # only what the first levels evaluate
+        seen[p.slots[p.slots >= 0]] = surf[p.slots[p.slots >= 0]]
+        seen[ident] = surf[ident]
+        on = p.lat_slot.reshape(g.lattice.shape)
+        assert all(on[c] == -2 if ident[g.lattice[c]] else p.slots[on[c]] == g.lattice[c] for c in zip(*np.nonzero(on != -1)))
+        # the first levels, then one round per level left
+        n_a = g.lattice.shape[0]
+        val = lambda c: np.inf if on[c] == -1 else seen[g.lattice[c]]
+        at = (g.za, g.zb)
+        low = val(at)
+        for lev in range(g.ltop, p.n_rounds - 1, -1):
+            s = 1 << lev
+            cand = ([(i, j) for j in range(0, n_b, s) for i in range(0, n_a, s)] if lev == g.ltop else
+                    [(min(max(at[0] + i * s, 0), n_a - 1), min(max(at[1] + j * s, 0), n_b - 1))
+                     for j in (-1, 0, 1) for i in (-1, 0, 1)])
+            best = min(range(len(cand)), key=lambda i: (val(cand[i]), i))
+            if val(cand[best]) < low:
+                at, low = cand[best], val(cand[best])
+        cell = int(g.lattice[at])
+        for r in range(p.n_rounds):
+            own = p.cell_slots[p.cell_group[r, cell]]
+            lst = {int(e) >> 24: int(e) & 0xFFFFFF for e in p.cell_list[r, cell] if e >= 0}
+            mn, to = np.inf, -1
+            for s in range(8):
+                q = int(p.cell_pairs[r, cell, s])
+                assert (own[s] == q and lst[s] == q) if q >= 0 else (own[s] == -1 and s not in lst)
+                d = surf[q] if q >= 0 else np.inf if q == -1 else surf[-2 - q]
+                if d < mn:
+                    mn, to = d, q if q >= 0 else -2 - q
+            if mn < low:
+                low, cell = mn, to
+        assert (cell, low) == full_descent(surf, g)
+
+
+@gpu
+@pytest.mark.parametrize("V,T,K,runs,n", [
+    (1, 40, 3, 1, None),      # one voxel
+    (63, 97, 8, 1, 33),       # a partial tile, T odd
+    (257, 200, 9, 2, 33),     # a row past two tiles; a run start inside a block of 16
+    (700, 250, 33, 3, 21),    # T % 4 == 2; two blocks of pairs per tile (K > 32)
+    (300, 160, 130, 1, 33),   # one pair per block of the projection
+    (4096, 128, 20, 1, 18),   # cells clamped at the lattice's edge, whole tiles
+    (1500, 72, 6, 4, 41),     # three rounds
+])
+def test_descent_equals_the_full_surface(V, T, K, runs, n, monkeypatch):
+    """best and the criterion there, bit for bit, with zero, constant, huge and NaN series among the voxels."""
+    from fastfuncstuff_gb300.glm import engine
+
+    Y, X, starts = arma_data(7, V, T, K, runs, baseline=50.0)
+    if V > 60:
+        Y[3], Y[17], Y[40], Y[41, 5] = 0.0, 12.5, Y[40] * 1e18, np.nan
+    g = grid_for(n)
+    Yd, Xd = torch.from_numpy(Y).to(DEV), torch.from_numpy(X).to(DEV)
+    f = engine.build_factors(Xd, g, G.run_layout(T, starts))
+    monkeypatch.setattr(engine, "DESCENT_MIN_WORK", 0)
+    monkeypatch.setattr(engine, "DESCENT_SHARE", 0)
+    assert engine._descent_plan(f, V) is not None
+    got = engine.search(Yd, f)
+    want = engine.search(Yd, f, keep_surface=True)
+    assert torch.equal(got.best, want.best)
+    assert torch.equal(got.best_crit.view(torch.int32), want.best_crit.view(torch.int32))
+    assert torch.equal(got.scale, want.scale) or V > 60
+
+
+@gpu
+@pytest.mark.parametrize("V,T,K,D,n", [(900, 100, 7, 3, 33), (2100, 133, 18, 5, 17), (40, 90, 40, 2, None)])
+def test_grouped_descent_equals_the_full_surface(V, T, K, D, n, monkeypatch):
+    """One design per group, groups of unequal size (one of them a single voxel), two runs."""
+    from fastfuncstuff_gb300.glm import engine
+
+    Y, X, starts = arma_data(9, V, T, K, 2)
+    Xs = np.stack([X + 0.1 * d * np.random.default_rng(d).standard_normal(X.shape).astype(np.float32) for d in range(D)])
+    gid = np.minimum(np.random.default_rng(2).zipf(1.5, V) - 1, D - 1)
+    gid[:] = np.where(gid == D - 1, 0, gid)
+    gid[5] = D - 1
+    g = grid_for(n)
+    Yd, Xd = torch.from_numpy(Y).to(DEV), torch.from_numpy(Xs.astype(np.float32)).to(DEV)
+    f = engine.build_factors(Xd, g, G.run_layout(T, starts))
+    slots = engine.design_slots(gid, D, K, g.P, DEV)
+    monkeypatch.setattr(engine, "DESCENT_SHARE", 0)
+    monkeypatch.setattr(engine, "DESCENT_MIN_WORK", 0)
+    got = engine.search_designs(Yd, f, slots)
+    monkeypatch.setattr(engine, "DESCENT_MIN_WORK", 1 << 60)
+    want = engine.search_designs(Yd, f, slots)
+    assert torch.equal(got.best, want.best) and torch.equal(got.best_crit, want.best_crit)
