@@ -18,6 +18,7 @@
 // kernel emits U = L^-T Q (the projection that lets the search skip the
 // whitening GEMM) and G = U L_xtx^-1 (the GLS solve), and the per-pair GLS
 // constants of fastfuncstuff/glm/arma.py:4853-4905.
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -213,94 +214,156 @@ struct BuildArgs {
   ffs_grid_out o;
 };
 
-// Phase 1 of an item: the per-run LDL' of pair p's AR-filtered tridiagonal
-// correlation, the serial recursion m_t = T_t,t-1 / D_t-1, D_t = T_tt - m_t
-// T_t,t-1 (one thread per run; unit gaps need no pow: a^1 = a and a^0 = 1
-// exactly), then sqrt, log and the reciprocals of every sample in parallel:
-// cms[t] = (c, m, D, 1/sqrt(D)) in shared memory, coef[p] and logdet_R[p].
-// *bad_r = 1 if a pivot D_t was not positive. Ends with a barrier.
-__device__ __forceinline__ void ldl_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p, double* cms, double* red,
-                            int* bad_r) {
+// Reciprocal of n by Newton's iteration r <- r (2 - n r) from the fp32 one
+// (error ~2^-24 -> 2^-48 -> below 2^-53), a quarter of the dependent FP64
+// operations of a correctly rounded division.
+__device__ __forceinline__ double rcp_newton(double n) {
+  if (!(n > 1e-30 && n < 1e30)) return 1.0 / n;
+  double r = (double)__frcp_rn((float)n);
+  r = r * fma(-n, r, 2.0);
+  return r * fma(-n, r, 2.0);
+}
+
+// Phase 1 of an item: the LDL' of pair p's AR-filtered tridiagonal correlation,
+// m_t = T_t,t-1 / D_t-1, D_t = T_tt - m_t T_t,t-1 within each run. D_t is the
+// ratio N_t / N_t-1 of the leading minors, which follow the three-term
+// recurrence N_t = T_tt N_t-1 - T_t,t-1^2 N_t-2: one dependent FMA per step (64
+// cycles of this GPU's FP64 pipe) where the recurrence of D takes a division
+// (about 480 cycles with Newton steps), and which a warp can scan in parallel.
+// The filter's entries before it and the reciprocals, square roots and outputs
+// after it are formed for every sample in parallel, and log|R| = 2 sum log(sqrt(D_t) + 1e-10) telescopes to the
+// log of each run's last minor + 2e-10 sum 1/sqrt(D_t) (the next term is 1e-20).
+// cc[t], cm[t], cr[t] = c, m, 1/sqrt(D); coef[p], logdet_R[p] written; tmp holds
+// 4 T doubles. *bad_r = 1 if a pivot D_t was not positive (it is replaced by 1).
+// Ends with a barrier.
+__device__ void ldl_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p, double* cc, double* cm, double* cr,
+                            double* tmp, double* red, int* bad_r) {
   const int T = d.T;
   const float af = d.a[p], bf = d.b[p];
   const double a = (double)af;
-  const double lam = d.lambda_fp32 ? (double)lambda_f32(af, bf) : lambda_f64(a, (double)bf);
-  if (threadIdx.x == 0) *bad_r = 0;
+  double *diag = tmp, *off2 = tmp + T, *num = tmp + 2 * T, *prev = tmp + 3 * T;
+  if (threadIdx.x == 0) {
+    *bad_r = 0;
+    red[0] = d.lambda_fp32 ? (double)lambda_f32(af, bf) : lambda_f64(a, (double)bf);
+  }
   __syncthreads();
-  for (int r = threadIdx.x; r < d.n_runs; r += blockDim.x) {
+  const double lam = red[0];
+  // lambda == 0: every lag correlation is zero, R = I exactly
+  const bool ident = lam == 0.0;
+  for (int t = threadIdx.x; t < T; t += blockDim.x) {
+    double c = 0.0, off = 0.0, dg = 1.0;
+    bool start = t == 0;
+    for (int r = 1; r < d.n_runs && !start; ++r) start = d.run_start[r] == t;
+    if (!start && !ident) {
+      const int gap = d.tau[t] - d.tau[t - 1];
+      // a^gap and a^(gap - 1) of small integer gaps by products (a^1 = a and
+      // a^0 = 1 exactly)
+      double ag1 = 1.0;
+      if (gap <= 16) {
+        for (int k = 1; k < gap; ++k) ag1 *= a;
+      } else {
+        ag1 = pow(a, (double)(gap - 1));
+      }
+      const double rho = lam * ag1;
+      c = ag1 * a;
+      dg = 1.0 + c * c - 2.0 * c * rho;
+      off = rho - c;
+    }
+    cc[t] = c;
+    cm[t] = off;
+    diag[t] = dg;
+    off2[t] = off * off;
+  }
+  __syncthreads();
+  // a warp per run: N_t, N_t-1 = A_t ... A_t0 (1, 1) with A_t = [T_tt, -off2; 1, 0].
+  // Each lane multiplies the matrices of its stretch, a scan over the lanes
+  // gives the minors before each stretch, and the lane walks it from there.
+  // (A warp has one FP64 instruction in flight, 64 cycles each: about 80 of
+  // them for a run of 200, where a walk by one lane takes 400.)
+  double ld = 0.0;
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < d.n_runs && !ident; r += blockDim.x >> 5) {
     const int t0 = d.run_start[r], t1 = d.run_start[r + 1];
-    double Dprev = 1.0, mprev = 0.0;
-    int prev_gap = 0;
-    for (int t = t0; t < t1; ++t) {
-      double c = 0.0, m = 0.0, D = 1.0;
-      // lambda == 0: every lag correlation is zero, R = I exactly
-      if (t > t0 && lam != 0.0) {
-        const int gap = d.tau[t] - d.tau[t - 1];
-        double rho;
-        if (gap == 1) {
-          c = a;
-          rho = lam;
-        } else {
-          // a^gap and a^(gap - 1) of small integer gaps by products
-          double ag1 = 1.0;
-          if (gap <= 16) {
-            for (int k = 1; k < gap; ++k) ag1 *= a;
-          } else {
-            ag1 = pow(a, (double)(gap - 1));
-          }
-          c = ag1 * a;
-          rho = lam * ag1;
-        }
-        const double Ttt = 1.0 + c * c - 2.0 * c * rho;
-        const double Toff = rho - c;
-        if (gap == 1 && prev_gap == 1 && Dprev == cms[4 * (t - 1) - 4 + 2]) {
-          // the previous step left D unchanged: the recursion has reached
-          // its fixed point, and every step of this stretch of unit gaps
-          // repeats it
-          m = mprev;
-          D = Dprev;
-        } else {
-          // 1/D_{t-1}: fp32 estimate refined by two Newton steps r (2 - D r)
-          // (error ~2^-24 -> ~2^-48 -> below 2^-53), cheaper than a
-          // correctly rounded FP64 division in this serial chain
-          if (Dprev > 1e-30 && Dprev < 1e30) {
-            double r = (double)__frcp_rn((float)Dprev);
-            r = r * fma(-Dprev, r, 2.0);
-            r = r * fma(-Dprev, r, 2.0);
-            m = Toff * r;
-          } else {
-            m = Toff / Dprev;
-          }
-          D = Ttt - m * Toff;
-        }
-        prev_gap = gap;
+    const int seg = (t1 - t0 + 31) >> 5;
+    const int s0 = min(t1, t0 + lane * seg), s1 = min(t1, s0 + seg);
+    double a0 = 1.0, a1 = 0.0, b0 = 0.0, b1 = 1.0;  // columns (a0, b0) and (a1, b1) of the product
+    int ex = 0;                                     // its scale, 2^ex
+    auto rescale = [&](double lead) {
+      const int e = ((__double2hiint(lead) >> 20) & 0x7ff) - 1023;
+      if (e > 64 || e < -64) {
+        const double sc = __hiloint2double((1023 - e) << 20, 0);
+        a0 *= sc;
+        a1 *= sc;
+        b0 *= sc;
+        b1 *= sc;
+        ex += e;
       }
-      if (!(D > 0.0)) {
-        *bad_r = 1;
-        D = 1.0;
-      }
-      double* cm = cms + 4 * t;
-      cm[0] = c; cm[1] = m; cm[2] = D;
-      Dprev = D;
-      mprev = m;
+    };
+    for (int t = s0; t < s1; ++t) {
+      const double dg = diag[t], of = off2[t];
+      const double na = fma(dg, a0, -(of * b0)), nb = fma(dg, a1, -(of * b1));
+      b0 = a0;
+      b1 = a1;
+      a0 = na;
+      a1 = nb;
+      if (((t - s0) & 7) == 7) rescale(a0);
     }
+    for (int o2 = 1; o2 < 32; o2 <<= 1) {  // inclusive: this lane's product times those before it
+      const double p0 = __shfl_up_sync(0xffffffffu, a0, o2), p1 = __shfl_up_sync(0xffffffffu, a1, o2);
+      const double q0 = __shfl_up_sync(0xffffffffu, b0, o2), q1 = __shfl_up_sync(0xffffffffu, b1, o2);
+      const int pe = __shfl_up_sync(0xffffffffu, ex, o2);
+      if (lane >= o2) {
+        const double c0 = fma(a0, p0, a1 * q0), c1 = fma(a0, p1, a1 * q1);
+        const double e0 = fma(b0, p0, b1 * q0), e1 = fma(b0, p1, b1 * q1);
+        a0 = c0;
+        a1 = c1;
+        b0 = e0;
+        b1 = e1;
+        ex += pe;
+        rescale(a0);
+      }
+    }
+    // (N, N of the step before) entering this lane's stretch; off2 = 0 at the
+    // run's start, so the second entry of the start vector is not read
+    double n1 = __shfl_up_sync(0xffffffffu, a0 + a1, 1), n0 = __shfl_up_sync(0xffffffffu, b0 + b1, 1);
+    int e2 = __shfl_up_sync(0xffffffffu, ex, 1);
+    if (lane == 0) {
+      n1 = n0 = 1.0;
+      e2 = 0;
+    }
+    for (int t = s0; t < s1; ++t) {
+      double n = fma(diag[t], n1, -(off2[t] * n0));
+      if (__double2hiint(n) <= 0) {  // not positive (NaN is caught by the Cholesky of X_w'X_w)
+        *bad_r = 1;
+        n = n1;
+      }
+      num[t] = n;
+      prev[t] = n1;
+      n0 = n1;
+      n1 = n;
+    }
+    if (s1 == t1 && s0 < s1) ld += log(n1) + (double)e2 * 0.693147180559945309417;
   }
   __syncthreads();
-  {
-    double ld = 0.0;
-    for (int t = threadIdx.x; t < T; t += blockDim.x) {
-      double* cm = cms + 4 * t;
-      const double D = cm[2];
-      const double sD = sqrt(D);
-      const double rsD = 1.0 / sD;
-      ld += 2.0 * log(sD + 1e-10);
-      cm[3] = rsD;
-      reinterpret_cast<float4*>(o.coef)[(size_t)p * T + t] =
-          make_float4((float)cm[0], (float)cm[1], (float)(1.0 / D), (float)rsD);
+  double rsum = 0.0;
+  for (int t = threadIdx.x; t < T; t += blockDim.x) {
+    double id = 1.0, rs = 1.0;
+    if (!ident && num[t] != prev[t]) {  // else D_t = 1
+      id = prev[t] * rcp_newton(num[t]);  // 1 / D_t
+      rs = id * rsqrt_newton(id);
     }
-    ld = block_sum(ld, red);
-    if (threadIdx.x == 0) o.logdet_R[p] = ld;
+    rsum += rs;
+    diag[t] = id;
+    cr[t] = rs;
   }
+  ld = block_sum(ld + 2e-10 * rsum, red);  // its barriers order diag
+  for (int t = threadIdx.x; t < T; t += blockDim.x) {
+    const double m = t > 0 ? cm[t] * diag[t - 1] : 0.0;
+    cm[t] = m;
+    reinterpret_cast<float4*>(o.coef)[(size_t)p * T + t] =
+        make_float4((float)cc[t], (float)m, (float)diag[t], (float)cr[t]);
+  }
+  if (threadIdx.x == 0) o.logdet_R[p] = ld;
   __syncthreads();
 }
 
@@ -394,23 +457,370 @@ __device__ void band_chol_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o,
 }
 
 // Phase 1 of every pair once, for the items of all designs (coef and
-// logdet_R depend on the pair only): cm [P][T][4] and bad [P] in the
-// workspace, read back by grid_build_kernel. With the banded R the pair's
-// band_L, band_coef, coef and logdet_R are written here, and cm keeps the
-// reciprocal diagonal and each row's band (the first 1.5 T doubles).
+// logdet_R depend on the pair only): c, m and 1/sqrt(D) ([P][3][T], stride 4 T
+// per pair) and bad [P] in the workspace, read back by the item kernels. With
+// the banded R the pair's band_L, band_coef, coef and logdet_R are written here,
+// and the workspace keeps the reciprocal diagonal and each row's band (the
+// first 1.5 T doubles).
 __global__ void __launch_bounds__(GB_THREADS) pair_ldl_kernel(BuildArgs args, double* cm, int* bad) {
   __shared__ double red[32];
   __shared__ int bad_r;
-  extern __shared__ double cms[];  // [T][4], or with the band as band_chol_of_pair lays it out
+  extern __shared__ double cms[];  // 4 T doubles, or with the band as band_chol_of_pair lays it out
   const int T = args.d.T;
+  double* dst = cm + (size_t)blockIdx.x * 4 * T;
   if (args.d.band)
     band_chol_of_pair(args.d, args.o, blockIdx.x, cms, reinterpret_cast<int*>(cms + T), cms + T + (T + 1) / 2, red,
                       &bad_r);
   else
-    ldl_of_pair(args.d, args.o, blockIdx.x, cms, red, &bad_r);
-  double2* dst = reinterpret_cast<double2*>(cm + (size_t)blockIdx.x * 4 * T);
-  for (int i = threadIdx.x; i < 2 * T; i += blockDim.x) dst[i] = reinterpret_cast<const double2*>(cms)[i];
+    ldl_of_pair(args.d, args.o, blockIdx.x, dst, dst + T, dst + 2 * T, cms, red, &bad_r);
+  if (args.d.band)
+    for (int i = threadIdx.x; i < 3 * T; i += blockDim.x) dst[i] = cms[i];
   if (threadIdx.x == 0) bad[blockIdx.x] = bad_r;
+}
+
+// The centring test of a design at its identity pair, where X_w = X: c =
+// (X'X)^-1 X'1 from the inverse factor Li (row stride ldi), accepted when
+// ||X c - 1||^2 <= 1e-12 T; *const_flag stays 1 only if every design passes.
+// w: 2 K doubles of scratch. Ends with a barrier.
+__device__ void const_of_design(const ffs_grid_desc& d, const ffs_grid_out& o, int dsg, const float* Xd,
+                                const double* Li, int ldi, bool chol, double* w, double* red) {
+  const int T = d.T, K = d.K;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  __syncthreads();
+  for (int j = wid; j < K; j += nw) {  // X'1
+    double x = 0.0;
+    for (int t = lane; t < T; t += 32) x += f2d_exact(Xd[(size_t)t * K + j]);
+    x = warp_sum_d(x);
+    if (lane == 0) w[K + j] = x;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < K; k += blockDim.x) {  // Lx^-1 X'1
+    double x = 0.0;
+    for (int j = 0; j <= k; ++j) x = fma(Li[k * ldi + j], w[K + j], x);
+    w[k] = x;
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < K; j += blockDim.x) {
+    double x = 0.0;
+    for (int k = j; k < K; ++k) x = fma(Li[k * ldi + j], w[k], x);
+    w[K + j] = x;
+  }
+  __syncthreads();
+  double part = 0.0;
+  for (int t = threadIdx.x; t < T; t += blockDim.x) {
+    double r = -1.0;
+    for (int j = 0; j < K; ++j) r = fma(f2d_exact(Xd[(size_t)t * K + j]), w[K + j], r);
+    part = fma(r, r, part);
+  }
+  const double ss = block_sum(part, red);
+  const bool ok = chol && ss <= 1e-12 * (double)T;
+  for (int j = threadIdx.x; j < K; j += blockDim.x) o.const_coef[(size_t)dsg * K + j] = ok ? (float)w[K + j] : 0.f;
+  if (threadIdx.x == 0 && !ok) atomicAnd(o.const_flag, 0);
+  __syncthreads();
+}
+
+// The end of an item: Gsum = G' 1 accumulated in FP64, the task-column F
+// matrix inv(A_task + 1e-8 I), the column sets' and the GLT variances c A c',
+// from s.Li with the scratch s.S and s.A. Starts and ends with a barrier.
+__device__ void item_tail(const ffs_grid_desc& d, const ffs_grid_out& o, const PairScratch& s, int pd, double* red,
+                          int* flag_s) {
+  const int T = d.T, K = d.K, LT = ld_t(T);
+  int& flag = *flag_s;
+  __syncthreads();
+  if (o.Gsum) {
+    for (int j = threadIdx.x; j < K; j += blockDim.x) {
+      double acc = 0.0;
+      for (int t = 0; t < T; ++t) acc += (double)o.G[((size_t)pd * K + j) * LT + t];
+      o.Gsum[(size_t)pd * K + j] = (float)acc;
+    }
+  }
+
+  // ---- 9. task-column F matrix inv(A_task + 1e-8 I) and GLT variances c A c'
+  const int nt = d.n_task;
+  if (d.n_glt > 0 && o.glt_var) {  // c A c' = ||Lx^-1 c||^2
+    for (int c = 0; c < d.n_glt; ++c) {
+      const float* gc = d.glt + (size_t)c * K;
+      double part = 0.0;
+      for (int k = threadIdx.x; k < K; k += blockDim.x) {
+        double w = 0.0;
+        for (int j = 0; j <= k; ++j) w += s.Li[k * K + j] * (double)gc[j];
+        part += w * w;
+      }
+      const double v = block_sum(part, red);
+      if (threadIdx.x == 0) o.glt_var[(size_t)pd * d.n_glt + c] = (float)v;
+    }
+  }
+  // the task block, then the column sets' blocks one after another
+  const int has_task = nt > 0 && o.Ftask ? 1 : 0;
+  const int nsets = o.Fsets ? d.n_sets : 0;
+  size_t msum = 0, off = 0;
+  for (int g = 0; g < nsets; ++g) {
+    const size_t q = (size_t)(d.set_ptr[g + 1] - d.set_ptr[g]);
+    msum += q * q;
+  }
+  for (int bk = 0; bk < has_task + nsets; ++bk) {
+    const bool task = bk < has_task;
+    const int g = bk - has_task;
+    const int n = task ? nt : d.set_ptr[g + 1] - d.set_ptr[g];
+    const int* idx = task ? d.task_idx : d.set_idx + d.set_ptr[g];
+    float* out = task ? o.Ftask + (size_t)pd * nt * nt : o.Fsets + (size_t)pd * msum + off;
+    sub_block_inverse(s, K, idx, n, &flag, out);
+    if (!task) off += (size_t)n * n;
+  }
+  __syncthreads();
+}
+
+// Phases 2 to 9 of one item with its matrices in the global scratch slot s,
+// after phase 1: cc, cm, cr as ldl_of_pair leaves them, or with the banded R cc
+// = the reciprocal diagonal and, behind it, each row's band. Any K and T.
+__device__ __noinline__ void item_global(const BuildArgs& args, const PairScratch& s, int p, int pd, const float* Xd,
+                                         const double* cc, const double* cm, const double* cr, int bad_r, double* red,
+                                         int* flag_s) {
+  const ffs_grid_desc& d = args.d;
+  const ffs_grid_out& o = args.o;
+  const int T = d.T, K = d.K, LT = ld_t(T);
+  int& flag = *flag_s;
+
+  // ---- 2. X_w = L^-1 X, one column per thread; the design samples of
+  // GB_PF steps are loaded ahead of the recursion that needs them (with the
+  // banded R: forward substitution against the band of each row)
+  if (d.band) {
+    const int W = d.band_w;
+    const double* Lb = o.band_L + (size_t)p * T * W;
+    const int* Jrow = reinterpret_cast<const int*>(cc + T);
+    for (int j = threadIdx.x; j < K; j += blockDim.x) {
+      double* xw = s.Xw + (size_t)j * T;
+      for (int t = 0; t < T; ++t) {
+        double acc = f2d_exact(__ldg(Xd + (size_t)t * K + j));
+        const double* row = Lb + (size_t)t * W;
+        for (int i = 1; i <= Jrow[t]; ++i) acc = fma(-row[i], xw[t - i], acc);
+        xw[t] = acc * cc[t];
+      }
+    }
+  }
+  for (int j = threadIdx.x; j < K && !d.band; j += blockDim.x) {
+    double xp = 0.0, vp = 0.0;
+    for (int t0 = 0; t0 < T; t0 += GB_PF) {
+      float xb[GB_PF];
+#pragma unroll
+      for (int k = 0; k < GB_PF; ++k) xb[k] = t0 + k < T ? __ldg(Xd + (size_t)(t0 + k) * K + j) : 0.f;
+#pragma unroll
+      for (int k = 0; k < GB_PF; ++k) {
+        const int t = t0 + k;
+        if (t < T) {
+          const double x = f2d_exact(xb[k]);
+          const double z = x - cc[t] * xp;
+          const double v = z - cm[t] * vp;
+          s.Xw[(size_t)j * T + t] = v * cr[t];
+          xp = x;
+          vp = v;
+        }
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- 3. X_w'X_w (full symmetric) into Lx, and the fp32 copy: one thread
+  // per lower-triangle entry (full warps), four chains each
+  for (int e = threadIdx.x; e < K * (K + 1) / 2; e += blockDim.x) {
+    int i, j;
+    tri_index(e, i, j);
+    Dot4 acc;
+    acc.run(s.Xw + (size_t)i * T, s.Xw + (size_t)j * T, T);
+    const double v = acc.sum();
+    s.Lx[i * K + j] = v;
+    s.Lx[j * K + i] = v;
+    o.XtX[(size_t)pd * K * K + i * K + j] = (float)v;
+    o.XtX[(size_t)pd * K * K + j * K + i] = (float)v;
+  }
+  __syncthreads();
+
+  // ---- 4. Cholesky of X_w'X_w, QR (modified Gram-Schmidt, twice) otherwise
+  // 1 / diag(Lx) goes to the A slot, free until phase 9
+  int info = 0;
+  const bool chol = block_cholesky(s.Lx, K, K, &flag, s.A);
+  if (!chol) {
+    info = 1;
+    // Q and R from X_w; Lx := R' (lower), so that X_w'X_w = Lx Lx'.
+    for (int idx = threadIdx.x; idx < K * K; idx += blockDim.x) s.Lx[idx] = 0.0;
+    __syncthreads();
+    for (int j = 0; j < K; ++j) {
+      double* q = s.Qm + (size_t)j * T;
+      for (int t = threadIdx.x; t < T; t += blockDim.x) q[t] = s.Xw[(size_t)j * T + t];
+      __syncthreads();
+      for (int pass = 0; pass < 2; ++pass) {
+        for (int i = 0; i < j; ++i) {
+          const double* qi = s.Qm + (size_t)i * T;
+          double part = 0.0;
+          for (int t = threadIdx.x; t < T; t += blockDim.x) part += qi[t] * q[t];
+          const double rij = block_sum(part, red);
+          for (int t = threadIdx.x; t < T; t += blockDim.x) q[t] -= rij * qi[t];
+          if (threadIdx.x == 0) s.Lx[j * K + i] += rij;
+          __syncthreads();
+        }
+      }
+      double part = 0.0;
+      for (int t = threadIdx.x; t < T; t += blockDim.x) part += q[t] * q[t];
+      const double nrm = sqrt(block_sum(part, red));
+      const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
+      for (int t = threadIdx.x; t < T; t += blockDim.x) q[t] *= inv;
+      if (threadIdx.x == 0) s.Lx[j * K + j] = nrm;
+      __syncthreads();
+    }
+  }
+  if (bad_r) info = 2;
+  __syncthreads();
+
+  if (threadIdx.x == 0) {
+    double ld = 0.0;
+    for (int j = 0; j < K; ++j) ld += 2.0 * log(fabs(s.Lx[j * K + j]) + 1e-10);
+    o.logdet_XtX[pd] = ld;
+    o.info[pd] = info;
+  }
+
+  // ---- 5. Q = X_w Lx^-T in fp32 (Q, U and G only leave as fp32 or fp16
+  // splits; the factorisation and the logdets above stay FP64). The two [K][T]
+  // FP64 slots are reused as fp32 arrays; the QR fallback converts its Q.
+  float* const xw_f = reinterpret_cast<float*>(s.Xw);
+  float* const qm_f = reinterpret_cast<float*>(s.Qm);
+  float* const lx_f = reinterpret_cast<float*>(s.S);  // [K][K] Lx, then Li in lx_f + K*K
+  float* qf;
+  float* uf;
+  for (int idx = threadIdx.x; idx < K * K; idx += blockDim.x) lx_f[idx] = (float)s.Lx[idx];
+  __syncthreads();
+  if (info != 1) {
+    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+      for (int j = 0; j < K; ++j) {
+        float acc = (float)s.Xw[(size_t)j * T + t];
+        for (int i = 0; i < j; ++i) acc = fmaf(-lx_f[j * K + i], qm_f[(size_t)i * T + t], acc);
+        qm_f[(size_t)j * T + t] = acc / lx_f[j * K + j];
+      }
+    }
+    qf = qm_f;
+    uf = xw_f;
+  } else {
+    for (int idx = threadIdx.x; idx < K * T; idx += blockDim.x) xw_f[idx] = (float)s.Qm[idx];
+    qf = xw_f;
+    uf = qm_f;
+  }
+  __syncthreads();
+
+  // ---- 6. U = L^-T Q = A' L~^-T D^-1/2 Q (backward recursions) in fp32, with
+  // the fp32 coefficients of phase 1
+  const float4* cf = reinterpret_cast<const float4*>(o.coef) + (size_t)p * T;
+  float umax_local = 0.f;
+  if (d.band) {
+    // back substitution against the band: u_t = (q_t - sum_i L(t + i, t)
+    // u_{t+i}) / L(t, t), the rows t + i of t's run within the band
+    const int W = d.band_w;
+    const double* Lb = o.band_L + (size_t)p * T * W;
+    const int* Jrow = reinterpret_cast<const int*>(cc + T);
+    for (int j = threadIdx.x; j < K; j += blockDim.x) {
+      const float* q = qf + (size_t)j * T;
+      float* u = uf + (size_t)j * T;
+      for (int t = T - 1; t >= 0; --t) {
+        double acc = (double)q[t];
+        for (int i = 1; t + i < T && i <= Jrow[t + i]; ++i) acc = fma(-Lb[(size_t)(t + i) * W + i], (double)u[t + i], acc);
+        const float ut = (float)(acc * cc[t]);
+        u[t] = ut;
+        o.U[((size_t)pd * K + j) * LT + t] = ut;
+        umax_local = fmaxf(umax_local, fabsf(ut));
+      }
+      for (int t = T; t < LT; ++t) o.U[((size_t)pd * K + j) * LT + t] = 0.f;
+    }
+  }
+  for (int j = threadIdx.x; j < K && !d.band; j += blockDim.x) {
+    const float* q = qf + (size_t)j * T;
+    float* u = uf + (size_t)j * T;
+    float xn = 0.f, mn = 0.f, cn = 0.f;  // x_{t+1}, m_{t+1}, c_{t+1}
+    for (int t1 = T - 1; t1 >= 0; t1 -= GB_PF) {  // GB_PF steps of q and coef loaded ahead
+      float qb[GB_PF];
+      float4 cb[GB_PF];
+#pragma unroll
+      for (int k = 0; k < GB_PF; ++k) {
+        const int t = t1 - k;
+        qb[k] = t >= 0 ? q[t] : 0.f;
+        cb[k] = t >= 0 ? cf[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int k = 0; k < GB_PF; ++k) {
+        const int t = t1 - k;
+        if (t >= 0) {
+          const float4 c4 = cb[k];  // (c, m, 1/D, 1/sqrt(D))
+          const float x = fmaf(-mn, xn, qb[k] * c4.w);
+          const float ut = fmaf(-cn, xn, x);
+          u[t] = ut;
+          o.U[((size_t)pd * K + j) * LT + t] = ut;
+          umax_local = fmaxf(umax_local, fabsf(ut));
+          xn = x;
+          mn = c4.y;
+          cn = c4.x;
+        }
+      }
+    }
+    for (int t = T; t < LT; ++t) o.U[((size_t)pd * K + j) * LT + t] = 0.f;
+  }
+  __syncthreads();
+  if (o.U_hi) {
+    // fp16 hi/lo split of U * 2^e, e placing max|U| in [128, 256)
+    double um = umax_local;
+    for (int off = 16; off > 0; off >>= 1) um = fmax(um, __shfl_xor_sync(0xffffffffu, um, off));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = um;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double mx = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mx = fmax(mx, red[w]);
+      red[0] = mx;
+    }
+    __syncthreads();
+    const int e = scale_exp((float)red[0]);
+    if (threadIdx.x == 0) o.uexp[pd] = e;
+    for (int idx = threadIdx.x; idx < K * d.ld_u; idx += blockDim.x) {
+      const int j = idx / d.ld_u, t = idx % d.ld_u;
+      uint16_t hi = 0, lo = 0;
+      if (t < T) split_fp16(ldexpf(uf[(size_t)j * T + t], e), hi, lo);
+      const size_t at = ((size_t)pd * K + j) * d.ld_u + t;
+      o.U_hi[at] = hi;
+      o.U_lo[at] = lo;
+    }
+  }
+  __syncthreads();
+
+  // ---- 7. Lx^-1 and diag(A), A = Lx^-T Lx^-1 = (X_w'X_w)^-1 (only the
+  // entries the statistics read are formed: the diagonal here, the task
+  // block and c A c' in phase 9)
+  block_tri_inverse(s.Lx, s.Li, K, K, chol ? s.A : nullptr);
+  for (int j = threadIdx.x; j < K; j += blockDim.x) {
+    double acc = 0.0;
+    for (int k = j; k < K; ++k) acc += s.Li[k * K + j] * s.Li[k * K + j];
+    o.Adiag[(size_t)pd * K + j] = (float)acc;
+  }
+  if (o.Afull) {  // all of A, for the per-voxel blocks of the -dsort fit
+    for (int e = threadIdx.x; e < K * K; e += blockDim.x) {
+      const int i = e / K, j = e % K;
+      double acc = 0.0;
+      for (int k = max(i, j); k < K; ++k) acc += s.Li[k * K + i] * s.Li[k * K + j];
+      o.Afull[(size_t)pd * K * K + e] = (float)acc;
+    }
+  }
+  __syncthreads();
+
+  if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, s.Li, K, chol, s.S, red);
+
+  // ---- 8. G = U Lx^-1 in fp32 (row t of G solves g Lx = u_t); Gsum = G' 1
+  // accumulated in FP64
+  float* const li_f = lx_f + (size_t)K * K;
+  for (int idx = threadIdx.x; idx < K * K; idx += blockDim.x) li_f[idx] = (float)s.Li[idx];
+  __syncthreads();
+  for (int t = threadIdx.x; t < LT; t += blockDim.x) {
+    for (int j = 0; j < K; ++j) {
+      float acc = 0.f;
+      if (t < T)
+        for (int i = j; i < K; ++i) acc = fmaf(uf[(size_t)i * T + t], li_f[i * K + j], acc);
+      o.G[((size_t)pd * K + j) * LT + t] = acc;
+    }
+  }
+  item_tail(d, o, s, pd, red, flag_s);
 }
 
 // Items are (design, pair) = (item / P, item % P); a CTA takes items
@@ -418,316 +828,614 @@ __global__ void __launch_bounds__(GB_THREADS) pair_ldl_kernel(BuildArgs args, do
 // Design-dependent outputs sit at pd = design * P + pair. With SHARED_LDL
 // (more than one design) phase 1 comes from pair_ldl_kernel (pair_cm,
 // pair_bad), which also wrote coef and logdet_R; without it every item
-// factors its pair's R itself. Capped at 64 registers (4 CTAs per SM): left
-// free, the compiler takes 80 to 126 of them.
+// factors its pair's R itself. This kernel takes the items that
+// grid_item_kernel does not (wide or long designs, the banded R). Capped at
+// 64 registers (4 CTAs per SM): left free, the compiler takes 80 to 126 of them.
 template <bool SHARED_LDL>
 __global__ void __launch_bounds__(GB_THREADS, 4) grid_build_kernel(BuildArgs args, int n_designs,
                                                                                   const double* pair_cm,
-                                                                                  const int* pair_bad) {
+                                                                                  const int* pair_bad, int tmp_smem) {
   const ffs_grid_desc& d = args.d;
   const ffs_grid_out& o = args.o;
-  const int T = d.T, K = d.K, LT = ld_t(T);
+  const int T = d.T, K = d.K;
   PairScratch s = scratch_of(o.work, blockIdx.x, T, K);
-
   __shared__ double red[32];
   __shared__ int flag, bad_r;
-  extern __shared__ double cms[];  // [T][4] c, m, D, 1/sqrt(D) of the current pair
-
+  extern __shared__ double cms[];  // c, m, 1/sqrt(D) of the current pair [3][T], then [4][T] with tmp_smem
   for (int item = blockIdx.x; item < d.P * n_designs; item += gridDim.x) {
-    const int p = item % d.P, pd = item;
-    const float* Xd = d.X + (size_t)(item / d.P) * T * K;
+    const int p = item % d.P;
     if constexpr (SHARED_LDL) {
       // the pre-pass factored R for every pair once: copy this pair's rows
-      const double2* src = reinterpret_cast<const double2*>(pair_cm + (size_t)p * 4 * T);
-      for (int i = threadIdx.x; i < 2 * T; i += blockDim.x) reinterpret_cast<double2*>(cms)[i] = src[i];
+      const double* src = pair_cm + (size_t)p * 4 * T;
+      for (int i = threadIdx.x; i < 3 * T; i += blockDim.x) cms[i] = src[i];
       if (threadIdx.x == 0) bad_r = pair_bad[p];
       __syncthreads();
     } else if (d.band) {
       band_chol_of_pair(d, o, p, cms, reinterpret_cast<int*>(cms + T), cms + T + (T + 1) / 2, red, &bad_r);
     } else {
-      ldl_of_pair(d, o, p, cms, red, &bad_r);
+      ldl_of_pair(d, o, p, cms, cms + T, cms + 2 * T, tmp_smem ? cms + 3 * T : s.cm, red, &bad_r);
     }
+    item_global(args, s, p, item, d.X + (size_t)(item / d.P) * T * K, cms, cms + T, cms + 2 * T, bad_r, red, &flag);
+  }
+}
 
-    // ---- 2. X_w = L^-1 X, one column per thread; the design samples of
-    // GB_PF steps are loaded ahead of the recursion that needs them (with the
-    // banded R: forward substitution against the band of each row)
-    if (d.band) {
-      const int W = d.band_w;
-      const double* Lb = o.band_L + (size_t)p * T * W;
-      const int* Jrow = reinterpret_cast<const int*>(cms + T);
-      for (int j = threadIdx.x; j < K; j += blockDim.x) {
-        double* xw = s.Xw + (size_t)j * T;
-        for (int t = 0; t < T; ++t) {
-          double acc = f2d_exact(__ldg(Xd + (size_t)t * K + j));
-          const double* row = Lb + (size_t)t * W;
-          for (int i = 1; i <= Jrow[t]; ++i) acc = fma(-row[i], xw[t - i], acc);
-          xw[t] = acc * cms[t];
-        }
-      }
-    }
-    for (int j = threadIdx.x; j < K && !d.band; j += blockDim.x) {
-      double xp = 0.0, vp = 0.0;
-      for (int t0 = 0; t0 < T; t0 += GB_PF) {
-        float xb[GB_PF];
-#pragma unroll
-        for (int k = 0; k < GB_PF; ++k) xb[k] = t0 + k < T ? __ldg(Xd + (size_t)(t0 + k) * K + j) : 0.f;
-#pragma unroll
-        for (int k = 0; k < GB_PF; ++k) {
-          const int t = t0 + k;
-          if (t < T) {
-            const double* cm = cms + 4 * t;
-            const double x = f2d_exact(xb[k]);
-            const double z = x - cm[0] * xp;
-            const double v = z - cm[1] * vp;
-            s.Xw[(size_t)j * T + t] = v * cm[3];
-            xp = x;
-            vp = v;
-          }
-        }
-      }
-    }
-    __syncthreads();
+// --------------------------------------------------------- Gram entries in integers
+// This GPU's FP64 pipe takes one warp instruction per 19 cycles and SM, its
+// integer multiply-add with a 64-bit sum one per cycle or better. A Gram entry
+// sum_t x_i[t] x_j[t] of FP64 series is therefore formed from 54-bit fixed-point
+// values: x = q 2^-s with s per column (|q| < 2^53, s from the column's largest
+// magnitude), q = hi 2^27 + lo with |hi|, |lo| <= 2^26, and the sums of hi hi',
+// hi lo' + lo hi' and lo lo' in 64-bit integers: exact for up to 1024 samples,
+// whatever the order. What remains is the rounding of x to the fixed point,
+// 2^-54 of the column's largest value at most twice over, where a chain of FP64
+// FMAs rounds every partial sum.
+constexpr int FX_TMAX = 1024;
 
-    // ---- 3. X_w'X_w (full symmetric) into Lx, and the fp32 copy: one thread
-    // per lower-triangle entry (full warps), four chains each
-    for (int e = threadIdx.x; e < K * (K + 1) / 2; e += blockDim.x) {
-      int i, j;
-      tri_index(e, i, j);
-      Dot4 acc;
-      acc.run(s.Xw + (size_t)i * T, s.Xw + (size_t)j * T, T);
-      const double v = acc.sum();
-      s.Lx[i * K + j] = v;
-      s.Lx[j * K + i] = v;
-      o.XtX[(size_t)pd * K * K + i * K + j] = (float)v;
-      o.XtX[(size_t)pd * K * K + j * K + i] = (float)v;
-    }
-    __syncthreads();
+// s for a column of largest magnitude mx: mx (1 + 1/32) < 2^(53 - s), the margin
+// for an mx found in fp32
+__device__ __forceinline__ int fixed_scale(float mx) {
+  int e = 0;
+  frexpf(mx * 1.03125f, &e);
+  return mx > 0.f ? 53 - e : 0;
+}
 
-    // ---- 4. Cholesky of X_w'X_w, QR (modified Gram-Schmidt, twice) otherwise
-    // 1 / diag(Lx) goes to the A slot, free until phase 9
-    int info = 0;
-    const bool chol = block_cholesky(s.Lx, K, K, &flag, s.A);
-    if (!chol) {
-      info = 1;
-      // Q and R from X_w; Lx := R' (lower), so that X_w'X_w = Lx Lx'.
-      for (int idx = threadIdx.x; idx < K * K; idx += blockDim.x) s.Lx[idx] = 0.0;
-      __syncthreads();
-      for (int j = 0; j < K; ++j) {
-        double* q = s.Qm + (size_t)j * T;
-        for (int t = threadIdx.x; t < T; t += blockDim.x) q[t] = s.Xw[(size_t)j * T + t];
-        __syncthreads();
-        for (int pass = 0; pass < 2; ++pass) {
-          for (int i = 0; i < j; ++i) {
-            const double* qi = s.Qm + (size_t)i * T;
-            double part = 0.0;
-            for (int t = threadIdx.x; t < T; t += blockDim.x) part += qi[t] * q[t];
-            const double rij = block_sum(part, red);
-            for (int t = threadIdx.x; t < T; t += blockDim.x) q[t] -= rij * qi[t];
-            if (threadIdx.x == 0) s.Lx[j * K + i] += rij;
-            __syncthreads();
-          }
-        }
-        double part = 0.0;
-        for (int t = threadIdx.x; t < T; t += blockDim.x) part += q[t] * q[t];
-        const double nrm = sqrt(block_sum(part, red));
-        const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
-        for (int t = threadIdx.x; t < T; t += blockDim.x) q[t] *= inv;
-        if (threadIdx.x == 0) s.Lx[j * K + j] = nrm;
-        __syncthreads();
-      }
-    }
-    if (bad_r) info = 2;
-    __syncthreads();
+// (hi, lo) of w 2^s rounded to an integer; over = true when it does not fit
+__device__ __forceinline__ int2 fixed_of(double w, int s, bool& over) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(w);
+  const int ex = (int)(b >> 52) & 0x7ff;
+  const int r = 1075 - ex - s;  // |w| 2^s = mantissa 2^-r
+  over = over || (r < 0 && ex != 0);
+  unsigned long long m = ((b << 1) & 0x1ffffffffffffeull) | 0x20000000000000ull;
+  m = (ex == 0 || r > 54) ? 0ull : ((m >> max(r, 0)) + 1) >> 1;
+  const long long q = (long long)b < 0 ? -(long long)m : (long long)m;
+  const int hi = (int)((q + (1 << 26)) >> 27);
+  return make_int2(hi, (int)(q - ((long long)hi << 27)));
+}
 
-    if (threadIdx.x == 0) {
-      double ld = 0.0;
-      for (int j = 0; j < K; ++j) ld += 2.0 * log(fabs(s.Lx[j * K + j]) + 1e-10);
-      o.logdet_XtX[pd] = ld;
-      o.info[pd] = info;
-    }
+// The sums of a Gram entry.
+struct FixedDot {
+  long long hh = 0, x = 0, ll = 0;
+  __device__ __forceinline__ void add(int2 a, int2 b) {
+    hh += (long long)a.x * b.x;
+    x += (long long)a.x * b.y;
+    x += (long long)a.y * b.x;
+    ll += (long long)a.y * b.y;
+  }
+  // the entry, for columns scaled by 2^si and 2^sj
+  __device__ __forceinline__ double value(int si, int sj) const {
+    const double v = fma((double)hh, 0x1p54, fma((double)x, 0x1p27, (double)ll));
+    return v * __hiloint2double((1023 - si - sj) << 20, 0);
+  }
+};
 
-    // ---- 5. Q = X_w Lx^-T in fp32 (Q, U and G only leave as fp32 or fp16
-    // splits; the factorisation and the logdets above stay FP64). The two [K][T]
-    // FP64 slots are reused as fp32 arrays; the QR fallback converts its Q.
-    float* const xw_f = reinterpret_cast<float*>(s.Xw);
-    float* const qm_f = reinterpret_cast<float*>(s.Qm);
-    float* const lx_f = reinterpret_cast<float*>(s.S);  // [K][K] Lx, then Li in lx_f + K*K
-    float* qf;
-    float* uf;
-    for (int idx = threadIdx.x; idx < K * K; idx += blockDim.x) lx_f[idx] = (float)s.Lx[idx];
-    __syncthreads();
-    if (info != 1) {
-      for (int t = threadIdx.x; t < T; t += blockDim.x) {
-        for (int j = 0; j < K; ++j) {
-          float acc = (float)s.Xw[(size_t)j * T + t];
-          for (int i = 0; i < j; ++i) acc = fmaf(-lx_f[j * K + i], qm_f[(size_t)i * T + t], acc);
-          qm_f[(size_t)j * T + t] = acc / lx_f[j * K + j];
-        }
-      }
-      qf = qm_f;
-      uf = xw_f;
+// float of a double, rounded to nearest even, by its bit fields (integer pipe);
+// anything but zeros and normal results takes the hardware conversion.
+__device__ __forceinline__ float d2f_exact(double w) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(w);
+  const unsigned long long m = b & 0x7fffffffffffffffull;
+  const uint32_t sg = (uint32_t)(b >> 32) & 0x80000000u;
+  if (m == 0) return __uint_as_float(sg);
+  const unsigned ex = (unsigned)(m >> 52);
+  if (ex - 897u >= 253u) return (float)w;
+  const unsigned long long r = m + 0x0fffffffull + ((m >> 29) & 1);
+  return __uint_as_float(sg | ((uint32_t)(r >> 29) - (896u << 23)));
+}
+
+// ------------------------------------------------------------- items in shared memory
+// Items of up to GI_KMAX columns and FX_TMAX samples whose matrices fit in
+// shared memory: the phases of item_global, arranged around the FP64 pipe,
+// which a warp fills with one instruction per 64 cycles whatever its lanes do.
+//   - X_w = L^-1 X in a pipeline over chunks of 8 to 32 samples of each time segment
+//     (segments start at run starts, where the recursion does), a chunk in each
+//     stage: z = x - c x' by all entry warps (full warps); v = z - m v' by the
+//     producer warps, a lane per column and segment, one FP64 instruction a
+//     step; w = v / sqrt(D) by the entry warps, in fixed point for the Gram
+//     matrix and as the fp32 copy that the later phases read; the Gram matrix in
+//     integers (above), blocks of 2 x 2 entries per thread, the samples split over
+//     SL threads of a block.
+//   - The Cholesky factorisation keeps each entry in its thread's register,
+//     two barriers a column; the producer warps then invert the factor while
+//     the others form Q, U and the fp16 splits in place in shared memory.
+// A rank-deficient item (a pivot that is not positive) or one whose series
+// leave the fixed point goes through item_global.
+// Builds, us, against item_global's phases with FP64 Gram chains: P = 117,
+// T = 200, K = 8: 238 -> 108; P = 561, T = 400, K = 20: 584 -> 307; K = 32: 1016
+// -> 676; T = 500, K = 40: 1319 -> 1059; 20 designs of T = 855, K = 18: 13629 ->
+// 7960. Bound now by latency: two or three CTAs an SM (their series fill the
+// shared memory), a barrier per chunk.
+constexpr int GI_KMAX = 40;       // 820 entry threads
+constexpr int GI_BUF = 4;         // chunks in the pipeline
+constexpr int GI_PROD = 96;       // most producer lanes (3 warps)
+constexpr int GI_VAL = 3;         // most values of a chunk per thread
+constexpr int GI_SMALL_K = 22;    // designs of up to this many columns need 256 + 96 threads
+constexpr int GI_SMALL = 256 + GI_PROD;
+
+struct ItemPlan {
+  // entries, their threads, rows (even), 2 x 2 blocks, slices, row stride, time
+  // segments, producer warps, log2 of a segment's samples per chunk
+  int E, GT, KR, NB, SL, rs, RP, PW, cs2;
+  int cm, xf, ring, L, Li, rd, lxf, lif, total;  // byte offsets
+};
+
+__host__ __device__ inline ItemPlan item_plan(int T, int K, int n_runs) {
+  ItemPlan m;
+  m.E = K * (K + 1) / 2;
+  m.GT = (m.E + 31) / 32 * 32;
+  if (m.GT < 256) m.GT = 256;
+  const int kb = (K + 1) / 2;
+  m.KR = 2 * kb;
+  m.NB = kb * (kb + 1) / 2;
+  m.SL = 1;
+  m.RP = 1;  // time segments: the fewest whose longest has the fewest runs
+  for (int rp = 2; rp <= n_runs && rp * K <= GI_PROD; ++rp)
+    if ((n_runs + rp - 1) / rp < (n_runs + m.RP - 1) / m.RP) m.RP = rp;
+  m.cs2 = 3;  // 8 samples, or 16 or 32 while a chunk is at most two values per thread
+  while (m.cs2 < 5 && (K * m.RP << (m.cs2 + 1)) <= 2 * m.GT) ++m.cs2;
+  const int cs = 1 << m.cs2;
+  while (2 * m.SL * m.NB <= m.GT && m.SL < 16 && m.SL < cs) m.SL *= 2;
+  m.rs = cs + (m.SL == 4 ? 2 : m.SL == 8 ? 4 : 1);  // a half-warp's blocks and slices in distinct banks
+  m.PW = (K * m.RP + 31) / 32;
+  const int K4 = (K + 3) & ~3;
+  int at = 0;
+  auto take = [&](size_t n) {
+    const int o = at;
+    at += (int)((n + 15) & ~(size_t)15);
+    return o;
+  };
+  m.cm = take(sizeof(double) * 3 * T);  // c, m, 1/sqrt(D); later the fp32 coefficients
+  // the fp32 series, whose region also holds phase 1's 4 T doubles
+  const size_t xf = sizeof(float) * (size_t)K * (T | 1), tmp = sizeof(double) * 4 * T;
+  m.xf = take(xf > tmp ? xf : tmp);
+  // [GI_BUF][RP][KR][rs] samples (FP64, then fixed point); afterwards 2 K^2 doubles of scratch
+  size_t ring = sizeof(int2) * GI_BUF * m.RP * m.KR * m.rs;
+  const size_t scr = sizeof(double) * 2 * K * K, cf = sizeof(float4) * T;  // before it, the fp32 coefficients
+  ring = ring > scr ? ring : scr;
+  m.ring = take(ring > cf ? ring : cf);
+  m.L = take(sizeof(double) * K * K);
+  m.Li = take(sizeof(double) * K * K);
+  m.rd = take(sizeof(double) * K);
+  m.lxf = take(sizeof(float) * K * K4);   // Lx transposed: [i][j], j contiguous
+  m.lif = take(sizeof(float) * K * K4);
+  m.total = at;
+  return m;
+}
+
+// Barrier of the first n threads (a multiple of 32) of the CTA.
+__device__ __forceinline__ void bar_sync(int id, int n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+template <bool SHARED_LDL, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == GI_SMALL ? 3 : 1) grid_item_kernel(BuildArgs args, int n_designs,
+                                                                                         const double* pair_cm,
+                                                                                         const int* pair_bad) {
+  const ffs_grid_desc& d = args.d;
+  const ffs_grid_out& o = args.o;
+  const int T = d.T, K = d.K, LT = ld_t(T), K4 = (K + 3) & ~3, ldx = T | 1;
+  const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, wid = tid >> 5;
+  extern __shared__ double2 gi_smem[];
+  char* sm = reinterpret_cast<char*>(gi_smem);
+  const ItemPlan pl = item_plan(T, K, d.n_runs);
+  const int GT = pl.GT, RP = pl.RP, rs = pl.rs;
+  double* cc = reinterpret_cast<double*>(sm + pl.cm);
+  double *cm = cc + T, *cr = cc + 2 * T;
+  float4* cfs = reinterpret_cast<float4*>(sm + pl.cm);     // after phase 4: (c, m, 1/D, 1/sqrt(D)) in fp32
+  float* xf = reinterpret_cast<float*>(sm + pl.xf);        // [K][ldx] X_w, then Q, then U
+  int2* ring = reinterpret_cast<int2*>(sm + pl.ring);      // [GI_BUF][RP][KR][rs]
+  const int bufw = RP * pl.KR * rs, cs2 = pl.cs2, CS = 1 << cs2;
+  double* scr = reinterpret_cast<double*>(sm + pl.ring);
+  double* L = reinterpret_cast<double*>(sm + pl.L);        // [K][K] X_w'X_w, then its factor
+  double* Li = reinterpret_cast<double*>(sm + pl.Li);
+  double* rd = reinterpret_cast<double*>(sm + pl.rd);      // 1 / diag(L)
+  float* lxf = reinterpret_cast<float*>(sm + pl.lxf);
+  float* lif = reinterpret_cast<float*>(sm + pl.lif);
+  __shared__ double red[32];
+  __shared__ float fred[32];
+  __shared__ int colmax[GI_KMAX], scale[GI_KMAX + 1];
+  __shared__ int seg[GI_PROD + 1];  // first sample of each time segment
+  __shared__ int flag, bad_r;
+  for (int q = tid; q <= RP; q += nth) seg[q] = d.run_start[q * d.n_runs / RP];
+  const bool entry = tid < pl.E;
+  int ei = 0, ej = 0;
+  if (entry) tri_index(tid, ei, ej);
+  int bi = 0, bj = 0;  // this thread's 2 x 2 block of the Gram matrix, and its slice of the samples
+  const bool gram = tid < pl.NB * pl.SL;
+  const int sl = tid % pl.SL;
+  if (gram) tri_index(tid / pl.SL, bi, bj);
+  const bool producer = tid >= GT && tid - GT < K * RP;
+  const int pj = producer ? (tid - GT) % K : 0, pq = producer ? (tid - GT) / K : 0;
+  __syncthreads();
+
+  for (int item = blockIdx.x; item < d.P * n_designs; item += gridDim.x) {
+    const int p = item % d.P, pd = item;
+    const float* Xd = d.X + (size_t)(item / d.P) * T * K;
+    if constexpr (SHARED_LDL) {
+      const double* src = pair_cm + (size_t)p * 4 * T;
+      for (int i = tid; i < 3 * T; i += nth) cc[i] = src[i];
+      if (tid == 0) bad_r = pair_bad[p];
     } else {
-      for (int idx = threadIdx.x; idx < K * T; idx += blockDim.x) xw_f[idx] = (float)s.Qm[idx];
-      qf = xw_f;
-      uf = qm_f;
+      ldl_of_pair(d, o, p, cc, cm, cr, reinterpret_cast<double*>(xf), red, &bad_r);
     }
+    if (tid == 0) flag = 0;
+    for (int j = tid; j < K; j += nth) colmax[j] = 0;
+    // the design into xf, where X_w replaces it, and the fp32 coefficients into
+    // the ring's region
+    const float4* cf = reinterpret_cast<const float4*>(o.coef) + (size_t)p * T;
+    float4* cfr = reinterpret_cast<float4*>(ring);
+    if (!SHARED_LDL) __syncthreads();  // phase 1's scratch is read no more
+    for (int t = tid; t < T; t += nth) cfr[t] = cf[t];
+#pragma unroll 4
+    for (int e = tid; e < K * T; e += nth) xf[(size_t)(e % K) * ldx + e / K] = __ldg(Xd + e);
     __syncthreads();
 
-    // ---- 6. U = L^-T Q = A' L~^-T D^-1/2 Q (backward recursions) in fp32, with
-    // the fp32 coefficients of phase 1
-    const float4* cf = reinterpret_cast<const float4*>(o.coef) + (size_t)p * T;
-    float umax_local = 0.f;
-    if (d.band) {
-      // back substitution against the band: u_t = (q_t - sum_i L(t + i, t)
-      // u_{t+i}) / L(t, t), the rows t + i of t's run within the band
-      const int W = d.band_w;
-      const double* Lb = o.band_L + (size_t)p * T * W;
-      const int* Jrow = reinterpret_cast<const int*>(cms + T);
-      for (int j = threadIdx.x; j < K; j += blockDim.x) {
-        const float* q = qf + (size_t)j * T;
-        float* u = uf + (size_t)j * T;
-        for (int t = T - 1; t >= 0; --t) {
-          double acc = (double)q[t];
-          for (int i = 1; t + i < T && i <= Jrow[t + i]; ++i) acc = fma(-Lb[(size_t)(t + i) * W + i], (double)u[t + i], acc);
-          const float ut = (float)(acc * cms[t]);
-          u[t] = ut;
-          o.U[((size_t)pd * K + j) * LT + t] = ut;
-          umax_local = fmaxf(umax_local, fabsf(ut));
-        }
-        for (int t = T; t < LT; ++t) o.U[((size_t)pd * K + j) * LT + t] = 0.f;
+    // ---- 2, 3. X_w and X_w'X_w
+    const int ps = producer ? seg[pq] : 0, pe = producer ? seg[pq + 1] : 0;
+    if (producer) {
+      // the columns' scales, from the recursion in fp32
+      const float* xs = xf + (size_t)pj * ldx;
+      float xp = 0.f, vp = 0.f, mx = 0.f;
+#pragma unroll 8
+      for (int t = ps; t < pe; ++t) {
+        const float x = xs[t];
+        const float4 q = cfr[t];
+        vp = fmaf(-q.y, vp, fmaf(-q.x, xp, x));
+        xp = x;
+        mx = fmaxf(mx, fabsf(vp * q.w));
       }
+      atomicMax(colmax + pj, __float_as_int(mx));
     }
-    for (int j = threadIdx.x; j < K && !d.band; j += blockDim.x) {
-      const float* q = qf + (size_t)j * T;
-      float* u = uf + (size_t)j * T;
-      float xn = 0.f, mn = 0.f, cn = 0.f;  // x_{t+1}, m_{t+1}, c_{t+1}
-      for (int t1 = T - 1; t1 >= 0; t1 -= GB_PF) {  // GB_PF steps of q and coef loaded ahead
-        float qb[GB_PF];
-        float4 cb[GB_PF];
+    __syncthreads();
+    if (pl.KR > K)  // the row past an odd K is zero
+      for (int e = tid; e < GI_BUF * RP * rs; e += nth) ring[(e / rs * pl.KR + K) * rs + e % rs] = make_int2(0, 0);
+    for (int j = tid; j < K; j += nth) scale[j] = fixed_scale(__int_as_float(colmax[j]));
+    __syncthreads();
+    int longest = 0;
+    for (int q = 0; q < RP; ++q) longest = max(longest, seg[q + 1] - seg[q]);
+    const int nch = (longest + CS - 1) >> cs2;
+    FixedDot acc[2][2];
+    {
+      // the values of a chunk this thread forms (z) and converts (w): slot in a
+      // ring buffer, sample of chunk 0 and its segment's end
+      int vs[GI_VAL], vt[GI_VAL], ve[GI_VAL], vj[GI_VAL];
 #pragma unroll
-        for (int k = 0; k < GB_PF; ++k) {
-          const int t = t1 - k;
-          qb[k] = t >= 0 ? q[t] : 0.f;
-          cb[k] = t >= 0 ? cf[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < GI_VAL; ++i) {
+        const int e = tid + i * GT;  // sample fastest: consecutive lanes, consecutive words
+        const bool on = tid < GT && e < K * RP << cs2;
+        const int k = e & (CS - 1), j = (e >> cs2) % K, q = on ? (e >> cs2) / K : 0;
+        vj[i] = j;
+        vs[i] = on ? (q * pl.KR + j) * rs + k : -1;
+        vt[i] = seg[q] + k;
+        ve[i] = seg[q + 1];
+      }
+      double vp = 0.0;
+      bool over = false;
+      for (int c = 0; c < nch + GI_BUF - 1; ++c) {
+        if (tid < GT) {
+          double* za = reinterpret_cast<double*>(ring) + (c % GI_BUF) * bufw;
+          if (c < nch) {
+#pragma unroll
+            for (int i = 0; i < GI_VAL; ++i) {
+              const int t = vt[i] + (c << cs2);
+              if (vs[i] >= 0 && t < ve[i]) {
+                const float* x = xf + (size_t)vj[i] * ldx + t;
+                za[vs[i]] = f2d_exact(x[0]) - cc[t] * f2d_exact(t > 0 ? x[-1] : 0.f);
+              }
+            }
+          }
+          if (c >= 2 && c < nch + 2) {
+            int2* wb = ring + ((c - 2) % GI_BUF) * bufw;
+#pragma unroll
+            for (int i = 0; i < GI_VAL; ++i) {
+              const int t = vt[i] + ((c - 2) << cs2);
+              if (vs[i] >= 0) {
+                int2 f = make_int2(0, 0);
+                if (t < ve[i]) {
+                  const double w = reinterpret_cast<double*>(wb)[vs[i]] * cr[t];
+                  f = fixed_of(w, scale[vj[i]], over);
+                  xf[(size_t)vj[i] * ldx + t] = d2f_exact(w);
+                }
+                wb[vs[i]] = f;
+              }
+            }
+          }
+          if (gram && c >= 3) {
+            const int2* rg = ring + ((c - 3) % GI_BUF) * bufw;
+            for (int u = sl; u < RP << cs2; u += pl.SL) {
+              const int2* r0 = rg + (u >> cs2) * pl.KR * rs + (u & (CS - 1));
+              const int2 *ai = r0 + 2 * bi * rs, *aj = r0 + 2 * bj * rs;
+              const int2 i0 = ai[0], i1 = ai[rs], j0 = aj[0], j1 = aj[rs];
+              acc[0][0].add(i0, j0);
+              acc[0][1].add(i0, j1);
+              acc[1][0].add(i1, j0);
+              acc[1][1].add(i1, j1);
+            }
+          }
+        } else if (producer && c >= 1 && c <= nch) {
+          double* v = reinterpret_cast<double*>(ring) + ((c - 1) % GI_BUF) * bufw + (pq * pl.KR + pj) * rs;
+          for (int k0 = 0; k0 < CS; k0 += 8, v += 8) {
+            const int t0 = ps + ((c - 1) << cs2) + k0;
+            double z[8], m[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              z[k] = v[k];
+              m[k] = cm[min(t0 + k, T - 1)];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) z[k] = vp = z[k] - m[k] * vp;  // past the segment: not read
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = z[k];
+          }
         }
+        __syncthreads();
+      }
+      if (over) flag = 1;
+    }
+    if (wid * 32 < pl.NB * pl.SL) {  // whole warps: the slices of a block lie in one
 #pragma unroll
-        for (int k = 0; k < GB_PF; ++k) {
-          const int t = t1 - k;
-          if (t >= 0) {
-            const float4 c4 = cb[k];  // (c, m, 1/D, 1/sqrt(D))
-            const float x = fmaf(-mn, xn, qb[k] * c4.w);
-            const float ut = fmaf(-cn, xn, x);
-            u[t] = ut;
-            o.U[((size_t)pd * K + j) * LT + t] = ut;
-            umax_local = fmaxf(umax_local, fabsf(ut));
-            xn = x;
-            mn = c4.y;
-            cn = c4.x;
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          FixedDot& f = acc[u][v];
+          for (int m = 1; m < pl.SL; m <<= 1) {
+            f.hh += __shfl_xor_sync(0xffffffffu, f.hh, m);
+            f.x += __shfl_xor_sync(0xffffffffu, f.x, m);
+            f.ll += __shfl_xor_sync(0xffffffffu, f.ll, m);
+          }
+          const int i = 2 * bi + u, j = 2 * bj + v;
+          if (gram && sl == 0 && i < K && j <= i) {
+            const double x = f.value(scale[i], scale[j]);
+            L[i * K + j] = x;
+            o.XtX[(size_t)pd * K * K + i * K + j] = (float)x;
+            o.XtX[(size_t)pd * K * K + j * K + i] = (float)x;
+          }
+        }
+    }
+    __syncthreads();
+    double mij = entry ? L[ei * K + ej] : 0.0;
+    const bool left = flag != 0;  // a series left the fixed point
+    __syncthreads();
+
+    // ---- 4. Cholesky, right-looking, an entry per thread: column k's entries
+    // are put down, the first warps scale them (full warps of the FP64 pipe), and
+    // every later entry takes its product off
+    for (int k = 0; k < K && !left; ++k) {
+      if (entry && ej == k) L[ei * K + k] = mij;
+      __syncthreads();
+      if (tid < (K + 31) / 32 * 32) {
+        const double dk = L[k * K + k];
+        const bool pos = dk > 0.0;
+        const double r = pos ? rsqrt_newton(dk) : 1.0;
+        __syncwarp();
+        if (tid > k && tid < K) L[tid * K + k] *= r;
+        if (tid == k) {
+          rd[k] = r;
+          scr[k] = pos ? dk * r : 1.0;  // the diagonal, put in place after the column's readers
+          if (!pos) flag = 1;
+        }
+      }
+      __syncthreads();
+      if (flag) break;
+      if (entry && ej > k) mij -= L[ei * K + k] * L[ej * K + k];
+    }
+    if (!flag) {
+      for (int k = tid; k < K; k += nth) L[k * K + k] = scr[k];
+    }
+    __syncthreads();
+    if (flag) {
+      __syncthreads();
+      const PairScratch s = scratch_of(o.work, blockIdx.x, T, K);
+      item_global(args, s, p, pd, Xd, cc, cm, cr, bad_r, red, &flag);
+      continue;
+    }
+    for (int e = tid; e < K * K4; e += nth) {
+      const int i = e / K4, j = e % K4;
+      lxf[e] = j < K && j >= i ? (float)L[j * K + i] : 0.f;
+    }
+    for (int t = tid; t < T; t += nth) cfs[t] = cf[t];  // c, m and 1/sqrt(D) in FP64 are done with
+    __syncthreads();
+
+    if (tid < GT) {
+      // ---- 5. Q = X_w Lx^-T in fp32, two samples per thread, four columns at a
+      // time: each earlier column is read once for them
+      for (int t = tid; t < T; t += 2 * GT) {
+        float* q = xf + t;
+        const int u1 = t + GT < T ? GT : 0;  // the second sample, or the first again
+        for (int j0 = 0; j0 < K; j0 += 4) {
+          float a4[4], b4[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            a4[c] = j0 + c < K ? q[(size_t)(j0 + c) * ldx] : 0.f;
+            b4[c] = j0 + c < K ? q[(size_t)(j0 + c) * ldx + u1] : 0.f;
+          }
+#pragma unroll 4
+          for (int i = 0; i < j0; ++i) {
+            const float qa = q[(size_t)i * ldx], qb = q[(size_t)i * ldx + u1];
+            const float4 l = *reinterpret_cast<const float4*>(lxf + i * K4 + j0);
+            a4[0] = fmaf(-l.x, qa, a4[0]);
+            b4[0] = fmaf(-l.x, qb, b4[0]);
+            a4[1] = fmaf(-l.y, qa, a4[1]);
+            b4[1] = fmaf(-l.y, qb, b4[1]);
+            a4[2] = fmaf(-l.z, qa, a4[2]);
+            b4[2] = fmaf(-l.z, qb, b4[2]);
+            a4[3] = fmaf(-l.w, qa, a4[3]);
+            b4[3] = fmaf(-l.w, qb, b4[3]);
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (j0 + c < K) {
+              const float* l = lxf + (j0 + c) * K4 + j0;
+              a4[c] = a4[c] / l[c];
+              b4[c] = b4[c] / l[c];
+#pragma unroll
+              for (int e = c + 1; e < 4; ++e) {
+                a4[e] = fmaf(-l[e], a4[c], a4[e]);
+                b4[e] = fmaf(-l[e], b4[c], b4[e]);
+              }
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (j0 + c < K) {
+              q[(size_t)(j0 + c) * ldx] = a4[c];
+              q[(size_t)(j0 + c) * ldx + u1] = b4[c];
+            }
           }
         }
       }
-      for (int t = T; t < LT; ++t) o.U[((size_t)pd * K + j) * LT + t] = 0.f;
-    }
-    __syncthreads();
-    if (o.U_hi) {
-      // fp16 hi/lo split of U * 2^e, e placing max|U| in [128, 256)
-      double um = umax_local;
-      for (int off = 16; off > 0; off >>= 1) um = fmax(um, __shfl_xor_sync(0xffffffffu, um, off));
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = um;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double mx = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mx = fmax(mx, red[w]);
-        red[0] = mx;
+      bar_sync(1, GT);
+      // ---- 6. U = L^-T Q, the backward recursions of each column and run
+      float umax = 0.f;
+      for (int e = tid; e < K * d.n_runs; e += GT) {
+        const int j = e % K, r = e / K;
+        float* u = xf + (size_t)j * ldx;
+        const int t0 = d.run_start[r];
+        float xn = 0.f, mn = 0.f, cn = 0.f;  // x_{t+1}, m_{t+1}, c_{t+1} (0 past a run's end)
+        constexpr int UB = 8;
+        float qn[UB];
+        float4 cb[UB];
+        auto load_c = [&](int t1) {
+#pragma unroll
+          for (int k = 0; k < UB; ++k) {
+            const int t = max(t1 - k, t0);
+            cb[k] = cfs[t];
+            qn[k] = u[t];
+          }
+        };
+        const int te = d.run_start[r + 1] - 1;
+        load_c(te);
+        for (int t1 = te; t1 >= t0; t1 -= UB) {
+          float qw[UB], mm[UB], ccv[UB];
+#pragma unroll
+          for (int k = 0; k < UB; ++k) {
+            qw[k] = qn[k] * cb[k].w;
+            mm[k] = cb[k].y;
+            ccv[k] = cb[k].x;
+          }
+          load_c(t1 - UB);  // the next batch's, before this one's stores
+#pragma unroll
+          for (int k = 0; k < UB; ++k) {
+            const float x = fmaf(-mn, xn, qw[k]);
+            qw[k] = fmaf(-cn, xn, x);
+            xn = x;
+            mn = mm[k];
+            cn = ccv[k];
+          }
+#pragma unroll
+          for (int k = 0; k < UB; ++k) {
+            if (t1 - k >= t0) {
+              u[t1 - k] = qw[k];
+              umax = fmaxf(umax, fabsf(qw[k]));
+            }
+          }
+        }
       }
-      __syncthreads();
-      const int e = scale_exp((float)red[0]);
-      if (threadIdx.x == 0) o.uexp[pd] = e;
-      for (int idx = threadIdx.x; idx < K * d.ld_u; idx += blockDim.x) {
-        const int j = idx / d.ld_u, t = idx % d.ld_u;
-        uint16_t hi = 0, lo = 0;
-        if (t < T) split_fp16(ldexpf(uf[(size_t)j * T + t], e), hi, lo);
-        const size_t at = ((size_t)pd * K + j) * d.ld_u + t;
-        o.U_hi[at] = hi;
-        o.U_lo[at] = lo;
+      for (int off = 16; off > 0; off >>= 1) umax = fmaxf(umax, __shfl_xor_sync(0xffffffffu, umax, off));
+      if (lane == 0) fred[wid] = umax;
+      bar_sync(1, GT);
+      float mx = 0.f;
+      for (int w = 0; w < GT / 32; ++w) mx = fmaxf(mx, fred[w]);
+      // fp16 hi/lo split of U * 2^e, e placing max|U| in [128, 256); x * 2^e as
+      // one product when 2^e is a normal float (ldexpf's value)
+      const int ex = scale_exp(mx);
+      if (o.U_hi && tid == 0) o.uexp[pd] = ex;
+      const bool pw = ex >= -126 && ex <= 127;
+      const float p2 = pw ? __int_as_float((ex + 127) << 23) : 0.f;
+      for (int j = wid; j < K; j += GT / 32) {  // a warp per column
+        const float* u = xf + (size_t)j * ldx;
+        float* uo = o.U + ((size_t)pd * K + j) * LT;
+#pragma unroll 4
+        for (int t = lane; t < LT; t += 32) uo[t] = t < T ? u[t] : 0.f;
+        if (o.U_hi) {
+          uint32_t* ho = reinterpret_cast<uint32_t*>(o.U_hi + ((size_t)pd * K + j) * d.ld_u);
+          uint32_t* lo = reinterpret_cast<uint32_t*>(o.U_lo + ((size_t)pd * K + j) * d.ld_u);
+#pragma unroll 4
+          for (int h = lane; h < (d.ld_u >> 1); h += 32) {
+            const int t = 2 * h;
+            uint16_t h0 = 0, l0 = 0, h1 = 0, l1 = 0;
+            if (t < T) split_fp16(pw ? __fmul_rn(u[t], p2) : ldexpf(u[t], ex), h0, l0);
+            if (t + 1 < T) split_fp16(pw ? __fmul_rn(u[t + 1], p2) : ldexpf(u[t + 1], ex), h1, l1);
+            ho[h] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+            lo[h] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+          }
+        }
+      }
+    } else {
+      // ---- 7. Li = Lx^-1, a column per lane: each entry formed takes its part
+      // off the rows below it; the logs of logdet beside it
+      for (int c = tid - GT; c < K; c += nth - GT) {
+        scr[c] = 2.0 * log(fabs(L[c * K + c]) + 1e-10);
+        for (int i = 0; i < K; ++i) Li[i * K + c] = i == c ? 1.0 : 0.0;
+        for (int k = c; k < K; ++k) {
+          const double v = Li[k * K + c] * rd[k];
+          Li[k * K + c] = v;
+#pragma unroll 4
+          for (int i = k + 1; i < K; ++i) Li[i * K + c] -= L[i * K + k] * v;
+        }
       }
     }
     __syncthreads();
 
-    // ---- 7. Lx^-1 and diag(A), A = Lx^-T Lx^-1 = (X_w'X_w)^-1 (only the
-    // entries the statistics read are formed: the diagonal here, the task
-    // block and c A c' in phase 9)
-    block_tri_inverse(s.Lx, s.Li, K, K, chol ? s.A : nullptr);
-    for (int j = threadIdx.x; j < K; j += blockDim.x) {
-      double acc = 0.0;
-      for (int k = j; k < K; ++k) acc += s.Li[k * K + j] * s.Li[k * K + j];
-      o.Adiag[(size_t)pd * K + j] = (float)acc;
+    if (tid == 0) {
+      double ld = 0.0;
+      for (int j = 0; j < K; ++j) ld += scr[j];
+      o.logdet_XtX[pd] = ld;
+      o.info[pd] = bad_r ? 2 : 0;
+    }
+    for (int e = tid; e < K * K4; e += nth) {
+      const int i = e / K4, j = e % K4;
+      lif[e] = j < K ? (float)Li[i * K + j] : 0.f;
+    }
+    for (int j = tid; j < K; j += nth) {
+      double a = 0.0;
+      for (int k = j; k < K; ++k) a += Li[k * K + j] * Li[k * K + j];
+      o.Adiag[(size_t)pd * K + j] = (float)a;
     }
     if (o.Afull) {  // all of A, for the per-voxel blocks of the -dsort fit
-      for (int e = threadIdx.x; e < K * K; e += blockDim.x) {
+      for (int e = tid; e < K * K; e += nth) {
         const int i = e / K, j = e % K;
-        double acc = 0.0;
-        for (int k = max(i, j); k < K; ++k) acc += s.Li[k * K + i] * s.Li[k * K + j];
-        o.Afull[(size_t)pd * K * K + e] = (float)acc;
+        double a = 0.0;
+        for (int k = max(i, j); k < K; ++k) a += Li[k * K + i] * Li[k * K + j];
+        o.Afull[(size_t)pd * K * K + e] = (float)a;
       }
     }
+    if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, Li, K, true, scr, red);
     __syncthreads();
 
-    // ---- 8. G = U Lx^-1 in fp32 (row t of G solves g Lx = u_t); Gsum = G' 1
-    // accumulated in FP64
-    float* const li_f = lx_f + (size_t)K * K;
-    for (int idx = threadIdx.x; idx < K * K; idx += blockDim.x) li_f[idx] = (float)s.Li[idx];
-    __syncthreads();
-    for (int t = threadIdx.x; t < LT; t += blockDim.x) {
-      for (int j = 0; j < K; ++j) {
-        float acc = 0.f;
-        if (t < T)
-          for (int i = j; i < K; ++i) acc = fmaf(uf[(size_t)i * T + t], li_f[i * K + j], acc);
-        o.G[((size_t)pd * K + j) * LT + t] = acc;
-      }
-    }
-    __syncthreads();
-    if (o.Gsum) {
-      for (int j = threadIdx.x; j < K; j += blockDim.x) {
-        double acc = 0.0;
-        for (int t = 0; t < T; ++t) acc += (double)o.G[((size_t)pd * K + j) * LT + t];
-        o.Gsum[(size_t)pd * K + j] = (float)acc;
-      }
-    }
-
-    // ---- 9. task-column F matrix inv(A_task + 1e-8 I) and GLT variances c A c'
-    const int nt = d.n_task;
-    if (d.n_glt > 0 && o.glt_var) {  // c A c' = ||Lx^-1 c||^2
-      for (int c = 0; c < d.n_glt; ++c) {
-        const float* gc = d.glt + (size_t)c * K;
-        double part = 0.0;
-        for (int k = threadIdx.x; k < K; k += blockDim.x) {
-          double w = 0.0;
-          for (int j = 0; j <= k; ++j) w += s.Li[k * K + j] * (double)gc[j];
-          part += w * w;
+    // ---- 8. G = U Lx^-1 in fp32, two samples per thread, four columns per pass over U
+    for (int t = tid; t < LT; t += 2 * nth) {
+      const float* u = xf + min(t, T - 1);
+      const bool two = t + nth < LT;
+      const int u1 = two ? min(t + nth, T - 1) - min(t, T - 1) : 0;
+      for (int j0 = 0; j0 < K; j0 += 4) {
+        float a4[4] = {0.f, 0.f, 0.f, 0.f}, b4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int i = j0; i < K; ++i) {  // Li is zero above its diagonal
+          const float ua = u[(size_t)i * ldx], ub = u[(size_t)i * ldx + u1];
+          const float4 l = *reinterpret_cast<const float4*>(lif + i * K4 + j0);
+          a4[0] = fmaf(ua, l.x, a4[0]);
+          b4[0] = fmaf(ub, l.x, b4[0]);
+          a4[1] = fmaf(ua, l.y, a4[1]);
+          b4[1] = fmaf(ub, l.y, b4[1]);
+          a4[2] = fmaf(ua, l.z, a4[2]);
+          b4[2] = fmaf(ub, l.z, b4[2]);
+          a4[3] = fmaf(ua, l.w, a4[3]);
+          b4[3] = fmaf(ub, l.w, b4[3]);
         }
-        const double v = block_sum(part, red);
-        if (threadIdx.x == 0) o.glt_var[(size_t)pd * d.n_glt + c] = (float)v;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (j0 + c < K) {
+            float* g = o.G + ((size_t)pd * K + j0 + c) * LT;
+            g[t] = t < T ? a4[c] : 0.f;
+            if (two) g[t + nth] = t + nth < T ? b4[c] : 0.f;
+          }
+        }
       }
     }
-    // the task block, then the column sets' blocks one after another
-    const int has_task = nt > 0 && o.Ftask ? 1 : 0;
-    const int nsets = o.Fsets ? d.n_sets : 0;
-    size_t msum = 0, off = 0;
-    for (int g = 0; g < nsets; ++g) {
-      const size_t q = (size_t)(d.set_ptr[g + 1] - d.set_ptr[g]);
-      msum += q * q;
-    }
-    for (int bk = 0; bk < has_task + nsets; ++bk) {
-      const bool task = bk < has_task;
-      const int g = bk - has_task;
-      const int n = task ? nt : d.set_ptr[g + 1] - d.set_ptr[g];
-      const int* idx = task ? d.task_idx : d.set_idx + d.set_ptr[g];
-      float* out = task ? o.Ftask + (size_t)pd * nt * nt : o.Fsets + (size_t)pd * msum + off;
-      sub_block_inverse(s, K, idx, n, &flag, out);
-      if (!task) off += (size_t)n * n;
-    }
-    __syncthreads();  // the next item reuses the scratch slot and the shared state
+    PairScratch s{};
+    s.Li = Li;
+    s.S = scr;
+    s.A = scr + (size_t)K * K;
+    item_tail(d, o, s, pd, red, &flag);
   }
 }
 
@@ -755,9 +1463,10 @@ inline int db_chunk(int T, int K) {
   return fit < t4 ? fit : t4;
 }
 
-__global__ void __launch_bounds__(256) design_gram_kernel(int T, int K, int chunk, const float* __restrict__ Xg,
-                                                          double* __restrict__ gram) {
-  extern __shared__ double xt[];  // [ncol][chunk + 1]: the columns this CTA reads, FP64, odd row stride
+__global__ void __launch_bounds__(256) design_gram_kernel(int T, int K, int chunk, int fixed,
+                                                          const float* __restrict__ Xg, double* __restrict__ gram) {
+  extern __shared__ double xt[];  // [ncol][chunk + 1]: the columns this CTA reads (FP64 or fixed point), odd row stride
+  __shared__ int cmax[GI_KMAX + 1];
   const int ne = db_entries(K);
   const int e0 = blockIdx.x * DB_ENTRIES;
   const int e1 = min(e0 + DB_ENTRIES, ne);
@@ -766,20 +1475,40 @@ __global__ void __launch_bounds__(256) design_gram_kernel(int T, int K, int chun
   const int ncol = ihi + 1;  // the entries' rows i <= ihi read columns 0..ihi (column K is the constant)
   const int ld = chunk + 1;
   const int e = e0 + (int)threadIdx.x;
+  const bool mine = threadIdx.x < 32 && e < e1;
   int i = 0, j = 0;
-  if (threadIdx.x < 32 && e < e1) tri_index(e, i, j);
+  if (mine) tri_index(e, i, j);
+  if (fixed) {  // the columns' scales
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) cmax[c] = c < K ? 0 : __float_as_int(1.f);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < T * min(ncol, K); idx += blockDim.x) {
+      const int t = idx / min(ncol, K), c = idx % min(ncol, K);
+      atomicMax(cmax + c, __float_as_int(fabsf(Xg[(size_t)t * K + c])));
+    }
+  }
+  int2* xi = reinterpret_cast<int2*>(xt);
   Dot4 acc;
+  FixedDot fx;
+  bool over = false;
   for (int t0 = 0; t0 < T; t0 += chunk) {
     const int n = min(chunk, T - t0);
     __syncthreads();
     for (int idx = threadIdx.x; idx < n * ncol; idx += blockDim.x) {
       const int t = idx / ncol, c = idx % ncol;
-      xt[c * ld + t] = c < K ? f2d_exact(Xg[(size_t)(t0 + t) * K + c]) : 1.0;
+      const double x = c < K ? f2d_exact(Xg[(size_t)(t0 + t) * K + c]) : 1.0;
+      if (fixed)
+        xi[c * ld + t] = fixed_of(x, fixed_scale(__int_as_float(cmax[c])), over);
+      else
+        xt[c * ld + t] = x;
     }
     __syncthreads();
-    if (threadIdx.x < 32 && e < e1) acc.run(xt + i * ld, xt + j * ld, n);
+    if (mine && fixed)
+      for (int t = 0; t < n; ++t) fx.add(xi[i * ld + t], xi[j * ld + t]);
+    else if (mine)
+      acc.run(xt + i * ld, xt + j * ld, n);
   }
-  if (threadIdx.x < 32 && e < e1) gram[e] = acc.sum();
+  if (mine)
+    gram[e] = fixed ? fx.value(fixed_scale(__int_as_float(cmax[i])), fixed_scale(__int_as_float(cmax[j]))) : acc.sum();
 }
 
 __global__ void __launch_bounds__(DB_THREADS) design_basis_kernel(int T, int K, const float* __restrict__ X,
@@ -916,7 +1645,9 @@ extern "C" int ffs_design_basis(int T, int K, const float* X, void* work, float*
   const size_t gsm = sizeof(double) * (size_t)(K + 1) * (chunk + 1);
   FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(design_gram_kernel), gsm));
   const int nb = ceil_div(db_entries(K), DB_ENTRIES);
-  design_gram_kernel<<<nb, 256, gsm, (cudaStream_t)stream>>>(T, K, chunk, X, gram);
+  // as the grid build forms its Gram matrices at these sizes
+  const int fixed = K <= GI_KMAX && T <= FX_TMAX && item_plan(T, K, 1).total <= 200 * 1024;
+  design_gram_kernel<<<nb, 256, gsm, (cudaStream_t)stream>>>(T, K, chunk, fixed, X, gram);
   if (const int rc = check_launch("design_gram_kernel")) return rc;
   const size_t fsm = K <= DB_SMEM_K ? sizeof(double) * 2 * K + sizeof(double) * (size_t)K * K +
                                           sizeof(float) * (size_t)K * K + sizeof(float) * (size_t)K * DB_THREADS
@@ -943,6 +1674,45 @@ extern "C" size_t ffs_grid_work_bytes_designs(int T, int K, int P, int n_designs
   size_t n = designs_slot_doubles(T, K, P, n_designs, max_ctas);
   if (n_designs > 1) n += (size_t)P * 4 * T + ((size_t)P + 1) / 2;
   return sizeof(double) * n;
+}
+
+// Shared memory of phase 1: 4 T doubles, or with the band invdiag [T], Jrow [T]
+// (ints) and the powers of a [band_w]. A T past 200 KB of it is refused.
+static size_t phase1_smem(const ffs_grid_desc& d) {
+  const size_t n = sizeof(double) * 4 * (size_t)d.T;
+  return d.band ? std::max(n, sizeof(double) * ((size_t)d.T + (d.T + 1) / 2 + (size_t)d.band_w + 1)) : n;
+}
+
+// The item kernel of a build: grid_item_kernel for designs of up to GI_KMAX
+// columns whose items fit in shared memory (half an SM's: two CTAs overlap
+// their latencies; one alone still beats global scratch, so up to 200 KB),
+// grid_build_kernel for the rest.
+static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, const double* pair_cm,
+                        const int* pair_bad, cudaStream_t st, const char* who) {
+  using namespace ffsk;
+  const ffs_grid_desc& d = args.d;
+  const ffs_grid_out& o = args.o;
+  FFS_REQUIRE(phase1_smem(d) <= 200 * 1024, "%s: T=%d too long", who, d.T);
+  FFS_REQUIRE(!o.const_flag == !o.const_coef && (!o.const_flag || (d.p0 >= 0 && d.p0 < d.P)),
+              "%s: const_flag and const_coef go together, with p0=%d in [0, P)", who, d.p0);
+  const ItemPlan pl = item_plan(d.T, d.K, d.n_runs);
+  if (d.K <= GI_KMAX && d.T <= FX_TMAX && !d.band && pl.total <= 200 * 1024 &&
+      (((uintptr_t)o.U_hi | (uintptr_t)o.U_lo) & 3) == 0) {
+    const bool small = d.K <= GI_SMALL_K;
+    auto kern = pair_cm ? (small ? grid_item_kernel<true, GI_SMALL> : grid_item_kernel<true, 1024>)
+                        : (small ? grid_item_kernel<false, GI_SMALL> : grid_item_kernel<false, 1024>);
+    FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), pl.total));
+    kern<<<grid, pl.GT + 32 * pl.PW, pl.total, st>>>(args, n_designs, pair_cm, pair_bad);
+    return check_launch("grid_item_kernel");
+  }
+  // phase 1's scratch beside the coefficients while that leaves room for four CTAs an SM
+  const int tmp_smem = !pair_cm && sizeof(double) * 7 * d.T <= 50 * 1024;
+  size_t smem = sizeof(double) * (tmp_smem ? 7 : 3) * d.T;
+  if (d.band) smem = std::max(smem, phase1_smem(d));
+  auto kern = pair_cm ? grid_build_kernel<true> : grid_build_kernel<false>;
+  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), smem));
+  kern<<<grid, GB_THREADS, smem, st>>>(args, n_designs, pair_cm, pair_bad, tmp_smem);
+  return check_launch("grid_build_kernel");
 }
 
 // n_sets needs its index arrays and the Fsets output
@@ -973,16 +1743,7 @@ extern "C" int ffs_grid_build(const ffs_grid_desc* d, const ffs_grid_out* o, voi
   FFS_REQUIRE(!d->band || (d->band_w >= 1 && d->band_w <= FFS_BAND_MAX_W && o->band_L && o->band_coef),
               "ffs_grid_build: the banded R needs 1 <= band_w=%d <= %d, band_L and band_coef", d->band_w,
               FFS_BAND_MAX_W);
-  BuildArgs args{*d, *o};
-  // shared memory: [T][4] doubles, or with the band invdiag [T], Jrow [T]
-  // (ints) and the powers of a [band_w]
-  size_t smem = sizeof(double) * 4 * (size_t)d->T;
-  if (d->band)
-    smem = std::max(smem, sizeof(double) * ((size_t)d->T + (d->T + 1) / 2 + (size_t)d->band_w + 1));
-  FFS_REQUIRE(smem <= 200 * 1024, "ffs_grid_build: T=%d too long", d->T);
-  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(grid_build_kernel<false>), smem));
-  grid_build_kernel<false><<<d->P, GB_THREADS, smem, (cudaStream_t)stream>>>(args, 1, nullptr, nullptr);
-  return check_launch("grid_build_kernel");
+  return launch_items(BuildArgs{*d, *o}, 1, d->P, nullptr, nullptr, (cudaStream_t)stream, "ffs_grid_build");
 }
 
 extern "C" int ffs_grid_build_designs(const ffs_grid_desc* d, int n_designs, int max_ctas, const ffs_grid_out* o,
@@ -1010,28 +1771,18 @@ extern "C" int ffs_grid_build_designs(const ffs_grid_desc* d, int n_designs, int
   const long long cap = max_ctas > 0 && max_ctas < FFS_GRID_MAX_SLOTS ? max_ctas : FFS_GRID_MAX_SLOTS;
   const int grid = (int)(items < cap ? items : cap);
   BuildArgs args{*d, *o};
-  const size_t smem = sizeof(double) * 4 * (size_t)d->T;
-  // phase 1 of the banded R also holds the powers of a (band_chol_of_pair)
-  const size_t smem1 = d->band ? std::max(smem, sizeof(double) * ((size_t)d->T + (d->T + 1) / 2 +
-                                                                  (size_t)d->band_w + 1))
-                               : smem;
-  FFS_REQUIRE(smem1 <= 200 * 1024, "ffs_grid_build_designs: T=%d too long", d->T);
-  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(grid_build_kernel<false>), smem1));
-  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(grid_build_kernel<true>), smem));
-  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(pair_ldl_kernel), smem1));
   double* pair_cm = nullptr;
   int* pair_bad = nullptr;
   if (n_designs > 1) {
+    const size_t smem = phase1_smem(*d);
+    FFS_REQUIRE(smem <= 200 * 1024, "ffs_grid_build_designs: T=%d too long", d->T);
+    FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(pair_ldl_kernel), smem));
     pair_cm = o->work + designs_slot_doubles(d->T, d->K, d->P, n_designs, max_ctas);
     pair_bad = reinterpret_cast<int*>(pair_cm + (size_t)d->P * 4 * d->T);
-    pair_ldl_kernel<<<d->P, GB_THREADS, smem1, (cudaStream_t)stream>>>(args, pair_cm, pair_bad);
+    pair_ldl_kernel<<<d->P, GB_THREADS, smem, (cudaStream_t)stream>>>(args, pair_cm, pair_bad);
     if (const int rc = check_launch("pair_ldl_kernel")) return rc;
   }
-  if (pair_cm)
-    grid_build_kernel<true><<<grid, GB_THREADS, smem, (cudaStream_t)stream>>>(args, n_designs, pair_cm, pair_bad);
-  else
-    grid_build_kernel<false><<<grid, GB_THREADS, smem1, (cudaStream_t)stream>>>(args, n_designs, nullptr, nullptr);
-  return check_launch("grid_build_kernel (designs)");
+  return launch_items(args, n_designs, grid, pair_cm, pair_bad, (cudaStream_t)stream, "ffs_grid_build_designs");
 }
 
 // ---------------------------------------------------------------------------
@@ -1116,11 +1867,5 @@ extern "C" int ffs_grid_build_noalloc(const ffs_grid_desc* d, const ffs_grid_out
   // the previous call's contents need no clearing
   BuildArgs args{*d, *o};
   args.o.work = scratch;
-  size_t smem = sizeof(double) * 4 * (size_t)d->T;  // as ffs_grid_build
-  if (d->band)
-    smem = std::max(smem, sizeof(double) * ((size_t)d->T + (d->T + 1) / 2 + (size_t)d->band_w + 1));
-  FFS_REQUIRE(smem <= 200 * 1024, "ffs_grid_build_noalloc: T=%d too long", d->T);
-  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(grid_build_kernel<false>), smem));
-  grid_build_kernel<false><<<d->P, GB_THREADS, smem, (cudaStream_t)stream>>>(args, 1, nullptr, nullptr);
-  return check_launch("grid_build_kernel (static scratch)");
+  return launch_items(args, 1, d->P, nullptr, nullptr, (cudaStream_t)stream, "ffs_grid_build_noalloc");
 }

@@ -26,7 +26,7 @@ import numpy as np
 import torch
 
 from .. import _lib
-from .grid import RemlGrid, RunLayout, descent_plan
+from .grid import RemlGrid, RunLayout, descent_plan, lambda_is_zero
 
 LD_ALIGN = 64  # k extent of one tcgen05 pipeline stage
 
@@ -408,7 +408,17 @@ def build_factors(X: torch.Tensor, grid: RemlGrid, layout: RunLayout, *, task_in
     nt = 0 if task_idx is None else task_idx.numel()
     ng = 0 if glt_t is None else glt_t.shape[0]
     lib = _lib.load()
-    cflag, ccoef = constant_flag(Xc) if center is None else center
+    own_center = False
+    if center is None:
+        if stream is None and lambda_is_zero(grid.a[grid.p0], grid.b[grid.p0]):
+            # the build itself tests the constant, at its identity pair's factor
+            own_center = True
+            center = (torch.ones(1, dtype=torch.int32, device=dev), torch.empty(D, K, **f32))
+        elif K <= DESIGN_BASIS_K and D == 1:
+            center = design_basis(Xc, with_constant=True)[1:]
+        else:
+            center = constant_flag(Xc)
+    cflag, ccoef = center
     single = D == 1 and max_ctas <= 0  # else the designs entry point, which takes a CTA cap
     wbytes = lib.ffs_grid_work_bytes(T, K, P) if single else lib.ffs_grid_work_bytes_designs(T, K, P, D, max_ctas)
     work = torch.empty(int(wbytes) // 8 + 1, dtype=torch.float64, device=dev)
@@ -459,12 +469,14 @@ def build_factors(X: torch.Tensor, grid: RemlGrid, layout: RunLayout, *, task_in
                       a=_p(a), b=_p(b), X=_p(Xc), lambda_fp32=0, ld_u=ld,
                       n_task=nt, task_idx=_p(task_idx), n_glt=ng, glt=_p(glt_t),
                       n_sets=sets.n_sets if f.Fsets is not None else 0, set_ptr=_p(sets_dev[0]),
-                      set_idx=_p(sets_dev[1]), band_w=f.band_w, band=_p(f.band))
+                      set_idx=_p(sets_dev[1]), band_w=f.band_w, band=_p(f.band), p0=grid.p0)
     # no Gsum from the kernel: G'1 is the FP64 coefficient vector of the constant (set below)
     o = _lib.GridOut(coef=_p(f.coef), logdet_R=_p(f.logdet_R), logdet_XtX=_p(f.logdet_XtX), U=_p(f.U),
                      U_hi=_p(f.U_hi), U_lo=_p(f.U_lo), uexp=_p(f.uexp), G=_p(f.G), Adiag=_p(f.Adiag), XtX=_p(f.XtX),
                      info=_p(f.info), Ftask=_p(f.Ftask), glt_var=_p(f.glt_var), Gsum=None, work=_p(work),
-                     Fsets=_p(f.Fsets), Afull=_p(f.Afull), band_L=_p(f.band_L), band_coef=_p(f.band_coef))
+                     Fsets=_p(f.Fsets), Afull=_p(f.Afull), band_L=_p(f.band_L), band_coef=_p(f.band_coef),
+                     const_flag=_p(cflag) if own_center else None, const_coef=_p(ccoef) if own_center else None)
+
     def launch():
         if single:
             _run("ffs_grid_build", lib.ffs_grid_build, C.byref(d), C.byref(o), _stream())
@@ -529,6 +541,8 @@ class PrepOut:
     yr_lo: torch.Tensor | None
     yexp: torch.Tensor | None
 
+
+DESIGN_BASIS_K = 64  # widest design whose basis kernel keeps its factor in shared memory
 
 # the one-CTA design basis pays off (beside the grid build) for small designs;
 # wider ones take Q0 from the grid build (U of the pair (0, 0))
@@ -1127,9 +1141,8 @@ class GroupedFitGraph:
     one CUDA graph: the FP64 grid build of every design, the residualisation
     of every voxel against its design, the tcgen05 projection work list, the
     criterion, the selection and the GLS, replayed as one unit. The data and
-    the designs are copied into the graph's static buffers; the centring test
-    of the designs (torch linear algebra) runs before the replay and its
-    result is copied in too. Results are returned as new tensors."""
+    the designs are copied into the graph's static buffers. Results are
+    returned as new tensors."""
 
     def __init__(self, Y: torch.Tensor, Xs: torch.Tensor, grid: RemlGrid, layout: RunLayout, slots: DesignSlots, *,
                  hierarchical: bool, do_scale: bool, gls_kw: dict, factor_kw: dict):
@@ -1138,7 +1151,6 @@ class GroupedFitGraph:
         self.Xs = Xs.float().contiguous().clone()
         self.grid, self.layout, self.slots = grid, layout, slots
         self.hierarchical, self.do_scale, self.gls_kw, self.factor_kw = hierarchical, do_scale, gls_kw, factor_kw
-        self.cflag, self.ccoef = constant_flag(self.Xs)
         self.Y.copy_(Y, non_blocking=True)
         self._body()  # fills the host-side caches a capture must not create
         torch.cuda.synchronize()
@@ -1147,18 +1159,14 @@ class GroupedFitGraph:
             self._body()
 
     def _body(self):
-        self.f = build_factors(self.Xs, self.grid, self.layout, center=(self.cflag, self.ccoef), **self.factor_kw)
+        self.f = build_factors(self.Xs, self.grid, self.layout, **self.factor_kw)
         self.so = search_designs(self.Y, self.f, self.slots, hierarchical=self.hierarchical, do_scale=self.do_scale)
         self.go = gls(self.Y, self.so.scale, self.so.best, self.f, self.Xs, design=self.slots.design, **self.gls_kw)
 
     def run(self, Y: torch.Tensor, Xs: torch.Tensor):
         """(SearchOut, GlsOut) of data Y (V, T) and designs Xs (D, T, K)."""
         self.Y.copy_(Y, non_blocking=True)
-        if not torch.equal(Xs, self.Xs):
-            self.Xs.copy_(Xs)
-            flag, coef = constant_flag(self.Xs)
-            self.cflag.copy_(flag)
-            self.ccoef.copy_(coef)
+        self.Xs.copy_(Xs)
         self.graph.replay()
         so = SearchOut(best=self.so.best.clone(), best_crit=self.so.best_crit.clone(), scale=self.so.scale.clone())
         go = GlsOut(**{k: (None if v is None else v.clone()) for k, v in vars(self.go).items()

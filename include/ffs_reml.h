@@ -108,6 +108,7 @@ typedef struct {
    * exact ARMA(1,1) R. */
   int band_w;
   const int* band;      /* device [P] or NULL                                    */
+  int p0;               /* a pair with lambda == 0 (read with const_flag)        */
 } ffs_grid_desc;
 
 typedef struct {
@@ -135,6 +136,12 @@ typedef struct {
    * whitening w_t = y_t band_coef[t][0] - sum_j band_coef[t][j] w_{t-j}. */
   double* band_L;
   float* band_coef;
+  /* The centring test of ffs_design_basis from pair p0's factor (both or
+   * neither): *const_flag, 1 on entry, is set to 0 when the constant series
+   * is not in the span of some design; const_coef [n_designs][K] its
+   * coefficients, 0 for such a design. */
+  int* const_flag;
+  float* const_coef;
 } ffs_grid_out;
 
 size_t ffs_grid_work_bytes(int T, int K, int P);
