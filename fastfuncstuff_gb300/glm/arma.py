@@ -341,11 +341,16 @@ def fit_glm_arma11(
         pa = _to_tensor(precomputed_arma_params).reshape(-1, 2)
         if pa.shape[0] != V:
             raise ValueError(f"precomputed_arma_params must have shape ({V}, 2), got {tuple(pa.shape)}")
-        pairs, inv = np.unique(pa.numpy().astype(np.float32), axis=0, return_inverse=True)
+        pa_np = pa.numpy()
+        found = engine.distinct_pairs(torch.from_numpy(pa_np), device)
+        if found is None:  # NaNs: np.unique keeps each as a row of its own
+            pairs, inv = np.unique(pa_np.astype(np.float32), axis=0, return_inverse=True)
+            best_all = torch.from_numpy(inv.reshape(-1).astype(np.int32))
+        else:
+            pairs, best_all = found
         grid = grid_of_pairs(pairs[:, 0], pairs[:, 1], use_double=use_double)
         factors = engine.build_factors(Xd, grid, layout, task_indices=ti, glt=glt, with_tc=False, sets=sets,
                                        afull=Dd is not None and bool(column_sets))
-        best_all = torch.from_numpy(inv.reshape(-1).astype(np.int32))
         crit_all = None
     else:
         if a_grid is None and b_grid is None:
@@ -686,7 +691,7 @@ def _apply_dsort(res, dchunks, ti, K, T, labels, want_nods, want_p, mode_p, want
 def _voxel_scale(Y: torch.Tensor, do_scale: bool) -> torch.Tensor:
     if not do_scale:
         return torch.ones(Y.shape[0], device=Y.device, dtype=torch.float32)
-    return Y.double().std(dim=1).float().clamp(min=1e-8)
+    return engine.voxel_scale(Y)
 
 
 def _partial_r2(res, tstats, r2, ti, K, dof, want_p, mode_p, want_s, mode_s, out):

@@ -46,7 +46,7 @@ LAUNCHES = {"ffs_grid_build": 1, "ffs_grid_build_designs": 1, "ffs_reml_prep": 1
             "ffs_reml_window": 1, "ffs_reml_project_tc_list": 1, "ffs_mlp_forward": 1, "ffs_reml_centers": 1,
             "ffs_design_basis": 2, "ffs_reml_strip": 1, "ffs_reml_near_line": 1, "ffs_reml_window_finish": 1,
             "ffs_reml_compact": 1, "ffs_merge_rows": 1, "ffs_reml_segment_items": 2,
-            "ffs_reml_band_sums": 1}
+            "ffs_reml_band_sums": 1, "ffs_series_sd": 1}
 
 
 class StageTimer:
@@ -1095,6 +1095,51 @@ def gls_dsort(Y: torch.Tensor, scale: torch.Tensor, best: torch.Tensor, f: GridF
     return o
 
 
+def voxel_scale(Y: torch.Tensor) -> torch.Tensor:
+    """(V,) max(std of each row, 1e-8) of Y (V, T) (``ffs_series_sd``)."""
+    Y = Y.to(dtype=torch.float32).contiguous()
+    V, T = Y.shape
+    scale = torch.empty(V, dtype=torch.float32, device=Y.device)
+    _run("ffs_series_sd", _lib.load().ffs_series_sd, V, T, _p(Y), _p(scale), None, _stream())
+    return scale
+
+
+def distinct_pairs(ab: torch.Tensor, dev) -> tuple[np.ndarray, torch.Tensor] | None:
+    """(pairs (P, 2) on the host, sorted as np.unique sorts rows; index (V,)
+    int32 on the device) of the given (a, b) (V, 2), or None when some value is
+    a NaN (``ffs_distinct_pairs``)."""
+    lib = _lib.load()
+    ab = ab.to(device=dev, dtype=torch.float32).contiguous()
+    V = ab.shape[0]
+    head = 2048  # pairs read back with the count
+    work = torch.empty(int(lib.ffs_distinct_pairs_work_bytes(V)) // 8 + 1, dtype=torch.int64, device=dev)
+    buf = torch.empty(2 + 2 * max(V, head), dtype=torch.float32, device=dev)  # counts, then the pairs
+    index = torch.empty(V, dtype=torch.int32, device=dev)
+    _run("ffs_distinct_pairs", lib.ffs_distinct_pairs, V, _p(ab), _p(work), buf.data_ptr() + 8, _p(index), _p(buf),
+         _stream(), launches=2)
+    host = buf[: 2 + 2 * head].cpu()
+    n, nan = host[:2].view(torch.int32).tolist()
+    if nan:
+        return None
+    pairs = (host[2 : 2 + 2 * n] if n <= head else buf[2 : 2 + 2 * n].cpu()).numpy().reshape(-1, 2)
+    order = np.lexsort((pairs[:, 1], pairs[:, 0]))
+    rank = np.empty(n, np.int32)
+    rank[order] = np.arange(n, dtype=np.int32)
+    return pairs[order], torch.from_numpy(rank).to(dev).index_select(0, index)
+
+
+def _maybe_constant(D: torch.Tensor) -> bool:
+    """False when no row of D (V, q, T) is constant and nonzero through time
+    (decided on the device by ``ffs_series_sd``; host data are looked at in
+    full)."""
+    if not D.is_cuda or D.numel() == 0:
+        return True
+    D = D.contiguous()
+    n = torch.empty(1, dtype=torch.int32, device=D.device)
+    _run("ffs_series_sd", _lib.load().ffs_series_sd, D.shape[0] * D.shape[1], D.shape[2], _p(D), None, _p(n), _stream())
+    return int(n.item()) > 0
+
+
 def dsort_prepare(dsort, V: int, T: int, run_bounds=None, dev=None) -> torch.Tensor:
     """The -dsort regressors as the kernel reads them, (V, q, T) float32 on the
     device: (V, T) taken as one dataset, the shape checked as the reference
@@ -1110,20 +1155,21 @@ def dsort_prepare(dsort, V: int, T: int, run_bounds=None, dev=None) -> torch.Ten
         Dt = Dt.unsqueeze(1)
     if Dt.ndim != 3 or Dt.shape[0] != V or Dt.shape[2] != T:
         raise ValueError(f"dsort must be (n_voxels={V}, n_dsort, n_timepoints={T}); got {tuple(Dt.shape)}")
-    sd = Dt.double().std(dim=2)
-    mabs = Dt.double().abs().mean(dim=2)
-    bad = (sd < 1e-8) & (mabs > 1e-8)
-    n_bad = int(bad.sum().item())
-    if n_bad:
-        Dt = Dt.clone()
-        for d in range(Dt.shape[1]):
-            bd = bad[:, d]
-            if bool(bd.any()):
-                good = ~bd
-                src = Dt[good, d] if bool(good.any()) else Dt[:, d]
-                Dt[bd, d] = src.double().mean(0).float()
-        warnings.warn(f"-dsort: {n_bad} voxel timeseries were ~constant through time and were replaced by "
-                      "their dataset mean (matches 3dREMLfit).", stacklevel=3)
+    if _maybe_constant(Dt):
+        sd = Dt.double().std(dim=2)
+        mabs = Dt.double().abs().mean(dim=2)
+        bad = (sd < 1e-8) & (mabs > 1e-8)
+        n_bad = int(bad.sum().item())
+        if n_bad:
+            Dt = Dt.clone()
+            for d in range(Dt.shape[1]):
+                bd = bad[:, d]
+                if bool(bd.any()):
+                    good = ~bd
+                    src = Dt[good, d] if bool(good.any()) else Dt[:, d]
+                    Dt[bd, d] = src.double().mean(0).float()
+            warnings.warn(f"-dsort: {n_bad} voxel timeseries were ~constant through time and were replaced by "
+                          "their dataset mean (matches 3dREMLfit).", stacklevel=3)
     if run_bounds is not None:
         rb = [int(x) for x in run_bounds]
         n_runs = len(rb) - 1

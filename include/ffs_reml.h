@@ -201,6 +201,22 @@ size_t ffs_design_basis_work_bytes(int T, int K);
 int ffs_design_basis(int T, int K, const float* X, void* work, float* Q0, int* info, int* const_flag,
                      float* const_coef, void* stream);
 
+/* Standard deviation of each of `rows` series of T samples (Y [rows][T]), N - 1
+ * divisor: scale[row] = max(sd, 1e-8), as fastfuncstuff/glm/arma.py:3952-3954
+ * takes it in float64 (here in compensated fp32 pairs, about 48 bits, then
+ * rounded once). With n_const (device int, or NULL) the number of rows that are
+ * constant and nonzero through time (sd < 1e-8, mean |x| > 1e-8, or within one
+ * part in 10^4 of that: 0 means that the -dsort guard of arma.py:3207-3245 has
+ * nothing to do). scale may be NULL with n_const. */
+int ffs_series_sd(int rows, int T, const float* Y, float* scale, int* n_const, void* stream);
+
+/* The distinct pairs of ab [V][2] (given (a, b) per voxel, arma.py:3744): pairs
+ * [<= V][2] in no particular order, index[v] the row of voxel v's pair,
+ * counts[0] their number, counts[1] = 1 if some value is a NaN (index is then
+ * not to be used). -0 counts as 0. work: ffs_distinct_pairs_work_bytes. */
+size_t ffs_distinct_pairs_work_bytes(int V);
+int ffs_distinct_pairs(int V, const float* ab, void* work, float* pairs, int* index, int* counts, void* stream);
+
 /* The device address of host_ptr: pinned host memory mapped into the device's
  * address space (cudaHostAlloc / cudaHostRegister), or device memory (returned
  * as it is). FFS_ERR_INVALID for pageable or unregistered host memory, which

@@ -225,3 +225,48 @@ def test_grouped_descent_equals_the_full_surface(V, T, K, D, n, monkeypatch):
     monkeypatch.setattr(engine, "DESCENT_MIN_WORK", 1 << 60)
     want = engine.search_designs(Yd, f, slots)
     assert torch.equal(got.best, want.best) and torch.equal(got.best_crit, want.best_crit)
+
+
+# ------------------------------------------------------------------ given (a, b)
+
+
+@gpu
+@pytest.mark.parametrize("V,levels", [(1, 1), (300, 3), (5000, 70), (40000, 40000)])
+def test_distinct_pairs_equal_np_unique(V, levels):
+    """One voxel, heavy repetition, more pairs than one read-back holds; -0 among them; NaN refused."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(V)
+    ab = rng.uniform(-0.9, 0.9, (levels, 2)).astype(np.float32)[rng.integers(0, levels, V)]
+    if V > 1:
+        ab[0], ab[V // 2] = (0.0, -0.0), (-0.0, 0.0)
+    pairs, index = engine.distinct_pairs(torch.from_numpy(ab), DEV)
+    want, inv = np.unique(ab, axis=0, return_inverse=True)
+    np.testing.assert_array_equal(pairs, want)
+    np.testing.assert_array_equal(index.cpu().numpy(), inv.reshape(-1))
+    ab[V - 1, 1] = np.nan
+    assert engine.distinct_pairs(torch.from_numpy(ab), DEV) is None
+
+
+@gpu
+@pytest.mark.parametrize("T", [2, 31, 33, 397, 1024])
+def test_series_sd_is_the_float_nearest_the_float64_value(T):
+    """Compensated sums carry about 48 bits, so the result is within 0.5 ulp
+    (+ 2^-20) of the float64 standard deviation, for large baselines, huge and
+    tiny values; constant rows and NaN as the float64 expression gives them."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(T)
+    Y = rng.standard_normal((70, T)).astype(np.float32)
+    Y[:20] += np.float32(1e4)
+    Y[20:30] *= np.float32(1e25)
+    Y[30:40] *= np.float32(1e-22)
+    Y[40], Y[41], Y[42, 0] = 0.0, 3.7, np.nan
+    got = engine.voxel_scale(torch.from_numpy(Y).to(DEV)).cpu().numpy()
+    want = Y.astype(np.float64).std(1, ddof=1)
+    assert np.isnan(got[42])
+    floor = want < 1e-8
+    assert (got[floor] == np.float32(1e-8)).all()
+    ok = ~floor & ~np.isnan(want)
+    ulp = np.spacing(want[ok].astype(np.float32)).astype(np.float64)
+    assert (np.abs(got[ok].astype(np.float64) - want[ok]) <= (0.5 + 2.0**-20) * ulp + 1e-15 * want[ok]).all()
