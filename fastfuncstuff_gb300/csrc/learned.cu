@@ -7,6 +7,8 @@
 //             sigma ~ U(0.5, 2); normals from Philox4x32-10 (Salmon et al.,
 //             SC'11) through Box-Muller.
 //   MLP       exact-erf GELU; loss sum (out - y)^2 / (2 B); Adam.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace ffsk {
@@ -123,151 +125,253 @@ constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + NH * NI, OFF_W2 = OFF_B1 + NH, OFF_B
               OFF_W3 = OFF_B2 + NH, OFF_B3 = OFF_W3 + NO * NH, N_PARAMS = OFF_B3 + NO;
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float z) {
-  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * expf(-0.5f * z * z) * 0.3989422804014327f;
+
+// gelu and its derivative, one erf for both
+__device__ __forceinline__ void gelu_both(float z, float& g, float& d) {
+  const float h = 0.5f * (1.0f + erff(z * 0.70710678118654752f));
+  g = 0.5f * z * (1.0f + erff(z * 0.70710678118654752f));
+  d = h + z * expf(-0.5f * z * z) * 0.3989422804014327f;
 }
 
-// Two samples per thread: every weight read from shared memory serves both,
-// and the two dependent FMA chains of a unit interleave.
-constexpr int FWD_PER_THREAD = 2;
+// A CTA of 256 threads works on tiles of MT samples held in shared memory with
+// the sample fastest (rows of MS floats: 16-byte loads of 8 rows fall in
+// distinct banks). A 64 x 64 layer over a tile is a small matrix product: each
+// thread forms 4 samples x 4 units, so a 16-byte load serves 16 FMAs, with the
+// units' sums in the order of a plain loop over the inputs (bias first). With
+// one or two samples per thread, every weight was read from shared memory for
+// one or two FMAs, and 8,192 samples gave 32 CTAs (forward 25 us, now 14; 200,000
+// samples 86 us, now 84).
+constexpr int MT = 64;
+constexpr int MS = MT + 4;
 
-__global__ void __launch_bounds__(128) mlp_forward_kernel(const float* __restrict__ prm, const float* __restrict__ x,
-                                                          int B, float* __restrict__ out) {
-  __shared__ float P[N_PARAMS];
-  for (int i = threadIdx.x; i < N_PARAMS; i += blockDim.x) P[i] = prm[i];
+struct MlpSmem {
+  float w1[NH * NI], b1[NH], w2t[NH][NH], b2[NH], w3[NO * NH], b3[NO + 2];
+  float x[NI + 1][MS];       // inputs
+  float h1[NH][MS], h2[NH][MS];
+};
+
+// Parameters, W2 transposed (input-major).
+__device__ __forceinline__ void mlp_load(const float* __restrict__ prm, MlpSmem& m) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  for (int i = tid; i < NH * NI; i += nt) m.w1[i] = prm[OFF_W1 + i];
+  for (int i = tid; i < NH; i += nt) {
+    m.b1[i] = prm[OFF_B1 + i];
+    m.b2[i] = prm[OFF_B2 + i];
+  }
+  for (int i = tid; i < NH * NH; i += nt) m.w2t[i % NH][i / NH] = prm[OFF_W2 + i];
+  for (int i = tid; i < NO * NH; i += nt) m.w3[i] = prm[OFF_W3 + i];
+  if (tid < NO) m.b3[tid] = prm[OFF_B3 + tid];
+}
+
+// The tile's inputs (rows idx[s0 + s], or s0 + s), zero past ns.
+__device__ __forceinline__ void mlp_inputs(const float* __restrict__ x, const int* __restrict__ idx, int s0, int ns,
+                                           MlpSmem& m) {
+  for (int i = threadIdx.x; i < MT * NI; i += blockDim.x) {
+    const int s = i / NI, k = i % NI;
+    m.x[k][s] = s < ns ? x[(size_t)(idx ? idx[s0 + s] : s0 + s) * NI + k] : 0.f;
+  }
+}
+
+// The two hidden layers of the tile; D1 and D2 (NULL for the forward pass
+// alone) receive the derivatives at their inputs. Starts and ends with a barrier.
+template <bool GRAD>
+__device__ __forceinline__ void mlp_hidden(MlpSmem& m, float (*d1)[MS], float (*d2)[MS]) {
+  const int tid = threadIdx.x;
   __syncthreads();
-  const int s0 = (blockIdx.x * blockDim.x + threadIdx.x) * FWD_PER_THREAD;
-  if (s0 >= B) return;
-  const bool two = s0 + 1 < B;
-  float xa[NI], xb[NI], ha[NH], hb[NH];
+  for (int i = tid; i < NH * MT; i += 256) {
+    const int u = i / MT, s = i % MT;
+    float z = m.b1[u];
 #pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    xa[i] = x[(size_t)s0 * NI + i];
-    xb[i] = two ? x[(size_t)(s0 + 1) * NI + i] : 0.f;
+    for (int k = 0; k < NI; ++k) z = fmaf(m.w1[u * NI + k], m.x[k][s], z);
+    if (GRAD)
+      gelu_both(z, m.h1[u][s], d1[u][s]);
+    else
+      m.h1[u][s] = gelu(z);
+  }
+  __syncthreads();
+  const int s4 = 4 * (tid >> 4), u4 = 4 * (tid & 15);
+  float z[4][4];  // [unit][sample]
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) z[j][i] = m.b2[u4 + j];
+#pragma unroll 8
+  for (int k = 0; k < NH; ++k) {
+    const float4 h = *reinterpret_cast<const float4*>(&m.h1[k][s4]);
+    const float4 w = *reinterpret_cast<const float4*>(&m.w2t[k][u4]);
+    const float hv[4] = {h.x, h.y, h.z, h.w}, wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) z[j][i] = fmaf(wv[j], hv[i], z[j][i]);
   }
 #pragma unroll
-  for (int u = 0; u < NH; ++u) {
-    float za = P[OFF_B1 + u], zb = za;
+  for (int j = 0; j < 4; ++j) {
+    float g[4], d[4];
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const float w = P[OFF_W1 + u * NI + i];
-      za = fmaf(w, xa[i], za);
-      zb = fmaf(w, xb[i], zb);
+    for (int i = 0; i < 4; ++i) {
+      if (GRAD)
+        gelu_both(z[j][i], g[i], d[i]);
+      else
+        g[i] = gelu(z[j][i]);
     }
-    ha[u] = gelu(za);
-    hb[u] = gelu(zb);
+    *reinterpret_cast<float4*>(&m.h2[u4 + j][s4]) = make_float4(g[0], g[1], g[2], g[3]);
+    if (GRAD) *reinterpret_cast<float4*>(&d2[u4 + j][s4]) = make_float4(d[0], d[1], d[2], d[3]);
   }
-  float oa0 = P[OFF_B3], oa1 = P[OFF_B3 + 1], ob0 = oa0, ob1 = oa1;
-  for (int u = 0; u < NH; ++u) {
-    float za = P[OFF_B2 + u], zb = za;
-#pragma unroll
-    for (int k = 0; k < NH; ++k) {
-      const float w = P[OFF_W2 + u * NH + k];
-      za = fmaf(w, ha[k], za);
-      zb = fmaf(w, hb[k], zb);
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) mlp_forward_kernel(const float* __restrict__ prm, const float* __restrict__ x,
+                                                          int B, float* __restrict__ out) {
+  extern __shared__ float4 mlp_smem[];
+  MlpSmem& m = *reinterpret_cast<MlpSmem*>(mlp_smem);
+  mlp_load(prm, m);
+  for (int s0 = blockIdx.x * MT; s0 < B; s0 += gridDim.x * MT) {
+    const int ns = min(MT, B - s0);
+    mlp_inputs(x, nullptr, s0, ns, m);
+    mlp_hidden<false>(m, nullptr, nullptr);
+    if (threadIdx.x < NO * MT) {
+      const int s = threadIdx.x >> 1, o = threadIdx.x & 1;
+      float z = m.b3[o];
+#pragma unroll 16
+      for (int u = 0; u < NH; ++u) z = fmaf(m.w3[o * NH + u], m.h2[u][s], z);
+      if (s < ns) out[(size_t)(s0 + s) * NO + o] = z;
     }
-    const float ga = gelu(za), gb = gelu(zb);
-    const float w0 = P[OFF_W3 + u], w1 = P[OFF_W3 + NH + u];
-    oa0 = fmaf(w0, ga, oa0);
-    oa1 = fmaf(w1, ga, oa1);
-    ob0 = fmaf(w0, gb, ob0);
-    ob1 = fmaf(w1, gb, ob1);
-  }
-  out[(size_t)s0 * NO] = oa0;
-  out[(size_t)s0 * NO + 1] = oa1;
-  if (two) {
-    out[(size_t)(s0 + 1) * NO] = ob0;
-    out[(size_t)(s0 + 1) * NO + 1] = ob1;
+    __syncthreads();  // the tile's arrays are free
   }
 }
 
-// One CTA = TILE samples. Forward, loss, backward into shared memory, then the
-// tile's parameter gradients are summed over its samples and added to grad.
-constexpr int TILE = 16;  // keeps the CTA's static shared memory under 48 KB
+// Forward, loss and backward of a CTA's tiles; the parameter gradients stay in
+// registers over them (16 entries of W2 per thread as 4 x 4 products summed over
+// the samples, the others 1 to 3) and are added to grad once per CTA. With 16
+// samples per CTA, 8,192 samples made 2.5 million global atomics: 160 us, now 21
+// (65,536 samples: 1024 us, now 98).
+struct MlpGradSmem {
+  MlpSmem m;
+  float w2[NH][NH];                  // unit-major
+  float d1[NH][MS], d2[NH][MS];      // derivatives, then the deltas
+  float dout[NO][MS];
+  float part[8];
+};
 
 __global__ void __launch_bounds__(256) mlp_grad_kernel(const float* __restrict__ prm, const float* __restrict__ x,
                                                        const float* __restrict__ y, const int* __restrict__ idx,
                                                        int B, float inv_n, float* __restrict__ grad,
                                                        float* __restrict__ loss) {
-  __shared__ float P[N_PARAMS];
-  __shared__ float X[TILE][NI];
-  __shared__ float Z1[TILE][NH], H1[TILE][NH], Z2[TILE][NH], H2[TILE][NH], D1[TILE][NH], D2[TILE][NH];
-  __shared__ float DO[TILE][NO];
-  __shared__ float lsum;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int s0 = blockIdx.x * TILE;
-  const int ns = min(TILE, B - s0);
-  for (int i = tid; i < N_PARAMS; i += nt) P[i] = prm[i];
-  for (int i = tid; i < TILE * NI; i += nt) {
-    const int s = i / NI, k = i % NI;
-    X[s][k] = s < ns ? x[(size_t)(idx ? idx[s0 + s] : s0 + s) * NI + k] : 0.f;
-  }
-  if (tid == 0) lsum = 0.f;
-  __syncthreads();
-  for (int i = tid; i < TILE * NH; i += nt) {
-    const int s = i / NH, u = i % NH;
-    float z = P[OFF_B1 + u];
-#pragma unroll
-    for (int k = 0; k < NI; ++k) z = fmaf(P[OFF_W1 + u * NI + k], X[s][k], z);
-    Z1[s][u] = z;
-    H1[s][u] = gelu(z);
-  }
-  __syncthreads();
-  for (int i = tid; i < TILE * NH; i += nt) {
-    const int s = i / NH, u = i % NH;
-    float z = P[OFF_B2 + u];
-    for (int k = 0; k < NH; ++k) z = fmaf(P[OFF_W2 + u * NH + k], H1[s][k], z);
-    Z2[s][u] = z;
-    H2[s][u] = gelu(z);
-  }
-  __syncthreads();
-  for (int i = tid; i < TILE * NO; i += nt) {
-    const int s = i / NO, o = i % NO;
-    float z = P[OFF_B3 + o];
-    for (int k = 0; k < NH; ++k) z = fmaf(P[OFF_W3 + o * NH + k], H2[s][k], z);
-    float e = 0.f;
-    if (s < ns) e = z - y[(size_t)(idx ? idx[s0 + s] : s0 + s) * NO + o];
-    DO[s][o] = e * inv_n;
-    atomicAdd(&lsum, 0.5f * e * e * inv_n);
-  }
-  __syncthreads();
-  for (int i = tid; i < TILE * NH; i += nt) {
-    const int s = i / NH, k = i % NH;
-    const float dh = P[OFF_W3 + k] * DO[s][0] + P[OFF_W3 + NH + k] * DO[s][1];
-    D2[s][k] = dh * gelu_grad(Z2[s][k]);
-  }
-  __syncthreads();
-  for (int i = tid; i < TILE * NH; i += nt) {
-    const int s = i / NH, k = i % NH;
-    float dh = 0.f;
-    for (int u = 0; u < NH; ++u) dh = fmaf(P[OFF_W2 + u * NH + k], D2[s][u], dh);
-    D1[s][k] = dh * gelu_grad(Z1[s][k]);
-  }
-  __syncthreads();
-  for (int pi = tid; pi < N_PARAMS; pi += nt) {
-    float g = 0.f;
-    if (pi < OFF_B1) {
-      const int u = pi / NI, k = pi % NI;
-      for (int s = 0; s < ns; ++s) g = fmaf(D1[s][u], X[s][k], g);
-    } else if (pi < OFF_W2) {
-      const int u = pi - OFF_B1;
-      for (int s = 0; s < ns; ++s) g += D1[s][u];
-    } else if (pi < OFF_B2) {
-      const int u = (pi - OFF_W2) / NH, k = (pi - OFF_W2) % NH;
-      for (int s = 0; s < ns; ++s) g = fmaf(D2[s][u], H1[s][k], g);
-    } else if (pi < OFF_W3) {
-      const int u = pi - OFF_B2;
-      for (int s = 0; s < ns; ++s) g += D2[s][u];
-    } else if (pi < OFF_B3) {
-      const int o = (pi - OFF_W3) / NH, k = (pi - OFF_W3) % NH;
-      for (int s = 0; s < ns; ++s) g = fmaf(DO[s][o], H2[s][k], g);
-    } else {
-      const int o = pi - OFF_B3;
-      for (int s = 0; s < ns; ++s) g += DO[s][o];
+  extern __shared__ float4 mlp_smem[];
+  MlpGradSmem& g = *reinterpret_cast<MlpGradSmem*>(mlp_smem);
+  MlpSmem& m = g.m;
+  const int tid = threadIdx.x, lane = tid & 31;
+  mlp_load(prm, m);
+  for (int i = tid; i < NH * NH; i += 256) g.w2[i / NH][i % NH] = prm[OFF_W2 + i];
+  const int tu = tid >> 4, tk = tid & 15;  // W2 entries (tu + 16 i, tk + 16 j)
+  float g2[4][4] = {}, g1[3] = {}, gb = 0.f, g3 = 0.f, lsum = 0.f;
+  auto row_dot = [&](const float* a, const float* b) {  // sum over the tile's samples
+    float r = 0.f;
+#pragma unroll 4
+    for (int s = 0; s < MT; s += 4) {
+      const float4 p = *reinterpret_cast<const float4*>(a + s), q = *reinterpret_cast<const float4*>(b + s);
+      r = fmaf(p.x, q.x, r);
+      r = fmaf(p.y, q.y, r);
+      r = fmaf(p.z, q.z, r);
+      r = fmaf(p.w, q.w, r);
     }
-    atomicAdd(grad + pi, g);
+    return r;
+  };
+  for (int s0 = blockIdx.x * MT; s0 < B; s0 += gridDim.x * MT) {
+    const int ns = min(MT, B - s0);
+    mlp_inputs(x, idx, s0, ns, m);
+    for (int s = tid; s < MT; s += 256) m.x[NI][s] = 1.f;  // the biases' input
+    mlp_hidden<true>(m, g.d1, g.d2);
+    if (tid < NO * MT) {
+      const int s = tid >> 1, o = tid & 1;
+      float z = m.b3[o];
+#pragma unroll 16
+      for (int u = 0; u < NH; ++u) z = fmaf(m.w3[o * NH + u], m.h2[u][s], z);
+      const float e = s < ns ? z - y[(size_t)(idx ? idx[s0 + s] : s0 + s) * NO + o] : 0.f;
+      g.dout[o][s] = e * inv_n;
+      lsum = fmaf(0.5f * e * e, inv_n, lsum);
+    }
+    __syncthreads();
+    for (int i = tid; i < NH * MT; i += 256) {
+      const int u = i / MT, s = i % MT;
+      g.d2[u][s] *= m.w3[u] * g.dout[0][s] + m.w3[NH + u] * g.dout[1][s];
+    }
+    __syncthreads();
+    {
+      const int s4 = 4 * (tid >> 4), k4 = 4 * (tid & 15);
+      float d[4][4] = {};  // [input][sample]
+#pragma unroll 8
+      for (int u = 0; u < NH; ++u) {
+        const float4 e = *reinterpret_cast<const float4*>(&g.d2[u][s4]);
+        const float4 w = *reinterpret_cast<const float4*>(&g.w2[u][k4]);
+        const float ev[4] = {e.x, e.y, e.z, e.w}, wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) d[j][i] = fmaf(wv[j], ev[i], d[j][i]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float4 f = *reinterpret_cast<float4*>(&g.d1[k4 + j][s4]);
+        f = make_float4(f.x * d[j][0], f.y * d[j][1], f.z * d[j][2], f.w * d[j][3]);
+        *reinterpret_cast<float4*>(&g.d1[k4 + j][s4]) = f;
+      }
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int s = 0; s < MT; s += 4) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[i] = *reinterpret_cast<const float4*>(&g.d2[tu + 16 * i][s]);
+        b[i] = *reinterpret_cast<const float4*>(&m.h1[tk + 16 * i][s]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float r = g2[i][j];
+          r = fmaf(a[i].x, b[j].x, r);
+          r = fmaf(a[i].y, b[j].y, r);
+          r = fmaf(a[i].z, b[j].z, r);
+          g2[i][j] = fmaf(a[i].w, b[j].w, r);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int e = tid + 256 * i;
+      if (e < NH * NI) g1[i] += row_dot(g.d1[e / NI], m.x[e % NI]);
+    }
+    if (tid < 2 * NH) {
+      gb += row_dot(tid < NH ? g.d1[tid] : g.d2[tid - NH], m.x[NI]);
+      if (tid < NO) g3 += row_dot(g.dout[tid], m.x[NI]);
+    } else {
+      const int e = tid - 2 * NH;
+      g3 += row_dot(g.dout[e / NH], m.h2[e % NH]);
+    }
+    __syncthreads();  // the tile's arrays are free
   }
-  if (tid == 0 && loss) atomicAdd(loss, lsum);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) atomicAdd(grad + OFF_W2 + (tu + 16 * i) * NH + tk + 16 * j, g2[i][j]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (tid + 256 * i < NH * NI) atomicAdd(grad + OFF_W1 + tid + 256 * i, g1[i]);
+  if (tid < 2 * NH) atomicAdd(grad + (tid < NH ? OFF_B1 + tid : OFF_B2 + tid - NH), gb);
+  if (tid < NO) atomicAdd(grad + OFF_B3 + tid, g3);
+  if (tid >= 2 * NH) atomicAdd(grad + OFF_W3 + tid - 2 * NH, g3);
+  if (loss) {
+    lsum = warp_sum(lsum);
+    if (lane == 0) g.part[tid >> 5] = lsum;
+    __syncthreads();
+    if (tid == 0) {
+      float r = 0.f;
+      for (int w = 0; w < 8; ++w) r += g.part[w];
+      atomicAdd(loss, r);
+    }
+  }
 }
 
 // Adam with bias correction; consumes and zeroes the gradient.
@@ -304,7 +408,12 @@ extern "C" int ffs_arma_simulate(int V, int T, int K, int n_runs, const int* run
 extern "C" int ffs_mlp_forward(const float* params, const float* x, int B, float* out, void* stream) {
   clear_error();
   FFS_REQUIRE(params && x && out && B > 0, "ffs_mlp_forward: bad arguments");
-  mlp_forward_kernel<<<ceil_div(B, 128 * FWD_PER_THREAD), 128, 0, (cudaStream_t)stream>>>(params, x, B, out);
+  // four CTAs an SM, each over its share of the tiles
+  int sms = 0;
+  FFS_CUDA(sm_count(&sms));
+  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(mlp_forward_kernel), sizeof(MlpSmem)));
+  mlp_forward_kernel<<<std::min(ceil_div(B, MT), 4 * sms), 256, sizeof(MlpSmem), (cudaStream_t)stream>>>(params, x, B,
+                                                                                                        out);
   return check_launch("mlp_forward_kernel");
 }
 
@@ -312,8 +421,11 @@ extern "C" int ffs_mlp_grad(const float* params, const float* x, const float* y,
                             float* grad, float* loss, void* stream) {
   clear_error();
   FFS_REQUIRE(params && x && y && grad && B > 0 && n_total > 0, "ffs_mlp_grad: bad arguments");
-  mlp_grad_kernel<<<ceil_div(B, TILE), 256, 0, (cudaStream_t)stream>>>(params, x, y, idx, B, 1.0f / (float)n_total,
-                                                                       grad, loss);
+  int sms = 0;
+  FFS_CUDA(sm_count(&sms));
+  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(mlp_grad_kernel), sizeof(MlpGradSmem)));
+  mlp_grad_kernel<<<std::min(ceil_div(B, MT), sms), 256, sizeof(MlpGradSmem), (cudaStream_t)stream>>>(
+      params, x, y, idx, B, 1.0f / (float)n_total, grad, loss);
   return check_launch("mlp_grad_kernel");
 }
 

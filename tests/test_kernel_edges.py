@@ -270,3 +270,30 @@ def test_series_sd_is_the_float_nearest_the_float64_value(T):
     ok = ~floor & ~np.isnan(want)
     ulp = np.spacing(want[ok].astype(np.float32)).astype(np.float64)
     assert (np.abs(got[ok].astype(np.float64) - want[ok]) <= (0.5 + 2.0**-20) * ulp + 1e-15 * want[ok]).all()
+
+
+# ------------------------------------------------------------------ the proposal network
+
+
+@gpu
+@pytest.mark.parametrize("B", [1, 63, 64, 65, 700, 10300])
+def test_mlp_tiles_against_the_oracle(B):
+    """Partial, single and several tiles per CTA (64 samples each), with an index list. Sums of B <= 10300 terms
+    of one sign pattern: relative error of each gradient below 64-term chains, CTA sums and atomics in float32,
+    against the gradient's largest entry: 2^-24 (64 + ceil(B / 64) + 64) <= 2e-5."""
+    from fastfuncstuff_gb300.glm import learned
+    from oracle import mlp as om
+
+    rng = np.random.default_rng(B)
+    p = (om.init(2) + 0.02 * rng.standard_normal(om.N_PARAMS)).astype(np.float32)
+    x = rng.standard_normal((B + 5, om.N_IN)).astype(np.float32)
+    y = (rng.standard_normal((B + 5, 2)) * 0.4).astype(np.float32)
+    idx = rng.permutation(B + 5)[:B].astype(np.int32)
+    pt, xt, yt, it = (torch.from_numpy(v).to(DEV) for v in (p, x, y, idx))
+    out = learned.ArmaProposal(pt).forward(xt[:B].contiguous()).cpu().numpy()
+    np.testing.assert_allclose(out, om.forward(p, x[:B]), rtol=1e-4, atol=1e-5)
+    grad, loss = torch.zeros(om.N_PARAMS, device=DEV), torch.zeros(1, device=DEV)
+    learned.mlp_grad(pt, xt, yt, it, B, grad, loss)
+    L, g = om.loss_and_grad(p.astype(np.float64), x[idx].astype(np.float64), y[idx].astype(np.float64))
+    assert np.abs(grad.cpu().numpy() - g).max() <= 2e-5 * np.abs(g).max()
+    assert float(loss.item()) == pytest.approx(L, rel=2e-5)
