@@ -402,6 +402,7 @@ def fit_glm_arma11(
                                              gls_kw=dict(want_residuals=want_residuals,
                                                          want_predicted=want_predicted),
                                              factor_kw=dict(task_indices=ti, glt=glt, with_tc=True))
+        if gplan is not None:
             slots = gplan.slots
         else:
             factors = engine.build_factors(Xs, grid, layout, task_indices=ti, glt=glt, with_tc=True, sets=sets,

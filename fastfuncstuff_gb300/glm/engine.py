@@ -804,45 +804,64 @@ class DesignSlots:
     design: torch.Tensor   # [V] int32 design of each voxel
     tile32: torch.Tensor   # [Vp / 32] int32
     tile256: torch.Tensor  # [Vp / 256] int32
-    items: torch.Tensor    # [n_items][6] int32 projection work list (ffs_tc_item)
-    n_items: torch.Tensor  # [1] int32
+    start: np.ndarray      # [D + 1] first slot of each design
+    K: int
+    P: int
     max_pairs: int
+    _list: tuple | None = None
+
+    def work_list(self) -> tuple[torch.Tensor, torch.Tensor]:
+        """The full grid's (design, voxel tile, pair block) projection work list
+        (``ffs_tc_item`` [n][6]) and its length [1], built when first asked
+        for (the descent does not read it)."""
+        if self._list is None:
+            P, K, g = self.P, self.K, self.max_pairs
+            p0 = np.arange(0, P, g, dtype=np.int64)
+            npair = np.minimum(g, P - p0)
+            rows = []
+            for d in range(self.start.size - 1):  # design-major, then voxel tile, then pair block
+                v0 = np.arange(int(self.start[d]), int(self.start[d + 1]), 128, dtype=np.int64)
+                vv, pp = np.meshgrid(v0, p0, indexing="ij")
+                nn = np.broadcast_to(npair, vv.shape)
+                rows.append(np.stack([vv, np.full_like(vv, 128), (d * P + pp) * K, nn, vv, pp], -1).reshape(-1, 6))
+            items = np.concatenate(rows).astype(np.int32) if rows else np.zeros((0, 6), np.int32)
+            dev = self.idx.device
+            self._list = (torch.from_numpy(items).to(dev),
+                          torch.tensor([items.shape[0]], dtype=torch.int32, device=dev))
+        return self._list
+
+    @property
+    def items(self) -> torch.Tensor:
+        return self.work_list()[0]
+
+    @property
+    def n_items(self) -> torch.Tensor:
+        return self.work_list()[1]
 
 
 def design_slots(gid: np.ndarray, n_designs: int, K: int, P: int, dev) -> DesignSlots:
-    """Slots and the (design, voxel tile, pair block) projection work list of a
-    grouped fit; ``gid`` [V] holds each voxel's design index (host)."""
-    gid = np.asarray(gid, dtype=np.int64).reshape(-1)
+    """Slots of a grouped fit; ``gid`` [V] holds each voxel's design index (host)."""
+    gid = np.asarray(gid).reshape(-1)
     V = gid.size
-    order = np.argsort(gid, kind="stable")
+    # 16-bit keys: numpy's stable sort is then a radix sort
+    order = np.argsort(gid.astype(np.int16 if n_designs <= 32767 else np.int64), kind="stable")
     counts = np.bincount(gid, minlength=n_designs)
     padded = (counts + 255) // 256 * 256
     start = np.concatenate([[0], np.cumsum(padded)])
-    first = np.concatenate([[0], np.cumsum(counts)])
     Vp = int(start[-1])
+    # the voxels in order, each design's shifted by the padding before it
+    shift = start[:-1] - np.concatenate([[0], np.cumsum(counts)[:-1]])
+    at = np.arange(V, dtype=np.int64) + np.repeat(shift, counts)
     idx = np.full(Vp, -1, np.int32)
+    idx[at] = order
     real = np.empty(V, np.int64)
-    for d in range(n_designs):
-        vox = order[first[d]:first[d + 1]]
-        idx[start[d]:start[d] + counts[d]] = vox
-        real[vox] = np.arange(start[d], start[d] + counts[d])
+    real[order] = at
     tile_of = np.repeat(np.arange(n_designs, dtype=np.int32), padded // 32)
-    g = max(1, min(P, 256 // K))
-    p0 = np.arange(0, P, g, dtype=np.int64)
-    npair = np.minimum(g, P - p0)
-    rows = []
-    for d in range(n_designs):  # design-major, then voxel tile, then pair block
-        v0 = np.arange(int(start[d]), int(start[d + 1]), 128, dtype=np.int64)
-        vv, pp = np.meshgrid(v0, p0, indexing="ij")
-        nn = np.broadcast_to(npair, vv.shape)
-        rows.append(np.stack([vv, np.full_like(vv, 128), (d * P + pp) * K, nn, vv, pp], -1).reshape(-1, 6))
-    items = np.concatenate(rows).astype(np.int32) if rows else np.zeros((0, 6), np.int32)
     return DesignSlots(V=V, Vp=Vp, idx=torch.from_numpy(idx).to(dev), real=torch.from_numpy(real).to(dev),
                        design=torch.from_numpy(gid.astype(np.int32)).to(dev),
                        tile32=torch.from_numpy(tile_of).to(dev),
                        tile256=torch.from_numpy(tile_of[::8].copy()).to(dev),
-                       items=torch.from_numpy(items).to(dev),
-                       n_items=torch.tensor([items.shape[0]], dtype=torch.int32, device=dev), max_pairs=g)
+                       start=start, K=K, P=P, max_pairs=max(1, min(P, 256 // K)))
 
 
 def search_designs(Y: torch.Tensor, f: GridFactors, slots: DesignSlots, *, hierarchical: bool = True,
@@ -886,9 +905,9 @@ def search_designs(Y: torch.Tensor, f: GridFactors, slots: DesignSlots, *, hiera
     ja = _lib.ProjectArgs(V=Vp, T=T, K=K, P=D * P, ld_y=ld, ld_u=ld, yr_hi=_p(yr_hi), yr_lo=_p(yr_lo),
                           u_hi=_p(f.U_hi), u_lo=_p(f.U_lo), yexp=_p(yexp), uexp=_p(f.uexp), yr_t=None, U=None,
                           proj=_p(proj), flag=_p(flag))
-    n_items = slots.items.shape[0]
-    _run("ffs_reml_project_tc_list", lib.ffs_reml_project_tc_list, C.byref(ja), _p(slots.items), _p(slots.n_items),
-         n_items, slots.max_pairs, 0, st)
+    items, n_items = slots.items, slots.n_items
+    _run("ffs_reml_project_tc_list", lib.ffs_reml_project_tc_list, C.byref(ja), _p(items), _p(n_items),
+         items.shape[0], slots.max_pairs, 0, st)
 
     surf = torch.empty(P, Vp, dtype=torch.float32, device=dev)
     crit0 = torch.empty(Vp, dtype=torch.float64, device=dev)
@@ -909,7 +928,7 @@ def search_designs(Y: torch.Tensor, f: GridFactors, slots: DesignSlots, *, hiera
     _run("ffs_reml_select", lib.ffs_reml_select, C.byref(se), st)
     out = SearchOut(best=best[slots.real], best_crit=best_crit[slots.real], scale=scale)
     out._flag = flag
-    out._keep = (q0, yr_t, yr_hi, yr_lo, yexp, proj, surf, crit0)
+    out._keep = (q0, yr_t, yr_hi, yr_lo, yexp, proj, surf, crit0, items, n_items)
     return out
 
 
@@ -1221,10 +1240,14 @@ class GroupedFitGraph:
 
 
 _GROUPED_GRAPHS: dict = {}
+_LAST_GROUPED: list = [None]  # the key of the last grouped fit
 
 
-def grouped_graph_for(Y, Xs, grid, layout, gid, *, hierarchical, do_scale, gls_kw, factor_kw) -> GroupedFitGraph:
-    """The cached GroupedFitGraph of this shape, grouping and options (built on first use)."""
+def grouped_graph_for(Y, Xs, grid, layout, gid, *, hierarchical, do_scale, gls_kw, factor_kw) -> GroupedFitGraph | None:
+    """The cached GroupedFitGraph of this shape, grouping and options. It is
+    built when a grouping comes twice in a row (capturing costs an eager fit
+    and a synchronisation, 30 ms at 100,000 voxels and 20 designs, and every
+    subject has a grouping of its own); None asks the caller to fit eagerly."""
     gid = np.asarray(gid, dtype=np.int32)
     fk = tuple((k, None if v is None else v.key() if hasattr(v, "key") else np.asarray(v).tobytes())
                for k, v in sorted(factor_kw.items()))
@@ -1233,6 +1256,9 @@ def grouped_graph_for(Y, Xs, grid, layout, gid, *, hierarchical, do_scale, gls_k
            layout.run_start.tobytes(), layout.tau.tobytes(), gid.tobytes(), hierarchical, do_scale,
            tuple(sorted(gls_kw.items())), fk)
     gr = _GROUPED_GRAPHS.get(key)
+    again, _LAST_GROUPED[0] = _LAST_GROUPED[0] == key, key
+    if gr is None and not again:
+        return None
     if gr is None:
         while len(_GROUPED_GRAPHS) >= 2:  # a plan holds a few GB of static buffers
             _GROUPED_GRAPHS.pop(next(iter(_GROUPED_GRAPHS)))
