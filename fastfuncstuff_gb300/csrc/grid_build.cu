@@ -367,101 +367,347 @@ __device__ void ldl_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p
   __syncthreads();
 }
 
+__device__ __forceinline__ void bar_sync(int id, int n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// Rows or columns of the band staged at a time by phases 2 and 6.
+constexpr int BD_STEPS = 32;
+
+__host__ __device__ inline int band_pitch(int W) { return W | 1; }
+// Runs factored side by side, each by half the block's warps: the chain of a
+// column's steps, not their work, takes the time. Two windows of W > 96 would
+// not leave room for the rest.
+__host__ __device__ inline int band_groups(int W, int n_runs) { return n_runs > 1 && W <= 96 ? 2 : 1; }
+// Shared doubles: the staged rows or columns of phases 2 and 6, and phase 1's
+// powers of a, index table, and per group a window and two columns (each raw and scaled).
+__host__ __device__ inline size_t band_stage_doubles(int W) { return (size_t)BD_STEPS * band_pitch(W); }
+__host__ __device__ inline size_t band_chol_doubles(int W, int n_runs) {
+  const size_t n = (size_t)(W + 1) + band_groups(W, n_runs) * ((size_t)W * W + 4 * (size_t)W) +
+                   ((size_t)W * (W + 1) / 2 + 3) / 4;
+  return n > band_stage_doubles(W) ? n : band_stage_doubles(W);
+}
+
+// d > 0, by the words (a compare on the FP64 pipe takes as long as a product)
+__device__ __forceinline__ bool positive(double d) {
+  const int hi = __double2hiint(d);
+  return hi > 0 ? hi < 0x7ff00000 || (hi == 0x7ff00000 && __double2loint(d) == 0) : hi == 0 && __double2loint(d) != 0;
+}
+
+// The factors of v / n = u + u p, u = v r: r the fp32 reciprocal of n and
+// p = e + e^2, e = 1 - n r (error e^3 ~ 2^-72). Positive n.
+__device__ __forceinline__ void rcp_factors(double n, double& r, double& p) {
+  const unsigned x = (unsigned)__double2hiint(n) >> 20;
+  r = x - (1023u - 100u) <= 200u ? f2d_exact(__frcp_rn((float)n)) : 1.0 / n;  // 2^-100 < n < 2^100
+  const double e = fma(-n, r, 1.0);
+  p = fma(e, e, e);
+}
+
 // Phase 1 of an item with AFNI's banded R (d.band): the Cholesky factor of
 // each run's block of R, where R(t, k) = lam a^(g-1) for 1 <= g = tau_t -
-// tau_k <= band[p] and 0 beyond. One warp per run, rows in order; row t has
-// J_t earlier rows of its run within the band (zero at a run start), and its
-// off-diagonal entries L(t, t - j) solve the triangular system of those rows
-// against R(t, t - j): the lanes hold the right-hand side (lane l the terms
-// j = l + 1 + 32 q), each solved entry is broadcast and taken off the terms
-// not yet solved. The diagonal is sqrt(1 - sum_j L(t, t - j)^2); a pivot that
-// is not positive flags the pair (bad_r) and is replaced by 1. FP64
-// throughout; band_L keeps the factor, band_coef its fp32 whitening
-// coefficients, invdiag and Jrow (shared memory) the reciprocal diagonal and
-// each row's band for phases 2 and 6. logdet_R = 2 sum log(L(t, t) + 1e-10)
-// as the reference takes it from its dense factor; coef is the identity.
-__device__ void band_chol_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p, double* invdiag, int* Jrow,
-                                  double* apow, double* red, int* bad_r) {
+// tau_k <= band[p] and 0 beyond. The rows of run r that column k reaches are
+// contiguous, k+1 .. end-1, and the fill stays inside the band, so the column
+// goes rightwards over a window of the last W rows in shared memory (row t in
+// slot t mod W, entry (t, t - j) at j): A(i, j) -= A(i, k) A(j, k) / D_k.
+// Warps 1.. update the window's triangle, one entry per lane through a table
+// of triangle indices (full warps: this GPU's FP64 pipe takes 19 cycles per
+// warp instruction whatever its lanes), and set up the rows that enter;
+// meanwhile warp 0 forms the next column with its pivot's reciprocal, so a
+// step costs one barrier and a chain of pivot, fp32 reciprocal, its two
+// correction terms and the scaling. The columns leave unscaled; the square roots,
+// L(t, t - j) = A(t, t - j) / sqrt(D_{t-j}), the fp32 whitening coefficients
+// and the logs follow for all entries in parallel. A pivot that is not
+// positive flags the pair (bad_r) and is replaced by 1.
+// FP64 throughout; band_L keeps the factor (zero outside a row's band),
+// band_coef its fp32 whitening coefficients, invdiag [T] (global scratch) the
+// reciprocal diagonal for phases 2 and 6. logdet_R = 2 sum log(L(t, t) +
+// 1e-10) as the reference takes it from its dense factor; coef is the
+// identity. The row-by-row form it replaces (a warp per run, every entry of a row
+// waiting for the one before through global memory) took most of the banded
+// build's 3110 us at T = 240, K = 11, 117 pairs of up to 42 lags; with phases 2
+// and 6 below the build takes 398 (this phase 150, phase 2 85, phase 6 105).
+// sm: band_chol_doubles shared doubles; invdiag: 1.5 T doubles
+// (each column's reach behind the diagonal). Ends with a barrier.
+__device__ __noinline__ void band_chol_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p, double* invdiag,
+                                               double* sm, double* red, int* bad_r) {
+  __builtin_assume(__isShared(sm));
   const int T = d.T, W = d.band_w, bw = d.band[p];
   const float af = d.a[p], bf = d.b[p];
   const double a = (double)af;
   const double lam = d.lambda_fp32 ? (double)lambda_f32(af, bf) : lambda_f64(a, (double)bf);
+  const bool zero = lam == 0.0;
+  const int* __restrict__ tau = d.tau;
   double* Lb = o.band_L + (size_t)p * T * W;
   float* Cb = o.band_coef + (size_t)p * T * W;
-  if (threadIdx.x == 0) {
+  const int ng = band_groups(W, d.n_runs), gw = (int)(blockDim.x >> 5) / ng;  // groups, warps of a group
+  const int grp = (int)(threadIdx.x >> 5) / gw, gtid = threadIdx.x - grp * gw * 32, gwarp = gtid >> 5;
+  double *apow = sm, *win = apow + W + 1 + grp * (W * W + 4 * W), *colA = win + (size_t)W * W, *colW = colA + 2 * W;
+  uint16_t* tri = reinterpret_cast<uint16_t*>(apow + W + 1 + ng * (W * W + 4 * W));
+  int* reach = reinterpret_cast<int*>(invdiag + T);  // first row past column t's band
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  if (tid == 0) {
     *bad_r = 0;
     double x = 1.0;
-    for (int k = 0; k < W; ++k) {  // a^k: corr(g) = lam a^(g - 1), 1 <= g < W
-      apow[k] = x;
+    for (int k = 0; k <= W; ++k) {  // lam a^k: corr(g) = lam a^(g - 1), 1 <= g < W
+      apow[k] = zero ? 0.0 : lam * x;
       x *= a;
     }
   }
+  for (int i = warp; i < W; i += nw)
+    for (int j = lane; j <= i; j += 32) tri[i * (i + 1) / 2 + j] = (uint16_t)(i << 8 | j);
+  for (int r = 0; r < d.n_runs; ++r)
+    for (int t = d.run_start[r] + tid; t < d.run_start[r + 1]; t += blockDim.x) {
+      int lo = t + 1, hi = min(t + bw + 1, d.run_start[r + 1]);
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (tau[mid] - tau[t] <= bw)
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      reach[t] = lo;
+    }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int r = warp; r < d.n_runs; r += nw) {
+
+  for (int r = grp; r < d.n_runs; r += ng) {
     const int t0 = d.run_start[r], t1 = d.run_start[r + 1];
-    for (int t = t0; t < t1; ++t) {
-      const int tt = d.tau[t];
-      int J = 0;
-      while (J < t - t0 && J < W - 1 && tt - d.tau[t - J - 1] <= bw) ++J;
-      double rj[4], own = 0.0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = lane + 1 + 32 * q;
-        rj[q] = (j <= J && lam != 0.0) ? lam * apow[tt - d.tau[t - j] - 1] : 0.0;
-      }
-      for (int j = J; j >= 1; --j) {
-        const int q = (j - 1) >> 5, owner = (j - 1) & 31;
-        const double mine = q == 0 ? rj[0] : q == 1 ? rj[1] : q == 2 ? rj[2] : rj[3];
-        const double ell = __shfl_sync(0xffffffffu, mine, owner) * invdiag[t - j];
-        if (lane == owner) {
-          Lb[(size_t)t * W + j] = ell;
-          own = fma(ell, ell, own);
+    int end = t0, cur = 0, slot1 = t0 % W;  // "column t0 - 1" reaches nothing: the first turn sets up column t0
+    int nend = t0 < t1 ? reach[t0] : t0;
+    for (int k = t0 - 1; k < t1 - 1; ++k) {
+      const double *cA = colA + cur * W, *cW = colW + cur * W;
+      const int C = end - 1 - k;  // rows k+1 .. k+C; row k + 1 in slot1
+      const int nnend = k + 2 < t1 ? reach[k + 2] : 0;
+      auto slot = [&](int i) { return slot1 + i >= W ? slot1 + i - W : slot1 + i; };  // of row k + 1 + i
+      if (gwarp == 0) {  // column k + 1: its entries less column k's share
+        double *nA = colA + (cur ^ 1) * W, *nW = colW + (cur ^ 1) * W;
+        const bool seen = C >= 1;  // row k + 1 is in the window
+        const double a1 = seen ? cA[1] : 0.0;
+        double dk = 1.0;
+        if (seen) dk = fma(-cW[1], a1, win[slot1 * W]);
+        if (!positive(dk)) {
+          if (lane == 0) *bad_r = 1;
+          dk = 1.0;
         }
+        double rk, pk;
+        rcp_factors(dk, rk, pk);
 #pragma unroll
-        for (int qq = 0; qq < 4; ++qq) {
-          const int jp = lane + 1 + 32 * qq;  // the term of row t - jp, column t - j
-          if (jp < j && j - jp <= Jrow[t - jp]) rj[qq] -= ell * Lb[(size_t)(t - jp) * W + (j - jp)];
+        for (int q = 0; q < 4; ++q) {
+          if (k + 2 + 32 * q >= nend) break;
+          const int i = 1 + lane + 32 * q, t = k + 1 + i;
+          if (t < nend) {
+            const double v = t < end ? fma(-cW[i + 1], a1, win[slot(i) * W + i]) : apow[tau[t] - tau[k + 1] - 1];
+            nA[i] = v;
+            const double u = v * rk;
+            nW[i] = fma(u, pk, u);
+            Lb[(size_t)t * W + i] = v;
+          }
+        }
+        if (lane == 0) invdiag[k + 1] = dk;
+      } else {
+        const int m = max(C - 1, 0);
+        for (int e = gtid - 32; e < m * (m + 1) / 2; e += 32 * (gw - 1)) {
+          const int ij = tri[e], i = ij >> 8, j = ij & 255;  // row k+2+i, column k+2+j
+          double* w = win + slot(i + 1) * W + (i - j);
+          *w = fma(-cW[i + 2], cA[j + 2], *w);
+        }
+        for (int t = max(end, k + 2) + gwarp - 1; t < nend; t += gw - 1) {  // rows that enter, from column k + 2
+          const int tt = tau[t];
+          for (int j = lane; j <= t - (k + 2); j += 32) {
+            const int g = tt - tau[t - j];
+            if (g <= bw) win[slot(t - k - 1) * W + j] = j == 0 ? 1.0 : apow[g - 1];
+          }
         }
       }
-      __syncwarp();  // the row's entries, written by their owner lanes, are read below
-      double d2 = 1.0 - warp_sum_d(own);
-      if (!(d2 > 0.0)) {
-        if (lane == 0) *bad_r = 1;
-        d2 = 1.0;
-      }
-      const double ltt = sqrt(d2);
-      const double inv = 1.0 / ltt;
-      for (int j = lane; j < W; j += 32) {
-        const double v = j == 0 ? ltt : (j <= J ? Lb[(size_t)t * W + j] : 0.0);
-        if (j > J) Lb[(size_t)t * W + j] = 0.0;
-        if (j == 0) Lb[(size_t)t * W] = ltt;
-        Cb[(size_t)t * W + j] = (float)(j == 0 ? inv : v * inv);
-      }
-      if (lane == 0) {
-        invdiag[t] = inv;
-        Jrow[t] = J;
-      }
-      __syncwarp();
+      end = nend;
+      nend = nnend;
+      cur ^= 1;
+      slot1 = slot1 + 1 == W ? 0 : slot1 + 1;
+      bar_sync(1 + grp, 32 * gw);
     }
   }
   __syncthreads();
+
   double ld = 0.0;
-  for (int t = threadIdx.x; t < T; t += blockDim.x) {
-    ld += 2.0 * log(Lb[(size_t)t * W] + 1e-10);
+  for (int t = tid; t < T; t += blockDim.x) {
+    const double ltt = sqrt(invdiag[t]);
+    ld += 2.0 * log(ltt + 1e-10);
+    invdiag[t] = 1.0 / ltt;
+    Lb[(size_t)t * W] = ltt;
     reinterpret_cast<float4*>(o.coef)[(size_t)p * T + t] = make_float4(0.f, 0.f, 1.f, 1.f);
   }
   ld = block_sum(ld, red);
-  if (threadIdx.x == 0) o.logdet_R[p] = ld;
+  if (tid == 0) o.logdet_R[p] = ld;
   __syncthreads();
+  constexpr int ROWS = 4;  // rows in flight per warp
+  for (int r = 0; r < d.n_runs; ++r) {
+    const int t0 = d.run_start[r], t1 = d.run_start[r + 1];
+    for (int tb = t0 + warp; tb < t1; tb += ROWS * nw)
+      for (int j = lane; j < W; j += 32) {
+        double l[ROWS], it[ROWS];
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) {
+          const int t = tb + q * nw;
+          const bool in = t < t1 && j >= 1 && t - j >= t0 && reach[t - j] > t;
+          it[q] = t < t1 ? invdiag[t] : 0.0;
+          l[q] = in ? Lb[(size_t)t * W + j] * invdiag[t - j] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) {
+          const int t = tb + q * nw;
+          if (t < t1) {
+            if (j >= 1) Lb[(size_t)t * W + j] = l[q];
+            Cb[(size_t)t * W + j] = (float)(j == 0 ? it[q] : l[q] * it[q]);
+          }
+        }
+      }
+  }
+  __syncthreads();
+}
+
+// Phase 2 with the band: X_w = L^-1 X, half a warp per column of X, rightwards.
+// Lane l of the half holds the column's rows k0 + l + 16 q of the running 16
+// steps; step k broadcasts row k and takes L(t, k) / L(k, k) times it off the
+// rows below, so the dependent chain of a step is one shuffle and one fma (the
+// leftward form, a dot product per row, waits for a whole row). Half warps
+// because the FP64 pipe's time goes by warp instructions: a band of 42 fills 42
+// of the 50 lanes a column then takes. The columns of BD_STEPS steps are staged
+// in shared memory for all the block's warps. NQ >= bw / 16 + 2. Whole blocks
+// only; ends with a barrier.
+template <int NQ>
+__device__ __noinline__ void band_whiten_cols(const double* Lb, const double* invd, const float* __restrict__ Xd,
+                                              double* Xw, double* st, int T, int K, int W, int bw) {
+  __builtin_assume(__isShared(st));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, pitch = band_pitch(W);
+  const int l16 = lane & 15;
+  for (int c0 = 0; c0 < K; c0 += 2 * nw) {
+    const int c = c0 + 2 * warp + (lane >> 4);
+    const bool live = c < K;
+    double x[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int t = l16 + 16 * q;
+      x[q] = live && t < T ? f2d_exact(__ldg(Xd + (size_t)t * K + c)) : 0.0;
+    }
+    for (int k0 = 0; k0 < T; k0 += 16) {
+      if (k0 % BD_STEPS == 0) {
+        __syncthreads();
+        for (int tb = k0 + 1 + warp; tb < k0 + BD_STEPS + bw; tb += 4 * nw)
+          for (int j = lane + 1; j <= bw; j += 32) {
+            double l[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int t = tb + q * nw, k = t - j;
+              l[q] = t < T && k >= k0 && k < k0 + BD_STEPS ? Lb[(size_t)t * W + j] * invd[k] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int k = tb + q * nw - j;
+              if (k >= k0 && k < k0 + BD_STEPS) st[(k - k0) * pitch + j] = l[q];
+            }
+          }
+        __syncthreads();
+      }
+      if (c0 + 2 * warp < K) {
+        const int n = min(16, T - k0);
+        const double* row = st + (k0 % BD_STEPS) * pitch + l16;
+#pragma unroll 4
+        for (int kk = 0; kk < n; ++kk, row += pitch - 1) {  // row[16 q] = step kk's entry i = l16 + 16 q - kk
+          const double xk = __shfl_sync(0xffffffffu, x[0], kk, 16);
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) {
+            if (16 * q - kk > bw) break;  // no lane's row is in reach
+            const int i = l16 + 16 * q - kk;
+            if (i >= 1 && i <= bw) x[q] = fma(-row[16 * q], xk, x[q]);
+          }
+        }
+        const int t = k0 + l16, tn = t + 16 * NQ;
+        if (live && t < T) Xw[(size_t)c * T + t] = x[0] * invd[t];
+#pragma unroll
+        for (int q = 0; q < NQ - 1; ++q) x[q] = x[q + 1];
+        x[NQ - 1] = live && tn < T ? f2d_exact(__ldg(Xd + (size_t)tn * K + c)) : 0.0;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Phase 6 with the band: U = L^-T Q by back substitution, u_t = (q_t - sum_i
+// L(t + i, t) u_{t+i}) / L(t, t) with the u of fp32, leftwards as phase 2 goes
+// rightwards (lane l holds rows k0 + l - 16 q; rows of L staged). Returns max
+// |u| of the thread's entries. Whole blocks only; ends with a barrier.
+template <int NQ>
+__device__ __noinline__ float band_back_cols(const double* Lb, const double* invd, const float* qf, float* uf, float* U,
+                                             double* st, int T, int LT, int K, int W, int bw) {
+  __builtin_assume(__isShared(st));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, pitch = band_pitch(W);
+  const int l16 = lane & 15;
+  float umax = 0.f;
+  for (int c0 = 0; c0 < K; c0 += 2 * nw) {
+    const int c = c0 + 2 * warp + (lane >> 4);
+    const bool live = c < K;
+    const int top = (T - 1) / 16 * 16;
+    double x[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int t = top + l16 - 16 * q;
+      x[q] = live && t >= 0 && t < T ? f2d_exact(qf[(size_t)c * T + t]) : 0.0;
+    }
+    for (int k0 = top; k0 >= 0; k0 -= 16) {
+      if (k0 == top || (k0 + 16) % BD_STEPS == 0) {
+        const int s0 = k0 / BD_STEPS * BD_STEPS;
+        __syncthreads();
+        for (int kb = warp; kb < BD_STEPS; kb += 4 * nw)
+          for (int j = lane + 1; j <= bw; j += 32) {
+            double l[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int kk = kb + q * nw;
+              l[q] = kk < BD_STEPS && s0 + kk < T ? Lb[(size_t)(s0 + kk) * W + j] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (kb + q * nw < BD_STEPS) st[(kb + q * nw) * pitch + j] = l[q];
+          }
+        __syncthreads();
+      }
+      if (c0 + 2 * warp < K) {
+        const int t = k0 + l16, n = min(16, T - k0);
+        const double iv = t < T ? invd[t] : 0.0;
+        const double* row = st + (k0 % BD_STEPS + n - 1) * pitch + (n - 1) - l16;
+#pragma unroll 4
+        for (int kk = n - 1; kk >= 0; --kk, row -= pitch + 1) {  // row[16 q] = step kk's entry i = kk - l16 + 16 q
+          const double ut = f2d_exact(__shfl_sync(0xffffffffu, (float)(x[0] * iv), kk, 16));
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) {
+            if (kk - 15 + 16 * q > bw) break;
+            const int i = kk - l16 + 16 * q;
+            if (i >= 1 && i <= bw) x[q] = fma(-row[16 * q], ut, x[q]);
+          }
+        }
+        if (live && t < T) {
+          const float ut = (float)(x[0] * iv);
+          uf[(size_t)c * T + t] = ut;
+          U[(size_t)c * LT + t] = ut;
+          umax = fmaxf(umax, fabsf(ut));
+        }
+        const int tn = t - 16 * NQ;
+#pragma unroll
+        for (int q = 0; q < NQ - 1; ++q) x[q] = x[q + 1];
+        x[NQ - 1] = live && tn >= 0 ? f2d_exact(qf[(size_t)c * T + tn]) : 0.0;
+      }
+    }
+    if (live)
+      for (int t = T + l16; t < LT; t += 16) U[(size_t)c * LT + t] = 0.f;
+  }
+  __syncthreads();
+  return umax;
 }
 
 // Phase 1 of every pair once, for the items of all designs (coef and
 // logdet_R depend on the pair only): c, m and 1/sqrt(D) ([P][3][T], stride 4 T
 // per pair) and bad [P] in the workspace, read back by the item kernels. With
 // the banded R the pair's band_L, band_coef, coef and logdet_R are written here,
-// and the workspace keeps the reciprocal diagonal and each row's band (the
-// first 1.5 T doubles).
+// and the workspace keeps the reciprocal diagonal (the first T doubles).
 __global__ void __launch_bounds__(GB_THREADS) pair_ldl_kernel(BuildArgs args, double* cm, int* bad) {
   __shared__ double red[32];
   __shared__ int bad_r;
@@ -469,12 +715,9 @@ __global__ void __launch_bounds__(GB_THREADS) pair_ldl_kernel(BuildArgs args, do
   const int T = args.d.T;
   double* dst = cm + (size_t)blockIdx.x * 4 * T;
   if (args.d.band)
-    band_chol_of_pair(args.d, args.o, blockIdx.x, cms, reinterpret_cast<int*>(cms + T), cms + T + (T + 1) / 2, red,
-                      &bad_r);
+    band_chol_of_pair(args.d, args.o, blockIdx.x, dst, cms, red, &bad_r);
   else
     ldl_of_pair(args.d, args.o, blockIdx.x, dst, dst + T, dst + 2 * T, cms, red, &bad_r);
-  if (args.d.band)
-    for (int i = threadIdx.x; i < 3 * T; i += blockDim.x) dst[i] = cms[i];
   if (threadIdx.x == 0) bad[blockIdx.x] = bad_r;
 }
 
@@ -572,33 +815,29 @@ __device__ void item_tail(const ffs_grid_desc& d, const ffs_grid_out& o, const P
 
 // Phases 2 to 9 of one item with its matrices in the global scratch slot s,
 // after phase 1: cc, cm, cr as ldl_of_pair leaves them, or with the banded R cc
-// = the reciprocal diagonal and, behind it, each row's band. Any K and T.
+// = the reciprocal diagonal and stage = band_stage_doubles shared doubles. Any K and T.
+template <bool BAND>
 __device__ __noinline__ void item_global(const BuildArgs& args, const PairScratch& s, int p, int pd, const float* Xd,
-                                         const double* cc, const double* cm, const double* cr, int bad_r, double* red,
-                                         int* flag_s) {
+                                         const double* cc, const double* cm, const double* cr, double* stage,
+                                         int bad_r, double* red, int* flag_s) {
   const ffs_grid_desc& d = args.d;
   const ffs_grid_out& o = args.o;
   const int T = d.T, K = d.K, LT = ld_t(T);
   int& flag = *flag_s;
 
   // ---- 2. X_w = L^-1 X, one column per thread; the design samples of
-  // GB_PF steps are loaded ahead of the recursion that needs them (with the
-  // banded R: forward substitution against the band of each row)
-  if (d.band) {
-    const int W = d.band_w;
-    const double* Lb = o.band_L + (size_t)p * T * W;
-    const int* Jrow = reinterpret_cast<const int*>(cc + T);
-    for (int j = threadIdx.x; j < K; j += blockDim.x) {
-      double* xw = s.Xw + (size_t)j * T;
-      for (int t = 0; t < T; ++t) {
-        double acc = f2d_exact(__ldg(Xd + (size_t)t * K + j));
-        const double* row = Lb + (size_t)t * W;
-        for (int i = 1; i <= Jrow[t]; ++i) acc = fma(-row[i], xw[t - i], acc);
-        xw[t] = acc * cc[t];
-      }
-    }
+  // GB_PF steps are loaded ahead of the recursion that needs them
+  if constexpr (BAND) {
+    const int bw = d.band[p];
+    const double* Lb = o.band_L + (size_t)p * T * d.band_w;
+    if (bw <= 16)
+      band_whiten_cols<3>(Lb, cc, Xd, s.Xw, stage, T, K, d.band_w, bw);
+    else if (bw <= 48)
+      band_whiten_cols<5>(Lb, cc, Xd, s.Xw, stage, T, K, d.band_w, bw);
+    else
+      band_whiten_cols<10>(Lb, cc, Xd, s.Xw, stage, T, K, d.band_w, bw);
   }
-  for (int j = threadIdx.x; j < K && !d.band; j += blockDim.x) {
+  for (int j = threadIdx.x; j < K && !BAND; j += blockDim.x) {
     double xp = 0.0, vp = 0.0;
     for (int t0 = 0; t0 < T; t0 += GB_PF) {
       float xb[GB_PF];
@@ -709,27 +948,18 @@ __device__ __noinline__ void item_global(const BuildArgs& args, const PairScratc
   // the fp32 coefficients of phase 1
   const float4* cf = reinterpret_cast<const float4*>(o.coef) + (size_t)p * T;
   float umax_local = 0.f;
-  if (d.band) {
-    // back substitution against the band: u_t = (q_t - sum_i L(t + i, t)
-    // u_{t+i}) / L(t, t), the rows t + i of t's run within the band
-    const int W = d.band_w;
-    const double* Lb = o.band_L + (size_t)p * T * W;
-    const int* Jrow = reinterpret_cast<const int*>(cc + T);
-    for (int j = threadIdx.x; j < K; j += blockDim.x) {
-      const float* q = qf + (size_t)j * T;
-      float* u = uf + (size_t)j * T;
-      for (int t = T - 1; t >= 0; --t) {
-        double acc = (double)q[t];
-        for (int i = 1; t + i < T && i <= Jrow[t + i]; ++i) acc = fma(-Lb[(size_t)(t + i) * W + i], (double)u[t + i], acc);
-        const float ut = (float)(acc * cc[t]);
-        u[t] = ut;
-        o.U[((size_t)pd * K + j) * LT + t] = ut;
-        umax_local = fmaxf(umax_local, fabsf(ut));
-      }
-      for (int t = T; t < LT; ++t) o.U[((size_t)pd * K + j) * LT + t] = 0.f;
-    }
+  if constexpr (BAND) {
+    const int bw = d.band[p];
+    const double* Lb = o.band_L + (size_t)p * T * d.band_w;
+    float* U = o.U + (size_t)pd * K * LT;
+    if (bw <= 16)
+      umax_local = band_back_cols<3>(Lb, cc, qf, uf, U, stage, T, LT, K, d.band_w, bw);
+    else if (bw <= 48)
+      umax_local = band_back_cols<5>(Lb, cc, qf, uf, U, stage, T, LT, K, d.band_w, bw);
+    else
+      umax_local = band_back_cols<10>(Lb, cc, qf, uf, U, stage, T, LT, K, d.band_w, bw);
   }
-  for (int j = threadIdx.x; j < K && !d.band; j += blockDim.x) {
+  for (int j = threadIdx.x; j < K && !BAND; j += blockDim.x) {
     const float* q = qf + (size_t)j * T;
     float* u = uf + (size_t)j * T;
     float xn = 0.f, mn = 0.f, cn = 0.f;  // x_{t+1}, m_{t+1}, c_{t+1}
@@ -831,8 +1061,8 @@ __device__ __noinline__ void item_global(const BuildArgs& args, const PairScratc
 // factors its pair's R itself. This kernel takes the items that
 // grid_item_kernel does not (wide or long designs, the banded R). Capped at
 // 64 registers (4 CTAs per SM): left free, the compiler takes 80 to 126 of them.
-template <bool SHARED_LDL>
-__global__ void __launch_bounds__(GB_THREADS, 4) grid_build_kernel(BuildArgs args, int n_designs,
+template <bool SHARED_LDL, bool BAND>
+__global__ void __launch_bounds__(GB_THREADS, BAND ? 2 : 4) grid_build_kernel(BuildArgs args, int n_designs,
                                                                                   const double* pair_cm,
                                                                                   const int* pair_bad, int tmp_smem) {
   const ffs_grid_desc& d = args.d;
@@ -841,21 +1071,27 @@ __global__ void __launch_bounds__(GB_THREADS, 4) grid_build_kernel(BuildArgs arg
   PairScratch s = scratch_of(o.work, blockIdx.x, T, K);
   __shared__ double red[32];
   __shared__ int flag, bad_r;
-  extern __shared__ double cms[];  // c, m, 1/sqrt(D) of the current pair [3][T], then [4][T] with tmp_smem
+  // c, m, 1/sqrt(D) of the current pair [3][T], then [4][T] with tmp_smem; or the band's scratch
+  extern __shared__ double cms[];
   for (int item = blockIdx.x; item < d.P * n_designs; item += gridDim.x) {
     const int p = item % d.P;
+    const double* cc = cms;
     if constexpr (SHARED_LDL) {
       // the pre-pass factored R for every pair once: copy this pair's rows
       const double* src = pair_cm + (size_t)p * 4 * T;
-      for (int i = threadIdx.x; i < 3 * T; i += blockDim.x) cms[i] = src[i];
+      if constexpr (BAND)
+        cc = src;
+      else
+        for (int i = threadIdx.x; i < 3 * T; i += blockDim.x) cms[i] = src[i];
       if (threadIdx.x == 0) bad_r = pair_bad[p];
       __syncthreads();
-    } else if (d.band) {
-      band_chol_of_pair(d, o, p, cms, reinterpret_cast<int*>(cms + T), cms + T + (T + 1) / 2, red, &bad_r);
+    } else if constexpr (BAND) {
+      band_chol_of_pair(d, o, p, s.cm, cms, red, &bad_r);
+      cc = s.cm;
     } else {
       ldl_of_pair(d, o, p, cms, cms + T, cms + 2 * T, tmp_smem ? cms + 3 * T : s.cm, red, &bad_r);
     }
-    item_global(args, s, p, item, d.X + (size_t)(item / d.P) * T * K, cms, cms + T, cms + 2 * T, bad_r, red, &flag);
+    item_global<BAND>(args, s, p, item, d.X + (size_t)(item / d.P) * T * K, cc, cms + T, cms + 2 * T, cms, bad_r, red, &flag);
   }
 }
 
@@ -1001,9 +1237,6 @@ __host__ __device__ inline ItemPlan item_plan(int T, int K, int n_runs) {
 }
 
 // Barrier of the first n threads (a multiple of 32) of the CTA.
-__device__ __forceinline__ void bar_sync(int id, int n) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
-}
 
 template <bool SHARED_LDL, int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS == GI_SMALL ? 3 : 1) grid_item_kernel(BuildArgs args, int n_designs,
@@ -1224,7 +1457,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == GI_SMALL ? 3 : 1) grid_ite
     if (flag) {
       __syncthreads();
       const PairScratch s = scratch_of(o.work, blockIdx.x, T, K);
-      item_global(args, s, p, pd, Xd, cc, cm, cr, bad_r, red, &flag);
+      item_global<false>(args, s, p, pd, Xd, cc, cm, cr, nullptr, bad_r, red, &flag);
       continue;
     }
     for (int e = tid; e < K * K4; e += nth) {
@@ -1676,11 +1909,16 @@ extern "C" size_t ffs_grid_work_bytes_designs(int T, int K, int P, int n_designs
   return sizeof(double) * n;
 }
 
-// Shared memory of phase 1: 4 T doubles, or with the band invdiag [T], Jrow [T]
-// (ints) and the powers of a [band_w]. A T past 200 KB of it is refused.
+// Shared memory of phase 1: 4 T doubles, or with the band its window and tables.
 static size_t phase1_smem(const ffs_grid_desc& d) {
-  const size_t n = sizeof(double) * 4 * (size_t)d.T;
-  return d.band ? std::max(n, sizeof(double) * ((size_t)d.T + (d.T + 1) / 2 + (size_t)d.band_w + 1)) : n;
+  return sizeof(double) * (d.band ? ffsk::band_chol_doubles(d.band_w, d.n_runs) : 4 * (size_t)d.T);
+}
+
+// A T past 200 KB of 4 T doubles is refused (with the band, past 200 KB of 1.5 T doubles and the powers of a too).
+static bool too_long(const ffs_grid_desc& d) {
+  size_t n = 4 * (size_t)d.T;
+  if (d.band) n = std::max(n, (size_t)d.T + (d.T + 1) / 2 + (size_t)d.band_w + 1);
+  return sizeof(double) * n > 200 * 1024;
 }
 
 // The item kernel of a build: grid_item_kernel for designs of up to GI_KMAX
@@ -1692,7 +1930,7 @@ static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, co
   using namespace ffsk;
   const ffs_grid_desc& d = args.d;
   const ffs_grid_out& o = args.o;
-  FFS_REQUIRE(phase1_smem(d) <= 200 * 1024, "%s: T=%d too long", who, d.T);
+  FFS_REQUIRE(!too_long(d), "%s: T=%d too long", who, d.T);
   FFS_REQUIRE(!o.const_flag == !o.const_coef && (!o.const_flag || (d.p0 >= 0 && d.p0 < d.P)),
               "%s: const_flag and const_coef go together, with p0=%d in [0, P)", who, d.p0);
   const ItemPlan pl = item_plan(d.T, d.K, d.n_runs);
@@ -1708,8 +1946,9 @@ static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, co
   // phase 1's scratch beside the coefficients while that leaves room for four CTAs an SM
   const int tmp_smem = !pair_cm && sizeof(double) * 7 * d.T <= 50 * 1024;
   size_t smem = sizeof(double) * (tmp_smem ? 7 : 3) * d.T;
-  if (d.band) smem = std::max(smem, phase1_smem(d));
-  auto kern = pair_cm ? grid_build_kernel<true> : grid_build_kernel<false>;
+  if (d.band) smem = pair_cm ? sizeof(double) * band_stage_doubles(d.band_w) : phase1_smem(d);
+  auto kern = d.band ? (pair_cm ? grid_build_kernel<true, true> : grid_build_kernel<false, true>)
+                     : (pair_cm ? grid_build_kernel<true, false> : grid_build_kernel<false, false>);
   FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), smem));
   kern<<<grid, GB_THREADS, smem, st>>>(args, n_designs, pair_cm, pair_bad, tmp_smem);
   return check_launch("grid_build_kernel");
@@ -1775,7 +2014,7 @@ extern "C" int ffs_grid_build_designs(const ffs_grid_desc* d, int n_designs, int
   int* pair_bad = nullptr;
   if (n_designs > 1) {
     const size_t smem = phase1_smem(*d);
-    FFS_REQUIRE(smem <= 200 * 1024, "ffs_grid_build_designs: T=%d too long", d->T);
+    FFS_REQUIRE(!too_long(*d), "ffs_grid_build_designs: T=%d too long", d->T);
     FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(pair_ldl_kernel), smem));
     pair_cm = o->work + designs_slot_doubles(d->T, d->K, d->P, n_designs, max_ctas);
     pair_bad = reinterpret_cast<int*>(pair_cm + (size_t)d->P * 4 * d->T);

@@ -297,3 +297,65 @@ def test_mlp_tiles_against_the_oracle(B):
     L, g = om.loss_and_grad(p.astype(np.float64), x[idx].astype(np.float64), y[idx].astype(np.float64))
     assert np.abs(grad.cpu().numpy() - g).max() <= 2e-5 * np.abs(g).max()
     assert float(loss.item()) == pytest.approx(L, rel=2e-5)
+
+
+@gpu
+@pytest.mark.parametrize("T,K,runs,hole,a_max,corcut", [
+    (16, 1, 1, (0, 0), 0.3, 1e-2),      # a history of 16, one column
+    (75, 17, 3, (20, 9), 0.8, 1e-4),    # a history of 48, odd runs, censored rows, two rounds of columns
+    (130, 5, 1, (60, 50), 0.8, 1e-4),   # one run; a gap wider than the band
+    (131, 33, 2, (0, 0), 0.8, 1e-12),   # a history of 128 (band 125), longer than a run
+    (40, 4, 4, (0, 0), 0.7, 1e-4),      # runs shorter than the band
+])
+def test_banded_factors_and_surface_against_dense_float64(T, K, runs, hole, a_max, corcut):
+    """AFNI's banded R: its factor, U = L^-T Q and the criterion's y'R^-1 y
+    against dense FP64 at the edges of the band's chunks and register
+    histories. band_L is FP64 throughout (1e-11 of 1); U leaves as fp32 after
+    an fp32 Q and substitution, its error below K fp32 roundings times ||L^-1||
+    (1e-5 of the largest entry); a sum of T squares of fp32 recurrences,
+    each step within band + 2 roundings that ||L^-1|| carries on, within 3e-5."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(T + K)
+    X = np.concatenate([np.ones((T, 1)), rng.standard_normal((T, K - 1))], 1)
+    keep = np.array([t for t in range(T + hole[1]) if not hole[0] <= t < hole[0] + hole[1]])
+    starts = [T * r // runs for r in range(runs)]
+    G.set_afni_mode(True, corcut)
+    try:
+        g = G.make_grid(torch.linspace(0.0, a_max, 4), torch.linspace(-0.8, 0.8, 5), use_double=True)
+        layout = G.run_layout(T, starts, tau=keep)
+        f = engine.build_factors(torch.from_numpy(X.astype(np.float32)).to(DEV), g, layout, with_tc=True)
+        V = 300
+        Y = torch.from_numpy((rng.standard_normal((V, T)) * 3 + 100).astype(np.float32)).to(DEV)
+        out = engine.search(Y, f, keep_surface=True, keep_yr=True)
+        torch.cuda.synchronize()
+    finally:
+        G.set_afni_mode(False)
+    assert int(f.info.abs().sum()) == 0
+    run_of = np.searchsorted(starts, np.arange(T), side="right")
+    gap = np.abs(keep[:, None] - keep[None, :])
+    X64 = X.astype(np.float32).astype(np.float64)
+    yr = out.yr_t.cpu().numpy().astype(np.float64)
+    surf = out.surf.cpu().numpy().astype(np.float64)
+    U0 = f.U[g.p0, :, :T].cpu().numpy().astype(np.float64)
+    rss0 = (yr ** 2).sum(0) - ((U0 @ yr) ** 2).sum(0)
+    base = float(f.logdet_R[g.p0] + f.logdet_XtX[g.p0])
+    for p in range(g.P):
+        bw = int(g.band[p])
+        a, b = float(np.float32(g.a[p])), float(np.float32(g.b[p]))
+        lam = (b + a) * (1 + a * b) / (1 + 2 * a * b + b * b)
+        R = np.where((gap > 0) & (gap <= bw) & (run_of[:, None] == run_of[None, :]),
+                     lam * a ** np.maximum(gap - 1, 0), 0.0) + np.eye(T)
+        got = np.zeros((T, T))
+        for j in range(f.band_w):
+            got[np.arange(j, T), np.arange(T - j)] = f.band_L[p, j:, j].cpu().numpy()
+        np.testing.assert_allclose(got, np.linalg.cholesky(R), rtol=0, atol=1e-11, err_msg=f"pair {p}")
+        Li = np.linalg.inv(got)
+        Xw = Li @ X64
+        U = f.U[p, :, :T].cpu().numpy().astype(np.float64)
+        want = np.linalg.solve(np.linalg.cholesky(Xw.T @ Xw), Xw.T) @ Li
+        assert np.abs(U - want).max() <= 1e-5 * np.abs(want).max()
+        ssw, proj = ((Li @ yr) ** 2).sum(0), ((want @ yr) ** 2).sum(0)
+        crit = float(f.logdet_R[p] + f.logdet_XtX[p]) - base + (T - K) * np.log1p((ssw - proj - rss0) / rss0)
+        scale = (ssw + proj) / np.minimum(ssw - proj, rss0)
+        assert (np.abs(surf[p] - crit) <= 3e-5 * (T - K) * scale + 1e-5 * np.abs(crit)).all()
