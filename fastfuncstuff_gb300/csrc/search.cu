@@ -496,63 +496,118 @@ __global__ void __launch_bounds__(SURF_THREADS, 2) surface_kernel(ffs_surface_ar
 }
 
 // ------------------------------------------------------------- banded surface
-// AFNI's banded R: one CTA per (pair, tile of SB_THREADS voxels), one thread
-// per voxel. Each step forms w_t = y_t c[t][0] - sum_{j <= band} c[t][j] w_{t-j}
-// against the last band_w - 1 values of w, kept per thread in a ring in
-// shared memory ([slot][thread], so a warp's accesses fall in distinct banks);
-// the coefficients of SB_STEPS steps are staged in shared memory at a time
-// and read by every thread (broadcast). y'R^-1 y = sum w_t^2, and the
-// criterion as the surface kernel forms it.
+// AFNI's banded R: one CTA per (pair, tile of 2 SB_THREADS voxels), two voxels
+// per thread. Each step forms w_t = y_t c[t][0] - sum_{j <= band} c[t][j] w_{t-j}
+// for j ascending, against the last values of w in registers: SB_UNROLL steps
+// are unrolled over a history of B values (every index is then static) that
+// moves down by SB_UNROLL after them. The coefficients of SB_STEPS steps are
+// staged in shared memory at a time and read as broadcast words of four that
+// serve both voxels, so a term costs 2 FFMA and a quarter of a load (a ring in
+// shared memory, one voxel per thread, took 2 loads, the ring's wrap and an
+// FFMA a term). y'R^-1 y = sum w_t^2, and the criterion as the surface kernel
+// forms it. 6000 voxels, T = 240, 117 pairs of up to 42 lags: 1147 -> 342 us;
+// bound by the FFMA chain of each step (82 us of FFMA issue).
 constexpr int SB_THREADS = 128;
-static_assert(256 % SB_THREADS == 0, "a CTA's voxels lie in one 256-voxel design tile");
+constexpr int SB_TILE = 2 * SB_THREADS;
+static_assert(256 % SB_TILE == 0, "a CTA's voxels lie in one 256-voxel design tile");
 constexpr int SB_STEPS = 32;
+constexpr int SB_UNROLL = 8;
 
-__global__ void __launch_bounds__(SB_THREADS) surface_band_kernel(ffs_surface_args a) {
-  extern __shared__ float sbm[];
-  const int W = a.band_w, T = a.T;
-  float* ring = sbm;                                  // [W][SB_THREADS]
-  float* cs = ring + (size_t)W * SB_THREADS;          // [SB_STEPS][W]
-  const int p = blockIdx.x, bw = a.band[p];
-  const int tid = threadIdx.x;
-  const int v = blockIdx.y * SB_THREADS + tid;
-  const bool live = v < a.V;
-  const float* cb = a.band_coef + (size_t)p * T * W;
-  for (int i = tid; i < W * SB_THREADS; i += blockDim.x) ring[i] = 0.f;
-  float yy = 0.f, ssw = 0.f;
-  int pos = 0;  // the ring slot of step t
+// Shared floats of a history of B: rows of c[t][0], 3 of padding, c[t][1 .. B]
+// (zero past the band and past T).
+constexpr int sb_floats(int B) { return SB_STEPS * (B + 4); }
+
+// ss, yy: sums of w_t^2 and y_t^2 of voxels v[0 .. NV), bw <= B (a multiple of 8).
+template <int B, int NV>
+__device__ __forceinline__ void band_sums(const float* __restrict__ cb, int W, int bw, int T,
+                                          const float* __restrict__ y, int V, const int* v, float* cs, float* ss,
+                                          float* yy) {
+  float h[NV][B + SB_UNROLL];
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    ss[n] = yy[n] = 0.f;
+#pragma unroll
+    for (int i = 0; i < B; ++i) h[n][i] = 0.f;
+  }
   for (int c0 = 0; c0 < T; c0 += SB_STEPS) {
-    const int cn = min(SB_STEPS, T - c0);
     __syncthreads();  // the previous chunk's coefficients are no longer read
-    for (int i = tid; i < cn * W; i += blockDim.x) cs[i] = cb[(size_t)c0 * W + i];
+    for (int i = threadIdx.x; i < SB_STEPS * (B + 1); i += SB_THREADS) {
+      const int s = i / (B + 1), j = i % (B + 1);
+      cs[s * (B + 4) + (j ? j + 3 : 0)] = c0 + s < T && j <= bw ? cb[(size_t)(c0 + s) * W + j] : 0.f;
+    }
     __syncthreads();
-    for (int s = 0; s < cn; ++s) {
-      const int t = c0 + s;
-      const float y = live ? a.yr_t[(size_t)t * a.V + v] : 0.f;
-      const float* c = cs + (size_t)s * W;
-      float acc = y * c[0];
-      const int jm = min(bw, t);
-      int q = pos;
-      for (int j = 1; j <= jm; ++j) {
-        q = q == 0 ? W - 1 : q - 1;
-        acc = fmaf(-c[j], ring[(size_t)q * SB_THREADS + tid], acc);
+    for (int s0 = 0; s0 < SB_STEPS && c0 + s0 < T; s0 += SB_UNROLL) {
+      float yv[NV][SB_UNROLL];
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+#pragma unroll
+        for (int s = 0; s < SB_UNROLL; ++s) {
+          const int t = c0 + s0 + s;
+          yv[n][s] = t < T && v[n] < V ? y[(size_t)t * V + v[n]] : 0.f;
+        }
+#pragma unroll
+      for (int s = 0; s < SB_UNROLL; ++s) {
+        const float* c = cs + (s0 + s) * (B + 4);
+        float acc[NV];
+#pragma unroll
+        for (int n = 0; n < NV; ++n) acc[n] = yv[n][s] * c[0];
+#pragma unroll
+        for (int j = 0; j < B; j += 8) {  // terms j + 1 .. j + 8
+          if (j >= bw) break;
+          const float4 p = *reinterpret_cast<const float4*>(c + 4 + j), q = *reinterpret_cast<const float4*>(c + 8 + j);
+          const float k[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int n = 0; n < NV; ++n) acc[n] = fmaf(-k[i], h[n][B + s - 1 - j - i], acc[n]);
+        }
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          h[n][B + s] = acc[n];
+          yy[n] = fmaf(yv[n][s], yv[n][s], yy[n]);
+          ss[n] = fmaf(acc[n], acc[n], ss[n]);
+        }
       }
-      ring[(size_t)pos * SB_THREADS + tid] = acc;
-      pos = pos + 1 == W ? 0 : pos + 1;
-      yy = fmaf(y, y, yy);
-      ssw = fmaf(acc, acc, ssw);
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+#pragma unroll
+        for (int i = 0; i < B; ++i) h[n][i] = h[n][i + SB_UNROLL];
     }
   }
-  if (!live) return;
+}
+
+// BMAX: the widest history of the launch (16, 48 or 128); a pair takes the
+// narrowest that holds its band, the registers of 128 one voxel at a time.
+template <int BMAX>
+__global__ void __launch_bounds__(SB_THREADS) surface_band_kernel(ffs_surface_args a) {
+  extern __shared__ float4 sbm4[];
+  float* cs = reinterpret_cast<float*>(sbm4);
+  const int p = blockIdx.x, bw = a.band[p];
+  const float* cb = a.band_coef + (size_t)p * a.T * a.band_w;
+  const int v[2] = {(int)(blockIdx.y * SB_TILE + threadIdx.x), (int)(blockIdx.y * SB_TILE + SB_THREADS + threadIdx.x)};
+  float ss[2], yy[2];
+  if (BMAX <= 16 || bw <= 16) {
+    band_sums<16, 2>(cb, a.band_w, bw, a.T, a.yr_t, a.V, v, cs, ss, yy);
+  } else if (BMAX <= 48 || bw <= 48) {
+    if constexpr (BMAX >= 48) band_sums<48, 2>(cb, a.band_w, bw, a.T, a.yr_t, a.V, v, cs, ss, yy);
+  } else if constexpr (BMAX >= 128) {
+#pragma unroll 1
+    for (int n = 0; n < 2; ++n) band_sums<128, 1>(cb, a.band_w, bw, a.T, a.yr_t, a.V, v + n, cs, ss + n, yy + n);
+  }
   const int Tk = a.T - a.K;
   // grouped fits: the design of this CTA's 256-voxel tile
-  const double* ldx = a.logdet_XtX + (a.tile_design ? (size_t)a.tile_design[blockIdx.y * SB_THREADS / 256] * a.P : 0);
+  const double* ldx = a.logdet_XtX + (a.tile_design ? (size_t)a.tile_design[blockIdx.y * SB_TILE / 256] * a.P : 0);
   const double c_p0 = a.logdet_R[a.p0] + ldx[a.p0];
-  const float rss0 = fmaxf(yy - a.proj[(size_t)a.p0 * a.V + v], 0.f);
-  const float den = rss0 + 1e-10f;
-  const float rss = fmaxf(ssw - a.proj[(size_t)p * a.V + v], 0.f);
   const float dc = (float)((a.logdet_R[p] + ldx[p]) - c_p0);
-  a.surf[(size_t)p * a.V + v] = dc + (float)Tk * log1pf((rss - rss0) / den);
-  if (p == 0) a.crit0[v] = c_p0 + (double)Tk * log((double)rss0 + 1e-10);
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    if (v[n] >= a.V) continue;
+    const float rss0 = fmaxf(yy[n] - a.proj[(size_t)a.p0 * a.V + v[n]], 0.f);
+    const float den = rss0 + 1e-10f;
+    const float rss = fmaxf(ss[n] - a.proj[(size_t)p * a.V + v[n]], 0.f);
+    a.surf[(size_t)p * a.V + v[n]] = dc + (float)Tk * log1pf((rss - rss0) / den);
+    if (p == 0) a.crit0[v[n]] = c_p0 + (double)Tk * log((double)rss0 + 1e-10);
+  }
 }
 
 // ---------------------------------------------------------------------- select
@@ -849,9 +904,10 @@ extern "C" int ffs_reml_surface(const ffs_surface_args* a, void* stream) {
     FFS_REQUIRE(a->yr_t && a->band && a->logdet_R && a->logdet_XtX && a->proj && a->surf && a->crit0,
                 "ffs_reml_surface: null buffer");
     FFS_REQUIRE(ceil_div(a->V, SB_THREADS) <= 65535, "ffs_reml_surface: V=%d exceeds one launch", a->V);
-    const size_t smem = sizeof(float) * (size_t)a->band_w * (SB_THREADS + SB_STEPS);
-    FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(surface_band_kernel), smem));
-    surface_band_kernel<<<dim3(a->P, ceil_div(a->V, SB_THREADS)), SB_THREADS, smem, (cudaStream_t)stream>>>(*a);
+    const int bw = a->band_w - 1;  // the widest band of the grid
+    auto kern = bw <= 16 ? surface_band_kernel<16> : bw <= 48 ? surface_band_kernel<48> : surface_band_kernel<128>;
+    const size_t smem = sizeof(float) * (bw <= 16 ? sb_floats(16) : bw <= 48 ? sb_floats(48) : sb_floats(128));
+    kern<<<dim3(a->P, ceil_div(a->V, SB_TILE)), SB_THREADS, smem, (cudaStream_t)stream>>>(*a);
     return check_launch("surface_band_kernel");
   }
   FFS_REQUIRE(a && a->V > 0 && a->T > 0 && a->P > 0 && a->n_chunks > 0, "ffs_reml_surface: bad sizes");
