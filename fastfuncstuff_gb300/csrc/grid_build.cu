@@ -1059,7 +1059,7 @@ __device__ __noinline__ void item_global(const BuildArgs& args, const PairScratc
 // (more than one design) phase 1 comes from pair_ldl_kernel (pair_cm,
 // pair_bad), which also wrote coef and logdet_R; without it every item
 // factors its pair's R itself. This kernel takes the items that
-// grid_item_kernel does not (wide or long designs, the banded R). Capped at
+// grid_item_kernel and grid_wide_kernel do not (long designs, the banded R). Capped at
 // 64 registers (4 CTAs per SM): left free, the compiler takes 80 to 126 of them.
 template <bool SHARED_LDL, bool BAND>
 __global__ void __launch_bounds__(GB_THREADS, BAND ? 2 : 4) grid_build_kernel(BuildArgs args, int n_designs,
@@ -1672,6 +1672,509 @@ __global__ void __launch_bounds__(THREADS, THREADS == GI_SMALL ? 3 : 1) grid_ite
   }
 }
 
+// ------------------------------------------------------------- wide designs
+// Items of more than GI_KMAX columns (single-trial designs), whose series do
+// not fit in shared memory: the series stay in the item's scratch slot (L2),
+// and shared memory holds what the CTA works on: staged samples of the Gram
+// matrix, then the packed K x K factor in FP64, then the fp32 factors that Q and
+// G read. Two CTAs share an SM, so that one's integer Gram matrix runs beside
+// the other's FP64 factorisation.
+//   - X_w = L^-1 X, a lane per column and run, to fixed point (as above, without
+//     the lo lo' sums: 2^-54 of a product of the columns' largest values, less
+//     than the rounding of the fixed point times their peak-to-rms ratio) and to
+//     fp32; the Gram matrix in blocks of 4 x 4 entries per thread (rows b, b + kb,
+//     b + 2 kb, b + 3 kb, so that a warp's blocks read consecutive rows) from
+//     double-buffered chunks of WI_CS samples.
+//   - X_w'X_w = Lu D Lu' and Lu^-1 in one pass over the packed lower triangle:
+//     step k takes w_r f_c off every entry (r, c) of the rows below k, w_r = A_rk / D_k,
+//     f = (row k of Lu^-1, 1, column k of A): left of column k the inverse grows
+//     where the factor's columns are no longer read. The first warps form the next
+//     step's f and w ahead of the others; one barrier a step.
+//   - Q = X_w Lx^-T and G = U Lx^-1 in fp32, 8 columns x 2 samples per thread.
+// A rank-deficient item or one whose series leave the fixed point goes through
+// item_global, whose general phases these replace: P = 561, T = 600, K = 130 in 3
+// runs: 13.7 -> 3.87 ms. What bounds an item: 0.73 M cycles of integer multiply-adds
+// (Gram) beside 0.57 M cycles of the FP64 pipe (X_w, factor and inverse).
+constexpr int WI_THREADS = 320;
+constexpr int WI_CS = 32;        // samples per chunk
+constexpr int WI_RS = WI_CS + 2; // row stride of a chunk (16-byte words of consecutive rows in distinct banks)
+constexpr int WI_KMAX = 255;     // 8-bit indices of the triangle's table
+
+struct WidePlan {
+  int KP, kb, NB, SL;           // K to a multiple of 8; 4 x 4 blocks a side, blocks, slices of the samples
+  int tri, fw, dk, scale, total;  // byte offsets (the work area is at 0)
+};
+
+__host__ __device__ inline WidePlan wide_plan(int T, int K) {
+  WidePlan m;
+  m.KP = (K + 7) & ~7;
+  m.kb = (K + 3) / 4;
+  m.NB = m.kb * (m.kb + 1) / 2;
+  m.SL = 1;
+  while (2 * m.SL * m.NB <= WI_THREADS && m.SL < 8) m.SL *= 2;
+  size_t area = sizeof(double) * 7 * T;  // phase 1
+  const size_t stage = sizeof(int2) * 2 * (size_t)(4 * m.kb) * WI_RS, pack = sizeof(double) * K * (K + 1) / 2,
+               f32 = sizeof(float) * (size_t)K * m.KP;
+  area = area > stage ? area : stage;
+  area = area > pack ? area : pack;
+  area = area > f32 ? area : f32;
+  size_t at = (area + 15) & ~(size_t)15;
+  auto take = [&](size_t n) {
+    const size_t o = at;
+    at += (n + 15) & ~(size_t)15;
+    return (int)o;
+  };
+  m.tri = take(sizeof(uint16_t) * (size_t)K * (K + 1) / 2);
+  m.fw = take(sizeof(double) * 4 * K);  // f and w, double-buffered
+  m.dk = take(sizeof(double) * 2 * K);  // D, 1 / sqrt(D)
+  m.scale = take(sizeof(int) * 2 * K);  // the columns' largest magnitudes (fp32 bits), their scales
+  m.total = (int)at;
+  return m;
+}
+
+// hh and x of FixedDot
+struct FixedDot2 {
+  long long hh = 0, x = 0;
+  __device__ __forceinline__ void add(int ax, int ay, int bx, int by) {
+    hh += (long long)ax * bx;
+    x += (long long)ax * by;
+    x += (long long)ay * bx;
+  }
+  __device__ __forceinline__ double value(int si, int sj) const {
+    return fma((double)hh, 0x1p54, (double)x * 0x1p27) * __hiloint2double((1023 - si - sj) << 20, 0);
+  }
+};
+
+template <bool SHARED_LDL>
+__global__ void __launch_bounds__(WI_THREADS, 2) grid_wide_kernel(BuildArgs args, int n_designs, const double* pair_cm,
+                                                                  const int* pair_bad) {
+  const ffs_grid_desc& d = args.d;
+  const ffs_grid_out& o = args.o;
+  const int T = d.T, K = d.K, LT = ld_t(T);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  constexpr int nth = WI_THREADS, NW = WI_THREADS / 32;
+  extern __shared__ double2 gi_smem[];
+  char* sm = reinterpret_cast<char*>(gi_smem);
+  const WidePlan pl = wide_plan(T, K);
+  const int KP = pl.KP, kb = pl.kb, SL = pl.SL;
+  double* area = reinterpret_cast<double*>(sm);
+  uint16_t* tri = reinterpret_cast<uint16_t*>(sm + pl.tri);
+  double* fw = reinterpret_cast<double*>(sm + pl.fw);
+  double *dk = reinterpret_cast<double*>(sm + pl.dk), *rs = dk + K;
+  int *colmax = reinterpret_cast<int*>(sm + pl.scale), *scale = colmax + K;
+  __shared__ double red[32];
+  __shared__ float fred[NW];
+  __shared__ int flag, bad_r;
+  for (int i = wid; i < K; i += NW)
+    for (int j = lane; j <= i; j += 32) tri[i * (i + 1) / 2 + j] = (uint16_t)(i << 8 | j);
+
+  for (int item = blockIdx.x; item < d.P * n_designs; item += gridDim.x) {
+    const int p = item % d.P, pd = item;
+    const float* Xd = d.X + (size_t)(item / d.P) * T * K;
+    const PairScratch s = scratch_of(o.work, blockIdx.x, T, K);
+    // the slot: X_w in fixed point and in fp32 (then Q), rows of LT samples
+    int2* fx = reinterpret_cast<int2*>(((uintptr_t)s.Xw + 15) & ~(uintptr_t)15);
+    float* xf = reinterpret_cast<float*>(fx + (size_t)K * LT);
+    const double *cc = area, *cm = area + T, *cr = area + 2 * T;
+    __syncthreads();  // the area's last use
+    if constexpr (SHARED_LDL) {
+      const double* src = pair_cm + (size_t)p * 4 * T;
+      for (int i = tid; i < 3 * T; i += nth) area[i] = src[i];
+      if (tid == 0) bad_r = pair_bad[p];
+    } else {
+      ldl_of_pair(d, o, p, area, area + T, area + 2 * T, area + 3 * T, red, &bad_r);
+    }
+    if (tid == 0) flag = 0;
+    for (int j = tid; j < K; j += nth) colmax[j] = 0;
+    __syncthreads();
+
+    // ---- 2. the columns' scales, from the recursion in fp32, then X_w
+    const float4* cf = reinterpret_cast<const float4*>(o.coef) + (size_t)p * T;
+    for (int e = tid; e < K * d.n_runs; e += nth) {
+      const int j = e % K, t0 = d.run_start[e / K], t1 = d.run_start[e / K + 1];
+      float xp = 0.f, vp = 0.f, mx = 0.f;
+#pragma unroll 8
+      for (int t = t0; t < t1; ++t) {
+        const float x = __ldg(Xd + (size_t)t * K + j);
+        const float4 q = cf[t];
+        vp = fmaf(-q.y, vp, fmaf(-q.x, xp, x));
+        xp = x;
+        mx = fmaxf(mx, fabsf(vp * q.w));
+      }
+      atomicMax(colmax + j, __float_as_int(mx));
+    }
+    __syncthreads();
+    for (int j = tid; j < K; j += nth) scale[j] = fixed_scale(__int_as_float(colmax[j]));
+    __syncthreads();
+    bool over = false;
+    for (int e = tid; e < K * d.n_runs; e += nth) {
+      const int j = e % K, t0 = d.run_start[e / K], t1 = d.run_start[e / K + 1], sc = scale[j];
+      int2* fr = fx + (size_t)j * LT;
+      float* xr = xf + (size_t)j * LT;
+      double xp = 0.0, vp = 0.0;  // c = m = 0 at the run's start
+      float xn[4];
+      auto load = [&](int tq) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) xn[k] = tq + k >= t0 && tq + k < t1 ? __ldg(Xd + (size_t)(tq + k) * K + j) : 0.f;
+      };
+      load(t0 & ~3);
+      for (int tq = t0 & ~3; tq < t1; tq += 4) {
+        const float xb[4] = {xn[0], xn[1], xn[2], xn[3]};
+        load(tq + 4);
+        int2 f[4];
+        float w4[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int t = tq + k;
+          f[k] = make_int2(0, 0);
+          w4[k] = 0.f;
+          if (t >= t0 && t < t1) {
+            const double x = f2d_exact(xb[k]);
+            const double z = x - cc[t] * xp;
+            vp = z - cm[t] * vp;
+            xp = x;
+            const double w = vp * cr[t];
+            f[k] = fixed_of(w, sc, over);
+            w4[k] = d2f_exact(w);
+          }
+        }
+        if (tq >= t0 && (tq + 4 <= t1 || t1 == T)) {  // whole, or the last of the row with its padding
+          *reinterpret_cast<int4*>(fr + tq) = make_int4(f[0].x, f[0].y, f[1].x, f[1].y);
+          *reinterpret_cast<int4*>(fr + tq + 2) = make_int4(f[2].x, f[2].y, f[3].x, f[3].y);
+          *reinterpret_cast<float4*>(xr + tq) = make_float4(w4[0], w4[1], w4[2], w4[3]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int t = tq + k;
+            if (t >= t0 && (t < t1 || t1 == T)) {
+              fr[t] = f[k];
+              xr[t] = w4[k];
+            }
+          }
+        }
+      }
+    }
+    if (over) flag = 1;
+    __syncthreads();
+    bool left = flag != 0;
+
+    // ---- 3. X_w'X_w, into XtX and (FP64) the slot's Lx
+    if (!left) {
+      int2* buf = reinterpret_cast<int2*>(area);
+      const int rows = 4 * kb, nch = (T + WI_CS - 1) / WI_CS;
+      auto stage = [&](int c) {
+        int2* b = buf + (c & 1) * rows * WI_RS;
+        for (int e = tid; e < rows * (WI_CS / 2); e += nth) {
+          const int j = e / (WI_CS / 2), h = e % (WI_CS / 2), t = c * WI_CS + 2 * h;
+          const bool in = j < K && t < LT;
+          const int2* src = in ? fx + (size_t)j * LT + t : fx;
+          const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(b + j * WI_RS + 2 * h));
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
+                       : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      for (int b0 = 0; b0 < pl.NB * SL; b0 += nth) {
+        const int b = b0 + tid, sl = b % SL;
+        const bool on = b < pl.NB * SL;
+        int bi = 0, bj = 0;
+        if (on) tri_index(b / SL, bi, bj);
+        FixedDot2 acc[4][4];
+        stage(0);
+        for (int c = 0; c < nch; ++c) {
+          if (c + 1 < nch) {
+            stage(c + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+          } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+          }
+          __syncthreads();
+          if (on) {
+            const int4* r0 = reinterpret_cast<const int4*>(buf + (c & 1) * rows * WI_RS);
+            const int4 *ri = r0 + bi * (WI_RS / 2), *rj = r0 + bj * (WI_RS / 2);
+            for (int h = sl; h < WI_CS / 2; h += SL) {
+              int4 x[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) x[u] = ri[u * kb * (WI_RS / 2) + h];
+#pragma unroll
+              for (int v = 0; v < 4; ++v) {
+                const int4 y = rj[v * kb * (WI_RS / 2) + h];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  acc[u][v].add(x[u].x, x[u].y, y.x, y.y);
+                  acc[u][v].add(x[u].z, x[u].w, y.z, y.w);
+                }
+              }
+            }
+          }
+          __syncthreads();
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            FixedDot2& f = acc[u][v];
+            for (int m = 1; m < SL; m <<= 1) {
+              f.hh += __shfl_xor_sync(0xffffffffu, f.hh, m);
+              f.x += __shfl_xor_sync(0xffffffffu, f.x, m);
+            }
+            const int i = bi + u * kb, j = bj + v * kb;
+            if (on && sl == 0 && i < K && j < K) {
+              const double x = f.value(scale[i], scale[j]);
+              s.Lx[i * K + j] = x;
+              s.Lx[j * K + i] = x;
+              o.XtX[(size_t)pd * K * K + i * K + j] = (float)x;
+              o.XtX[(size_t)pd * K * K + j * K + i] = (float)x;
+            }
+          }
+      }
+      __syncthreads();
+
+      // ---- 4. the factor and its inverse. A holds the packed triangle; column
+      // k of A (before its division by sqrt(D_k)) goes to row k of s.Lx
+      double* A = area;
+      for (int e = tid; e < K * (K + 1) / 2; e += nth) {
+        const int rc = tri[e];
+        A[e] = s.Lx[(rc >> 8) * K + (rc & 255)];
+      }
+      __syncthreads();
+      constexpr int LA = 32;  // entries of f per warp of the look-ahead
+      const int nla = (K + LA - 1) / LA;
+      for (int k = -1; k < K - 1; ++k) {
+        bool bad = false;
+        const double *f = fw + (k & 1) * 2 * K, *w = f + K;
+        double *fn = fw + ((k + 1) & 1) * 2 * K, *wn = fn + K;
+        const int k1 = k + 1, row1 = k1 * (k1 + 1) / 2;
+        if (wid < nla) {
+          const int i = wid * LA + lane;
+          const double w1 = k >= 0 ? w[k1] : 0.0, f1 = k >= 0 ? f[k1] : 0.0;
+          double dn = A[row1 + k1];
+          if (k >= 0) dn = fma(-w1, f1, dn);
+          bad = !positive(dn);
+          if (bad) dn = 1.0;
+          double v = 1.0, r, pc;
+          if (i < k1) {  // row k + 1 of the inverse
+            v = fma(-w1, f[i], i == k ? 0.0 : A[row1 + i]);
+            A[row1 + i] = v;
+          } else if (i > k1 && i < K) {
+            v = A[i * (i + 1) / 2 + k1];
+            if (k >= 0) v = fma(-w[i], f1, v);
+            s.Lx[k1 * K + i] = v;
+          }
+          rcp_factors(dn, r, pc);
+          if (i < K) {
+            const double u = v * r;
+            fn[i] = v;
+            wn[i] = fma(u, pc, u);
+          }
+          if (i == k1) dk[k1] = dn;
+        }
+        if (k >= 0) {
+          const int E = K * (K + 1) / 2;
+#pragma unroll 2
+          for (int e = (k + 2) * (k + 3) / 2 + tid; e < E; e += nth) {
+            const int rc = tri[e], r = rc >> 8, c = rc & 255;
+            if (c != k1) A[e] = fma(-w[r], f[c], c == k ? 0.0 : A[e]);
+          }
+        }
+        left = __syncthreads_or(bad);
+        if (left) break;
+      }
+    }
+    __syncthreads();
+    if (left) {
+      if constexpr (SHARED_LDL) {
+        const double* src = pair_cm + (size_t)p * 4 * T;
+        for (int i = tid; i < 3 * T; i += nth) area[i] = src[i];
+        __syncthreads();
+      } else {
+        ldl_of_pair(d, o, p, area, area + T, area + 2 * T, area + 3 * T, red, &bad_r);
+      }
+      item_global<false>(args, s, p, pd, Xd, cc, cm, cr, nullptr, bad_r, red, &flag);
+      continue;
+    }
+    double* A = area;
+    // the last row's rank-1 share went no further than f; Li = D^-1/2 Lu^-1
+    for (int k = tid; k < K; k += nth) {
+      const double r = rsqrt_newton(dk[k]);
+      rs[k] = r;
+      fw[k] = 2.0 * log(fabs(dk[k] * r) + 1e-10);
+    }
+    __syncthreads();
+    if (tid == 0) {
+      double ld = 0.0;
+      for (int j = 0; j < K; ++j) ld += fw[j];
+      o.logdet_XtX[pd] = ld;
+      o.info[pd] = bad_r ? 2 : 0;
+    }
+    for (int e = tid; e < K * (K + 1) / 2; e += nth) {
+      const int rc = tri[e], i = rc >> 8, j = rc & 255;
+      const double v = i == j ? rs[i] : A[e] * rs[i];
+      A[e] = v;
+      s.Li[i * K + j] = v;
+    }
+    __syncthreads();
+    for (int j = tid; j < K; j += nth) {
+      double acc = 0.0;
+      for (int k = j; k < K; ++k) {
+        const double v = A[k * (k + 1) / 2 + j];
+        acc = fma(v, v, acc);
+      }
+      o.Adiag[(size_t)pd * K + j] = (float)acc;
+    }
+    if (o.Afull) {  // all of A, for the per-voxel blocks of the -dsort fit
+      for (int e = tid; e < K * (K + 1) / 2; e += nth) {
+        const int rc = tri[e], i = rc >> 8, j = rc & 255;
+        double acc = 0.0;
+        for (int k = i; k < K; ++k) acc = fma(A[k * (k + 1) / 2 + i], A[k * (k + 1) / 2 + j], acc);
+        o.Afull[(size_t)pd * K * K + i * K + j] = (float)acc;
+        o.Afull[(size_t)pd * K * K + j * K + i] = (float)acc;
+      }
+    }
+    __syncthreads();
+
+    // ---- 5. Q = X_w Lx^-T in fp32; lx[i][j], j contiguous
+    float* lx = reinterpret_cast<float*>(area);
+    for (int e = tid; e < K * KP; e += nth) {
+      const int i = e / KP, j = e % KP;
+      lx[e] = j < K && j >= i ? (float)(j == i ? dk[i] * rs[i] : s.Lx[i * K + j] * rs[i]) : 0.f;
+    }
+    __syncthreads();
+    for (int t2 = tid; t2 < LT / 2; t2 += nth) {
+      float2* q = reinterpret_cast<float2*>(xf) + t2;
+      for (int j0 = 0; j0 < K; j0 += 8) {
+        float2 a[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) a[c] = j0 + c < K ? q[(size_t)(j0 + c) * (LT / 2)] : make_float2(0.f, 0.f);
+#pragma unroll 4
+        for (int i = 0; i < j0; ++i) {
+          const float2 qi = q[(size_t)i * (LT / 2)];
+          const float4 l0 = *reinterpret_cast<const float4*>(lx + i * KP + j0);
+          const float4 l1 = *reinterpret_cast<const float4*>(lx + i * KP + j0 + 4);
+          const float l[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            a[c].x = fmaf(-l[c], qi.x, a[c].x);
+            a[c].y = fmaf(-l[c], qi.y, a[c].y);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          if (j0 + c < K) {
+            const float* l = lx + (j0 + c) * KP + j0;
+            a[c].x /= l[c];
+            a[c].y /= l[c];
+#pragma unroll
+            for (int e = c + 1; e < 8; ++e) {
+              a[e].x = fmaf(-l[e], a[c].x, a[e].x);
+              a[e].y = fmaf(-l[e], a[c].y, a[e].y);
+            }
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (j0 + c < K) q[(size_t)(j0 + c) * (LT / 2)] = a[c];
+      }
+    }
+    __syncthreads();
+
+    // ---- 6. U = L^-T Q, the backward recursions of each column and run
+    float* const U = o.U + (size_t)pd * K * LT;
+    float umax = 0.f;
+    for (int e = tid; e < K * d.n_runs; e += nth) {
+      const int j = e % K, t0 = d.run_start[e / K], t1 = d.run_start[e / K + 1];
+      const float* q = xf + (size_t)j * LT;
+      float* u = U + (size_t)j * LT;
+      if (t1 == T)
+        for (int t = T; t < LT; ++t) u[t] = 0.f;
+      float xn = 0.f, mn = 0.f, cn = 0.f;  // x_{t+1}, m_{t+1}, c_{t+1} (0 past a run's end)
+      auto step = [&](float qt, float4 c4) {
+        const float x = fmaf(-mn, xn, qt * c4.w);
+        const float ut = fmaf(-cn, xn, x);
+        xn = x;
+        mn = c4.y;
+        cn = c4.x;
+        umax = fmaxf(umax, fabsf(ut));
+        return ut;
+      };
+      int t = t1 - 1;
+      for (; t >= t0 && (t & 3) != 3; --t) u[t] = step(q[t], cf[t]);
+#pragma unroll 2
+      for (; t - 3 >= t0; t -= 4) {
+        const float4 q4 = *reinterpret_cast<const float4*>(q + t - 3);
+        const float4 c3 = cf[t], c2 = cf[t - 1], c1 = cf[t - 2], c0 = cf[t - 3];
+        float4 r;
+        r.w = step(q4.w, c3);
+        r.z = step(q4.z, c2);
+        r.y = step(q4.y, c1);
+        r.x = step(q4.x, c0);
+        *reinterpret_cast<float4*>(u + t - 3) = r;
+      }
+      for (; t >= t0; --t) u[t] = step(q[t], cf[t]);
+    }
+    for (int off = 16; off > 0; off >>= 1) umax = fmaxf(umax, __shfl_xor_sync(0xffffffffu, umax, off));
+    if (lane == 0) fred[wid] = umax;
+    // Lx^-1 for G, beside
+    float* li = reinterpret_cast<float*>(area);
+    for (int e = tid; e < K * KP; e += nth) {
+      const int i = e / KP, j = e % KP;
+      li[e] = j <= i ? (float)s.Li[i * K + j] : 0.f;
+    }
+    __syncthreads();
+    if (o.U_hi) {
+      // fp16 hi/lo split of U * 2^e, e placing max|U| in [128, 256)
+      float mx = 0.f;
+      for (int w = 0; w < NW; ++w) mx = fmaxf(mx, fred[w]);
+      const int ex = scale_exp(mx);
+      if (tid == 0) o.uexp[pd] = ex;
+      const bool pw = ex >= -126 && ex <= 127;
+      const float p2 = pw ? __int_as_float((ex + 127) << 23) : 0.f;
+      for (int j = wid; j < K; j += NW) {  // a warp per column
+        const float2* u = reinterpret_cast<const float2*>(U + (size_t)j * LT);
+        uint32_t* ho = reinterpret_cast<uint32_t*>(o.U_hi + ((size_t)pd * K + j) * d.ld_u);
+        uint32_t* lo = reinterpret_cast<uint32_t*>(o.U_lo + ((size_t)pd * K + j) * d.ld_u);
+#pragma unroll 4
+        for (int h = lane; h < (d.ld_u >> 1); h += 32) {
+          const float2 y = 2 * h < LT ? u[h] : make_float2(0.f, 0.f);
+          uint16_t h0, l0, h1, l1;
+          split_fp16(pw ? __fmul_rn(y.x, p2) : ldexpf(y.x, ex), h0, l0);
+          split_fp16(pw ? __fmul_rn(y.y, p2) : ldexpf(y.y, ex), h1, l1);
+          ho[h] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+          lo[h] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+        }
+      }
+    }
+    if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, s.Li, K, true, s.S, red);
+
+    // ---- 8. G = U Lx^-1 in fp32
+    for (int t2 = tid; t2 < LT / 2; t2 += nth) {
+      const float2* u = reinterpret_cast<const float2*>(U) + t2;
+      float2* g = reinterpret_cast<float2*>(o.G + (size_t)pd * K * LT) + t2;
+      for (int j0 = 0; j0 < K; j0 += 8) {
+        float2 a[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) a[c] = make_float2(0.f, 0.f);
+#pragma unroll 4
+        for (int i = j0; i < K; ++i) {  // li is zero above its diagonal
+          const float2 ui = u[(size_t)i * (LT / 2)];
+          const float4 l0 = *reinterpret_cast<const float4*>(li + i * KP + j0);
+          const float4 l1 = *reinterpret_cast<const float4*>(li + i * KP + j0 + 4);
+          const float l[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            a[c].x = fmaf(ui.x, l[c], a[c].x);
+            a[c].y = fmaf(ui.y, l[c], a[c].y);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (j0 + c < K) g[(size_t)(j0 + c) * (LT / 2)] = a[c];
+      }
+    }
+    item_tail(d, o, s, pd, red, &flag);
+  }
+}
+
 // ---- Design basis: Q0 = X Lx^-T, Lx the FP64 Cholesky factor of X'X (Q0 is
 // U of the pair (0, 0), where R = I and X_w = X, and comes out bit for bit
 // equal to the grid build's: the same Dot4 entries, block_cholesky and fp32
@@ -1924,7 +2427,9 @@ static bool too_long(const ffs_grid_desc& d) {
 // The item kernel of a build: grid_item_kernel for designs of up to GI_KMAX
 // columns whose items fit in shared memory (half an SM's: two CTAs overlap
 // their latencies; one alone still beats global scratch, so up to 200 KB),
-// grid_build_kernel for the rest.
+// grid_wide_kernel for wider ones whose factor does, grid_build_kernel for the
+// rest (more than FX_TMAX samples, whose sums leave the integers' range, and the
+// banded R).
 static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, const double* pair_cm,
                         const int* pair_bad, cudaStream_t st, const char* who) {
   using namespace ffsk;
@@ -1942,6 +2447,14 @@ static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, co
     FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), pl.total));
     kern<<<grid, pl.GT + 32 * pl.PW, pl.total, st>>>(args, n_designs, pair_cm, pair_bad);
     return check_launch("grid_item_kernel");
+  }
+  const WidePlan wp = wide_plan(d.T, d.K);
+  if (d.K > GI_KMAX && d.K <= WI_KMAX && d.T <= FX_TMAX && !d.band && wp.total <= 200 * 1024 &&
+      (((uintptr_t)o.U_hi | (uintptr_t)o.U_lo) & 3) == 0 && (((uintptr_t)o.U | (uintptr_t)o.G) & 15) == 0) {
+    auto kern = pair_cm ? grid_wide_kernel<true> : grid_wide_kernel<false>;
+    FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), wp.total));
+    kern<<<grid, WI_THREADS, wp.total, st>>>(args, n_designs, pair_cm, pair_bad);
+    return check_launch("grid_wide_kernel");
   }
   // phase 1's scratch beside the coefficients while that leaves room for four CTAs an SM
   const int tmp_smem = !pair_cm && sizeof(double) * 7 * d.T <= 50 * 1024;

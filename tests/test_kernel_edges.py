@@ -359,3 +359,62 @@ def test_banded_factors_and_surface_against_dense_float64(T, K, runs, hole, a_ma
         crit = float(f.logdet_R[p] + f.logdet_XtX[p]) - base + (T - K) * np.log1p((ssw - proj - rss0) / rss0)
         scale = (ssw + proj) / np.minimum(ssw - proj, rss0)
         assert (np.abs(surf[p] - crit) <= 3e-5 * (T - K) * scale + 1e-5 * np.abs(crit)).all()
+
+
+@gpu
+@pytest.mark.parametrize("T,K,runs,dup", [
+    (161, 41, 1, False),   # the narrowest wide design, four sample slices, T odd
+    (203, 57, 3, False),   # runs that start inside a word of four
+    (400, 72, 2, False),   # two slices
+    (301, 103, 3, False),  # two rounds of blocks
+    (600, 130, 1, False),
+    (400, 150, 2, False),
+    (203, 57, 3, True),    # a repeated column: the general phases' QR
+])
+def test_wide_designs_against_dense_float64(T, K, runs, dup):
+    """Builds of more than 40 columns: Gram matrix, logdets, diag((X'R^-1X)^-1),
+    U = L^-T Q and G against dense FP64. The Gram matrix, the factor and its
+    inverse are FP64 or finer and leave as fp32 (one rounding, 1e-6 with room
+    for the factor's); Q, U and G go through fp32 sums of up to K terms on a
+    design of condition below 30 (K 2^-24 30: 3e-4 of the largest entry at
+    the widest)."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(T + K)
+    X = rng.standard_normal((T, K)).astype(np.float32)
+    X[:, 0] = 1.0
+    if dup:
+        X[:, 7] = X[:, 3]
+    starts = [T * r // runs for r in range(runs)]
+    g = G.make_grid(torch.linspace(0.0, 0.8, 3), torch.linspace(-0.4, 0.4, 3), use_double=True)
+    f = engine.build_factors(torch.from_numpy(X).to(DEV), g, G.run_layout(T, starts), with_tc=True)
+    torch.cuda.synchronize()
+    info = f.info.cpu().numpy()
+    if dup:
+        assert (info == 1).any() or np.isfinite(f.U.cpu().numpy()).all()
+        return
+    assert (info == 0).all()
+    run_of = np.searchsorted(starts, np.arange(T), side="right")
+    gap = np.abs(np.arange(T)[:, None] - np.arange(T)[None, :])
+    tol = K * 2.0 ** -24 * 30
+    for p in range(g.P):
+        a, b = float(np.float32(g.a[p])), float(np.float32(g.b[p]))
+        lam = (b + a) * (1 + a * b) / (1 + 2 * a * b + b * b)
+        R = np.where((gap > 0) & (run_of[:, None] == run_of[None, :]), lam * a ** np.maximum(gap - 1, 0), 0.0) + np.eye(T)
+        Li = np.linalg.inv(np.linalg.cholesky(R))
+        Xw = Li @ X.astype(np.float64)
+        N = Xw.T @ Xw
+        C = np.linalg.cholesky(N)
+        Ci = np.linalg.inv(C)
+        U = (Ci @ Xw.T) @ Li
+        np.testing.assert_allclose(float(f.logdet_XtX[p]), 2 * np.log(np.diag(C) + 1e-10).sum(), rtol=1e-9, atol=1e-9)
+        np.testing.assert_allclose(f.XtX[p].cpu().numpy(), N, rtol=1e-6, atol=1e-6 * np.abs(N).max())
+        np.testing.assert_allclose(f.Adiag[p].cpu().numpy(), np.diag(Ci.T @ Ci), rtol=1e-6)
+        got = f.U[p, :, :T].cpu().numpy()
+        assert np.abs(got - U).max() <= tol * np.abs(U).max()
+        Gm = Ci.T @ U
+        assert np.abs(f.G[p, :, :T].cpu().numpy() - Gm).max() <= tol * np.abs(Gm).max()
+        assert (f.U[p, :, T:] == 0).all() and (f.G[p, :, T:] == 0).all()
+        hi, lo = (x.view(f.P, K, -1)[p].view(torch.float16).double() for x in (f.U_hi, f.U_lo))
+        back = ((hi + lo) * 2.0 ** -float(f.uexp[p])).cpu().numpy()[:, :T]
+        assert np.abs(back - got).max() <= 2.0 ** -20 * np.abs(got).max()
