@@ -416,14 +416,26 @@ __device__ void gls_finish_tile(const ffs_gls_args& a, int g, int j0, int n, flo
     const int l = tid & 31, ks = tid >> 5;
     float part = 0.f;
     if (l < n) {
-      for (int k = ks; k < nk; k += TILE_WARPS) {
-        const int ck = a.n_task > 0 ? a.task_idx[k] : k;
-        float s = 0.f;
-        for (int c = 0; c < nk; ++c) {
-          const int cl = a.n_task > 0 ? a.task_idx[c] : c;
-          s = fmaf(Mq[k * nk + c], C0[cl * TILE_V + l], s);
+      constexpr int KR = 4;  // rows at a time, their loads in flight together
+      for (int k0 = ks; k0 < nk; k0 += KR * TILE_WARPS) {
+        float s[KR];
+        const float* row[KR];
+#pragma unroll
+        for (int u = 0; u < KR; ++u) {
+          s[u] = 0.f;
+          row[u] = Mq + (size_t)min(k0 + u * TILE_WARPS, nk - 1) * nk;
         }
-        part = fmaf(C0[ck * TILE_V + l], s, part);
+#pragma unroll 4
+        for (int c = 0; c < nk; ++c) {
+          const float b = C0[(a.n_task > 0 ? a.task_idx[c] : c) * TILE_V + l];
+#pragma unroll
+          for (int u = 0; u < KR; ++u) s[u] = fmaf(row[u][c], b, s[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < KR; ++u) {
+          const int k = k0 + u * TILE_WARPS;
+          if (k < nk) part = fmaf(C0[(a.n_task > 0 ? a.task_idx[k] : k) * TILE_V + l], s[u], part);
+        }
       }
     }
     red[ks * TILE_V + l] = part;
@@ -465,9 +477,12 @@ __device__ void gls_finish_tile(const ffs_gls_args& a, int g, int j0, int n, flo
   }
 }
 
-__global__ void __launch_bounds__(TILE_WARPS * 32, 3) gls_tile_kernel(ffs_gls_args a, GlsExtra x, const int* end,
-                                                                   const int* tile_start, int P, int ld, int kp,
-                                                                   int hb, int msz) {
+// WIDE: designs of more than TILE_TC_K columns, whose tiles leave room for two CTAs an SM.
+template <bool WIDE>
+__global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel(ffs_gls_args a, GlsExtra x,
+                                                                                 const int* end, const int* tile_start,
+                                                                                 int P, int ld, int kp, int hb,
+                                                                                 int msz) {
   extern __shared__ float4 sm4[];
   const int T = a.T, K = a.K, LT = ld_t(T), nq = LT >> 2;
   const bool vec = (T & 3) == 0;  // 16-byte rows of the [V][T] outputs
@@ -570,7 +585,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, 3) gls_tile_kernel(ffs_gls_ar
   const float* Xt = a.Xt + (size_t)design_of(a, g) * K * LT;
   // b0 = G'y; SS_tot; r = y - X b0. Warp w takes the rows 4w .. 4w+3 in the
   // row passes, lanes over quads.
-  tile_project(Gg, LT, Ys, ld, K, C0);
+  tile_project<WIDE>(Gg, LT, Ys, ld, K, C0);
 #pragma unroll
   for (int i = 0; i < TILE_SUB_VB; ++i) {
     const int l = TILE_SUB_VB * wid + i;
@@ -592,9 +607,9 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, 3) gls_tile_kernel(ffs_gls_ar
     sst = warp_sum(sst);
     if (lane == 0) st[4 * TILE_V + l] = sst;
   }
-  tile_subtract_any(Xt, LT, C0, Ys, ld, K);
+  tile_subtract_any<WIDE>(Xt, LT, C0, Ys, ld, K);
   // the refinement d = G'r; SS_res and the unwhitened outputs
-  tile_project(Gg, LT, Ys, ld, K, C1);
+  tile_project<WIDE>(Gg, LT, Ys, ld, K, C1);
 #pragma unroll
   for (int i = 0; i < TILE_SUB_VB; ++i) {
     const int l = TILE_SUB_VB * wid + i;
@@ -1268,8 +1283,8 @@ extern "C" int ffs_reml_gls_grouped(const ffs_gls_args* a, int lj_h, const int* 
   FFS_REQUIRE(lj_h >= 0 && lj_h <= a->T / 2, "ffs_reml_gls_grouped: Ljung-Box lag %d out of range", lj_h);
   FFS_REQUIRE(lj_h == 0 || (lj_w && ljung_box), "ffs_reml_gls_grouped: Ljung-Box buffers");
   const int ld = tile_ld(a->T);
-  const int kp = (a->K + 3) & ~3;
-  const int hb = (lj_h + 4) & ~3;
+  const int kp = lj_h > 0 ? (a->K + 3) & ~3 : 0;  // per-warp scratch of the Ljung-Box form
+  const int hb = lj_h > 0 ? (lj_h + 4) & ~3 : 0;
   const int nm = a->n_task > 0 ? a->n_task : a->K;
   const int msz = nm * nm <= 4096 ? nm * nm : 0;  // F matrix staged per tile when it is small
   size_t smem = sizeof(float) * ((size_t)TILE_V * ld + 2 * (size_t)a->K * TILE_V +
@@ -1283,9 +1298,10 @@ extern "C" int ffs_reml_gls_grouped(const ffs_gls_args* a, int lj_h, const int* 
   cudaStream_t st = (cudaStream_t)stream;
   GlsExtra x{lj_h, lj_tau, lj_w, ljung_box, lj_tab};
   gls_tile_scan<<<1, 1024, 0, st>>>(P, group_end, tile_start);
-  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(gls_tile_kernel), smem));
+  auto kern = a->K > TILE_TC_K ? gls_tile_kernel<true> : gls_tile_kernel<false>;
+  FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), smem));
   const int max_tiles = ceil_div(a->V, GLS_TILE) + P;
-  gls_tile_kernel<<<max_tiles, TILE_WARPS * 32, smem, st>>>(*a, x, group_end, tile_start, P, ld, kp, hb, msz);
+  kern<<<max_tiles, TILE_WARPS * 32, smem, st>>>(*a, x, group_end, tile_start, P, ld, kp, hb, msz);
   return check_launch("gls_tile_kernel");
 }
 

@@ -145,7 +145,8 @@ __global__ void __launch_bounds__(256) prep_kernel(ffs_prep_args a, int ld_s) {
 // (fastfuncstuff/glm/arma.py:1554-1571). Rows of Y are read as 16-byte words
 // when T % 4 == 0 and as single samples otherwise; the tile's samples
 // T .. ld_t(T) stay zero.
-__global__ void __launch_bounds__(TILE_WARPS * 32, 3) prep_tile_kernel(ffs_prep_args a, int ld) {
+template <bool WIDE>
+__global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kernel(ffs_prep_args a, int ld) {
   extern __shared__ float4 sm4[];
   float* Ys = reinterpret_cast<float*>(sm4);       // [32][ld]
   float* Cq = Ys + (size_t)TILE_V * ld;            // [K][32]
@@ -224,8 +225,8 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, 3) prep_tile_kernel(ffs_prep_
   __syncthreads();
   if (K > 0) {
     const float* Q0 = a.Q0 + (a.tile_design ? (size_t)a.tile_design[blockIdx.x] * K * LT : 0);
-    tile_project(Q0, LT, Ys, ld, K, Cq);
-    tile_subtract_any(Q0, LT, Cq, Ys, ld, K);
+    tile_project<WIDE>(Q0, LT, Ys, ld, K, Cq);
+    tile_subtract_any<WIDE>(Q0, LT, Cq, Ys, ld, K);
   }
   __syncthreads();
   if (a.feats) {
@@ -882,8 +883,9 @@ extern "C" int ffs_reml_prep(const ffs_prep_args* a, void* stream) {
     const size_t smem = sizeof(float) * ((size_t)TILE_V * ld + (size_t)a->K * TILE_V);
     FFS_REQUIRE(smem <= 200 * 1024 || !a->Y_ref, "ffs_reml_prep: Y_ref needs the tiled prep (T=%d too long)", a->T);
     if (smem <= 200 * 1024) {
-      FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(prep_tile_kernel), smem));
-      prep_tile_kernel<<<ceil_div(a->V, TILE_V), TILE_WARPS * 32, smem, (cudaStream_t)stream>>>(*a, ld);
+      auto kern = a->K > TILE_TC_K ? prep_tile_kernel<true> : prep_tile_kernel<false>;
+      FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), smem));
+      kern<<<ceil_div(a->V, TILE_V), TILE_WARPS * 32, smem, (cudaStream_t)stream>>>(*a, ld);
       return check_launch("prep_tile_kernel");
     }
   }

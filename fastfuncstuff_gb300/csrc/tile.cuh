@@ -17,7 +17,7 @@
 // FMA is therefore bound by that path, not by the FMA pipe. Each thread here
 // keeps a block of operands in registers instead: in the projection 8 voxels
 // x up to 5 columns (every loaded matrix entry serves 8 voxels, every loaded
-// sample up to 5 columns), in the update 4 voxels x up to 10 columns.
+// sample up to 5 columns), in the update 8 voxels x 4 samples.
 #pragma once
 #include "common.cuh"
 
@@ -28,8 +28,9 @@ constexpr int TILE_WARPS = 8;    // warps per CTA
 constexpr int TILE_SLICES = 16;  // time slices of tile_project (lane bits 0..3)
 constexpr int TILE_VB = 8;       // voxels per thread in tile_project
 constexpr int TILE_KB_MAX = 5;   // columns per thread and pass in tile_project
-constexpr int TILE_SUB_VB = 4;   // voxels per warp in tile_subtract (warp w: 4w .. 4w+3)
-constexpr int TILE_SUB_KC = 10;  // columns per pass in tile_subtract
+constexpr int TILE_SUB_VB = 4;   // voxels per warp in the row passes (warp w: 4w .. 4w+3)
+constexpr int TILE_SUB_PF = 4;   // columns loaded ahead in tile_subtract
+constexpr int TILE_TC_K = 32;    // widest design of the tensor-core update
 
 // Row stride (floats) of a tile: a multiple of 4 with ld / 4 odd, so 128-bit
 // loads of 8 lanes from 8 different rows fall in distinct banks.
@@ -80,7 +81,9 @@ __device__ __forceinline__ void tile_stage_rows(const float* __restrict__ Y, int
 // partials are summed by recursive halving across lane bits 3, 2, 1 (each
 // exchange ships half of the remaining values) and a final exchange across
 // bit 0; lanes s and s ^ 1 then hold the KB sums of voxel s >> 1.
-template <int KB>
+// PF: the matrix entries of a thread's next quad are loaded before this one's
+// products (more registers; for matrices that do not stay in the L1 cache).
+template <int KB, bool PF>
 __device__ __forceinline__ void tile_project_kb(const float* __restrict__ M, int lm, const float* Ys, int ld, int K,
                                                 float* C) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -95,11 +98,22 @@ __device__ __forceinline__ void tile_project_kb(const float* __restrict__ M, int
 #pragma unroll
     for (int i = 0; i < TILE_VB * KB; ++i) acc[i] = 0.f;
     const float4* mb = reinterpret_cast<const float4*>(M + (size_t)min(jb, K - 1) * lm);  // row jb, stride nq
-    for (int q = s; q < nq; q += TILE_SLICES) {
-      float4 m[KB];
+    float4 next[PF ? KB : 1];
+    auto load = [&](float4* to, int q) {
 #pragma unroll
       for (int k = 0; k < KB; ++k)
-        m[k] = (jb + k < K) ? __ldg(mb + (size_t)k * nq + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        to[k] = (jb + k < K) && q < nq ? __ldg(mb + (size_t)k * nq + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if constexpr (PF) load(next, s);
+    for (int q = s; q < nq; q += TILE_SLICES) {
+      float4 m[KB];
+      if constexpr (PF) {
+#pragma unroll
+        for (int k = 0; k < KB; ++k) m[k] = next[k];
+        load(next, q + TILE_SLICES);
+      } else {
+        load(m, q);
+      }
 #pragma unroll
       for (int i = 0; i < TILE_VB; ++i) {
         const float4 y = y4[(size_t)i * ld4 + q];
@@ -139,55 +153,69 @@ __device__ __forceinline__ void tile_project_kb(const float* __restrict__ M, int
 
 // C[j][l] = sum_t M[j][t] Ys[l][t] for j < K, l < 32 (C is [K][32]; M has
 // row stride lm). Ends with a barrier.
+template <bool PF = false>
 __device__ __forceinline__ void tile_project(const float* __restrict__ M, int lm, const float* Ys, int ld, int K,
                                              float* C) {
   const int passes = (K + 4 * TILE_KB_MAX - 1) / (4 * TILE_KB_MAX);
   const int kb = (K + 4 * passes - 1) / (4 * passes);  // columns per thread and pass, <= TILE_KB_MAX
   switch (kb) {
-    case 1: tile_project_kb<1>(M, lm, Ys, ld, K, C); break;
-    case 2: tile_project_kb<2>(M, lm, Ys, ld, K, C); break;
-    case 3: tile_project_kb<3>(M, lm, Ys, ld, K, C); break;
-    case 4: tile_project_kb<4>(M, lm, Ys, ld, K, C); break;
-    default: tile_project_kb<5>(M, lm, Ys, ld, K, C); break;
+    case 1: tile_project_kb<1, PF>(M, lm, Ys, ld, K, C); break;
+    case 2: tile_project_kb<2, PF>(M, lm, Ys, ld, K, C); break;
+    case 3: tile_project_kb<3, PF>(M, lm, Ys, ld, K, C); break;
+    case 4: tile_project_kb<4, PF>(M, lm, Ys, ld, K, C); break;
+    default: tile_project_kb<5, PF>(M, lm, Ys, ld, K, C); break;
   }
   __syncthreads();
 }
 
-// Ys[l][t] -= sum_j N[j][t] C[j][l] (N has row stride lm). Warp w updates the rows 4w .. 4w+3
-// (lanes over quads), so a thread's later reads of those rows need no
-// barrier; rows of other warps do. No barrier.
+// Ys[l][t] -= sum_j N[j][t] C[j][l] (N has row stride lm), j ascending, on the
+// CUDA cores: a thread keeps 8 voxels x 1 quad and goes over all K columns, so
+// that the series are read and written once and an entry of N, loaded
+// TILE_SUB_PF columns ahead (a wide N comes from L2), serves 8 voxels. Half
+// warps take the voxel groups of 8, lanes the quads. No barrier. (With 4 voxels
+// a warp and every entry of N loaded where it was used, each load's latency was
+// waited for: 30,000 voxels, T = 600, K = 130: two thirds of prep's 0.88 ms and 43%
+// of the GLS refit's 2.55 ms; with the loads ahead here, in the projections and in
+// the F statistic, the fit takes 6.37 ms where it took 8.70.)
 __device__ __forceinline__ void tile_subtract(const float* __restrict__ N, int lm, const float* C, float* Ys, int ld,
                                               int K) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nq = lm >> 2, ld4 = ld >> 2;
-  float4* r4 = reinterpret_cast<float4*>(Ys) + (size_t)(TILE_SUB_VB * w) * ld4;
-  for (int j0 = 0; j0 < K; j0 += TILE_SUB_KC) {
-    float c[TILE_SUB_VB][TILE_SUB_KC];
+  for (int task = w; task < 2 * ((nq + 15) >> 4); task += TILE_WARPS) {
+    const int vg = 2 * (task & 1) + (lane >> 4), q = 16 * (task >> 1) + (lane & 15);
+    const bool on = q < nq;
+    const float4* n4 = reinterpret_cast<const float4*>(N) + (on ? q : 0);
+    float4* r4 = reinterpret_cast<float4*>(Ys) + (size_t)(TILE_VB * vg) * ld4 + (on ? q : 0);
+    const float4* c4 = reinterpret_cast<const float4*>(C) + 2 * vg;
+    float4 r[TILE_VB], next[TILE_SUB_PF];
 #pragma unroll
-    for (int k = 0; k < TILE_SUB_KC; ++k) {
+    for (int i = 0; i < TILE_VB; ++i) r[i] = r4[(size_t)i * ld4];
 #pragma unroll
-      for (int i = 0; i < TILE_SUB_VB; ++i)
-        c[i][k] = (j0 + k < K) ? C[(size_t)(j0 + k) * TILE_V + TILE_SUB_VB * w + i] : 0.f;
-    }
-    for (int q = lane; q < nq; q += 32) {
-      float4 r[TILE_SUB_VB];
+    for (int k = 0; k < TILE_SUB_PF; ++k) next[k] = __ldg(n4 + (size_t)min(k, K - 1) * nq);
+    for (int j0 = 0; j0 < K; j0 += TILE_SUB_PF) {
+      float4 n[TILE_SUB_PF];
 #pragma unroll
-      for (int i = 0; i < TILE_SUB_VB; ++i) r[i] = r4[(size_t)i * ld4 + q];
+      for (int k = 0; k < TILE_SUB_PF; ++k) n[k] = next[k];
 #pragma unroll
-      for (int k = 0; k < TILE_SUB_KC; ++k) {
+      for (int k = 0; k < TILE_SUB_PF; ++k) next[k] = __ldg(n4 + (size_t)min(j0 + TILE_SUB_PF + k, K - 1) * nq);
+#pragma unroll
+      for (int k = 0; k < TILE_SUB_PF; ++k) {
         if (j0 + k < K) {
-          const float4 n = __ldg(reinterpret_cast<const float4*>(N + (size_t)(j0 + k) * lm) + q);
+          const float4 ca = c4[(size_t)(j0 + k) * (TILE_V / 4)], cb = c4[(size_t)(j0 + k) * (TILE_V / 4) + 1];
+          const float c[TILE_VB] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
 #pragma unroll
-          for (int i = 0; i < TILE_SUB_VB; ++i) {
-            r[i].x = fmaf(-n.x, c[i][k], r[i].x);
-            r[i].y = fmaf(-n.y, c[i][k], r[i].y);
-            r[i].z = fmaf(-n.z, c[i][k], r[i].z);
-            r[i].w = fmaf(-n.w, c[i][k], r[i].w);
+          for (int i = 0; i < TILE_VB; ++i) {
+            r[i].x = fmaf(-n[k].x, c[i], r[i].x);
+            r[i].y = fmaf(-n[k].y, c[i], r[i].y);
+            r[i].z = fmaf(-n[k].z, c[i], r[i].z);
+            r[i].w = fmaf(-n[k].w, c[i], r[i].w);
           }
         }
       }
+    }
+    if (on) {
 #pragma unroll
-      for (int i = 0; i < TILE_SUB_VB; ++i) r4[(size_t)i * ld4 + q] = r[i];
+      for (int i = 0; i < TILE_VB; ++i) r4[(size_t)i * ld4] = r[i];
     }
   }
 }
@@ -295,19 +323,21 @@ __device__ __forceinline__ void tile_subtract_tc(const float* __restrict__ N, in
   }
 }
 
-// Ys -= (N C)' with the tensor cores for K <= 32 and the register-blocked
-// CUDA-core pass otherwise. Starts with a barrier and ends with one.
+// Ys -= (N C)' with the tensor cores for K <= TILE_TC_K and the register-blocked
+// CUDA-core pass otherwise (WIDE). Starts with a barrier and ends with one.
+template <bool WIDE>
 __device__ __forceinline__ void tile_subtract_any(const float* __restrict__ N, int lm, const float* C, float* Ys,
                                                   int ld, int K) {
-  switch ((K + 7) >> 3) {
-    case 1: tile_subtract_tc<1>(N, lm, C, Ys, ld, K); break;
-    case 2: tile_subtract_tc<2>(N, lm, C, Ys, ld, K); break;
-    case 3: tile_subtract_tc<3>(N, lm, C, Ys, ld, K); break;
-    case 4: tile_subtract_tc<4>(N, lm, C, Ys, ld, K); break;
-    default:
-      __syncthreads();
-      tile_subtract(N, lm, C, Ys, ld, K);
-      break;
+  if constexpr (WIDE) {
+    __syncthreads();
+    tile_subtract(N, lm, C, Ys, ld, K);
+  } else {
+    switch ((K + 7) >> 3) {
+      case 1: tile_subtract_tc<1>(N, lm, C, Ys, ld, K); break;
+      case 2: tile_subtract_tc<2>(N, lm, C, Ys, ld, K); break;
+      case 3: tile_subtract_tc<3>(N, lm, C, Ys, ld, K); break;
+      default: tile_subtract_tc<4>(N, lm, C, Ys, ld, K); break;
+    }
   }
   __syncthreads();
 }
