@@ -1174,30 +1174,27 @@ __device__ __forceinline__ float d2f_exact(double w) {
 //     the others form Q, U and the fp16 splits in place in shared memory.
 // A rank-deficient item (a pivot that is not positive) or one whose series
 // leave the fixed point goes through item_global.
-// Builds, us, against item_global's phases with FP64 Gram chains: P = 117,
-// T = 200, K = 8: 238 -> 108; P = 561, T = 400, K = 20: 584 -> 307; K = 32: 1016
-// -> 676; T = 500, K = 40: 1319 -> 1059; 20 designs of T = 855, K = 18: 13629 ->
-// 7960. Bound now by latency: two or three CTAs an SM (their series fill the
-// shared memory), a barrier per chunk.
-constexpr int GI_KMAX = 40;       // 820 entry threads
+// P = 117, T = 200, K = 8: 238 -> 107 us against item_global's phases with FP64 Gram
+// chains; P = 561, T = 400, K = 20: 584 -> 307. Bound by latency: two or three CTAs
+// an SM (their series fill the shared memory), a barrier per chunk.
+constexpr int GI_KMAX = 22;       // 253 entries, one per entry thread
 constexpr int GI_BUF = 4;         // chunks in the pipeline
 constexpr int GI_PROD = 96;       // most producer lanes (3 warps)
 constexpr int GI_VAL = 3;         // most values of a chunk per thread
-constexpr int GI_SMALL_K = 22;    // designs of up to this many columns need 256 + 96 threads
-constexpr int GI_SMALL = 256 + GI_PROD;
+constexpr int GI_ENTRY = 256;     // entry threads
+constexpr int GI_CTAS = 3;        // CTAs an SM, by registers
 
 struct ItemPlan {
-  // entries, their threads, rows (even), 2 x 2 blocks, slices, row stride, time
+  // entries, rows (even), 2 x 2 blocks, slices, row stride, time
   // segments, producer warps, log2 of a segment's samples per chunk
-  int E, GT, KR, NB, SL, rs, RP, PW, cs2;
+  int E, KR, NB, SL, rs, RP, PW, cs2;
   int cm, xf, ring, L, Li, rd, lxf, lif, total;  // byte offsets
 };
 
 __host__ __device__ inline ItemPlan item_plan(int T, int K, int n_runs) {
   ItemPlan m;
   m.E = K * (K + 1) / 2;
-  m.GT = (m.E + 31) / 32 * 32;
-  if (m.GT < 256) m.GT = 256;
+  constexpr int GT = GI_ENTRY;
   const int kb = (K + 1) / 2;
   m.KR = 2 * kb;
   m.NB = kb * (kb + 1) / 2;
@@ -1206,9 +1203,9 @@ __host__ __device__ inline ItemPlan item_plan(int T, int K, int n_runs) {
   for (int rp = 2; rp <= n_runs && rp * K <= GI_PROD; ++rp)
     if ((n_runs + rp - 1) / rp < (n_runs + m.RP - 1) / m.RP) m.RP = rp;
   m.cs2 = 3;  // 8 samples, or 16 or 32 while a chunk is at most two values per thread
-  while (m.cs2 < 5 && (K * m.RP << (m.cs2 + 1)) <= 2 * m.GT) ++m.cs2;
+  while (m.cs2 < 5 && (K * m.RP << (m.cs2 + 1)) <= 2 * GT) ++m.cs2;
   const int cs = 1 << m.cs2;
-  while (2 * m.SL * m.NB <= m.GT && m.SL < 16 && m.SL < cs) m.SL *= 2;
+  while (2 * m.SL * m.NB <= GT && m.SL < 16 && m.SL < cs) m.SL *= 2;
   m.rs = cs + (m.SL == 4 ? 2 : m.SL == 8 ? 4 : 1);  // a half-warp's blocks and slices in distinct banks
   m.PW = (K * m.RP + 31) / 32;
   const int K4 = (K + 3) & ~3;
@@ -1238,10 +1235,10 @@ __host__ __device__ inline ItemPlan item_plan(int T, int K, int n_runs) {
 
 // Barrier of the first n threads (a multiple of 32) of the CTA.
 
-template <bool SHARED_LDL, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == GI_SMALL ? 3 : 1) grid_item_kernel(BuildArgs args, int n_designs,
-                                                                                         const double* pair_cm,
-                                                                                         const int* pair_bad) {
+template <bool SHARED_LDL>
+__global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(BuildArgs args, int n_designs,
+                                                                                const double* pair_cm,
+                                                                                const int* pair_bad) {
   const ffs_grid_desc& d = args.d;
   const ffs_grid_out& o = args.o;
   const int T = d.T, K = d.K, LT = ld_t(T), K4 = (K + 3) & ~3, ldx = T | 1;
@@ -1249,7 +1246,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == GI_SMALL ? 3 : 1) grid_ite
   extern __shared__ double2 gi_smem[];
   char* sm = reinterpret_cast<char*>(gi_smem);
   const ItemPlan pl = item_plan(T, K, d.n_runs);
-  const int GT = pl.GT, RP = pl.RP, rs = pl.rs;
+  constexpr int GT = GI_ENTRY;
+  const int RP = pl.RP, rs = pl.rs;
   double* cc = reinterpret_cast<double*>(sm + pl.cm);
   double *cm = cc + T, *cr = cc + 2 * T;
   float4* cfs = reinterpret_cast<float4*>(sm + pl.cm);     // after phase 4: (c, m, 1/D, 1/sqrt(D)) in fp32
@@ -1672,18 +1670,16 @@ __global__ void __launch_bounds__(THREADS, THREADS == GI_SMALL ? 3 : 1) grid_ite
   }
 }
 
-// ------------------------------------------------------------- wide designs
-// Items of more than GI_KMAX columns (single-trial designs), whose series do
-// not fit in shared memory: the series stay in the item's scratch slot (L2),
-// and shared memory holds what the CTA works on: staged samples of the Gram
-// matrix, then the packed K x K factor in FP64, then the fp32 factors that Q and
-// G read. Two CTAs share an SM, so that one's integer Gram matrix runs beside
-// the other's FP64 factorisation.
+// ------------------------------------------------------------- many or wide items
+// The series stay in the item's scratch slot (L2), and shared memory holds what
+// the CTA works on: staged samples of the Gram matrix, then the packed K x K
+// factor in FP64, then the fp32 factors that Q and G read. So several CTAs share
+// an SM, and one's integer Gram matrix runs beside another's FP64 recursions.
 //   - X_w = L^-1 X, a lane per column and run, to fixed point (as above, without
 //     the lo lo' sums: 2^-54 of a product of the columns' largest values, less
 //     than the rounding of the fixed point times their peak-to-rms ratio) and to
-//     fp32; the Gram matrix in blocks of 4 x 4 entries per thread (rows b, b + kb,
-//     b + 2 kb, b + 3 kb, so that a warp's blocks read consecutive rows) from
+//     fp32; the Gram matrix in blocks of 4 x 4 or 2 x 2 entries per thread (rows b,
+//     b + kb, ..., so that a warp's blocks read consecutive rows) from
 //     double-buffered chunks of WI_CS samples.
 //   - X_w'X_w = Lu D Lu' and Lu^-1 in one pass over the packed lower triangle:
 //     step k takes w_r f_c off every entry (r, c) of the rows below k, w_r = A_rk / D_k,
@@ -1693,27 +1689,32 @@ __global__ void __launch_bounds__(THREADS, THREADS == GI_SMALL ? 3 : 1) grid_ite
 //   - Q = X_w Lx^-T and G = U Lx^-1 in fp32, 8 columns x 2 samples per thread.
 // A rank-deficient item or one whose series leave the fixed point goes through
 // item_global, whose general phases these replace: P = 561, T = 600, K = 130 in 3
-// runs: 13.7 -> 3.87 ms. What bounds an item: 0.73 M cycles of integer multiply-adds
-// (Gram) beside 0.57 M cycles of the FP64 pipe (X_w, factor and inverse).
-constexpr int WI_THREADS = 320;
+// runs: 13.7 -> 3.87 ms; 20 designs of T = 855, K = 18: 13.6 -> 4.55 (in shared
+// memory with three CTAs an SM: 8.0). What bounds an item at K = 130: 0.73 M cycles of
+// integer multiply-adds (Gram) beside 0.57 M cycles of the FP64 pipe (X_w, factor
+// and inverse); narrow ones the latency of their phases.
+constexpr int WI_WIDE = 320;     // threads: 2 CTAs an SM, blocks of 4 x 4
+constexpr int WI_NARROW = 128;   // 5 (many designs: 8), blocks of 2 x 2
+constexpr int WI_NARROW_K = 56;
 constexpr int WI_CS = 32;        // samples per chunk
 constexpr int WI_RS = WI_CS + 2; // row stride of a chunk (16-byte words of consecutive rows in distinct banks)
 constexpr int WI_KMAX = 255;     // 8-bit indices of the triangle's table
 
 struct WidePlan {
-  int KP, kb, NB, SL;           // K to a multiple of 8; 4 x 4 blocks a side, blocks, slices of the samples
+  int KP, kb, NB, SL;           // K to a multiple of 8; blocks a side, blocks, slices of the samples
   int tri, fw, dk, scale, total;  // byte offsets (the work area is at 0)
 };
 
-__host__ __device__ inline WidePlan wide_plan(int T, int K) {
+__host__ __device__ inline WidePlan wide_plan(int T, int K, bool shared_ldl, int threads) {
   WidePlan m;
   m.KP = (K + 7) & ~7;
-  m.kb = (K + 3) / 4;
+  const int tb = threads == WI_WIDE ? 4 : 2;  // rows of a block
+  m.kb = (K + tb - 1) / tb;
   m.NB = m.kb * (m.kb + 1) / 2;
   m.SL = 1;
-  while (2 * m.SL * m.NB <= WI_THREADS && m.SL < 8) m.SL *= 2;
-  size_t area = sizeof(double) * 7 * T;  // phase 1
-  const size_t stage = sizeof(int2) * 2 * (size_t)(4 * m.kb) * WI_RS, pack = sizeof(double) * K * (K + 1) / 2,
+  while (2 * m.SL * m.NB <= threads && m.SL < 8) m.SL *= 2;
+  size_t area = sizeof(double) * (shared_ldl ? 3 : 7) * T;  // phase 1
+  const size_t stage = sizeof(int2) * 2 * (size_t)(tb * m.kb) * WI_RS, pack = sizeof(double) * K * (K + 1) / 2,
                f32 = sizeof(float) * (size_t)K * m.KP;
   area = area > stage ? area : stage;
   area = area > pack ? area : pack;
@@ -1745,17 +1746,17 @@ struct FixedDot2 {
   }
 };
 
-template <bool SHARED_LDL>
-__global__ void __launch_bounds__(WI_THREADS, 2) grid_wide_kernel(BuildArgs args, int n_designs, const double* pair_cm,
-                                                                  const int* pair_bad) {
+template <bool SHARED_LDL, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ? 8 : 5)
+    grid_wide_kernel(BuildArgs args, int n_designs, const double* pair_cm, const int* pair_bad) {
   const ffs_grid_desc& d = args.d;
   const ffs_grid_out& o = args.o;
   const int T = d.T, K = d.K, LT = ld_t(T);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  constexpr int nth = WI_THREADS, NW = WI_THREADS / 32;
+  constexpr int nth = THREADS, NW = THREADS / 32, TB = THREADS == WI_WIDE ? 4 : 2;
   extern __shared__ double2 gi_smem[];
   char* sm = reinterpret_cast<char*>(gi_smem);
-  const WidePlan pl = wide_plan(T, K);
+  const WidePlan pl = wide_plan(T, K, SHARED_LDL, THREADS);
   const int KP = pl.KP, kb = pl.kb, SL = pl.SL;
   double* area = reinterpret_cast<double*>(sm);
   uint16_t* tri = reinterpret_cast<uint16_t*>(sm + pl.tri);
@@ -1861,7 +1862,7 @@ __global__ void __launch_bounds__(WI_THREADS, 2) grid_wide_kernel(BuildArgs args
     // ---- 3. X_w'X_w, into XtX and (FP64) the slot's Lx
     if (!left) {
       int2* buf = reinterpret_cast<int2*>(area);
-      const int rows = 4 * kb, nch = (T + WI_CS - 1) / WI_CS;
+      const int rows = TB * kb, nch = (T + WI_CS - 1) / WI_CS;
       auto stage = [&](int c) {
         int2* b = buf + (c & 1) * rows * WI_RS;
         for (int e = tid; e < rows * (WI_CS / 2); e += nth) {
@@ -1879,7 +1880,7 @@ __global__ void __launch_bounds__(WI_THREADS, 2) grid_wide_kernel(BuildArgs args
         const bool on = b < pl.NB * SL;
         int bi = 0, bj = 0;
         if (on) tri_index(b / SL, bi, bj);
-        FixedDot2 acc[4][4];
+        FixedDot2 acc[TB][TB];
         stage(0);
         for (int c = 0; c < nch; ++c) {
           if (c + 1 < nch) {
@@ -1893,14 +1894,14 @@ __global__ void __launch_bounds__(WI_THREADS, 2) grid_wide_kernel(BuildArgs args
             const int4* r0 = reinterpret_cast<const int4*>(buf + (c & 1) * rows * WI_RS);
             const int4 *ri = r0 + bi * (WI_RS / 2), *rj = r0 + bj * (WI_RS / 2);
             for (int h = sl; h < WI_CS / 2; h += SL) {
-              int4 x[4];
+              int4 x[TB];
 #pragma unroll
-              for (int u = 0; u < 4; ++u) x[u] = ri[u * kb * (WI_RS / 2) + h];
+              for (int u = 0; u < TB; ++u) x[u] = ri[u * kb * (WI_RS / 2) + h];
 #pragma unroll
-              for (int v = 0; v < 4; ++v) {
+              for (int v = 0; v < TB; ++v) {
                 const int4 y = rj[v * kb * (WI_RS / 2) + h];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < TB; ++u) {
                   acc[u][v].add(x[u].x, x[u].y, y.x, y.y);
                   acc[u][v].add(x[u].z, x[u].w, y.z, y.w);
                 }
@@ -1910,9 +1911,9 @@ __global__ void __launch_bounds__(WI_THREADS, 2) grid_wide_kernel(BuildArgs args
           __syncthreads();
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < TB; ++u)
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
+          for (int v = 0; v < TB; ++v) {
             FixedDot2& f = acc[u][v];
             for (int m = 1; m < SL; m <<= 1) {
               f.hh += __shfl_xor_sync(0xffffffffu, f.hh, m);
@@ -2185,6 +2186,7 @@ __global__ void __launch_bounds__(WI_THREADS, 2) grid_wide_kernel(BuildArgs args
 // doubles (QR fallback), then K x K doubles when K > DB_SMEM_K.
 
 constexpr int DB_ENTRIES = 32;   // Gram entries per CTA: one warp's lanes
+constexpr int DB_FIXED_K = 40;   // Gram entries in fixed point up to this K (wider: too few of them per staged column)
 constexpr int DB_SMEM_K = 64;    // the factor stays in shared memory up to this K
 constexpr int DB_THREADS = 256;  // the finishing CTA (its MGS fallback's sums depend on it)
 
@@ -2202,7 +2204,7 @@ inline int db_chunk(int T, int K) {
 __global__ void __launch_bounds__(256) design_gram_kernel(int T, int K, int chunk, int fixed,
                                                           const float* __restrict__ Xg, double* __restrict__ gram) {
   extern __shared__ double xt[];  // [ncol][chunk + 1]: the columns this CTA reads (FP64 or fixed point), odd row stride
-  __shared__ int cmax[GI_KMAX + 1];
+  __shared__ int cmax[DB_FIXED_K + 1];
   const int ne = db_entries(K);
   const int e0 = blockIdx.x * DB_ENTRIES;
   const int e1 = min(e0 + DB_ENTRIES, ne);
@@ -2381,8 +2383,7 @@ extern "C" int ffs_design_basis(int T, int K, const float* X, void* work, float*
   const size_t gsm = sizeof(double) * (size_t)(K + 1) * (chunk + 1);
   FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(design_gram_kernel), gsm));
   const int nb = ceil_div(db_entries(K), DB_ENTRIES);
-  // as the grid build forms its Gram matrices at these sizes
-  const int fixed = K <= GI_KMAX && T <= FX_TMAX && item_plan(T, K, 1).total <= 200 * 1024;
+  const int fixed = K <= DB_FIXED_K && T <= FX_TMAX;
   design_gram_kernel<<<nb, 256, gsm, (cudaStream_t)stream>>>(T, K, chunk, fixed, X, gram);
   if (const int rc = check_launch("design_gram_kernel")) return rc;
   const size_t fsm = K <= DB_SMEM_K ? sizeof(double) * 2 * K + sizeof(double) * (size_t)K * K +
@@ -2424,12 +2425,17 @@ static bool too_long(const ffs_grid_desc& d) {
   return sizeof(double) * n > 200 * 1024;
 }
 
-// The item kernel of a build: grid_item_kernel for designs of up to GI_KMAX
-// columns whose items fit in shared memory (half an SM's: two CTAs overlap
-// their latencies; one alone still beats global scratch, so up to 200 KB),
-// grid_wide_kernel for wider ones whose factor does, grid_build_kernel for the
-// rest (more than FX_TMAX samples, whose sums leave the integers' range, and the
-// banded R).
+// The item kernel of a build. grid_item_kernel has the shorter latency and
+// takes the builds of up to GI_KMAX columns whose items run in one wave of its
+// CTAs (two up to 16 columns); grid_wide_kernel does less work on more CTAs and
+// takes the others whose factor fits: with 128 threads while the items
+// outnumber two CTAs an SM and the columns are at most WI_NARROW_K, else with 320.
+// us, grid_item_kernel / 128 / 320 threads: P = 117, T = 331, K = 13: 106 / 120 /
+// 128; P = 231, T = 600, K = 20: 197 / 262 / 239; P = 561, T = 331, K = 13: 140 / 165 /
+// 277; T = 400, K = 20: 307 / 248 / 344; P = 231, K = 32: - / 242 / 215; P = 561,
+// K = 44: - / 502 / 639, K = 64: - / 1300 / 1184; 20 designs of T = 855, K = 18: 8006 /
+// 4545 / 8732. grid_build_kernel takes the rest (more than FX_TMAX samples, whose
+// sums leave the integers' range, and the banded R).
 static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, const double* pair_cm,
                         const int* pair_bad, cudaStream_t st, const char* who) {
   using namespace ffsk;
@@ -2438,22 +2444,31 @@ static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, co
   FFS_REQUIRE(!too_long(d), "%s: T=%d too long", who, d.T);
   FFS_REQUIRE(!o.const_flag == !o.const_coef && (!o.const_flag || (d.p0 >= 0 && d.p0 < d.P)),
               "%s: const_flag and const_coef go together, with p0=%d in [0, P)", who, d.p0);
+  int sms = 0;
+  FFS_CUDA(sm_count(&sms));
+  const long long items = (long long)d.P * n_designs;
+  const bool fixed = d.T <= FX_TMAX && !d.band && (((uintptr_t)o.U_hi | (uintptr_t)o.U_lo) & 3) == 0;
+  const bool narrow = d.K <= WI_NARROW_K && items > 2 * sms;
+  const WidePlan wp = wide_plan(d.T, d.K, pair_cm != nullptr, narrow ? WI_NARROW : WI_WIDE);
+  const bool wide = fixed && d.K <= WI_KMAX && wp.total <= 200 * 1024 && (((uintptr_t)o.U | (uintptr_t)o.G) & 15) == 0;
   const ItemPlan pl = item_plan(d.T, d.K, d.n_runs);
-  if (d.K <= GI_KMAX && d.T <= FX_TMAX && !d.band && pl.total <= 200 * 1024 &&
-      (((uintptr_t)o.U_hi | (uintptr_t)o.U_lo) & 3) == 0) {
-    const bool small = d.K <= GI_SMALL_K;
-    auto kern = pair_cm ? (small ? grid_item_kernel<true, GI_SMALL> : grid_item_kernel<true, 1024>)
-                        : (small ? grid_item_kernel<false, GI_SMALL> : grid_item_kernel<false, 1024>);
-    FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), pl.total));
-    kern<<<grid, pl.GT + 32 * pl.PW, pl.total, st>>>(args, n_designs, pair_cm, pair_bad);
-    return check_launch("grid_item_kernel");
+  if (fixed && d.K <= GI_KMAX && pl.total <= 200 * 1024) {
+    const long long wave = sms * std::min<long long>(GI_CTAS, 225 * 1024 / (pl.total + 2048));
+    if (!wide || items <= (d.K <= 16 ? 2 : 1) * wave) {
+      auto kern = pair_cm ? grid_item_kernel<true> : grid_item_kernel<false>;
+      FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), pl.total));
+      kern<<<grid, GI_ENTRY + 32 * pl.PW, pl.total, st>>>(args, n_designs, pair_cm, pair_bad);
+      return check_launch("grid_item_kernel");
+    }
   }
-  const WidePlan wp = wide_plan(d.T, d.K);
-  if (d.K > GI_KMAX && d.K <= WI_KMAX && d.T <= FX_TMAX && !d.band && wp.total <= 200 * 1024 &&
-      (((uintptr_t)o.U_hi | (uintptr_t)o.U_lo) & 3) == 0 && (((uintptr_t)o.U | (uintptr_t)o.G) & 15) == 0) {
-    auto kern = pair_cm ? grid_wide_kernel<true> : grid_wide_kernel<false>;
+  if (wide) {
+    auto kern = pair_cm ? (narrow ? grid_wide_kernel<true, WI_NARROW> : grid_wide_kernel<true, WI_WIDE>)
+                        : (narrow ? grid_wide_kernel<false, WI_NARROW> : grid_wide_kernel<false, WI_WIDE>);
     FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), wp.total));
-    kern<<<grid, WI_THREADS, wp.total, st>>>(args, n_designs, pair_cm, pair_bad);
+    // no more CTAs than run at once: a slot's series are then still in L2 when its
+    // next item overwrites them (20 designs: 4767 -> 4545 us)
+    if (narrow) grid = std::min(grid, 8 * sms);
+    kern<<<grid, narrow ? WI_NARROW : WI_WIDE, wp.total, st>>>(args, n_designs, pair_cm, pair_bad);
     return check_launch("grid_wide_kernel");
   }
   // phase 1's scratch beside the coefficients while that leaves room for four CTAs an SM
