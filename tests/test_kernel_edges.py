@@ -418,3 +418,42 @@ def test_wide_designs_against_dense_float64(T, K, runs, dup):
         hi, lo = (x.view(f.P, K, -1)[p].view(torch.float16).double() for x in (f.U_hi, f.U_lo))
         back = ((hi + lo) * 2.0 ** -float(f.uexp[p])).cpu().numpy()[:, :T]
         assert np.abs(back - got).max() <= 2.0 ** -20 * np.abs(got).max()
+
+
+@gpu
+@pytest.mark.parametrize("T", [3, 4, 30, 127, 128, 390, 855])
+@pytest.mark.parametrize("V", [1, 33, 300])
+def test_prep_scaling_is_the_correctly_rounded_quotient(T, V):
+    """(y - m) / s without a design, by corrected products where the values
+    are of ordinary size and by divisions elsewhere: the correctly rounded
+    quotient, bit for bit, for samples of any magnitude; and the fp16 split of
+    it (hi the nearest fp16 of y 2^e, lo of the rest), zero past T."""
+    import ctypes as C
+
+    from fastfuncstuff_gb300 import _lib
+
+    rng = np.random.default_rng(T * 1000 + V)
+    y = rng.standard_normal((V, T)) * 10.0 ** rng.uniform(-3, 3, (V, 1))
+    y[rng.random((V, T)) < 0.05] = 0.0
+    y[0, :2] = 1e-25, -3e-22
+    if V > 1:
+        y[1] = 7.25  # a constant series: the floor of the scale
+        y[2 % V] *= 1e18
+    Y = torch.from_numpy(y.astype(np.float32)).to(DEV)
+    ld = (T + 7) // 8 * 8
+    scale = torch.empty(V, device=DEV)
+    rows = torch.empty(V, T, device=DEV)
+    hi, lo = (torch.full((V, ld), 77, dtype=torch.int16, device=DEV) for _ in range(2))
+    yexp = torch.empty(V, dtype=torch.int32, device=DEV)
+    a = _lib.PrepArgs(V=V, T=T, K=0, Y=Y.data_ptr(), do_scale=1, center=0, ld_y=ld, scale=scale.data_ptr(),
+                      yr_hi=hi.data_ptr(), yr_lo=lo.data_ptr(), yexp=yexp.data_ptr(), yr_rows=rows.data_ptr())
+    _lib.check(_lib.load().ffs_reml_prep(C.byref(a), torch.cuda.current_stream().cuda_stream), "ffs_reml_prep")
+    torch.cuda.synchronize()
+    want = Y.cpu().numpy() / scale.cpu().numpy()[:, None]
+    assert np.array_equal(rows.cpu().numpy(), want)
+    x = np.ldexp(want.astype(np.float64), yexp.cpu().numpy()[:, None]).astype(np.float32)
+    h = x.astype(np.float16)
+    low = (x - h.astype(np.float32)).astype(np.float16)
+    assert np.array_equal(hi.view(torch.float16).cpu().numpy()[:, :T], h)
+    assert np.array_equal(lo.view(torch.float16).cpu().numpy()[:, :T], low)
+    assert (hi[:, T:] == 0).all() and (lo[:, T:] == 0).all()
