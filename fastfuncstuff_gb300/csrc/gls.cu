@@ -103,6 +103,50 @@ __device__ __forceinline__ void band_whiten(const ffs_gls_args& a, int p, const 
   band_whiten_rows(a.band_coef + (size_t)p * T * a.band_w, a.band_w, a.band[p], r, w, T);
 }
 
+// The same for a tile's 32 rows (in place, row stride ld), and ssw[l] = sum of
+// squares of row l: 8 lanes per row take the band's lags in turn (NI of them
+// each, bw <= 8 NI) and sum their shares by shuffles, the coefficients of the
+// next step loaded a step ahead. One lane per row over all lags waited for
+// every 8 lags' loads (6,000 voxels, T = 240, bands of up to 42: the kernel
+// 200 -> 83 us).
+template <int NI>
+__device__ __noinline__ void band_whiten_tile(const float* __restrict__ cb, int W, int bw, float* Ys, int ld, int T,
+                                              float* ssw) {
+  const int lane = threadIdx.x & 31, l = 4 * (threadIdx.x >> 5) + (lane >> 3), r = lane & 7;
+  float* row = Ys + (size_t)l * ld;
+  float next[NI], c0n = 0.f, ss = 0.f;
+  auto load = [&](int t) {
+    const float* c = cb + (size_t)t * W;
+    c0n = t < T ? c[0] : 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int j = r + 1 + 8 * i;
+      next[i] = t < T && j <= bw && j <= t ? c[j] : 0.f;
+    }
+  };
+  load(0);
+  for (int t = 0; t < T; ++t) {
+    float k[NI];
+    const float c0 = c0n;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) k[i] = next[i];
+    load(t + 1);
+    float acc = r == 0 ? row[t] * c0 : 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int j = r + 1 + 8 * i;
+      if (8 * i >= bw) break;
+      if (j <= bw && j <= t) acc = fmaf(-k[i], row[t - j], acc);
+    }
+    for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    __syncwarp();
+    if (r == 0) row[t] = acc;
+    ss = fmaf(acc, acc, ss);
+    __syncwarp();
+  }
+  if (r == 0) ssw[l] = ss;
+}
+
 // GLS of one voxel v at pair g, executed by one warp. Gp = G of pair g and Xt
 // (the transposed design) may live in shared or global memory; ys, r, beta and
 // bins are this warp's shared scratch.
@@ -664,18 +708,28 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
   float4* rr = reinterpret_cast<float4*>(Ys + (size_t)lane * ld);
 
   if (a.band_coef) {
-    // the banded R's whitening: one lane per voxel over the whole series, in
-    // place, and the sums of squares
-    if (wid == 0) {
-      float* row = Ys + (size_t)lane * ld;
+    // the banded R's whitening, in place, and the sums of squares
+#pragma unroll
+    for (int i = 0; i < TILE_SUB_VB; ++i) {
+      const int l = TILE_SUB_VB * wid + i;
+      const float4* r4 = reinterpret_cast<const float4*>(Ys + (size_t)l * ld);
       float ssr = 0.f;
-      for (int t = 0; t < T; ++t) ssr = fmaf(row[t], row[t], ssr);
-      st[3 * TILE_V + lane] = ssr;
-      band_whiten(a, pair_of(a, g), row, row, T);
-      float ssw = 0.f;
-      for (int t = 0; t < T; ++t) ssw = fmaf(row[t], row[t], ssw);
-      st[5 * TILE_V + lane] = ssw;
+      for (int q = lane; q < nq; q += 32) {
+        const float4 r = r4[q];
+        ssr = fmaf(r.w, r.w, fmaf(r.z, r.z, fmaf(r.y, r.y, fmaf(r.x, r.x, ssr))));
+      }
+      ssr = warp_sum(ssr);
+      if (lane == 0) st[3 * TILE_V + l] = ssr;
     }
+    __syncthreads();
+    const int p = pair_of(a, g), bw = a.band[p];
+    const float* cb = a.band_coef + (size_t)p * T * a.band_w;
+    if (bw <= 16)
+      band_whiten_tile<2>(cb, a.band_w, bw, Ys, ld, T, st + 5 * TILE_V);
+    else if (bw <= 48)
+      band_whiten_tile<6>(cb, a.band_w, bw, Ys, ld, T, st + 5 * TILE_V);
+    else
+      band_whiten_tile<16>(cb, a.band_w, bw, Ys, ld, T, st + 5 * TILE_V);
     __syncthreads();
   } else {
   // whitened residual by segments of the time axis
@@ -685,7 +739,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
   float rp = s0 > 0 ? Ys[(size_t)lane * ld + s0 - 1] : 0.f;
   __syncthreads();
   {
-    float vp = 0.f, H = 1.f, ssr = 0.f;
+    float vp = 0.f, H = 1.f, ssr[4] = {0.f, 0.f, 0.f, 0.f};  // short chains
     for (int t = s0; t < s1; t += 4) {
       const float4 r = rr[t >> 2];
       const float rv[4] = {r.x, r.y, r.z, r.w};
@@ -700,24 +754,25 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) gls_tile_kernel
           rp = rv[k];
           vp = vt;
           H *= -q.y;
-          ssr = fmaf(rv[k], rv[k], ssr);
+          ssr[k] = fmaf(rv[k], rv[k], ssr[k]);
         }
       }
       rr[t >> 2] = make_float4(o[0], o[1], o[2], o[3]);
     }
     vend[wid * TILE_V + lane] = vp;
-    red[wid * TILE_V + lane] = ssr;
+    red[wid * TILE_V + lane] = (ssr[0] + ssr[1]) + (ssr[2] + ssr[3]);
     if (lane == 0) Hs[wid] = H;
   }
   __syncthreads();
   if (wid == 0) {
-    float vin = 0.f, ssr = 0.f;
+    float vin = 0.f, ssr[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
     for (int k = 0; k < TILE_WARPS; ++k) {
       carry[k * TILE_V + lane] = vin;
       vin = fmaf(Hs[k], vin, vend[k * TILE_V + lane]);
-      ssr += red[k * TILE_V + lane];
+      ssr[k >> 1] += red[k * TILE_V + lane];
     }
-    st[3 * TILE_V + lane] = ssr;
+    st[3 * TILE_V + lane] = (ssr[0] + ssr[1]) + (ssr[2] + ssr[3]);
   }
   __syncthreads();
   {

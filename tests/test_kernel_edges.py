@@ -457,3 +457,35 @@ def test_prep_scaling_is_the_correctly_rounded_quotient(T, V):
     assert np.array_equal(hi.view(torch.float16).cpu().numpy()[:, :T], h)
     assert np.array_equal(lo.view(torch.float16).cpu().numpy()[:, :T], low)
     assert (hi[:, T:] == 0).all() and (lo[:, T:] == 0).all()
+
+
+@gpu
+@pytest.mark.parametrize("a_max,corcut,lags", [(0.3, 1e-2, 16), (0.8, 1e-4, 48), (0.8, 1e-12, 127)])
+def test_banded_gls_whitening_against_dense_float64(a_max, corcut, lags):
+    """sigma^2 of the GLS under AFNI's banded R, its tile whitened by 8 lanes a
+    row over up to 16, 48 or 127 lags, against the dense FP64 whitening of the
+    same fit's residual (fp32 residuals and sums of T squares: 1e-4)."""
+    from fastfuncstuff_gb300.glm.arma import fit_glm_arma11
+
+    V, T, K = 70, 131, 4
+    Y, X, starts = arma_data(11, V, T, K, runs=2)
+    grids = torch.linspace(0.0, a_max, 4), torch.linspace(-0.4, 0.4, 5)
+    G.set_afni_mode(True, corcut)
+    try:
+        g = G.make_grid(*grids)
+        r = fit_glm_arma11(torch.from_numpy(Y), torch.from_numpy(X), 2.0, *grids, run_starts=starts, device="cuda",
+                           verbose=False)
+    finally:
+        G.set_afni_mode(False)
+    assert lags // 3 < g.band.max() <= lags or lags == 16
+    run_of = np.searchsorted(starts, np.arange(T), side="right")
+    gap = np.abs(np.arange(T)[:, None] - np.arange(T)[None, :])
+    band = {(np.float32(a), np.float32(b)): int(w) for a, b, w in zip(g.a, g.b, g.band)}
+    betas, sigma2 = r.betas.numpy().astype(np.float64), r.sigma2.numpy()
+    for v in range(V):
+        a, b = (np.float32(x) for x in r.arma_params[v].numpy())
+        bw, a, b = band[a, b], float(a), float(b)
+        lam = (b + a) * (1 + a * b) / (1 + 2 * a * b + b * b)
+        R = np.where((gap > 0) & (gap <= bw) & (run_of[:, None] == run_of[None, :]), lam * a ** np.maximum(gap - 1, 0), 0.0)
+        w = np.linalg.solve(np.linalg.cholesky(R + np.eye(T)), Y[v] - X.astype(np.float64) @ betas[v])
+        assert abs(float(sigma2[v]) - (w @ w) / (T - K)) <= 1e-4 * (w @ w) / (T - K)
