@@ -257,13 +257,21 @@ def _roofline(dom: str, ms_step: float, T: int, K: int, P: int, pk: dict, sm_mhz
                 "frac": ach / fp32_peak, "traffic": None, "peak_src": "152 SMs x 128 FMA/clk at the sampled clock",
                 "work": "G'y, X b0 and G'r (3 K x T products) and the whitening recurrence per voxel"}
     if dom in ("ffs_grid_build", "ffs_grid_build_designs"):
-        # FP64: the whitened design (2 T K) and its Gram matrix (T K (K + 1)) per (design, pair)
+        # FP64 per (design, pair): the whitened design (3 operations a sample) and X_w'X_w's factor with its
+        # inverse (K^3 / 3 FMAs); the Gram matrix runs on the integer pipe
         items = P * work.get("designs", 1)
-        flops = items * (2.0 * T * K * (K + 1) + 4.0 * T * K)
+        flops = items * (6.0 * T * K + 2.0 * K ** 3 / 3.0)
         ach = flops / sec / 1e12
         return {"kernel": dom, "bound": "fp64", "achieved": ach, "peak": 1.25, "unit": "TFLOP/s",
                 "frac": ach / 1.25, "traffic": None, "peak_src": "nominal GB300 FP64 (not measured)",
-                "work": "FP64 X_w = L^-1 X and X_w'X_w per (design, pair)"}
+                "work": "FP64 X_w = L^-1 X, factor and inverse of X_w'X_w per (design, pair)"}
+    if dom == "ffs_reml_descent":
+        # the pairs the selector reads on the 33 x 33 lattice: 9 of the top level, 8 more in each of 4 rounds
+        flops = V * 41 * (4.0 * T + 2.0 * K * T)
+        ach = flops / sec / 1e12
+        return {"kernel": dom, "bound": "fp32", "achieved": ach, "peak": fp32_peak, "unit": "TFLOP/s",
+                "frac": ach / fp32_peak, "traffic": None, "peak_src": "152 SMs x 128 FMA/clk at the sampled clock",
+                "work": "recurrence and projection (tcgen05) of the pairs the hierarchical selector reads"}
     # the rest stream HBM (prep: Y in; rows/time-major and the fp16 split out)
     ld = (T + 63) // 64 * 64
     byts = V * (T * 4 + T * 4 + 2 * ld * 2 + 16)

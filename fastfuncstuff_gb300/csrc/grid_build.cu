@@ -2177,12 +2177,11 @@ __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ?
 }
 
 // ---- Design basis: Q0 = X Lx^-T, Lx the FP64 Cholesky factor of X'X (Q0 is
-// U of the pair (0, 0), where R = I and X_w = X, and comes out bit for bit
-// equal to the grid build's: the same Dot4 entries, block_cholesky and fp32
-// recursion), and the centring test c = (X'X)^-1 X'1. Two launches: the Gram
-// entries of [X | 1] spread over CTAs (each entry a chain of FP64 FMAs whose
-// latency, not the FP64 rate, bounds it), then one CTA for the factor, Q0 and
-// c. work: [NE] Gram entries of [X | 1] (packed lower triangle), [K][T]
+// U of the pair (0, 0), where R = I and X_w = X: the grid build's to the rounding
+// of FP64, so of its fp32 form almost always the same bits), and the centring
+// test c = (X'X)^-1 X'1. Two launches: the Gram entries of [X | 1] spread over
+// CTAs (in fixed point up to DB_FIXED_K columns, else each a chain of FP64 FMAs
+// whose latency bounds it), then one CTA for the factor, Q0 and c. work: [NE] Gram entries of [X | 1] (packed lower triangle), [K][T]
 // doubles (QR fallback), then K x K doubles when K > DB_SMEM_K.
 
 constexpr int DB_ENTRIES = 32;   // Gram entries per CTA: one warp's lanes
