@@ -289,7 +289,11 @@ struct TopArgs {
   float* best_crit;
 };
 
-__global__ void __launch_bounds__(TOP_ROWS * TOP_GROUPS, 1) descent_top_kernel(TopArgs a) {
+// At most 80 registers: with the 118 that the compiler takes by itself one CTA
+// of 384 threads fills an SM, and its 12 warps waited at each block's barrier
+// (ncu: 46% of the issue slots); two run at 80, without spills. 200,000 voxels of T
+// = 400: 871 -> 626 us, 100,000 of T = 855: 1284 -> 950 (64 registers: 654, 1001).
+__global__ void __maxnreg__(80) descent_top_kernel(TopArgs a) {
   extern __shared__ float4 dsm4[];
   __shared__ int rows[TOP_ROWS];
   __shared__ float dc[TOP_GROUPS * D_SLOTS], rss0_s[TOP_ROWS];
