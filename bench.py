@@ -267,11 +267,12 @@ def _roofline(dom: str, ms_step: float, T: int, K: int, P: int, pk: dict, sm_mhz
                 "work": "FP64 X_w = L^-1 X, factor and inverse of X_w'X_w per (design, pair)"}
     if dom == "ffs_reml_descent":
         # the pairs the selector reads on the 33 x 33 lattice: 9 of the top level, 8 more in each of 4 rounds
-        flops = V * 41 * (4.0 * T + 2.0 * K * T)
+        flops = V * 41 * 4.0 * T
         ach = flops / sec / 1e12
         return {"kernel": dom, "bound": "fp32", "achieved": ach, "peak": fp32_peak, "unit": "TFLOP/s",
                 "frac": ach / fp32_peak, "traffic": None, "peak_src": "152 SMs x 128 FMA/clk at the sampled clock",
-                "work": "recurrence and projection (tcgen05) of the pairs the hierarchical selector reads"}
+                "work": "2 FMA per (voxel, pair, time point) for the pairs the hierarchical selector reads; their "
+                        "projections run on the tensor cores in the same call"}
     # the rest stream HBM (prep: Y in; rows/time-major and the fp16 split out)
     ld = (T + 63) // 64 * 64
     byts = V * (T * 4 + T * 4 + 2 * ld * 2 + 16)
