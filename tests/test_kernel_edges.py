@@ -489,3 +489,43 @@ def test_banded_gls_whitening_against_dense_float64(a_max, corcut, lags):
         R = np.where((gap > 0) & (gap <= bw) & (run_of[:, None] == run_of[None, :]), lam * a ** np.maximum(gap - 1, 0), 0.0)
         w = np.linalg.solve(np.linalg.cholesky(R + np.eye(T)), Y[v] - X.astype(np.float64) @ betas[v])
         assert abs(float(sigma2[v]) - (w @ w) / (T - K)) <= 1e-4 * (w @ w) / (T - K)
+
+
+@gpu
+@pytest.mark.parametrize("T,K,runs,D", [(150, 20, 1, 1), (203, 23, 3, 1), (301, 56, 2, 1), (130, 9, 2, 4), (199, 18, 3, 3)])
+def test_many_items_builds_against_dense_float64(T, K, runs, D):
+    """Builds of more items than the latency kernel takes (33 x 33 lattice, one
+    design or several): logdet, diag((X'R^-1X)^-1), U and G of some pairs
+    against dense FP64, to the bounds of the wide designs' test."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(T + K)
+    X = rng.standard_normal((D, T, K)).astype(np.float32)
+    X[:, :, 0] = 1.0
+    starts = [T * r // runs for r in range(runs)]
+    ax = torch.linspace(-0.8, 0.8, 33)
+    g = G.make_grid(ax, ax, use_double=True)
+    Xd = torch.from_numpy(X if D > 1 else X[0]).to(DEV)
+    f = engine.build_factors(Xd, g, G.run_layout(T, starts), with_tc=True)
+    torch.cuda.synchronize()
+    assert (f.info.cpu().numpy() == 0).all()
+    run_of = np.searchsorted(starts, np.arange(T), side="right")
+    gap = np.abs(np.arange(T)[:, None] - np.arange(T)[None, :])
+    same = (gap > 0) & (run_of[:, None] == run_of[None, :])
+    for dsg in range(D):
+        for p in range(5, g.P, 90):
+            a, b = float(np.float32(g.a[p])), float(np.float32(g.b[p]))
+            lam = (b + a) * (1 + a * b) / (1 + 2 * a * b + b * b)
+            R = np.where(same, lam * a ** np.maximum(gap - 1, 0), 0.0) + np.eye(T)
+            Li = np.linalg.inv(np.linalg.cholesky(R))
+            Xw = Li @ X[dsg].astype(np.float64)
+            C = np.linalg.cholesky(Xw.T @ Xw)
+            Ci = np.linalg.inv(C)
+            U = (Ci @ Xw.T) @ Li
+            tol = K * 2.0 ** -24 * max(30.0, np.linalg.cond(Xw))
+            pd = dsg * g.P + p
+            np.testing.assert_allclose(float(f.logdet_XtX[pd]), 2 * np.log(np.diag(C) + 1e-10).sum(), rtol=1e-9, atol=1e-9)
+            np.testing.assert_allclose(f.Adiag[pd].cpu().numpy(), np.diag(Ci.T @ Ci), rtol=1e-6)
+            assert np.abs(f.U[pd, :, :T].cpu().numpy() - U).max() <= tol * np.abs(U).max()
+            Gm = Ci.T @ U
+            assert np.abs(f.G[pd, :, :T].cpu().numpy() - Gm).max() <= tol * np.abs(Gm).max()
