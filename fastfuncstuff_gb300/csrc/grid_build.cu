@@ -724,7 +724,8 @@ __global__ void __launch_bounds__(GB_THREADS) pair_ldl_kernel(BuildArgs args, do
 // The centring test of a design at its identity pair, where X_w = X: c =
 // (X'X)^-1 X'1 from the inverse factor Li (row stride ldi), accepted when
 // ||X c - 1||^2 <= 1e-12 T; *const_flag stays 1 only if every design passes.
-// w: 2 K doubles of scratch. Ends with a barrier.
+// w: 2 K doubles of scratch (a slot's A, whose K x K doubles the S of the same
+// size follows: S alone is too short at K = 1). Ends with a barrier.
 __device__ void const_of_design(const ffs_grid_desc& d, const ffs_grid_out& o, int dsg, const float* Xd,
                                 const double* Li, int ldi, bool chol, double* w, double* red) {
   const int T = d.T, K = d.K;
@@ -1035,7 +1036,7 @@ __device__ __noinline__ void item_global(const BuildArgs& args, const PairScratc
   }
   __syncthreads();
 
-  if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, s.Li, K, chol, s.S, red);
+  if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, s.Li, K, chol, s.A, red);
 
   // ---- 8. G = U Lx^-1 in fp32 (row t of G solves g Lx = u_t); Gsum = G' 1
   // accumulated in FP64
@@ -2145,7 +2146,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ?
         }
       }
     }
-    if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, s.Li, K, true, s.S, red);
+    if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, s.Li, K, true, s.A, red);
 
     // ---- 8. G = U Lx^-1 in fp32
     for (int t2 = tid; t2 < LT / 2; t2 += nth) {
