@@ -1734,6 +1734,12 @@ __host__ __device__ inline WidePlan wide_plan(int T, int K, bool shared_ldl, int
   return m;
 }
 
+// The series of an item, rows of LT samples in fixed point (8 bytes) and fp32 (4)
+// from a 16-byte boundary, lie in the slot's X_w and Q (16 bytes a sample in rows
+// of T, 8-byte aligned): too long for them at T = 1, 2, 3, 5, 6 and 9, which the
+// item kernel takes.
+__host__ __device__ inline bool wide_slot_fits(int T) { return 3 * ld_t(T) + 2 <= 4 * T; }
+
 // hh and x of FixedDot
 struct FixedDot2 {
   long long hh = 0, x = 0;
@@ -2450,7 +2456,8 @@ static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, co
   const bool fixed = d.T <= FX_TMAX && !d.band && (((uintptr_t)o.U_hi | (uintptr_t)o.U_lo) & 3) == 0;
   const bool narrow = d.K <= WI_NARROW_K && items > 2 * sms;
   const WidePlan wp = wide_plan(d.T, d.K, pair_cm != nullptr, narrow ? WI_NARROW : WI_WIDE);
-  const bool wide = fixed && d.K <= WI_KMAX && wp.total <= 200 * 1024 && (((uintptr_t)o.U | (uintptr_t)o.G) & 15) == 0;
+  const bool wide = fixed && d.K <= WI_KMAX && wide_slot_fits(d.T) && wp.total <= 200 * 1024 &&
+                    (((uintptr_t)o.U | (uintptr_t)o.G) & 15) == 0;
   const ItemPlan pl = item_plan(d.T, d.K, d.n_runs);
   if (fixed && d.K <= GI_KMAX && pl.total <= 200 * 1024) {
     const long long wave = sms * std::min<long long>(GI_CTAS, 225 * 1024 / (pl.total + 2048));

@@ -73,3 +73,24 @@ def test_centring_test_of_one_column_stays_in_its_scratch(T, banded, monkeypatch
     p = g.p0 + 1
     assert int(f.info.abs().sum()) == 0
     check_pair(f, p, p, X, starts, 1e-5, int(g.band[p]) if banded else None)
+
+
+@gpu
+@pytest.mark.parametrize("T,K,runs,D", [(2, 1, 1, 3), (5, 2, 1, 2), (5, 4, 1, 3), (6, 3, 2, 2), (9, 5, 2, 2), (10, 4, 1, 2)])
+def test_many_short_series_against_dense_float64(T, K, runs, D):
+    """More items than two waves of series of a few samples, rows padded to a
+    multiple of 4 wider than the series. Designs of condition below 30 (fp32
+    sums of up to K terms: K 2^-24 30, at least 1e-5)."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(10 * T + K)
+    X = np.stack([np.linalg.qr(rng.standard_normal((T, K)))[0] + 0.05 * d for d in range(D)]).astype(np.float32)
+    starts = [T * r // runs for r in range(runs)]
+    ax = torch.linspace(-0.8, 0.8, 33)
+    g = G.make_grid(ax, ax, use_double=True)
+    f = engine.build_factors(torch.from_numpy(X).to(DEV), g, G.run_layout(T, starts), with_tc=True)
+    torch.cuda.synchronize()
+    assert (f.info.cpu().numpy() == 0).all()
+    for d in range(D):
+        for p in range(3, g.P, 50):
+            check_pair(f, p, d * g.P + p, X[d], starts, max(1e-5, K * 2.0**-24 * 30))
