@@ -233,9 +233,11 @@ __device__ __forceinline__ double rcp_newton(double n) {
 // The filter's entries before it and the reciprocals, square roots and outputs
 // after it are formed for every sample in parallel, and log|R| = 2 sum log(sqrt(D_t) + 1e-10) telescopes to the
 // log of each run's last minor + 2e-10 sum 1/sqrt(D_t) (the next term is 1e-20).
+// A minor is a product of the pivots, down to 1e-4 each for (a, b) near 1, so the
+// products and the walks over them carry a power of two beside them.
 // cc[t], cm[t], cr[t] = c, m, 1/sqrt(D); coef[p], logdet_R[p] written; tmp holds
-// 4 T doubles. *bad_r = 1 if a pivot D_t was not positive (it is replaced by 1).
-// Ends with a barrier.
+// 4 T doubles. A run with a pivot D_t that is not positive goes through the
+// recurrence of D instead, which replaces it by 1 and sets *bad_r. Ends with a barrier.
 __device__ void ldl_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p, double* cc, double* cm, double* cr,
                             double* tmp, double* red, int* bad_r) {
   const int T = d.T;
@@ -331,18 +333,39 @@ __device__ void ldl_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p
       n1 = n0 = 1.0;
       e2 = 0;
     }
+    bool bad = false;
     for (int t = s0; t < s1; ++t) {
-      double n = fma(diag[t], n1, -(off2[t] * n0));
-      if (__double2hiint(n) <= 0) {  // not positive (NaN is caught by the Cholesky of X_w'X_w)
-        *bad_r = 1;
-        n = n1;
-      }
+      const double n = fma(diag[t], n1, -(off2[t] * n0));
       num[t] = n;
       prev[t] = n1;
+      const int hi = __double2hiint(n);
+      bad = bad || hi <= 0 || hi >= 0x7ff00000;  // not positive, or not finite
       n0 = n1;
       n1 = n;
+      const int e = (hi >> 20) - 1023;
+      if (((t - s0) & 7) == 7 && !bad && (e > 64 || e < -64)) {
+        const double sc = __hiloint2double((1023 - e) << 20, 0);
+        n0 *= sc;
+        n1 *= sc;
+        e2 += e;
+      }
     }
-    if (s1 == t1 && s0 < s1) ld += log(n1) + (double)e2 * 0.693147180559945309417;
+    __syncwarp();  // a walk by lane 0 rewrites num and prev
+    if (!__any_sync(0xffffffffu, bad)) {
+      if (s1 == t1 && s0 < s1) ld += log(n1) + (double)e2 * 0.693147180559945309417;
+    } else if (lane == 0) {  // R is singular or not a correlation
+      double D = 1.0;
+      for (int t = t0; t < t1; ++t) {
+        D = diag[t] - off2[t] / D;
+        if (!(D > 0.0)) {
+          *bad_r = 1;
+          D = 1.0;
+        }
+        num[t] = D;
+        prev[t] = 1.0;
+        ld += log(D);
+      }
+    }
   }
   __syncthreads();
   double rsum = 0.0;

@@ -3,6 +3,8 @@ singular correlations, designs the fixed point cannot hold, many designs."""
 
 from __future__ import annotations
 
+import copy
+
 import numpy as np
 import pytest
 import torch
@@ -94,3 +96,68 @@ def test_many_short_series_against_dense_float64(T, K, runs, D):
     for d in range(D):
         for p in range(3, g.P, 50):
             check_pair(f, p, d * g.P + p, X[d], starts, max(1e-5, K * 2.0**-24 * 30))
+
+
+def pivots(a, b, starts, T):
+    """(D, m, c) of every sample by the recurrence of D in extended precision; D = 1 where it is not positive."""
+    a, b = np.longdouble(np.float32(a)), np.longdouble(np.float32(b))
+    lam = (b + a) * (1 + a * b) / (1 + 2 * a * b + b * b)
+    D, m, c = np.ones(T, np.longdouble), np.zeros(T, np.longdouble), np.zeros(T, np.longdouble)
+    for t in range(T):
+        if t not in starts and lam != 0:
+            off, c[t] = lam - a, a
+            m[t] = off / D[t - 1]
+            D[t] = 1 + a * a - 2 * a * lam - m[t] * off
+            D[t] = D[t] if D[t] > 0 else 1
+    return D, m, c
+
+
+@gpu
+@pytest.mark.parametrize("T,runs,K", [(1024, 1, 4), (1500, 1, 1), (4500, 1, 3), (6400, 1, 1), (6400, 2, 2), (1024, 1, 40)])
+def test_long_runs_near_unit_roots(T, runs, K):
+    """The LDL' of R where the leading minors leave FP64's range (0.005 a sample
+    at (0.99, 0.99)), against the recurrence of D: D to 1e-11 (a rounding of
+    the three-term recurrence is amplified by up to 1 / min D), m = off / D
+    relative to the largest |m| likewise, then one rounding to fp32."""
+    from fastfuncstuff_gb300.glm import engine
+
+    X = np.random.default_rng(T).standard_normal((T, K)).astype(np.float32)
+    starts = [T * r // runs for r in range(runs)]
+    a, b = np.array([0.0, 0.95, 0.99, 0.99, -0.9, 0.999]), np.array([0.0, 0.95, 0.99, -0.5, -0.9, 0.999])
+    ok = (a + b >= 0)
+    g = G.grid_of_pairs(a[ok], b[ok], use_double=True)
+    f = engine.build_factors(torch.from_numpy(X).to(DEV), g, G.run_layout(T, starts), with_tc=True)
+    torch.cuda.synchronize()
+    assert int(f.info.abs().sum()) == 0
+    coef = f.coef.cpu().numpy().astype(np.float64)
+    for p in range(g.P):
+        D, m, c = (x.astype(np.float64) for x in pivots(g.a[p], g.b[p], starts, T))
+        tol = 1e-11 + 2.0**-24
+        for k, want in enumerate((c, m, 1 / D, 1 / np.sqrt(D))):
+            assert np.abs(coef[p, :, k] - want).max() <= tol * np.abs(want).max(), (p, k)
+        assert float(f.logdet_R[p]) == pytest.approx(2 * np.log(np.sqrt(D) + 1e-10).sum(), rel=1e-11, abs=1e-9)
+
+
+@gpu
+@pytest.mark.parametrize("T,K,D", [(200, 3, 1), (200, 30, 1), (1500, 2, 1), (200, 3, 12)])
+def test_singular_correlation_replaces_its_pivots(T, K, D):
+    """a = 1: R is all ones, every pivot after a run's first is zero and is
+    replaced by 1 (info 2), so logdet R is that of the identity; the other
+    pairs have theirs. The item kernel, the wide one and the general one, and
+    many designs."""
+    from fastfuncstuff_gb300.glm import engine
+
+    X = np.random.default_rng(T).standard_normal((D, T, K)).astype(np.float32)
+    starts = [0, T // 2]
+    g = copy.deepcopy(G.make_grid(torch.tensor([0.0, 0.5, 0.7]), torch.tensor([0.0, 0.5]), use_double=True))
+    g.a[g.a == np.float32(0.7)] = 1.0
+    f = engine.build_factors(torch.from_numpy(X if D > 1 else X[0]).to(DEV), g, G.run_layout(T, starts), with_tc=True)
+    torch.cuda.synchronize()
+    info, coef = f.info.cpu().numpy().reshape(D, g.P), f.coef.cpu().numpy()
+    one = g.a == 1.0
+    assert one.any() and (info[:, one] == 2).all() and (info[:, ~one] == 0).all()
+    for p in range(g.P):
+        Dp, m, c = (x.astype(np.float64) for x in pivots(g.a[p], g.b[p], starts, T))
+        want = np.stack([c, m, 1 / Dp, 1 / np.sqrt(Dp)], 1)
+        assert np.abs(coef[p] - want).max() <= 1e-6 * np.abs(want).max()
+        assert float(f.logdet_R[p]) == pytest.approx(2 * np.log(np.sqrt(Dp) + 1e-10).sum(), rel=1e-11, abs=1e-9)
