@@ -1139,14 +1139,16 @@ __device__ __forceinline__ int fixed_scale(float mx) {
   return mx > 0.f ? 53 - e : 0;
 }
 
-// (hi, lo) of w 2^s rounded to an integer; over = true when it does not fit
+// (hi, lo) of w 2^s rounded to an integer; over = true when that is 2^(53 + SHIFT)
+// or more in magnitude (with SHIFT = 5, |hi| may be 2^31, for the caller to refuse)
+template <int SHIFT>
 __device__ __forceinline__ int2 fixed_of(double w, int s, bool& over) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(w);
   const int ex = (int)(b >> 52) & 0x7ff;
-  const int r = 1075 - ex - s;  // |w| 2^s = mantissa 2^-r
+  const int r = 1075 + SHIFT - ex - s;  // |w| 2^s = mantissa 2^(SHIFT - r)
   over = over || (r < 0 && ex != 0);
   unsigned long long m = ((b << 1) & 0x1ffffffffffffeull) | 0x20000000000000ull;
-  m = (ex == 0 || r > 54) ? 0ull : ((m >> max(r, 0)) + 1) >> 1;
+  m = (ex == 0 || r > 54 + SHIFT) ? 0ull : (((m << SHIFT) >> max(r, 0)) + 1) >> 1;
   const long long q = (long long)b < 0 ? -(long long)m : (long long)m;
   const int hi = (int)((q + (1 << 26)) >> 27);
   return make_int2(hi, (int)(q - ((long long)hi << 27)));
@@ -1386,7 +1388,7 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
                 int2 f = make_int2(0, 0);
                 if (t < ve[i]) {
                   const double w = reinterpret_cast<double*>(wb)[vs[i]] * cr[t];
-                  f = fixed_of(w, scale[vj[i]], over);
+                  f = fixed_of<0>(w, scale[vj[i]], over);
                   xf[(size_t)vj[i] * ldx + t] = d2f_exact(w);
                 }
                 wb[vs[i]] = f;
@@ -1699,10 +1701,8 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
 // the CTA works on: staged samples of the Gram matrix, then the packed K x K
 // factor in FP64, then the fp32 factors that Q and G read. So several CTAs share
 // an SM, and one's integer Gram matrix runs beside another's FP64 recursions.
-//   - X_w = L^-1 X, a lane per column and run, to fixed point (as above, without
-//     the lo lo' sums: 2^-54 of a product of the columns' largest values, less
-//     than the rounding of the fixed point times their peak-to-rms ratio) and to
-//     fp32; the Gram matrix in blocks of 4 x 4 or 2 x 2 entries per thread (rows b,
+//   - X_w = L^-1 X, a lane per column and run, to fixed point (scaled by the columns'
+//     norms, without the lo lo' sums: norm_scale) and to fp32; the Gram matrix in blocks of 4 x 4 or 2 x 2 entries per thread (rows b,
 //     b + kb, ..., so that a warp's blocks read consecutive rows) from
 //     double-buffered chunks of WI_CS samples.
 //   - X_w'X_w = Lu D Lu' and Lu^-1 in one pass over the packed lower triangle:
@@ -1752,7 +1752,7 @@ __host__ __device__ inline WidePlan wide_plan(int T, int K, bool shared_ldl, int
   m.tri = take(sizeof(uint16_t) * (size_t)K * (K + 1) / 2);
   m.fw = take(sizeof(double) * 4 * K);  // f and w, double-buffered
   m.dk = take(sizeof(double) * 2 * K);  // D, 1 / sqrt(D)
-  m.scale = take(sizeof(int) * 2 * K);  // the columns' largest magnitudes (fp32 bits), their scales
+  m.scale = take(sizeof(int) * 2 * K);  // the columns' sums of squares (fp32 bits), their scales
   m.total = (int)at;
   return m;
 }
@@ -1762,6 +1762,25 @@ __host__ __device__ inline WidePlan wide_plan(int T, int K, bool shared_ldl, int
 // of T, 8-byte aligned): too long for them at T = 1, 2, 3, 5, 6 and 9, which the
 // item kernel takes.
 __host__ __device__ inline bool wide_slot_fits(int T) { return 3 * ld_t(T) + 2 <= 4 * T; }
+
+// The columns' scales of FixedDot2, from their norms: s with B 4^(s - 27) < 2^61, B
+// (at least the column's sum of squares, found in fp32: + 1/16) in 1e-30 .. 1e30;
+// false otherwise. A dense column then has |hi| of about 2^26, a sample that stands
+// out up to 2^31, and every column's hi a norm below 2^30.8 (norm_fits holds the
+// samples as they come out to it), so that whatever the columns
+//   |hh| <= 2^61.6, |x| <= 2 * 2^30.8 * 2^26 sqrt(1024) = 2^62.8 in 64 bits, and
+//   |ll| <= 2^52 T, 2^-51 of the product of the norms at worst and 2^-60 at random,
+// which FixedDot2 leaves out. Measured against 64 bits (largest error of an entry
+// over |x_i| |x_j|, whitened designs of the ranges in use, peaked and graded columns):
+// FP64 FMA chains 1.2e-16 to 7e-15, this 7e-18 to 3.1e-16.
+__device__ __forceinline__ bool norm_scale(float b, int& s) {
+  int e = 0;
+  frexpf(b * 1.0625f, &e);
+  const bool ok = b > 1e-30f && b < 1e30f;
+  s = ok ? 27 + ((61 - e) >> 1) : 0;
+  return ok;
+}
+__device__ __forceinline__ bool norm_fits(float b, int s) { return ldexpf(b, 2 * (s - 27)) <= 0x1.8p61f; }
 
 // hh and x of FixedDot
 struct FixedDot2 {
@@ -1792,7 +1811,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ?
   uint16_t* tri = reinterpret_cast<uint16_t*>(sm + pl.tri);
   double* fw = reinterpret_cast<double*>(sm + pl.fw);
   double *dk = reinterpret_cast<double*>(sm + pl.dk), *rs = dk + K;
-  int *colmax = reinterpret_cast<int*>(sm + pl.scale), *scale = colmax + K;
+  int *colss = reinterpret_cast<int*>(sm + pl.scale), *scale = colss + K;
   __shared__ double red[32];
   __shared__ float fred[NW];
   __shared__ int flag, bad_r;
@@ -1816,33 +1835,37 @@ __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ?
       ldl_of_pair(d, o, p, area, area + T, area + 2 * T, area + 3 * T, red, &bad_r);
     }
     if (tid == 0) flag = 0;
-    for (int j = tid; j < K; j += nth) colmax[j] = 0;
+    for (int j = tid; j < K; j += nth) colss[j] = 0;
     __syncthreads();
 
-    // ---- 2. the columns' scales, from the recursion in fp32, then X_w
+    // ---- 2. the columns' scales, from the recursion in fp32 (the largest sum of
+    // squares of a run times their number), then X_w
     const float4* cf = reinterpret_cast<const float4*>(o.coef) + (size_t)p * T;
     for (int e = tid; e < K * d.n_runs; e += nth) {
       const int j = e % K, t0 = d.run_start[e / K], t1 = d.run_start[e / K + 1];
-      float xp = 0.f, vp = 0.f, mx = 0.f;
+      float xp = 0.f, vp = 0.f, ss = 0.f;
 #pragma unroll 8
       for (int t = t0; t < t1; ++t) {
         const float x = __ldg(Xd + (size_t)t * K + j);
         const float4 q = cf[t];
         vp = fmaf(-q.y, vp, fmaf(-q.x, xp, x));
         xp = x;
-        mx = fmaxf(mx, fabsf(vp * q.w));
+        const float w = vp * q.w;
+        ss = fmaf(w, w, ss);
       }
-      atomicMax(colmax + j, __float_as_int(mx));
+      atomicMax(colss + j, __float_as_int(ss));
     }
     __syncthreads();
-    for (int j = tid; j < K; j += nth) scale[j] = fixed_scale(__int_as_float(colmax[j]));
-    __syncthreads();
     bool over = false;
+    for (int j = tid; j < K; j += nth)
+      over = !norm_scale(__int_as_float(colss[j]) * (float)d.n_runs, scale[j]) || over;
+    __syncthreads();
     for (int e = tid; e < K * d.n_runs; e += nth) {
       const int j = e % K, t0 = d.run_start[e / K], t1 = d.run_start[e / K + 1], sc = scale[j];
       int2* fr = fx + (size_t)j * LT;
       float* xr = xf + (size_t)j * LT;
       double xp = 0.0, vp = 0.0;  // c = m = 0 at the run's start
+      float ss = 0.f;
       float xn[4];
       auto load = [&](int tq) {
 #pragma unroll
@@ -1865,8 +1888,9 @@ __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ?
             vp = z - cm[t] * vp;
             xp = x;
             const double w = vp * cr[t];
-            f[k] = fixed_of(w, sc, over);
+            f[k] = fixed_of<5>(w, sc, over);
             w4[k] = d2f_exact(w);
+            ss = fmaf(w4[k], w4[k], ss);
           }
         }
         if (tq >= t0 && (tq + 4 <= t1 || t1 == T)) {  // whole, or the last of the row with its padding
@@ -1884,6 +1908,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ?
           }
         }
       }
+      over = over || !norm_fits(ss * (float)d.n_runs, sc);
     }
     if (over) flag = 1;
     __syncthreads();
@@ -2264,7 +2289,7 @@ __global__ void __launch_bounds__(256) design_gram_kernel(int T, int K, int chun
       const int t = idx / ncol, c = idx % ncol;
       const double x = c < K ? f2d_exact(Xg[(size_t)(t0 + t) * K + c]) : 1.0;
       if (fixed)
-        xi[c * ld + t] = fixed_of(x, fixed_scale(__int_as_float(cmax[c])), over);
+        xi[c * ld + t] = fixed_of<0>(x, fixed_scale(__int_as_float(cmax[c])), over);
       else
         xt[c * ld + t] = x;
     }

@@ -161,3 +161,41 @@ def test_singular_correlation_replaces_its_pivots(T, K, D):
         want = np.stack([c, m, 1 / Dp, 1 / np.sqrt(Dp)], 1)
         assert np.abs(coef[p] - want).max() <= 1e-6 * np.abs(want).max()
         assert float(f.logdet_R[p]) == pytest.approx(2 * np.log(np.sqrt(Dp) + 1e-10).sum(), rel=1e-11, abs=1e-9)
+
+
+@gpu
+@pytest.mark.parametrize("T,K,n", [(400, 24, 3), (600, 130, 3), (1024, 41, 3), (400, 20, 33), (855, 18, 33)])
+@pytest.mark.parametrize("kind", ["gaussian", "outlier", "graded", "constant"])
+def test_gram_matrix_of_wide_builds_against_exact_sums(T, K, n, kind):
+    """X'X at (0, 0), where the whitened design is the design, as the build
+    forms it in FP64 (the lower triangle of the slot's factor, which the
+    factorisation leaves) against sums in extended precision, whatever the
+    columns' profile. Error of an entry over |x_i| |x_j|: a fixed point of
+    norm 2^56.4 or more rounds each sample by half a unit (sqrt(T) 2^-56.4 for
+    both columns), the products of the low halves left out are at most T 2^52
+    of 2^112.8, and the value takes two FP64 roundings."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(T + K)
+    X = rng.standard_normal((T, K))
+    if kind == "outlier":
+        X[T // 3] *= 1e4
+    elif kind == "graded":
+        X *= 10.0 ** rng.uniform(-6, 6, (T, K))
+    elif kind == "constant":  # every low half alike, no two columns parallel
+        X = np.where(np.arange(T)[:, None] % (K + 1) == np.arange(K)[None, :], 2.0, 1.0) * np.linspace(1.0, 1.9, K)
+    X = X.astype(np.float32)
+    ax = torch.linspace(-0.8, 0.8, n)
+    g = G.make_grid(ax, ax, use_double=True)
+    f = engine.build_factors(torch.from_numpy(X).to(DEV), g, G.run_layout(T, [0]), with_tc=True)
+    torch.cuda.synchronize()
+    assert int(f.info[g.p0]) == 0
+    slot = 4 * T + 2 * K * T + 4 * K * K
+    at = g.p0 * slot + 4 * T + 2 * K * T
+    got = f._keep[3][at : at + K * K].cpu().numpy().reshape(K, K)
+    Xl = X.astype(np.longdouble)
+    want = Xl.T @ Xl
+    norm = np.sqrt(np.diag(want))
+    err = np.abs(got - want) / (norm[:, None] * norm[None, :])
+    tol = np.sqrt(T) * 2.0**-56.4 + T * 2.0**-60.8 + 2.0**-52
+    assert (err[np.tril_indices(K)] <= tol).all(), float(err[np.tril_indices(K)].max())
