@@ -76,6 +76,28 @@ __device__ double block_sum(double v, double* red) {
   return red[0];
 }
 
+// sum_t f(t), t < n, as block_sum adds it over 256 threads (f(t) in the thread t mod
+// 256) whatever the CTA's width: a pair's factor does not depend on the kernel that
+// forms it. Starts and ends with a barrier.
+template <typename F>
+__device__ __forceinline__ double block_sum256(int n, F f, double* red) {
+  const int lane = threadIdx.x & 31;
+  __syncthreads();
+  for (int w = threadIdx.x >> 5; w < 8; w += blockDim.x >> 5) {
+    double v = 0.0;
+    for (int t = 32 * w + lane; t < n; t += 256) v += f(t);
+    v = warp_sum_d(v);
+    if (lane == 0) red[w] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double v = warp_sum_d(lane < 8 ? red[lane] : 0.0);
+    if (lane == 0) red[0] = v;
+  }
+  __syncthreads();
+  return red[0];
+}
+
 // 1/sqrt(d) by the Newton-Raphson iteration r <- r + r (1 - d r^2) / 2 from
 // the fp32 estimate (relative error about 2^-22; each step squares it, so two
 // steps reach FP64 rounding). On this GPU an FP64 square root or division
@@ -281,8 +303,8 @@ __device__ void ldl_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p
   // Each lane multiplies the matrices of its stretch, a scan over the lanes
   // gives the minors before each stretch, and the lane walks it from there.
   // (A warp has one FP64 instruction in flight, 64 cycles each: about 80 of
-  // them for a run of 200, where a walk by one lane takes 400.)
-  double ld = 0.0;
+  // them for a run of 200, where a walk by one lane takes 400.) A run's log goes to
+  // off2 of its first sample, which its warp has read by then.
   const int lane = threadIdx.x & 31;
   for (int r = threadIdx.x >> 5; r < d.n_runs && !ident; r += blockDim.x >> 5) {
     const int t0 = d.run_start[r], t1 = d.run_start[r + 1];
@@ -352,9 +374,9 @@ __device__ void ldl_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p
     }
     __syncwarp();  // a walk by lane 0 rewrites num and prev
     if (!__any_sync(0xffffffffu, bad)) {
-      if (s1 == t1 && s0 < s1) ld += log(n1) + (double)e2 * 0.693147180559945309417;
+      if (s1 == t1 && s0 < s1) off2[t0] = log(n1) + (double)e2 * 0.693147180559945309417;
     } else if (lane == 0) {  // R is singular or not a correlation
-      double D = 1.0;
+      double D = 1.0, ld = 0.0;
       for (int t = t0; t < t1; ++t) {
         D = diag[t] - off2[t] / D;
         if (!(D > 0.0)) {
@@ -365,28 +387,32 @@ __device__ void ldl_of_pair(const ffs_grid_desc& d, const ffs_grid_out& o, int p
         prev[t] = 1.0;
         ld += log(D);
       }
+      off2[t0] = ld;
     }
   }
   __syncthreads();
-  double rsum = 0.0;
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
     double id = 1.0, rs = 1.0;
     if (!ident && num[t] != prev[t]) {  // else D_t = 1
       id = prev[t] * rcp_newton(num[t]);  // 1 / D_t
       rs = id * rsqrt_newton(id);
     }
-    rsum += rs;
     diag[t] = id;
     cr[t] = rs;
   }
-  ld = block_sum(ld + 2e-10 * rsum, red);  // its barriers order diag
+  const double rsum = block_sum256(T, [&](int t) { return cr[t]; }, red);  // its barriers order diag
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
     const double m = t > 0 ? cm[t] * diag[t - 1] : 0.0;
     cm[t] = m;
     reinterpret_cast<float4*>(o.coef)[(size_t)p * T + t] =
         make_float4((float)cc[t], (float)m, (float)diag[t], (float)cr[t]);
   }
-  if (threadIdx.x == 0) o.logdet_R[p] = ld;
+  if (threadIdx.x == 0) {
+    double ld = 2e-10 * rsum;
+    for (int r = 0; r < d.n_runs && !ident; ++r)
+      if (d.run_start[r] < d.run_start[r + 1]) ld += off2[d.run_start[r]];
+    o.logdet_R[p] = ld;
+  }
   __syncthreads();
 }
 
@@ -914,17 +940,13 @@ __device__ __noinline__ void item_global(const BuildArgs& args, const PairScratc
       for (int pass = 0; pass < 2; ++pass) {
         for (int i = 0; i < j; ++i) {
           const double* qi = s.Qm + (size_t)i * T;
-          double part = 0.0;
-          for (int t = threadIdx.x; t < T; t += blockDim.x) part += qi[t] * q[t];
-          const double rij = block_sum(part, red);
+          const double rij = block_sum256(T, [&](int t) { return qi[t] * q[t]; }, red);
           for (int t = threadIdx.x; t < T; t += blockDim.x) q[t] -= rij * qi[t];
           if (threadIdx.x == 0) s.Lx[j * K + i] += rij;
           __syncthreads();
         }
       }
-      double part = 0.0;
-      for (int t = threadIdx.x; t < T; t += blockDim.x) part += q[t] * q[t];
-      const double nrm = sqrt(block_sum(part, red));
+      const double nrm = sqrt(block_sum256(T, [&](int t) { return q[t] * q[t]; }, red));
       const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
       for (int t = threadIdx.x; t < T; t += blockDim.x) q[t] *= inv;
       if (threadIdx.x == 0) s.Lx[j * K + j] = nrm;
@@ -1170,6 +1192,38 @@ struct FixedDot {
   }
 };
 
+// The columns' scales of FixedDot2, from their norms: s with B 4^(s - 27) < 2^61, B
+// (at least the column's sum of squares, found in fp32: + 1/16) in 1e-30 .. 1e30;
+// false otherwise. A dense column then has |hi| of about 2^26, a sample that stands
+// out up to 2^31, and every column's hi a norm below 2^30.8 (norm_fits holds the
+// samples as they come out to it), so that whatever the columns
+//   |hh| <= 2^61.6, |x| <= 2 * 2^30.8 * 2^26 sqrt(1024) = 2^62.8 in 64 bits, and
+//   |ll| <= 2^52 T, 2^-51 of the product of the norms at worst and 2^-60 at random,
+// which FixedDot2 leaves out. Measured against 64 bits (largest error of an entry
+// over |x_i| |x_j|, whitened designs of the ranges in use, peaked and graded columns):
+// FP64 FMA chains 1.2e-16 to 7e-15, this 7e-18 to 3.1e-16.
+__device__ __forceinline__ bool norm_scale(float b, int& s) {
+  int e = 0;
+  frexpf(b * 1.0625f, &e);
+  const bool ok = b > 1e-30f && b < 1e30f;
+  s = ok ? 27 + ((61 - e) >> 1) : 0;
+  return ok;
+}
+__device__ __forceinline__ bool norm_fits(float b, int s) { return ldexpf(b, 2 * (s - 27)) <= 0x1.8p61f; }
+
+// hh and x of FixedDot
+struct FixedDot2 {
+  long long hh = 0, x = 0;
+  __device__ __forceinline__ void add(int ax, int ay, int bx, int by) {
+    hh += (long long)ax * bx;
+    x += (long long)ax * by;
+    x += (long long)ay * bx;
+  }
+  __device__ __forceinline__ double value(int si, int sj) const {
+    return fma((double)hh, 0x1p54, (double)x * 0x1p27) * __hiloint2double((1023 - si - sj) << 20, 0);
+  }
+};
+
 // float of a double, rounded to nearest even, by its bit fields (integer pipe);
 // anything but zeros and normal results takes the hardware conversion.
 __device__ __forceinline__ float d2f_exact(double w) {
@@ -1181,6 +1235,54 @@ __device__ __forceinline__ float d2f_exact(double w) {
   if (ex - 897u >= 253u) return (float)w;
   const unsigned long long r = m + 0x0fffffffull + ((m >> 29) & 1);
   return __uint_as_float(sg | ((uint32_t)(r >> 29) - (896u << 23)));
+}
+
+// The factor of X_w'X_w = Lu D Lu' and Lu^-1 in one pass over its packed lower
+// triangle A, for the kernels below: step k takes w_r f_c off every entry (r, c) of
+// the rows below k + 1, w_r = A_rk / D_k, f = (row k of Lu^-1, 1, column k of A): left
+// of column k the inverse grows where the factor's columns are no longer read.
+// Some warps form the next step's f and w ahead of the others (fold_ahead, lane
+// by lane i < K); one barrier a step, for k = -1 .. K - 2. fw: f and w, double-
+// buffered [2][2][K]; column k of A, before its division by sqrt(D_k), goes to row k of
+// Lx [K][K], right of its diagonal; dk [K] receives D.
+struct Fold {
+  double *A, *fw, *dk, *Lx;
+  int K;
+};
+
+// Returns true when pivot k + 1 is not positive.
+__device__ __forceinline__ bool fold_ahead(const Fold& m, int k, int i) {
+  const double *f = m.fw + (k & 1) * 2 * m.K, *w = f + m.K;
+  double *fn = m.fw + ((k + 1) & 1) * 2 * m.K, *wn = fn + m.K;
+  const int k1 = k + 1, row1 = k1 * (k1 + 1) / 2;
+  const double w1 = k >= 0 ? w[k1] : 0.0, f1 = k >= 0 ? f[k1] : 0.0;
+  double dn = m.A[row1 + k1];
+  if (k >= 0) dn = fma(-w1, f1, dn);
+  const bool bad = !positive(dn);
+  if (bad) dn = 1.0;
+  double v = 1.0, r, pc;
+  if (i < k1) {  // row k + 1 of the inverse
+    v = fma(-w1, f[i], i == k ? 0.0 : m.A[row1 + i]);
+    m.A[row1 + i] = v;
+  } else if (i > k1 && i < m.K) {
+    v = m.A[i * (i + 1) / 2 + k1];
+    if (k >= 0) v = fma(-w[i], f1, v);
+    m.Lx[k1 * m.K + i] = v;
+  }
+  rcp_factors(dn, r, pc);
+  if (i < m.K) {
+    const double u = v * r;
+    fn[i] = v;
+    wn[i] = fma(u, pc, u);
+  }
+  if (i == k1) m.dk[k1] = dn;
+  return bad;
+}
+
+// Step k >= 0 at entry e = (r, c), r > k + 1.
+__device__ __forceinline__ void fold_entry(const Fold& m, int k, int e, int r, int c) {
+  const double *f = m.fw + (k & 1) * 2 * m.K, *w = f + m.K;
+  if (c != k + 1) m.A[e] = fma(-w[r], f[c], c == k ? 0.0 : m.A[e]);
 }
 
 // ------------------------------------------------------------- items in shared memory
@@ -1195,9 +1297,10 @@ __device__ __forceinline__ float d2f_exact(double w) {
 //     matrix and as the fp32 copy that the later phases read; the Gram matrix in
 //     integers (above), blocks of 2 x 2 entries per thread, the samples split over
 //     SL threads of a block.
-//   - The Cholesky factorisation keeps each entry in its thread's register,
-//     two barriers a column; the producer warps then invert the factor while
-//     the others form Q, U and the fp16 splits in place in shared memory.
+//   - The factor and its inverse (Fold), an entry per thread; then Q, U and the fp16
+//     splits in place in shared memory.
+// The sums, the factor and the fp32 phases are grid_wide_kernel's to the bit, so a
+// design's factors do not depend on how many others are built beside it.
 // A rank-deficient item (a pivot that is not positive) or one whose series
 // leave the fixed point goes through item_global.
 // P = 117, T = 200, K = 8: 238 -> 107 us against item_global's phases with FP64 Gram
@@ -1247,19 +1350,21 @@ __host__ __device__ inline ItemPlan item_plan(int T, int K, int n_runs) {
   m.xf = take(xf > tmp ? xf : tmp);
   // [GI_BUF][RP][KR][rs] samples (FP64, then fixed point); afterwards 2 K^2 doubles of scratch
   size_t ring = sizeof(int2) * GI_BUF * m.RP * m.KR * m.rs;
-  const size_t scr = sizeof(double) * 2 * K * K, cf = sizeof(float4) * T;  // before it, the fp32 coefficients
+  // before it, the fp32 coefficients; first the packed triangle, f and w
+  const size_t fold = (size_t)m.E + 4 * K, kk = (size_t)2 * K * K;
+  const size_t scr = sizeof(double) * (fold > kk ? fold : kk), cf = sizeof(float4) * T;
   ring = ring > scr ? ring : scr;
   m.ring = take(ring > cf ? ring : cf);
-  m.L = take(sizeof(double) * K * K);
+  m.L = take(sizeof(double) * K * K);     // [k][i]: column k of the factor, times sqrt(D_k)
   m.Li = take(sizeof(double) * K * K);
-  m.rd = take(sizeof(double) * K);
+  m.rd = take(sizeof(double) * 2 * K);    // D, 1 / sqrt(D)
   m.lxf = take(sizeof(float) * K * K4);   // Lx transposed: [i][j], j contiguous
   m.lif = take(sizeof(float) * K * K4);
   m.total = at;
   return m;
 }
 
-// Barrier of the first n threads (a multiple of 32) of the CTA.
+
 
 template <bool SHARED_LDL>
 __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(BuildArgs args, int n_designs,
@@ -1281,14 +1386,16 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
   int2* ring = reinterpret_cast<int2*>(sm + pl.ring);      // [GI_BUF][RP][KR][rs]
   const int bufw = RP * pl.KR * rs, cs2 = pl.cs2, CS = 1 << cs2;
   double* scr = reinterpret_cast<double*>(sm + pl.ring);
-  double* L = reinterpret_cast<double*>(sm + pl.L);        // [K][K] X_w'X_w, then its factor
+  double* L = reinterpret_cast<double*>(sm + pl.L);
   double* Li = reinterpret_cast<double*>(sm + pl.Li);
-  double* rd = reinterpret_cast<double*>(sm + pl.rd);      // 1 / diag(L)
+  double *dk = reinterpret_cast<double*>(sm + pl.rd), *rsd = dk + K;
+  const Fold fold{scr, scr + pl.E, dk, L, K};              // X_w'X_w, then the inverse, packed
   float* lxf = reinterpret_cast<float*>(sm + pl.lxf);
   float* lif = reinterpret_cast<float*>(sm + pl.lif);
   __shared__ double red[32];
   __shared__ float fred[32];
-  __shared__ int colmax[GI_KMAX], scale[GI_KMAX + 1];
+  __shared__ int colss[GI_KMAX], scale[GI_KMAX + 1];
+  __shared__ float colsum[GI_KMAX];
   __shared__ int seg[GI_PROD + 1];  // first sample of each time segment
   __shared__ int flag, bad_r;
   for (int q = tid; q <= RP; q += nth) seg[q] = d.run_start[q * d.n_runs / RP];
@@ -1314,7 +1421,10 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
       ldl_of_pair(d, o, p, cc, cm, cr, reinterpret_cast<double*>(xf), red, &bad_r);
     }
     if (tid == 0) flag = 0;
-    for (int j = tid; j < K; j += nth) colmax[j] = 0;
+    for (int j = tid; j < K; j += nth) {
+      colss[j] = 0;
+      colsum[j] = 0.f;
+    }
     // the design into xf, where X_w replaces it, and the fp32 coefficients into
     // the ring's region
     const float4* cf = reinterpret_cast<const float4*>(o.coef) + (size_t)p * T;
@@ -1326,34 +1436,40 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
     __syncthreads();
 
     // ---- 2, 3. X_w and X_w'X_w
-    const int ps = producer ? seg[pq] : 0, pe = producer ? seg[pq + 1] : 0;
+    const int ps = producer ? seg[pq] : 0;
     if (producer) {
-      // the columns' scales, from the recursion in fp32
+      // the columns' scales, from the recursion in fp32 (the largest sum of squares
+      // of a run times their number)
       const float* xs = xf + (size_t)pj * ldx;
-      float xp = 0.f, vp = 0.f, mx = 0.f;
+      for (int r = pq * d.n_runs / RP; r < (pq + 1) * d.n_runs / RP; ++r) {
+        const int t1 = d.run_start[r + 1];
+        float xp = 0.f, vp = 0.f, ss = 0.f;
 #pragma unroll 8
-      for (int t = ps; t < pe; ++t) {
-        const float x = xs[t];
-        const float4 q = cfr[t];
-        vp = fmaf(-q.y, vp, fmaf(-q.x, xp, x));
-        xp = x;
-        mx = fmaxf(mx, fabsf(vp * q.w));
+        for (int t = d.run_start[r]; t < t1; ++t) {
+          const float x = xs[t];
+          const float4 q = cfr[t];
+          vp = fmaf(-q.y, vp, fmaf(-q.x, xp, x));
+          xp = x;
+          const float w = vp * q.w;
+          ss = fmaf(w, w, ss);
+        }
+        atomicMax(colss + pj, __float_as_int(ss));
       }
-      atomicMax(colmax + pj, __float_as_int(mx));
     }
     __syncthreads();
     if (pl.KR > K)  // the row past an odd K is zero
       for (int e = tid; e < GI_BUF * RP * rs; e += nth) ring[(e / rs * pl.KR + K) * rs + e % rs] = make_int2(0, 0);
-    for (int j = tid; j < K; j += nth) scale[j] = fixed_scale(__int_as_float(colmax[j]));
+    bool over = tid < K && !norm_scale(__int_as_float(colss[tid]) * (float)d.n_runs, scale[tid]);
     __syncthreads();
     int longest = 0;
     for (int q = 0; q < RP; ++q) longest = max(longest, seg[q + 1] - seg[q]);
     const int nch = (longest + CS - 1) >> cs2;
-    FixedDot acc[2][2];
+    FixedDot2 acc[2][2];
     {
       // the values of a chunk this thread forms (z) and converts (w): slot in a
       // ring buffer, sample of chunk 0 and its segment's end
       int vs[GI_VAL], vt[GI_VAL], ve[GI_VAL], vj[GI_VAL];
+      float ss[GI_VAL];
 #pragma unroll
       for (int i = 0; i < GI_VAL; ++i) {
         const int e = tid + i * GT;  // sample fastest: consecutive lanes, consecutive words
@@ -1363,9 +1479,9 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
         vs[i] = on ? (q * pl.KR + j) * rs + k : -1;
         vt[i] = seg[q] + k;
         ve[i] = seg[q + 1];
+        ss[i] = 0.f;
       }
       double vp = 0.0;
-      bool over = false;
       for (int c = 0; c < nch + GI_BUF - 1; ++c) {
         if (tid < GT) {
           double* za = reinterpret_cast<double*>(ring) + (c % GI_BUF) * bufw;
@@ -1388,8 +1504,10 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
                 int2 f = make_int2(0, 0);
                 if (t < ve[i]) {
                   const double w = reinterpret_cast<double*>(wb)[vs[i]] * cr[t];
-                  f = fixed_of<0>(w, scale[vj[i]], over);
-                  xf[(size_t)vj[i] * ldx + t] = d2f_exact(w);
+                  f = fixed_of<5>(w, scale[vj[i]], over);
+                  const float wf = d2f_exact(w);
+                  ss[i] = fmaf(wf, wf, ss[i]);
+                  xf[(size_t)vj[i] * ldx + t] = wf;
                 }
                 wb[vs[i]] = f;
               }
@@ -1401,10 +1519,10 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
               const int2* r0 = rg + (u >> cs2) * pl.KR * rs + (u & (CS - 1));
               const int2 *ai = r0 + 2 * bi * rs, *aj = r0 + 2 * bj * rs;
               const int2 i0 = ai[0], i1 = ai[rs], j0 = aj[0], j1 = aj[rs];
-              acc[0][0].add(i0, j0);
-              acc[0][1].add(i0, j1);
-              acc[1][0].add(i1, j0);
-              acc[1][1].add(i1, j1);
+              acc[0][0].add(i0.x, i0.y, j0.x, j0.y);
+              acc[0][1].add(i0.x, i0.y, j1.x, j1.y);
+              acc[1][0].add(i1.x, i1.y, j0.x, j0.y);
+              acc[1][1].add(i1.x, i1.y, j1.x, j1.y);
             }
           }
         } else if (producer && c >= 1 && c <= nch) {
@@ -1425,68 +1543,58 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
         }
         __syncthreads();
       }
-      if (over) flag = 1;
+      if (tid < GT) {
+#pragma unroll
+        for (int i = 0; i < GI_VAL; ++i) {  // CS lanes a column
+          for (int m = 1; m < CS; m <<= 1) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], m);
+          if (vs[i] >= 0 && (lane & (CS - 1)) == 0) atomicAdd(colsum + vj[i], ss[i]);
+        }
+      }
     }
     if (wid * 32 < pl.NB * pl.SL) {  // whole warps: the slices of a block lie in one
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
-          FixedDot& f = acc[u][v];
+          FixedDot2& f = acc[u][v];
           for (int m = 1; m < pl.SL; m <<= 1) {
             f.hh += __shfl_xor_sync(0xffffffffu, f.hh, m);
             f.x += __shfl_xor_sync(0xffffffffu, f.x, m);
-            f.ll += __shfl_xor_sync(0xffffffffu, f.ll, m);
           }
           const int i = 2 * bi + u, j = 2 * bj + v;
           if (gram && sl == 0 && i < K && j <= i) {
             const double x = f.value(scale[i], scale[j]);
-            L[i * K + j] = x;
+            fold.A[i * (i + 1) / 2 + j] = x;
             o.XtX[(size_t)pd * K * K + i * K + j] = (float)x;
             o.XtX[(size_t)pd * K * K + j * K + i] = (float)x;
           }
         }
     }
     __syncthreads();
-    double mij = entry ? L[ei * K + ej] : 0.0;
-    const bool left = flag != 0;  // a series left the fixed point
-    __syncthreads();
+    over = over || (tid < K && !norm_fits(colsum[tid], scale[tid]));
+    bool left = __syncthreads_or(over);  // a series left the fixed point
 
-    // ---- 4. Cholesky, right-looking, an entry per thread: column k's entries
-    // are put down, the first warps scale them (full warps of the FP64 pipe), and
-    // every later entry takes its product off
-    for (int k = 0; k < K && !left; ++k) {
-      if (entry && ej == k) L[ei * K + k] = mij;
-      __syncthreads();
-      if (tid < (K + 31) / 32 * 32) {
-        const double dk = L[k * K + k];
-        const bool pos = dk > 0.0;
-        const double r = pos ? rsqrt_newton(dk) : 1.0;
-        __syncwarp();
-        if (tid > k && tid < K) L[tid * K + k] *= r;
-        if (tid == k) {
-          rd[k] = r;
-          scr[k] = pos ? dk * r : 1.0;  // the diagonal, put in place after the column's readers
-          if (!pos) flag = 1;
-        }
-      }
-      __syncthreads();
-      if (flag) break;
-      if (entry && ej > k) mij -= L[ei * K + k] * L[ej * K + k];
+    // ---- 4. the factor and its inverse, an entry per thread
+    for (int k = -1; k < K - 1 && !left; ++k) {
+      const bool bad = wid == 0 && fold_ahead(fold, k, lane);
+      if (k >= 0 && entry && ei > k + 1) fold_entry(fold, k, tid, ei, ej);
+      left = __syncthreads_or(bad);
     }
-    if (!flag) {
-      for (int k = tid; k < K; k += nth) L[k * K + k] = scr[k];
-    }
-    __syncthreads();
-    if (flag) {
-      __syncthreads();
+    if (left) {
       const PairScratch s = scratch_of(o.work, blockIdx.x, T, K);
       item_global<false>(args, s, p, pd, Xd, cc, cm, cr, nullptr, bad_r, red, &flag);
       continue;
     }
+    for (int k = tid; k < K; k += nth) {
+      const double r = rsqrt_newton(dk[k]);
+      rsd[k] = r;
+      fold.fw[k] = 2.0 * log(fabs(dk[k] * r) + 1e-10);
+    }
+    __syncthreads();
+    if (entry) Li[ei * K + ej] = ei == ej ? rsd[ei] : fold.A[tid] * rsd[ei];  // Li = D^-1/2 Lu^-1
     for (int e = tid; e < K * K4; e += nth) {
       const int i = e / K4, j = e % K4;
-      lxf[e] = j < K && j >= i ? (float)L[j * K + i] : 0.f;
+      lxf[e] = j < K && j >= i ? (float)(j == i ? dk[i] * rsd[i] : L[i * K + j] * rsd[i]) : 0.f;
     }
     for (int t = tid; t < T; t += nth) cfs[t] = cf[t];  // c, m and 1/sqrt(D) in FP64 are done with
     __syncthreads();
@@ -1617,41 +1725,30 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
         }
       }
     } else {
-      // ---- 7. Li = Lx^-1, a column per lane: each entry formed takes its part
-      // off the rows below it; the logs of logdet beside it
-      for (int c = tid - GT; c < K; c += nth - GT) {
-        scr[c] = 2.0 * log(fabs(L[c * K + c]) + 1e-10);
-        for (int i = 0; i < K; ++i) Li[i * K + c] = i == c ? 1.0 : 0.0;
-        for (int k = c; k < K; ++k) {
-          const double v = Li[k * K + c] * rd[k];
-          Li[k * K + c] = v;
-#pragma unroll 4
-          for (int i = k + 1; i < K; ++i) Li[i * K + c] -= L[i * K + k] * v;
-        }
+      // ---- 7. logdet, diag(A) and the fp32 copy of Li beside them
+      if (tid == GT) {
+        double ld = 0.0;
+        for (int j = 0; j < K; ++j) ld += fold.fw[j];
+        o.logdet_XtX[pd] = ld;
+        o.info[pd] = bad_r ? 2 : 0;
+      }
+      for (int e = tid - GT; e < K * K4; e += nth - GT) {
+        const int i = e / K4, j = e % K4;
+        lif[e] = j <= i ? (float)Li[i * K + j] : 0.f;
+      }
+      for (int j = tid - GT; j < K; j += nth - GT) {
+        double a = 0.0;
+        for (int k = j; k < K; ++k) a = fma(Li[k * K + j], Li[k * K + j], a);
+        o.Adiag[(size_t)pd * K + j] = (float)a;
       }
     }
     __syncthreads();
 
-    if (tid == 0) {
-      double ld = 0.0;
-      for (int j = 0; j < K; ++j) ld += scr[j];
-      o.logdet_XtX[pd] = ld;
-      o.info[pd] = bad_r ? 2 : 0;
-    }
-    for (int e = tid; e < K * K4; e += nth) {
-      const int i = e / K4, j = e % K4;
-      lif[e] = j < K ? (float)Li[i * K + j] : 0.f;
-    }
-    for (int j = tid; j < K; j += nth) {
-      double a = 0.0;
-      for (int k = j; k < K; ++k) a += Li[k * K + j] * Li[k * K + j];
-      o.Adiag[(size_t)pd * K + j] = (float)a;
-    }
     if (o.Afull) {  // all of A, for the per-voxel blocks of the -dsort fit
       for (int e = tid; e < K * K; e += nth) {
         const int i = e / K, j = e % K;
         double a = 0.0;
-        for (int k = max(i, j); k < K; ++k) a += Li[k * K + i] * Li[k * K + j];
+        for (int k = max(i, j); k < K; ++k) a = fma(Li[k * K + i], Li[k * K + j], a);
         o.Afull[(size_t)pd * K * K + e] = (float)a;
       }
     }
@@ -1705,11 +1802,7 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
 //     norms, without the lo lo' sums: norm_scale) and to fp32; the Gram matrix in blocks of 4 x 4 or 2 x 2 entries per thread (rows b,
 //     b + kb, ..., so that a warp's blocks read consecutive rows) from
 //     double-buffered chunks of WI_CS samples.
-//   - X_w'X_w = Lu D Lu' and Lu^-1 in one pass over the packed lower triangle:
-//     step k takes w_r f_c off every entry (r, c) of the rows below k, w_r = A_rk / D_k,
-//     f = (row k of Lu^-1, 1, column k of A): left of column k the inverse grows
-//     where the factor's columns are no longer read. The first warps form the next
-//     step's f and w ahead of the others; one barrier a step.
+//   - X_w'X_w = Lu D Lu' and Lu^-1 in one pass (Fold).
 //   - Q = X_w Lx^-T and G = U Lx^-1 in fp32, 8 columns x 2 samples per thread.
 // A rank-deficient item or one whose series leave the fixed point goes through
 // item_global, whose general phases these replace: P = 561, T = 600, K = 130 in 3
@@ -1762,38 +1855,6 @@ __host__ __device__ inline WidePlan wide_plan(int T, int K, bool shared_ldl, int
 // of T, 8-byte aligned): too long for them at T = 1, 2, 3, 5, 6 and 9, which the
 // item kernel takes.
 __host__ __device__ inline bool wide_slot_fits(int T) { return 3 * ld_t(T) + 2 <= 4 * T; }
-
-// The columns' scales of FixedDot2, from their norms: s with B 4^(s - 27) < 2^61, B
-// (at least the column's sum of squares, found in fp32: + 1/16) in 1e-30 .. 1e30;
-// false otherwise. A dense column then has |hi| of about 2^26, a sample that stands
-// out up to 2^31, and every column's hi a norm below 2^30.8 (norm_fits holds the
-// samples as they come out to it), so that whatever the columns
-//   |hh| <= 2^61.6, |x| <= 2 * 2^30.8 * 2^26 sqrt(1024) = 2^62.8 in 64 bits, and
-//   |ll| <= 2^52 T, 2^-51 of the product of the norms at worst and 2^-60 at random,
-// which FixedDot2 leaves out. Measured against 64 bits (largest error of an entry
-// over |x_i| |x_j|, whitened designs of the ranges in use, peaked and graded columns):
-// FP64 FMA chains 1.2e-16 to 7e-15, this 7e-18 to 3.1e-16.
-__device__ __forceinline__ bool norm_scale(float b, int& s) {
-  int e = 0;
-  frexpf(b * 1.0625f, &e);
-  const bool ok = b > 1e-30f && b < 1e30f;
-  s = ok ? 27 + ((61 - e) >> 1) : 0;
-  return ok;
-}
-__device__ __forceinline__ bool norm_fits(float b, int s) { return ldexpf(b, 2 * (s - 27)) <= 0x1.8p61f; }
-
-// hh and x of FixedDot
-struct FixedDot2 {
-  long long hh = 0, x = 0;
-  __device__ __forceinline__ void add(int ax, int ay, int bx, int by) {
-    hh += (long long)ax * bx;
-    x += (long long)ax * by;
-    x += (long long)ay * bx;
-  }
-  __device__ __forceinline__ double value(int si, int sj) const {
-    return fma((double)hh, 0x1p54, (double)x * 0x1p27) * __hiloint2double((1023 - si - sj) << 20, 0);
-  }
-};
 
 template <bool SHARED_LDL, int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ? 8 : 5)
@@ -1996,42 +2057,13 @@ __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ?
       __syncthreads();
       constexpr int LA = 32;  // entries of f per warp of the look-ahead
       const int nla = (K + LA - 1) / LA;
+      const Fold fold{A, fw, dk, s.Lx, K};
       for (int k = -1; k < K - 1; ++k) {
-        bool bad = false;
-        const double *f = fw + (k & 1) * 2 * K, *w = f + K;
-        double *fn = fw + ((k + 1) & 1) * 2 * K, *wn = fn + K;
-        const int k1 = k + 1, row1 = k1 * (k1 + 1) / 2;
-        if (wid < nla) {
-          const int i = wid * LA + lane;
-          const double w1 = k >= 0 ? w[k1] : 0.0, f1 = k >= 0 ? f[k1] : 0.0;
-          double dn = A[row1 + k1];
-          if (k >= 0) dn = fma(-w1, f1, dn);
-          bad = !positive(dn);
-          if (bad) dn = 1.0;
-          double v = 1.0, r, pc;
-          if (i < k1) {  // row k + 1 of the inverse
-            v = fma(-w1, f[i], i == k ? 0.0 : A[row1 + i]);
-            A[row1 + i] = v;
-          } else if (i > k1 && i < K) {
-            v = A[i * (i + 1) / 2 + k1];
-            if (k >= 0) v = fma(-w[i], f1, v);
-            s.Lx[k1 * K + i] = v;
-          }
-          rcp_factors(dn, r, pc);
-          if (i < K) {
-            const double u = v * r;
-            fn[i] = v;
-            wn[i] = fma(u, pc, u);
-          }
-          if (i == k1) dk[k1] = dn;
-        }
+        const bool bad = wid < nla && fold_ahead(fold, k, wid * LA + lane);
         if (k >= 0) {
           const int E = K * (K + 1) / 2;
 #pragma unroll 2
-          for (int e = (k + 2) * (k + 3) / 2 + tid; e < E; e += nth) {
-            const int rc = tri[e], r = rc >> 8, c = rc & 255;
-            if (c != k1) A[e] = fma(-w[r], f[c], c == k ? 0.0 : A[e]);
-          }
+          for (int e = (k + 2) * (k + 3) / 2 + tid; e < E; e += nth) fold_entry(fold, k, e, tri[e] >> 8, tri[e] & 255);
         }
         left = __syncthreads_or(bad);
         if (left) break;

@@ -199,3 +199,42 @@ def test_gram_matrix_of_wide_builds_against_exact_sums(T, K, n, kind):
     err = np.abs(got - want) / (norm[:, None] * norm[None, :])
     tol = np.sqrt(T) * 2.0**-56.4 + T * 2.0**-60.8 + 2.0**-52
     assert (err[np.tril_indices(K)] <= tol).all(), float(err[np.tril_indices(K)].max())
+
+
+@gpu
+@pytest.mark.parametrize("T,K,runs,D,n,zero", [
+    (200, 8, 1, 20, None, False),   # one design: the item kernel; all: the wide one, 128 threads
+    (331, 13, 2, 9, None, False),
+    (300, 20, 3, 7, 21, False),
+    (850, 22, 1, 2, 21, False),     # the wide one, 320 threads
+    (150, 18, 11, 12, None, False),  # more runs than a warp per run, several runs a time segment
+    (97, 1, 1, 30, None, False),
+    (120, 7, 2, 20, None, True),    # rank deficient: Gram-Schmidt in every kernel
+    (240, 40, 2, 3, 21, True),
+    (1100, 6, 2, 3, None, False),   # the general phases
+])
+def test_a_design_factors_are_its_own_whatever_is_built_beside_it(T, K, runs, D, n, zero):
+    """The factors of each design of a build of many equal those of its build
+    alone, bit for bit, across the kernels that the number of items selects."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(T + K)
+    X = rng.standard_normal((D, T, K)).astype(np.float32)
+    X[:, :, 0] += 3.0
+    if zero:
+        X[1, :, K // 2] = 0.0
+    layout = G.run_layout(T, [T * r // runs for r in range(runs)])
+    ax = G.get_default_arma_grids() if n is None else (torch.linspace(-0.8, 0.8, n),) * 2
+    g = G.make_grid(*ax)
+    kw = dict(task_indices=[0, K // 2], glt=np.eye(K, dtype=np.float32)[:1], with_tc=True, afull=True) if K > 1 else {}
+    Xd = torch.from_numpy(X).to(DEV)
+    f = engine.build_factors(Xd, g, layout, **kw)
+    for d in (0, 1, D - 1):
+        one, part = engine.build_factors(Xd[d], g, layout, **kw), engine.design_view(f, d)
+        torch.cuda.synchronize()
+        assert int(one.info.max()) == (1 if zero and d == 1 else 0)
+        for name in ("coef", "logdet_R", "logdet_XtX", "U", "G", "Adiag", "XtX", "info", "Ftask", "glt_var", "uexp",
+                     "Afull", "U_hi", "U_lo"):
+            a, b = getattr(one, name), getattr(part, name)
+            if a is not None:
+                assert torch.equal(a.reshape(-1).view(torch.uint8), b.reshape(-1).view(torch.uint8)), (d, name)
