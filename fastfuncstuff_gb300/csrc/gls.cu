@@ -251,9 +251,9 @@ __device__ void gls_voxel(const ffs_gls_args& a, const GlsExtra& x, const int v,
 // sums reduced together, and each lane forms its own lag's term in FP64.
 // Adding every product into a shared bin instead serialised the warp, whose
 // lanes share a lag (4,099 voxels, T = 331, 30 lags: 1977 us; with the table
-// 37 us, by the difference of the fits). Without a table (tau not rising, or no room for it) the products
-// are binned in bins ([h + 1] floats of shared memory) by atomics. The value is
-// returned on lane 0.
+// 37 us, by the difference of the fits). Without a table (tau not rising, or no room
+// for it) bins ([h + 1] floats of shared memory) takes a lag's sum, or with tau the
+// products by atomics. The value is returned on lane 0.
 __device__ float ljung_box_warp(int h, const int* tau, const float* w, const float* ys, int T, float ssw,
                                 float* bins, const LjTab& tab) {
   const int lane = threadIdx.x & 31;
@@ -293,8 +293,15 @@ __device__ float ljung_box_warp(int h, const int* tau, const float* w, const flo
     for (int k = lane; k <= h; k += 32) bins[k] = 0.f;
     __syncwarp();
     for (int k = 1; k <= h; ++k) {
+      if (!tau) {  // every pair in one bin: summed by shuffles
+        float part = 0.f;
+        for (int t = lane; t + k < T; t += 32) part = fmaf(ys[t], ys[t + k], part);
+        part = warp_sum(part);
+        if (lane == 0) bins[k] = part;
+        continue;
+      }
       for (int t = lane; t + k < T; t += 32) {
-        const int dj = tau ? tau[t + k] - tau[t] : k;
+        const int dj = tau[t + k] - tau[t];
         if (dj > 0 && dj <= h) atomicAdd(bins + dj, ys[t] * ys[t + k]);
       }
     }
