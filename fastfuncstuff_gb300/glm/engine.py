@@ -20,6 +20,7 @@ from __future__ import annotations
 import copy
 import ctypes as C
 import math
+import threading
 from dataclasses import dataclass
 
 import numpy as np
@@ -1240,14 +1241,19 @@ class GroupedFitGraph:
 
 
 _GROUPED_GRAPHS: dict = {}
-_LAST_GROUPED: list = [None]  # the key of the last grouped fit
+GROUPED_GRAPHS_MAX = 2  # a plan holds a few GB of static buffers
+_GROUPED_RECENT: dict = {}  # per device, hashes of the keys of the last grouped fits
+_GROUPED_LOCK = threading.Lock()
 
 
 def grouped_graph_for(Y, Xs, grid, layout, gid, *, hierarchical, do_scale, gls_kw, factor_kw) -> GroupedFitGraph | None:
     """The cached GroupedFitGraph of this shape, grouping and options. It is
-    built when a grouping comes twice in a row (capturing costs an eager fit
-    and a synchronisation, 30 ms at 100,000 voxels and 20 designs, and every
-    subject has a grouping of its own); None asks the caller to fit eagerly."""
+    built when a grouping comes back while it is among the last
+    GROUPED_GRAPHS_MAX of its device, as many as are kept: a repeated one, or
+    two that alternate (capturing costs an eager fit and a synchronisation, 30
+    ms at 100,000 voxels and 20 designs, and every subject has a grouping of
+    its own; with more that take turns each would evict the next). None asks
+    the caller to fit eagerly."""
     gid = np.asarray(gid, dtype=np.int32)
     fk = tuple((k, None if v is None else v.key() if hasattr(v, "key") else np.asarray(v).tobytes())
                for k, v in sorted(factor_kw.items()))
@@ -1256,11 +1262,17 @@ def grouped_graph_for(Y, Xs, grid, layout, gid, *, hierarchical, do_scale, gls_k
            layout.run_start.tobytes(), layout.tau.tobytes(), gid.tobytes(), hierarchical, do_scale,
            tuple(sorted(gls_kw.items())), fk)
     gr = _GROUPED_GRAPHS.get(key)
-    again, _LAST_GROUPED[0] = _LAST_GROUPED[0] == key, key
+    with _GROUPED_LOCK:
+        recent = _GROUPED_RECENT.setdefault(str(Xs.device), [])
+        again = hash(key) in recent
+        if again:
+            recent.remove(hash(key))
+        recent.append(hash(key))
+        del recent[:-GROUPED_GRAPHS_MAX]
     if gr is None and not again:
         return None
     if gr is None:
-        while len(_GROUPED_GRAPHS) >= 2:  # a plan holds a few GB of static buffers
+        while len(_GROUPED_GRAPHS) >= GROUPED_GRAPHS_MAX:
             _GROUPED_GRAPHS.pop(next(iter(_GROUPED_GRAPHS)))
         slots = design_slots(gid, Xs.shape[0], Xs.shape[2], grid.P, Xs.device)
         gr = GroupedFitGraph(Y, Xs, grid, layout, slots, hierarchical=hierarchical, do_scale=do_scale,

@@ -32,3 +32,64 @@ def test_ljung_box_without_room_for_its_table(T, K, runs):
     e = ((-(-T // 32) if runs == 1 else T) + 12) * 2.0**-24
     tol = 2 * e * slope + e * e * T * (T + 2.0) * plan[2].sum() + 4e-7 * want
     assert (np.abs(got.ljung_box.numpy() - want) <= tol).all()
+
+
+@pytest.mark.parametrize("order,captured", [("AA", "A"), ("AAA", "A"), ("ABAB", "AB"), ("ABBA", "BA"), ("ABCABC", ""),
+                                            ("AABABA", "AB"), ("ABCCAB", "C")])
+def test_grouped_graphs_are_captured_for_groupings_that_come_back(order, captured, monkeypatch):
+    """Captured at the second of two in a row or of two that alternate; three
+    in turn, of which the cache would evict each before it returns, never."""
+    from fastfuncstuff_gb300.glm import engine
+
+    built = []
+
+    class Plan:
+        def __init__(self, Y, Xs, grid, layout, slots, **kw):
+            built.append(chr(ord("A") + int(slots.design[0])))
+
+    monkeypatch.setattr(engine, "GroupedFitGraph", Plan)
+    monkeypatch.setattr(engine, "_GROUPED_GRAPHS", {})
+    monkeypatch.setattr(engine, "_GROUPED_RECENT", {})
+    Y, Xs = torch.zeros(6, 20), torch.zeros(3, 20, 2)
+    g, layout = G.make_grid(*G.get_default_arma_grids()), G.run_layout(20)
+    for name in order:
+        gid = np.full(6, ord(name) - ord("A"))
+        engine.grouped_graph_for(Y, Xs, g, layout, gid, hierarchical=True, do_scale=True, gls_kw={}, factor_kw={})
+    assert "".join(built) == captured
+
+
+@gpu
+def test_grouped_graph_replays_other_data_and_other_designs(monkeypatch):
+    """A captured grouped fit replayed on other data, on designs whose span
+    lost the constant (the centring flag computed inside the graph goes to 0)
+    and on the first ones again equals the eager fit bit for bit; so does one
+    of two groupings that alternate."""
+    from fastfuncstuff_gb300 import fit_glm_arma11_grouped, synth
+    from fastfuncstuff_gb300.glm import engine
+
+    w = synth.workload(2, V=5000)
+    keep = np.isin(w.groups, np.arange(4))
+    Y, gid = w.Y[keep], w.groups[keep]
+    designs = {h: w.designs[h] for h in range(4)}
+    assert all(engine.constant_in_span(x) for x in designs.values())
+    ramp = dict(designs)
+    ramp[2] = designs[2] * (1.0 + np.linspace(0.0, 0.5, Y.shape[1], dtype=np.float32)[:, None])
+    assert not engine.constant_in_span(ramp[2])
+    other = np.roll(gid, 7)
+    kw = dict(a_grid=np.linspace(-0.8, 0.8, 33), b_grid=np.linspace(-0.8, 0.8, 33), run_starts=w.run_starts, tau=w.tau,
+              device=DEV, verbose=False, want_residuals=True)
+    monkeypatch.setattr(engine, "_GROUPED_GRAPHS", {})
+    monkeypatch.setattr(engine, "_GROUPED_RECENT", {})
+    monkeypatch.setattr(engine, "DESCENT_MIN_WORK", 0)
+    runs, real = [], engine.GroupedFitGraph.run
+    monkeypatch.setattr(engine.GroupedFitGraph, "run", lambda self, *a: (runs.append(self), real(self, *a))[1])
+    steps = [(Y, designs, gid, 0), (Y, designs, gid, 1), (Y[:, ::-1].copy(), designs, gid, 2), (Y, ramp, gid, 3),
+             (Y, designs, gid, 4), (Y, designs, other, 4), (Y, designs, gid, 5), (Y, ramp, other, 6), (Y, ramp, gid, 7)]
+    for data, xs, groups, replays in steps:
+        graph = fit_glm_arma11_grouped(data, xs, groups, tr=2.0, cuda_graphs=True, **kw)
+        assert len(runs) == replays
+        eager = fit_glm_arma11_grouped(data, xs, groups, tr=2.0, cuda_graphs=False, **kw)
+        for name in ("arma_params", "reml_likelihood", "betas", "tstats", "sigma2", "fstats", "r2", "residuals",
+                     "residuals_whitened"):
+            np.testing.assert_array_equal(getattr(graph, name).numpy(), getattr(eager, name).numpy(), err_msg=name)
+    assert len(engine._GROUPED_GRAPHS) == 2
