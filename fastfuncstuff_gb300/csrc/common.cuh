@@ -174,6 +174,12 @@ inline cudaError_t ensure_dyn_smem(const void* fn, size_t bytes) {
   return e;
 }
 
+// Shared memory of surface_kernel's tables for series of T samples (search.cu), and the
+// most it may be: a series whose tables do not fit has no criterion, whichever kernel
+// forms it, so that the selectors take the same series whatever the number of voxels.
+size_t surface_smem(int T);
+constexpr size_t SURFACE_SMEM_MAX = 227 * 1024;
+
 // SM count of the current device, looked up once per device
 inline cudaError_t sm_count(int* n) {
   static std::mutex mu;

@@ -523,6 +523,7 @@ int check_descent(const ffs_descent_args* a) {
   FFS_REQUIRE(a && a->V > 0 && a->T > a->K && a->K > 0 && a->K <= 256 && a->P > 0 && a->n_designs > 0 &&
                   a->ld >= a->T && a->ld % 64 == 0,
               "ffs_reml_descent: bad sizes");
+  FFS_REQUIRE(surface_smem(a->T) <= SURFACE_SMEM_MAX, "ffs_reml_descent: T=%d too long", a->T);
   FFS_REQUIRE((long long)a->P * a->n_designs < (1 << 24), "ffs_reml_descent: too many pairs");
   FFS_REQUIRE(a->p0 >= 0 && a->p0 < a->P && a->za >= 0 && a->za < a->n_a && a->zb >= 0 && a->zb < a->n_b,
               "ffs_reml_descent: (0, 0) outside the lattice");

@@ -930,6 +930,10 @@ __global__ void __launch_bounds__(128) project_simt_kernel(ffs_project_args a) {
 
 }  // namespace
 
+size_t surface_smem(int T) {
+  return (sizeof(float4) * (SURF_G2 + 1) + 1) * (size_t)T + sizeof(float) * SURF_G + ceil_div(T, SURF_TB);
+}
+
 }  // namespace ffsk
 
 using namespace ffsk;
@@ -982,9 +986,8 @@ extern "C" int ffs_reml_surface(const ffs_surface_args* a, void* stream) {
   FFS_REQUIRE(a->yr_t && a->coef && a->logdet_R && a->logdet_XtX && a->proj && a->chunk_start &&
                   a->chunk_pairs && a->surf && a->crit0,
               "ffs_reml_surface: null buffer");
-  const size_t smem = (sizeof(float4) * (SURF_G2 + 1) + 1) * (size_t)a->T + sizeof(float) * SURF_G +
-                      ceil_div(a->T, SURF_TB);
-  FFS_REQUIRE(smem <= 227 * 1024, "ffs_reml_surface: T=%d too long", a->T);
+  const size_t smem = surface_smem(a->T);
+  FFS_REQUIRE(smem <= SURFACE_SMEM_MAX, "ffs_reml_surface: T=%d too long", a->T);
   FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(surface_kernel), smem));
   FFS_REQUIRE(ceil_div(a->V, SURF_THREADS) <= 65535, "ffs_reml_surface: V=%d exceeds one launch", a->V);
   dim3 grid(a->n_chunks, ceil_div(a->V, SURF_THREADS));

@@ -93,3 +93,27 @@ def test_grouped_graph_replays_other_data_and_other_designs(monkeypatch):
                      "residuals_whitened"):
             np.testing.assert_array_equal(getattr(graph, name).numpy(), getattr(eager, name).numpy(), err_msg=name)
     assert len(engine._GROUPED_GRAPHS) == 2
+
+
+@pytest.mark.parametrize("T,takes", [(1000, True), (1601, True), (1602, False), (2000, False)])
+def test_the_descent_takes_the_series_that_the_surface_takes(T, takes):
+    """Length limits are checked on the host: a hierarchical fit is refused for
+    the same series whether its voxels are many (descent) or few (surface)."""
+    import ctypes as C
+
+    from fastfuncstuff_gb300 import _lib
+
+    lib, fake = _lib.load(), 256
+    ld = (T + 63) // 64 * 64
+    d = _lib.DescentArgs(V=100, T=T, K=5, P=545, n_designs=1, ld=ld, n_a=33, n_b=33, za=16, zb=16, ltop=4, n_groups=6,
+                         n_list=49, n_rounds=2, n_cell_groups=500, n_chunks=40)
+    n = lib.ffs_reml_descent_work_bytes(C.byref(d))
+    assert (n > 0) == takes
+    if not takes:
+        assert "too long" in lib.ffs_last_error().decode()
+        s = _lib.SurfaceArgs(V=100, T=T, K=5, P=545, p0=0, n_chunks=40, **{k: fake for k in (
+            "yr_t", "coef", "logdet_R", "logdet_XtX", "proj", "chunk_start", "chunk_pairs", "surf", "crit0")})
+        assert lib.ffs_reml_surface(C.byref(s), None) == _lib.FFS_ERR_INVALID
+        assert "too long" in lib.ffs_last_error().decode()
+    d.T, d.ld = 100, 128
+    assert lib.ffs_reml_descent_work_bytes(C.byref(d)) > 0  # leaves no message behind
