@@ -287,6 +287,7 @@ struct TopArgs {
   double* crit0;             // [V]
   int* best;                 // outputs of the last level
   float* best_crit;
+  const int* flag;           // set: a projection gave up, and the criterion is a NaN
 };
 
 // At most 80 registers: with the 118 that the compiler takes by itself one CTA
@@ -365,7 +366,7 @@ __global__ void __maxnreg__(80) descent_top_kernel(TopArgs a) {
   a.crit0[vo] = cr0;
   if (a.lev_stop == 0) {
     a.best[vo] = p;
-    a.best_crit[vo] = (float)(cr0 + (double)bl);
+    a.best_crit[vo] = *a.flag ? NAN : (float)(cr0 + (double)bl);
   }
 }
 
@@ -414,6 +415,7 @@ struct RoundArgs {
   float* low;
   int* best;                 // last round only
   float* best_crit;
+  const int* flag;
 };
 
 // A thread per row of the tile, its cell's 8 neighbours in registers; the
@@ -461,7 +463,7 @@ __global__ void __launch_bounds__(ROUND_ROWS, 5) descent_round_kernel(RoundArgs 
   }
   if (a.best) {
     a.best[v] = p;
-    a.best_crit[v] = (float)(a.crit0[v] + (double)bl);
+    a.best_crit[v] = *a.flag ? NAN : (float)(a.crit0[v] + (double)bl);
   } else {
     a.key[v] = dsg * a.P + p;
     a.low[v] = bl;
@@ -593,7 +595,7 @@ extern "C" int ffs_reml_descent(const ffs_descent_args* a, void* stream) {
 
   TopArgs ta{a->V, T, T - a->K, a->P, a->p0, a->n_groups, a->n_a, a->n_b, a->za, a->zb, a->ltop, a->n_rounds,
              a->rows, w.top, a->slots, a->lat_slot, a->lattice, w.proj, a->logdet_R, a->logdet_XtX, a->tile_design,
-             w.key, w.low, w.rss0, w.crit0, a->best, a->best_crit};
+             w.key, w.low, w.rss0, w.crit0, a->best, a->best_crit, a->flag};
   const size_t top_smem = sizeof(Stage<2>) * D_BUF * a->n_groups +
                           sizeof(float) * TOP_ROWS * (D_BUF * D_LD + a->n_groups * D_SLOTS);
   FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(descent_top_kernel), top_smem));
@@ -625,7 +627,8 @@ extern "C" int ffs_reml_descent(const ffs_descent_args* a, void* stream) {
     const bool last = r + 1 == a->n_rounds;
     RoundArgs ra{T, T - a->K, a->P, a->p0, a->rows, w.order, w.tiles, w.counts, w.cells,
                  a->cell_group + (size_t)r * a->P, a->cell_pairs + (size_t)r * a->P * D_SLOTS, w.proj, a->logdet_R,
-                 a->logdet_XtX, w.rss0, w.crit0, w.key, w.low, last ? a->best : nullptr, a->best_crit};
+                 a->logdet_XtX, w.rss0, w.crit0, w.key, w.low, last ? a->best : nullptr, a->best_crit,
+                 a->flag};
     FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(descent_round_kernel), round_smem));
     descent_round_kernel<<<max_tiles, ROUND_ROWS, round_smem, st>>>(ra);
   }

@@ -435,7 +435,7 @@ def fit_glm_arma11(
     chunks = {k: [] for k in ("best", "crit", "surf", "betas", "tstats", "sigma2", "fstats", "r2", "lam",
                               "cb", "ct", "resid", "resid_w", "pred", "lb", "scale")}
     factors_used = factors
-    dchunks = []
+    dchunks, waits = [], []  # waits: device flags of the searches' bounded waits
     proj = "tc" if factors is None else _projector(factors)
     if proposal is not None and best_all is None:
         from . import learned
@@ -501,12 +501,14 @@ def fit_glm_arma11(
             so, go = gplan.run(Yb, _group_designs[0])
             factors_used = gplan.f
             best, scale = so.best, so.scale
+            waits.append(so._flag)
             chunks["best"].append(best)
             chunks["crit"].append(so.best_crit)
         elif slots is not None:
             so = engine.search_designs(Yb, factors, slots, hierarchical=not force_exhaustive_search,
                                        do_scale=not use_double)
             best, scale = so.best, so.scale
+            waits.append(so._flag)
             chunks["best"].append(best)
             chunks["crit"].append(so.best_crit)
             go = engine.gls(Yb, scale, best, factors, _group_designs[0], want_residuals=want_residuals,
@@ -515,6 +517,7 @@ def fit_glm_arma11(
             so = engine.search(Yb, factors, hierarchical=not force_exhaustive_search, projector=proj,
                                do_scale=not use_double, keep_surface=save_profile_likelihoods, q0=q0, join=join)
             best, scale = so.best, so.scale
+            waits.append(so._flag)
             chunks["best"].append(best)
             chunks["crit"].append(so.best_crit)
             if save_profile_likelihoods:
@@ -627,8 +630,13 @@ def fit_glm_arma11(
         res.voxel_mask = spatial_metadata.get("voxel_mask")
         res.full_shape = spatial_metadata.get("volume_shape")
         res.affine = spatial_metadata.get("affine")
+    gave_up = None
+    if waits and not return_device:  # results left on the device are not waited for
+        gave_up = out(waits[0] if len(waits) == 1 else torch.cat(waits), torch.int32)
     if pending:
         torch.cuda.current_stream(device).synchronize()
+    if gave_up is not None and any(gave_up.tolist()):
+        raise RuntimeError("ffs_reml_project_tc: a bounded wait expired in the search; its results are not valid")
     if verbose:
         print(f"ARMA(1,1) REML: {V:,} voxels x {P} pairs, T={T}, K={K} on {torch.cuda.get_device_name(device)}")
     return res

@@ -1237,6 +1237,7 @@ class GroupedFitGraph:
         so = SearchOut(best=self.so.best.clone(), best_crit=self.so.best_crit.clone(), scale=self.so.scale.clone())
         go = GlsOut(**{k: (None if v is None else v.clone()) for k, v in vars(self.go).items()
                        if not k.startswith("_")})
+        so._flag = self.so._flag
         return so, go
 
 

@@ -427,7 +427,8 @@ int ffs_reml_select(const ffs_select_args* a, void* stream);
  * chunk_start / chunk_pairs: the grid's surface chunks (ffs_surface_args): they
  * decide how each pair's sums are blocked. Rows of several designs come in
  * tiles of 256 of one design (tile_design), as ffs_reml_prep lays them out;
- * U and logdet_XtX are then [n_designs][P]. flag as in ffs_project_args. */
+ * U and logdet_XtX are then [n_designs][P]. flag as in ffs_project_args; when it is
+ * set, best_crit is a NaN. Series as long as ffs_reml_surface takes them. */
 typedef struct {
   int V, T, K, P, n_designs, ld;
   int p0, n_a, n_b, za, zb, ltop;

@@ -117,3 +117,36 @@ def test_the_descent_takes_the_series_that_the_surface_takes(T, takes):
         assert "too long" in lib.ffs_last_error().decode()
     d.T, d.ld = 100, 128
     assert lib.ffs_reml_descent_work_bytes(C.byref(d)) > 0  # leaves no message behind
+
+
+@gpu
+@pytest.mark.parametrize("path", ["surface", "descent", "grouped"])
+def test_a_wait_that_ran_out_in_the_search_is_reported(path, monkeypatch):
+    """The projection kernels leave at once when their flag is set, as they do
+    after a wait that ran out: results for the host raise, and the descent's
+    criterion on the device is a NaN."""
+    from fastfuncstuff_gb300 import fit_glm_arma11, fit_glm_arma11_grouped
+    from fastfuncstuff_gb300.glm import engine
+
+    Y, X, _ = arma_data(5, 300, 90, 4)
+    ax = np.linspace(-0.8, 0.8, 33)
+    kw = dict(a_grid=ax, b_grid=ax, device=DEV, verbose=False)
+    monkeypatch.setattr(engine, "DESCENT_MIN_WORK", 1 << 60 if path == "surface" else 0)
+
+    def fit(**more):
+        if path == "grouped":
+            return fit_glm_arma11_grouped(Y, {0: X, 1: X[::-1].copy()}, np.arange(300) % 2, tr=2.0, cuda_graphs=False,
+                                          **kw, **more)
+        return fit_glm_arma11(Y, X, tr=2.0, **kw, **more)
+
+    assert torch.isfinite(fit().reml_likelihood).all()
+    real = torch.zeros
+
+    def preset(*size, **k):
+        return real(*size, **k).fill_(1) if size == (1,) and k.get("dtype") is torch.int32 else real(*size, **k)
+
+    monkeypatch.setattr(engine.torch, "zeros", preset)
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        fit()
+    if path != "surface":
+        assert torch.isnan(fit(return_device=True).reml_likelihood).all()
