@@ -150,3 +150,17 @@ def test_a_wait_that_ran_out_in_the_search_is_reported(path, monkeypatch):
         fit()
     if path != "surface":
         assert torch.isnan(fit(return_device=True).reml_likelihood).all()
+
+
+def test_small_batches_are_not_split_by_the_free_memory(monkeypatch):
+    """The free memory decides the batch only where it is large: a fit of a few
+    hundred voxels does not ask for it."""
+    from fastfuncstuff_gb300.glm import arma
+
+    asked = []
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d=None: (asked.append(d), (1 << 28, 1 << 30))[1])
+    assert arma._batch_size(200, 200, 117, 8, None, DEV) == 200 and not asked
+    assert arma._batch_size(0, 200, 117, 8, None, DEV) == 1 and not asked
+    assert arma._batch_size(200, 200, 117, 8, 64, DEV) == 64 and not asked
+    per_voxel = 4 * (3 * 545 + 6 * 400 + 4 * 20 + 16)
+    assert arma._batch_size(200_000, 400, 545, 20, None, DEV) == (1 << 27) // per_voxel and len(asked) == 1
