@@ -31,7 +31,7 @@ class GridDesc(C.Structure):
         ("X", C.c_void_p), ("lambda_fp32", C.c_int), ("ld_u", C.c_int),
         ("n_task", C.c_int), ("task_idx", C.c_void_p), ("n_glt", C.c_int), ("glt", C.c_void_p),
         ("n_sets", C.c_int), ("set_ptr", C.c_void_p), ("set_idx", C.c_void_p),
-        ("band_w", C.c_int), ("band", C.c_void_p), ("p0", C.c_int),
+        ("band_w", C.c_int), ("band", C.c_void_p),
     ]
 
 
@@ -43,7 +43,6 @@ class GridOut(C.Structure):
         ("Adiag", C.c_void_p), ("XtX", C.c_void_p), ("info", C.c_void_p), ("Ftask", C.c_void_p),
         ("glt_var", C.c_void_p), ("Gsum", C.c_void_p), ("work", C.c_void_p), ("Fsets", C.c_void_p),
         ("Afull", C.c_void_p), ("band_L", C.c_void_p), ("band_coef", C.c_void_p),
-        ("const_flag", C.c_void_p), ("const_coef", C.c_void_p),
     ]
 
 
@@ -168,6 +167,8 @@ SIGNATURES = {
     "ffs_grid_build": ([C.POINTER(GridDesc), C.POINTER(GridOut), C.c_void_p], C.c_int),
     "ffs_grid_work_bytes_designs": ([C.c_int, C.c_int, C.c_int, C.c_int, C.c_int], C.c_size_t),
     "ffs_grid_build_designs": ([C.POINTER(GridDesc), C.c_int, C.c_int, C.POINTER(GridOut), C.c_void_p], C.c_int),
+    "ffs_grid_build_centred": ([C.POINTER(GridDesc), C.c_int, C.c_int, C.POINTER(GridOut), C.c_int, C.c_void_p,
+                                C.c_void_p, C.c_void_p], C.c_int),
     "ffs_grid_build_noalloc": ([C.POINTER(GridDesc), C.POINTER(GridOut), C.c_void_p], C.c_int),
     "ffs_reml_prep": ([C.POINTER(PrepArgs), C.c_void_p], C.c_int),
     "ffs_reml_project_tc": ([C.POINTER(ProjectArgs), C.c_void_p], C.c_int),

@@ -234,6 +234,10 @@ __device__ __forceinline__ void sub_block_inverse(const PairScratch& s, int K, c
 struct BuildArgs {
   ffs_grid_desc d;
   ffs_grid_out o;
+  // the centring test (ffs_grid_build_centred), or NULL
+  int p0;
+  int* const_flag;
+  float* const_coef;
 };
 
 // Reciprocal of n by Newton's iteration r <- r (2 - n r) from the fp32 one
@@ -775,9 +779,9 @@ __global__ void __launch_bounds__(GB_THREADS) pair_ldl_kernel(BuildArgs args, do
 // ||X c - 1||^2 <= 1e-12 T; *const_flag stays 1 only if every design passes.
 // w: 2 K doubles of scratch (a slot's A, whose K x K doubles the S of the same
 // size follows: S alone is too short at K = 1). Ends with a barrier.
-__device__ void const_of_design(const ffs_grid_desc& d, const ffs_grid_out& o, int dsg, const float* Xd,
-                                const double* Li, int ldi, bool chol, double* w, double* red) {
-  const int T = d.T, K = d.K;
+__device__ void const_of_design(const BuildArgs& args, int dsg, const float* Xd, const double* Li, int ldi, bool chol,
+                                double* w, double* red) {
+  const int T = args.d.T, K = args.d.K;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();
   for (int j = wid; j < K; j += nw) {  // X'1
@@ -807,8 +811,8 @@ __device__ void const_of_design(const ffs_grid_desc& d, const ffs_grid_out& o, i
   }
   const double ss = block_sum(part, red);
   const bool ok = chol && ss <= 1e-12 * (double)T;
-  for (int j = threadIdx.x; j < K; j += blockDim.x) o.const_coef[(size_t)dsg * K + j] = ok ? (float)w[K + j] : 0.f;
-  if (threadIdx.x == 0 && !ok) atomicAnd(o.const_flag, 0);
+  for (int j = threadIdx.x; j < K; j += blockDim.x) args.const_coef[(size_t)dsg * K + j] = ok ? (float)w[K + j] : 0.f;
+  if (threadIdx.x == 0 && !ok) atomicAnd(args.const_flag, 0);
   __syncthreads();
 }
 
@@ -1081,7 +1085,7 @@ __device__ __noinline__ void item_global(const BuildArgs& args, const PairScratc
   }
   __syncthreads();
 
-  if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, s.Li, K, chol, s.A, red);
+  if (args.const_flag && p == args.p0) const_of_design(args, pd / d.P, Xd, s.Li, K, chol, s.A, red);
 
   // ---- 8. G = U Lx^-1 in fp32 (row t of G solves g Lx = u_t); Gsum = G' 1
   // accumulated in FP64
@@ -1752,7 +1756,7 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
         o.Afull[(size_t)pd * K * K + e] = (float)a;
       }
     }
-    if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, Li, K, true, scr, red);
+    if (args.const_flag && p == args.p0) const_of_design(args, pd / d.P, Xd, Li, K, true, scr, red);
     __syncthreads();
 
     // ---- 8. G = U Lx^-1 in fp32, two samples per thread, four columns per pass over U
@@ -2232,7 +2236,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == WI_WIDE ? 2 : SHARED_LDL ?
         }
       }
     }
-    if (o.const_flag && p == d.p0) const_of_design(d, o, pd / d.P, Xd, s.Li, K, true, s.A, red);
+    if (args.const_flag && p == args.p0) const_of_design(args, pd / d.P, Xd, s.Li, K, true, s.A, red);
 
     // ---- 8. G = U Lx^-1 in fp32
     for (int t2 = tid; t2 < LT / 2; t2 += nth) {
@@ -2528,8 +2532,6 @@ static int launch_items(const ffsk::BuildArgs& args, int n_designs, int grid, co
   const ffs_grid_desc& d = args.d;
   const ffs_grid_out& o = args.o;
   FFS_REQUIRE(!too_long(d), "%s: T=%d too long", who, d.T);
-  FFS_REQUIRE(!o.const_flag == !o.const_coef && (!o.const_flag || (d.p0 >= 0 && d.p0 < d.P)),
-              "%s: const_flag and const_coef go together, with p0=%d in [0, P)", who, d.p0);
   int sms = 0;
   FFS_CUDA(sm_count(&sms));
   const long long items = (long long)d.P * n_designs;
@@ -2577,7 +2579,14 @@ static int check_sets(const ffs_grid_desc* d, const ffs_grid_out* o, const char*
   return FFS_OK;
 }
 
-extern "C" int ffs_grid_build(const ffs_grid_desc* d, const ffs_grid_out* o, void* stream) {
+// The centring test of a build (ffs_grid_build_centred).
+struct Centring {
+  int p0;
+  int* flag;
+  float* coef;
+};
+
+static int build_single(const ffs_grid_desc* d, const ffs_grid_out* o, const Centring& c, void* stream) {
   using namespace ffsk;
   clear_error();
   FFS_REQUIRE(d && o, "ffs_grid_build: null descriptor");
@@ -2597,11 +2606,16 @@ extern "C" int ffs_grid_build(const ffs_grid_desc* d, const ffs_grid_out* o, voi
   FFS_REQUIRE(!d->band || (d->band_w >= 1 && d->band_w <= FFS_BAND_MAX_W && o->band_L && o->band_coef),
               "ffs_grid_build: the banded R needs 1 <= band_w=%d <= %d, band_L and band_coef", d->band_w,
               FFS_BAND_MAX_W);
-  return launch_items(BuildArgs{*d, *o}, 1, d->P, nullptr, nullptr, (cudaStream_t)stream, "ffs_grid_build");
+  return launch_items(BuildArgs{*d, *o, c.p0, c.flag, c.coef}, 1, d->P, nullptr, nullptr, (cudaStream_t)stream,
+                      "ffs_grid_build");
 }
 
-extern "C" int ffs_grid_build_designs(const ffs_grid_desc* d, int n_designs, int max_ctas, const ffs_grid_out* o,
-                                      void* stream) {
+extern "C" int ffs_grid_build(const ffs_grid_desc* d, const ffs_grid_out* o, void* stream) {
+  return build_single(d, o, Centring{}, stream);
+}
+
+static int build_designs(const ffs_grid_desc* d, int n_designs, int max_ctas, const ffs_grid_out* o, const Centring& c,
+                         void* stream) {
   using namespace ffsk;
   clear_error();
   FFS_REQUIRE(d && o, "ffs_grid_build_designs: null descriptor");
@@ -2624,7 +2638,7 @@ extern "C" int ffs_grid_build_designs(const ffs_grid_desc* d, int n_designs, int
   const long long items = (long long)d->P * n_designs;
   const long long cap = max_ctas > 0 && max_ctas < FFS_GRID_MAX_SLOTS ? max_ctas : FFS_GRID_MAX_SLOTS;
   const int grid = (int)(items < cap ? items : cap);
-  BuildArgs args{*d, *o};
+  BuildArgs args{*d, *o, c.p0, c.flag, c.coef};
   double* pair_cm = nullptr;
   int* pair_bad = nullptr;
   if (n_designs > 1) {
@@ -2637,6 +2651,21 @@ extern "C" int ffs_grid_build_designs(const ffs_grid_desc* d, int n_designs, int
     if (const int rc = check_launch("pair_ldl_kernel")) return rc;
   }
   return launch_items(args, n_designs, grid, pair_cm, pair_bad, (cudaStream_t)stream, "ffs_grid_build_designs");
+}
+
+extern "C" int ffs_grid_build_designs(const ffs_grid_desc* d, int n_designs, int max_ctas, const ffs_grid_out* o,
+                                      void* stream) {
+  return build_designs(d, n_designs, max_ctas, o, Centring{}, stream);
+}
+
+extern "C" int ffs_grid_build_centred(const ffs_grid_desc* d, int n_designs, int max_ctas, const ffs_grid_out* o, int p0,
+                                      int* const_flag, float* const_coef, void* stream) {
+  ffsk::clear_error();
+  FFS_REQUIRE(d && const_flag && const_coef, "ffs_grid_build_centred: null argument");
+  FFS_REQUIRE(p0 >= 0 && p0 < d->P, "ffs_grid_build_centred: p0=%d outside [0, P)", p0);
+  const Centring c{p0, const_flag, const_coef};
+  return n_designs == 1 && max_ctas <= 0 ? build_single(d, o, c, stream)
+                                         : build_designs(d, n_designs, max_ctas, o, c, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -2719,7 +2748,7 @@ extern "C" int ffs_grid_build_noalloc(const ffs_grid_desc* d, const ffs_grid_out
   if (!scratch) return st;
   // every scratch entry the kernel reads it writes first in the same launch, so
   // the previous call's contents need no clearing
-  BuildArgs args{*d, *o};
+  BuildArgs args{*d, *o, 0, nullptr, nullptr};
   args.o.work = scratch;
   return launch_items(args, 1, d->P, nullptr, nullptr, (cudaStream_t)stream, "ffs_grid_build_noalloc");
 }

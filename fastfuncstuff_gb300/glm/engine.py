@@ -470,16 +470,18 @@ def build_factors(X: torch.Tensor, grid: RemlGrid, layout: RunLayout, *, task_in
                       a=_p(a), b=_p(b), X=_p(Xc), lambda_fp32=0, ld_u=ld,
                       n_task=nt, task_idx=_p(task_idx), n_glt=ng, glt=_p(glt_t),
                       n_sets=sets.n_sets if f.Fsets is not None else 0, set_ptr=_p(sets_dev[0]),
-                      set_idx=_p(sets_dev[1]), band_w=f.band_w, band=_p(f.band), p0=grid.p0)
+                      set_idx=_p(sets_dev[1]), band_w=f.band_w, band=_p(f.band))
     # no Gsum from the kernel: G'1 is the FP64 coefficient vector of the constant (set below)
     o = _lib.GridOut(coef=_p(f.coef), logdet_R=_p(f.logdet_R), logdet_XtX=_p(f.logdet_XtX), U=_p(f.U),
                      U_hi=_p(f.U_hi), U_lo=_p(f.U_lo), uexp=_p(f.uexp), G=_p(f.G), Adiag=_p(f.Adiag), XtX=_p(f.XtX),
                      info=_p(f.info), Ftask=_p(f.Ftask), glt_var=_p(f.glt_var), Gsum=None, work=_p(work),
-                     Fsets=_p(f.Fsets), Afull=_p(f.Afull), band_L=_p(f.band_L), band_coef=_p(f.band_coef),
-                     const_flag=_p(cflag) if own_center else None, const_coef=_p(ccoef) if own_center else None)
+                     Fsets=_p(f.Fsets), Afull=_p(f.Afull), band_L=_p(f.band_L), band_coef=_p(f.band_coef))
 
     def launch():
-        if single:
+        if own_center:
+            _run("ffs_grid_build" if single else "ffs_grid_build_designs", lib.ffs_grid_build_centred, C.byref(d), D,
+                 max_ctas, C.byref(o), grid.p0, _p(cflag), _p(ccoef), _stream(), launches=2 if D > 1 else 1)
+        elif single:
             _run("ffs_grid_build", lib.ffs_grid_build, C.byref(d), C.byref(o), _stream())
         else:
             # more than one design: a pre-pass factors R once per pair

@@ -108,7 +108,6 @@ typedef struct {
    * exact ARMA(1,1) R. */
   int band_w;
   const int* band;      /* device [P] or NULL                                    */
-  int p0;               /* a pair with lambda == 0 (read with const_flag)        */
 } ffs_grid_desc;
 
 typedef struct {
@@ -136,12 +135,6 @@ typedef struct {
    * whitening w_t = y_t band_coef[t][0] - sum_j band_coef[t][j] w_{t-j}. */
   double* band_L;
   float* band_coef;
-  /* The centring test of ffs_design_basis from pair p0's factor (both or
-   * neither): *const_flag, 1 on entry, is set to 0 when the constant series
-   * is not in the span of some design; const_coef [n_designs][K] its
-   * coefficients, 0 for such a design. */
-  int* const_flag;
-  float* const_coef;
 } ffs_grid_out;
 
 size_t ffs_grid_work_bytes(int T, int K, int P);
@@ -162,6 +155,13 @@ int ffs_grid_build(const ffs_grid_desc* d, const ffs_grid_out* o, void* stream);
 #define FFS_GRID_MAX_SLOTS 2048
 size_t ffs_grid_work_bytes_designs(int T, int K, int P, int n_designs, int max_ctas);
 int ffs_grid_build_designs(const ffs_grid_desc* d, int n_designs, int max_ctas, const ffs_grid_out* o, void* stream);
+
+/* ffs_grid_build (n_designs = 1, max_ctas = 0) or ffs_grid_build_designs, with the
+ * centring test of ffs_design_basis from the factor of pair p0, one with lambda == 0:
+ * *const_flag, 1 on entry, is set to 0 when the constant series is not in the span
+ * of some design; const_coef [n_designs][K] its coefficients, 0 for such a design. */
+int ffs_grid_build_centred(const ffs_grid_desc* d, int n_designs, int max_ctas, const ffs_grid_out* o, int p0,
+                           int* const_flag, float* const_coef, void* stream);
 
 /* ffs_grid_build without a workspace argument: this variant has no counterpart
  * in the reference. It is for callers that cannot allocate device memory where

@@ -156,3 +156,14 @@ def C_sizeof(py) -> int:
     import ctypes
 
     return ctypes.sizeof(py)
+
+
+def test_structures_that_callers_fill_keep_their_layout():
+    """The grid build's structures as programs were compiled against them: a
+    longer one would be read past its end. New arguments come by new entry
+    points (ffs_grid_build_centred)."""
+    assert (C_sizeof(_lib.GridDesc), _lib.GridDesc.band.offset) == (136, 128)
+    assert (C_sizeof(_lib.GridOut), _lib.GridOut.band_coef.offset) == (152, 144)
+    lib = _lib.load()
+    assert lib.ffs_grid_build_centred(None, 1, 0, None, 0, None, None, None) == _lib.FFS_ERR_INVALID
+    assert "ffs_grid_build_centred" in lib.ffs_last_error().decode()
