@@ -304,11 +304,13 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kerne
       if (lane == 0) a.yexp[v] = e;
       if (!a.yr_hi) continue;
       const float4* row4 = reinterpret_cast<const float4*>(Ys + (size_t)i * ld);
-      // four samples per lane: 8-byte words of hi and lo (ld_y is a multiple of 8);
+      // four samples per lane: 8-byte words of hi and lo (ld_y is a multiple of 8),
+      // 4-byte ones where the buffers start between them;
       // x * 2^e as one product when 2^e is a normal float (then the same
       // correctly rounded value as ldexpf)
-      uint2* hi = reinterpret_cast<uint2*>(a.yr_hi + (size_t)v * a.ld_y);
-      uint2* lo = reinterpret_cast<uint2*>(a.yr_lo + (size_t)v * a.ld_y);
+      uint32_t* hi = reinterpret_cast<uint32_t*>(a.yr_hi + (size_t)v * a.ld_y);
+      uint32_t* lo = reinterpret_cast<uint32_t*>(a.yr_lo + (size_t)v * a.ld_y);
+      const bool word8 = (((uintptr_t)a.yr_hi | (uintptr_t)a.yr_lo) & 7) == 0;
       const bool pw = e >= -126 && e <= 127;
       const float p2 = pw ? __int_as_float((e + 127) << 23) : 0.f;
       for (int q = lane; q < (a.ld_y >> 2); q += 32) {
@@ -320,8 +322,15 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kerne
         uint2 h, l;
         split_fp16x2(x.x, x.y, h.x, l.x);
         split_fp16x2(x.z, x.w, h.y, l.y);
-        hi[q] = h;
-        lo[q] = l;
+        if (word8) {
+          reinterpret_cast<uint2*>(hi)[q] = h;
+          reinterpret_cast<uint2*>(lo)[q] = l;
+        } else {
+          hi[2 * q] = h.x;
+          hi[2 * q + 1] = h.y;
+          lo[2 * q] = l.x;
+          lo[2 * q + 1] = l.y;
+        }
       }
     }
   }

@@ -164,3 +164,27 @@ def test_small_batches_are_not_split_by_the_free_memory(monkeypatch):
     assert arma._batch_size(200, 200, 117, 8, 64, DEV) == 64 and not asked
     per_voxel = 4 * (3 * 545 + 6 * 400 + 4 * 20 + 16)
     assert arma._batch_size(200_000, 400, 545, 20, None, DEV) == (1 << 27) // per_voxel and len(asked) == 1
+
+
+@gpu
+@pytest.mark.parametrize("T", [3, 130])
+def test_prep_writes_splits_that_start_between_eight_byte_words(T):
+    """The fp16 splits into buffers on 4-byte boundaries equal those on 8-byte
+    ones (stored by narrower words)."""
+    import ctypes as C
+
+    from fastfuncstuff_gb300 import _lib
+
+    V, ld = 37, (T + 7) // 8 * 8
+    Y = torch.randn(V, T, device=DEV)
+    scale, yexp = torch.empty(V, device=DEV), torch.empty(V, dtype=torch.int32, device=DEV)
+    out = []
+    for off in (0, 2):
+        hi, lo = (torch.full((V * ld + 8,), 77, dtype=torch.int16, device=DEV) for _ in range(2))
+        a = _lib.PrepArgs(V=V, T=T, K=0, Y=Y.data_ptr(), do_scale=1, center=0, ld_y=ld, scale=scale.data_ptr(),
+                          yr_hi=hi.data_ptr() + 2 * off, yr_lo=lo.data_ptr() + 2 * off, yexp=yexp.data_ptr())
+        _lib.check(_lib.load().ffs_reml_prep(C.byref(a), torch.cuda.current_stream().cuda_stream), "ffs_reml_prep")
+        torch.cuda.synchronize()
+        assert all((x[:off] == 77).all() and (x[off + V * ld :] == 77).all() for x in (hi, lo))
+        out.append(torch.stack([hi[off : off + V * ld], lo[off : off + V * ld]]))
+    assert torch.equal(out[0], out[1])
