@@ -2335,8 +2335,10 @@ __global__ void __launch_bounds__(256) design_gram_kernel(int T, int K, int chun
     else if (mine)
       acc.run(xt + i * ld, xt + j * ld, n);
   }
+  // a sample that is not finite leaves the fixed point: no factor, as its FP64 sums give none
+  if (fixed) over = __syncthreads_or(over);
   if (mine)
-    gram[e] = fixed ? fx.value(fixed_scale(__int_as_float(cmax[i])), fixed_scale(__int_as_float(cmax[j]))) : acc.sum();
+    gram[e] = over ? (double)NAN : fixed ? fx.value(fixed_scale(__int_as_float(cmax[i])), fixed_scale(__int_as_float(cmax[j]))) : acc.sum();
 }
 
 __global__ void __launch_bounds__(DB_THREADS) design_basis_kernel(int T, int K, const float* __restrict__ X,

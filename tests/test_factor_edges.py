@@ -238,3 +238,21 @@ def test_a_design_factors_are_its_own_whatever_is_built_beside_it(T, K, runs, D,
             a, b = getattr(one, name), getattr(part, name)
             if a is not None:
                 assert torch.equal(a.reshape(-1).view(torch.uint8), b.reshape(-1).view(torch.uint8)), (d, name)
+
+
+@gpu
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("T,K", [(150, 5), (400, 40), (150, 50), (1100, 5)])
+def test_design_basis_of_a_design_that_is_not_finite(value, T, K):
+    """A sample of the design that is not finite leaves no basis of its column
+    (none of it finite) and no centring, whichever way the Gram entries are
+    summed (fixed point up to 40 columns and 1,024 samples, else FP64)."""
+    from fastfuncstuff_gb300.glm import engine
+
+    X = np.random.default_rng(K).standard_normal((T, K)).astype(np.float32)
+    X[:, 0] = 1.0
+    X[T // 2, 2] = value
+    q0, flag, coef = engine.design_basis(torch.from_numpy(X).to(DEV), with_constant=True)
+    torch.cuda.synchronize()
+    assert not torch.isfinite(q0[2, :T]).any()
+    assert int(flag) == 0 and (coef == 0).all()
