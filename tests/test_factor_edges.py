@@ -256,3 +256,52 @@ def test_design_basis_of_a_design_that_is_not_finite(value, T, K):
     torch.cuda.synchronize()
     assert not torch.isfinite(q0[2, :T]).any()
     assert int(flag) == 0 and (coef == 0).all()
+
+
+@gpu
+@pytest.mark.parametrize("T,K,runs,n", [(150, 8, 1, None), (203, 20, 3, 33), (203, 57, 3, None), (400, 130, 2, 3),
+                                        (1100, 6, 1, None)])
+def test_a_zero_column_goes_through_the_general_phases(T, K, runs, n):
+    """A column of zeros has no positive pivot: every kernel of the build sends
+    the item to the general phases (info 1), whose basis spans the other
+    columns: U'U = L^-T Q Q'L^-1 against a float64 QR of them (sums of K fp32
+    products on designs of condition below 30: K 2^-24 30, at least 1e-5)."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(T + K)
+    X = rng.standard_normal((T, K)).astype(np.float32)
+    X[:, K // 2] = 0.0
+    starts = [T * r // runs for r in range(runs)]
+    ax = G.get_default_arma_grids() if n is None else (torch.linspace(-0.8, 0.8, n),) * 2
+    g = G.make_grid(*ax, use_double=True)
+    f = engine.build_factors(torch.from_numpy(X).to(DEV), g, G.run_layout(T, starts), with_tc=True)
+    torch.cuda.synchronize()
+    assert (f.info.cpu().numpy() == 1).all()
+    rest = np.delete(X, K // 2, 1)
+    for p in range(0, g.P, max(1, g.P // 4)):
+        _, ld_x, U, _ = dense_factors(rest, g.a[p], g.b[p], starts)
+        got = f.U[p, :, :T].cpu().numpy().astype(np.float64)
+        assert (got[K // 2] == 0).all()
+        want = U.T @ U
+        assert np.abs(got.T @ got - want).max() <= max(1e-5, K * 2.0**-24 * 30) * np.abs(want).max()
+        # log |R_jj| + 1e-10 of the zero column
+        assert float(f.logdet_XtX[p]) == pytest.approx(ld_x + 2 * np.log(1e-10), rel=1e-9)
+
+
+@gpu
+@pytest.mark.parametrize("T,K,runs", [(200, 8, 1), (331, 13, 2), (400, 20, 4), (300, 31, 1), (1100, 12, 2)])
+def test_design_basis_is_the_grid_builds_to_rounding(T, K, runs):
+    """Q0 and U of (0, 0) come from FP64 factors that agree to their rounding
+    (the Gram entries' fixed points differ), rounded to fp32 each and carried
+    through the same fp32 recursion: within 4 roundings a column, K 2^-22 of
+    the largest entry on designs of condition below 4."""
+    from fastfuncstuff_gb300.glm import engine
+
+    X = np.random.default_rng(T).standard_normal((T, K)).astype(np.float32)
+    assert np.linalg.cond(X.astype(np.float64)) < 4
+    g = G.make_grid(*G.get_default_arma_grids())
+    Xd = torch.from_numpy(X).to(DEV)
+    f = engine.build_factors(Xd, g, G.run_layout(T, [T * r // runs for r in range(runs)]))
+    q0 = engine.design_basis(Xd)
+    torch.cuda.synchronize()
+    assert float((q0 - f.U[g.p0]).abs().max()) <= K * 2.0**-22 * float(q0.abs().max())

@@ -188,3 +188,32 @@ def test_prep_writes_splits_that_start_between_eight_byte_words(T):
         assert all((x[:off] == 77).all() and (x[off + V * ld :] == 77).all() for x in (hi, lo))
         out.append(torch.stack([hi[off : off + V * ld], lo[off : off + V * ld]]))
     assert torch.equal(out[0], out[1])
+
+
+@gpu
+def test_descent_scales_the_voxels_as_the_surface_does(monkeypatch):
+    """The voxel scales of both searches bit for bit, of zero, constant, huge and NaN series too."""
+    from fastfuncstuff_gb300.glm import engine
+
+    V, T, K = 260, 130, 7
+    Y, X, starts = arma_data(7, V, T, K, 2, baseline=50.0)
+    Y[3], Y[17], Y[40], Y[41, 5] = 0.0, 12.5, Y[40] * 1e18, np.nan
+    ax = torch.linspace(-0.8, 0.8, 33)
+    Yd = torch.from_numpy(Y).to(DEV)
+    f = engine.build_factors(torch.from_numpy(X).to(DEV), G.make_grid(ax, ax), G.run_layout(T, starts))
+    monkeypatch.setattr(engine, "DESCENT_MIN_WORK", 0)
+    assert engine._descent_plan(f, V) is not None
+    got, want = engine.search(Yd, f), engine.search(Yd, f, keep_surface=True)
+    assert torch.equal(got.scale.view(torch.int32), want.scale.view(torch.int32))
+
+
+@pytest.mark.parametrize("a_max,corcut,lags", [(0.3, 1e-2, 16), (0.8, 1e-4, 48), (0.8, 1e-12, 128)])
+def test_bands_of_the_banded_tests_reach_their_register_history(a_max, corcut, lags):
+    """The grids that the banded GLS and surface tests use take the history of
+    16, 48 and 128 lags that they are written for."""
+    G.set_afni_mode(True, corcut)
+    try:
+        band = int(G.make_grid(torch.linspace(0.0, a_max, 4), torch.linspace(-0.4, 0.4, 5)).band.max())
+    finally:
+        G.set_afni_mode(False)
+    assert {16: 0, 48: 16, 128: 48}[lags] < band <= lags
