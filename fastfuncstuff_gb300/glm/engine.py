@@ -671,6 +671,8 @@ def _descent_plan(f: GridFactors, V: int):
     better searched by it than over the full surface, else None."""
     if f.U_hi is None or f.band_coef is not None or V * f.P * f.T < DESCENT_MIN_WORK:
         return None
+    if f.P * f.n_designs >= DESCENT_MAX_KEYS:
+        return None
     g, dev = f.grid, f.coef.device
     cached = g.__dict__.setdefault("_descent", {})
     if "plan" not in cached:
@@ -692,6 +694,7 @@ def _descent_plan(f: GridFactors, V: int):
 # which the descent could read more than half takes the surface too.
 DESCENT_MIN_WORK = 600_000_000
 DESCENT_SHARE = 2
+DESCENT_MAX_KEYS = 1 << 24  # (design, pair) keys that the lists' entries hold beside a slot
 
 
 def descent(pr: PrepOut, f: GridFactors, plan, *, tile_design: torch.Tensor | None = None):

@@ -217,3 +217,18 @@ def test_bands_of_the_banded_tests_reach_their_register_history(a_max, corcut, l
     finally:
         G.set_afni_mode(False)
     assert {16: 0, 48: 16, 128: 48}[lags] < band <= lags
+
+
+def test_builds_of_more_keys_than_the_descent_holds_keep_the_surface():
+    """(design, pair) keys share a word with a slot in the descent's lists; a
+    build of more of them is searched over the surface, which has no such limit."""
+    import types
+
+    from fastfuncstuff_gb300.glm import engine
+
+    ax = torch.linspace(-0.8, 0.8, 33)
+    g = G.make_grid(ax, ax)
+    f = types.SimpleNamespace(U_hi=0, band_coef=None, P=g.P, T=100, grid=g, coef=torch.zeros(1))
+    for n, takes in (((1 << 24) // g.P, True), ((1 << 24) // g.P + 1, False)):
+        f.n_designs = n
+        assert (engine._descent_plan(f, 1_000_000) is not None) == takes
