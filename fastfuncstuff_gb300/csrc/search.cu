@@ -160,7 +160,8 @@ __device__ __forceinline__ float div_rn(float x, float d, float r) {
 // rows scaled together with their divisions and roots in four lanes, samples
 // divided by corrected products, the split four samples a lane. 200,000 voxels of
 // T = 400, K = 20 in two launches: 798 -> 658 us.
-template <bool WIDE>
+// WORD8: yr_hi and yr_lo lie on 8-byte boundaries (4-byte ones otherwise).
+template <bool WIDE, bool WORD8>
 __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kernel(ffs_prep_args a, int ld) {
   extern __shared__ float4 sm4[];
   float* Ys = reinterpret_cast<float*>(sm4);       // [32][ld]
@@ -304,13 +305,11 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kerne
       if (lane == 0) a.yexp[v] = e;
       if (!a.yr_hi) continue;
       const float4* row4 = reinterpret_cast<const float4*>(Ys + (size_t)i * ld);
-      // four samples per lane: 8-byte words of hi and lo (ld_y is a multiple of 8),
-      // 4-byte ones where the buffers start between them;
+      // four samples per lane (ld_y is a multiple of 8);
       // x * 2^e as one product when 2^e is a normal float (then the same
       // correctly rounded value as ldexpf)
       uint32_t* hi = reinterpret_cast<uint32_t*>(a.yr_hi + (size_t)v * a.ld_y);
       uint32_t* lo = reinterpret_cast<uint32_t*>(a.yr_lo + (size_t)v * a.ld_y);
-      const bool word8 = (((uintptr_t)a.yr_hi | (uintptr_t)a.yr_lo) & 7) == 0;
       const bool pw = e >= -126 && e <= 127;
       const float p2 = pw ? __int_as_float((e + 127) << 23) : 0.f;
       for (int q = lane; q < (a.ld_y >> 2); q += 32) {
@@ -322,7 +321,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, WIDE ? 2 : 3) prep_tile_kerne
         uint2 h, l;
         split_fp16x2(x.x, x.y, h.x, l.x);
         split_fp16x2(x.z, x.w, h.y, l.y);
-        if (word8) {
+        if constexpr (WORD8) {
           reinterpret_cast<uint2*>(hi)[q] = h;
           reinterpret_cast<uint2*>(lo)[q] = l;
         } else {
@@ -961,7 +960,9 @@ extern "C" int ffs_reml_prep(const ffs_prep_args* a, void* stream) {
     const size_t smem = sizeof(float) * ((size_t)TILE_V * ld + (size_t)a->K * TILE_V);
     FFS_REQUIRE(smem <= 200 * 1024 || !a->Y_ref, "ffs_reml_prep: Y_ref needs the tiled prep (T=%d too long)", a->T);
     if (smem <= 200 * 1024) {
-      auto kern = a->K > TILE_TC_K ? prep_tile_kernel<true> : prep_tile_kernel<false>;
+      const bool word8 = (((uintptr_t)a->yr_hi | (uintptr_t)a->yr_lo) & 7) == 0;
+      auto kern = a->K > TILE_TC_K ? (word8 ? prep_tile_kernel<true, true> : prep_tile_kernel<true, false>)
+                                   : (word8 ? prep_tile_kernel<false, true> : prep_tile_kernel<false, false>);
       FFS_CUDA(ensure_dyn_smem(reinterpret_cast<const void*>(kern), smem));
       kern<<<ceil_div(a->V, TILE_V), TILE_WARPS * 32, smem, (cudaStream_t)stream>>>(*a, ld);
       return check_launch("prep_tile_kernel");
