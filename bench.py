@@ -266,7 +266,8 @@ def _roofline(dom: str, ms_step: float, T: int, K: int, P: int, pk: dict, sm_mhz
                 "frac": ach / 1.25, "traffic": None, "peak_src": "nominal GB300 FP64 (not measured)",
                 "work": "FP64 X_w = L^-1 X, factor and inverse of X_w'X_w per (design, pair)"}
     if dom == "ffs_reml_descent":
-        # the pairs the selector reads on the 33 x 33 lattice: 9 of the top level, 8 more in each of 4 rounds
+        # the pairs the selector reads on the 33 x 33 lattice: 9 of the top level, 8 more in each of 4 rounds (the
+        # kernels evaluate 52: the 36 of the first three levels for every voxel, at most 16 in rounds)
         flops = V * 41 * 4.0 * T
         ach = flops / sec / 1e12
         return {"kernel": dom, "bound": "fp32", "achieved": ach, "peak": fp32_peak, "unit": "TFLOP/s",

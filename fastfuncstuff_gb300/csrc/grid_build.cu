@@ -447,8 +447,9 @@ __device__ __forceinline__ bool positive(double d) {
   return hi > 0 ? hi < 0x7ff00000 || (hi == 0x7ff00000 && __double2loint(d) == 0) : hi == 0 && __double2loint(d) != 0;
 }
 
-// The factors of v / n = u + u p, u = v r: r the fp32 reciprocal of n and
-// p = e + e^2, e = 1 - n r (error e^3 ~ 2^-72). Positive n.
+// The factors of v / n = u + u p, u = v r: r the fp32 reciprocal of n and p = e + e^2,
+// e = 1 - n r, the cubic form of the reciprocal's Newton iteration (Householder's; error
+// e^3 ~ 2^-72). Positive n.
 __device__ __forceinline__ void rcp_factors(double n, double& r, double& p) {
   const unsigned x = (unsigned)__double2hiint(n) >> 20;
   r = x - (1023u - 100u) <= 200u ? f2d_exact(__frcp_rn((float)n)) : 1.0 / n;  // 2^-100 < n < 2^100
@@ -1148,13 +1149,13 @@ __global__ void __launch_bounds__(GB_THREADS, BAND ? 2 : 4) grid_build_kernel(Bu
 // --------------------------------------------------------- Gram entries in integers
 // This GPU's FP64 pipe takes one warp instruction per 19 cycles and SM, its
 // integer multiply-add with a 64-bit sum one per cycle or better. A Gram entry
-// sum_t x_i[t] x_j[t] of FP64 series is therefore formed from 54-bit fixed-point
-// values: x = q 2^-s with s per column (|q| < 2^53, s from the column's largest
-// magnitude), q = hi 2^27 + lo with |hi|, |lo| <= 2^26, and the sums of hi hi',
+// sum_t x_i[t] x_j[t] of FP64 series is therefore formed from fixed-point values
+// x = q 2^-s, s per column, q = hi 2^27 + lo with |lo| <= 2^26, and the sums of hi hi',
 // hi lo' + lo hi' and lo lo' in 64-bit integers: exact for up to 1024 samples,
-// whatever the order. What remains is the rounding of x to the fixed point,
-// 2^-54 of the column's largest value at most twice over, where a chain of FP64
-// FMAs rounds every partial sum.
+// whatever the order. What remains is the rounding of x to the fixed point, where a
+// chain of FP64 FMAs rounds every partial sum. s comes from the column's largest
+// magnitude (|q| < 2^53, |hi| <= 2^26: the design basis, which forms all three sums) or
+// from its norm (|hi| up to 2^31: the grid build, which leaves lo lo' out).
 constexpr int FX_TMAX = 1024;
 
 // s for a column of largest magnitude mx: mx (1 + 1/32) < 2^(53 - s), the margin
@@ -1180,7 +1181,7 @@ __device__ __forceinline__ int2 fixed_of(double w, int s, bool& over) {
   return make_int2(hi, (int)(q - ((long long)hi << 27)));
 }
 
-// The sums of a Gram entry.
+// The sums of a Gram entry, for columns scaled by fixed_scale.
 struct FixedDot {
   long long hh = 0, x = 0, ll = 0;
   __device__ __forceinline__ void add(int2 a, int2 b) {
@@ -1367,8 +1368,6 @@ __host__ __device__ inline ItemPlan item_plan(int T, int K, int n_runs) {
   m.total = at;
   return m;
 }
-
-
 
 template <bool SHARED_LDL>
 __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(BuildArgs args, int n_designs,
@@ -1803,7 +1802,8 @@ __global__ void __launch_bounds__(GI_ENTRY + GI_PROD, GI_CTAS) grid_item_kernel(
 // factor in FP64, then the fp32 factors that Q and G read. So several CTAs share
 // an SM, and one's integer Gram matrix runs beside another's FP64 recursions.
 //   - X_w = L^-1 X, a lane per column and run, to fixed point (scaled by the columns'
-//     norms, without the lo lo' sums: norm_scale) and to fp32; the Gram matrix in blocks of 4 x 4 or 2 x 2 entries per thread (rows b,
+//     norms, without the lo lo' sums: norm_scale) and to fp32; the Gram matrix in
+//     blocks of 4 x 4 or 2 x 2 entries per thread (rows b,
 //     b + kb, ..., so that a warp's blocks read consecutive rows) from
 //     double-buffered chunks of WI_CS samples.
 //   - X_w'X_w = Lu D Lu' and Lu^-1 in one pass (Fold).
@@ -2517,7 +2517,8 @@ static bool too_long(const ffs_grid_desc& d) {
   return sizeof(double) * n > 200 * 1024;
 }
 
-// The item kernel of a build. grid_item_kernel has the shorter latency and
+// The item kernel of a build; the two kernels and their widths give the same bits.
+// grid_item_kernel has the shorter latency and
 // takes the builds of up to GI_KMAX columns whose items run in one wave of its
 // CTAs (two up to 16 columns); grid_wide_kernel does less work on more CTAs and
 // takes the others whose factor fits: with 128 threads while the items
