@@ -207,6 +207,8 @@ def _side_stream(device) -> torch.cuda.Stream:
     return _SIDE[key]
 
 
+WAIT_RAN_OUT = "ffs_reml_project_tc: a bounded wait expired in the search; its results are not valid"
+
 # A batch of up to this many bytes is no more than a fit allocates whatever its batch
 # (factors and workspace of the default grid: 8 MB at T = 200, K = 8), so the free
 # memory is not asked for: the query takes 35 us of a small fit's 890.
@@ -383,6 +385,8 @@ def fit_glm_arma11(
         ym = Y.to(device=device, dtype=out_dtype).mean(0, keepdim=True).float()
         so = engine.search(ym, factors, hierarchical=False, projector=_projector(factors), do_scale=False)
         best_all = so.best.expand(V).to(torch.int32).cpu()
+        if int(so._flag):
+            raise RuntimeError(WAIT_RAN_OUT)
         global_crit = so.best_crit[:1].expand(V)
     P = grid.P
     bs = _batch_size(V, T, P, K, batch_size, device)
@@ -644,7 +648,7 @@ def fit_glm_arma11(
     if pending:
         torch.cuda.current_stream(device).synchronize()
     if gave_up is not None and any(gave_up.tolist()):
-        raise RuntimeError("ffs_reml_project_tc: a bounded wait expired in the search; its results are not valid")
+        raise RuntimeError(WAIT_RAN_OUT)
     if verbose:
         print(f"ARMA(1,1) REML: {V:,} voxels x {P} pairs, T={T}, K={K} on {torch.cuda.get_device_name(device)}")
     return res

@@ -120,7 +120,7 @@ def test_the_descent_takes_the_series_that_the_surface_takes(T, takes):
 
 
 @gpu
-@pytest.mark.parametrize("path", ["surface", "descent", "grouped"])
+@pytest.mark.parametrize("path", ["surface", "descent", "grouped", "global"])
 def test_a_wait_that_ran_out_in_the_search_is_reported(path, monkeypatch):
     """The projection kernels leave at once when their flag is set, as they do
     after a wait that ran out: results for the host raise, and the descent's
@@ -137,7 +137,7 @@ def test_a_wait_that_ran_out_in_the_search_is_reported(path, monkeypatch):
         if path == "grouped":
             return fit_glm_arma11_grouped(Y, {0: X, 1: X[::-1].copy()}, np.arange(300) % 2, tr=2.0, cuda_graphs=False,
                                           **kw, **more)
-        return fit_glm_arma11(Y, X, tr=2.0, **kw, **more)
+        return fit_glm_arma11(Y, X, tr=2.0, estimate_per_voxel=path != "global", **kw, **more)
 
     assert torch.isfinite(fit().reml_likelihood).all()
     real = torch.zeros
@@ -148,7 +148,7 @@ def test_a_wait_that_ran_out_in_the_search_is_reported(path, monkeypatch):
     monkeypatch.setattr(engine.torch, "zeros", preset)
     with pytest.raises(RuntimeError, match="bounded wait"):
         fit()
-    if path != "surface":
+    if path in ("descent", "grouped"):
         assert torch.isnan(fit(return_device=True).reml_likelihood).all()
 
 
