@@ -305,3 +305,26 @@ def test_design_basis_is_the_grid_builds_to_rounding(T, K, runs):
     q0 = engine.design_basis(Xd)
     torch.cuda.synchronize()
     assert float((q0 - f.U[g.p0]).abs().max()) <= K * 2.0**-22 * float(q0.abs().max())
+
+
+@gpu
+@pytest.mark.parametrize("T,K,n", [(200, 8, None), (300, 20, 33), (400, 24, 3), (600, 70, 3)])
+@pytest.mark.parametrize("low,high", [(-10, 10), (-17, 17)])
+def test_columns_of_any_magnitude(T, K, n, low, high):
+    """Columns from 10^low to 10^high: within the fixed point's norms and past
+    them (the general phases). The basis does not depend on the columns'
+    magnitudes: U against dense float64 (condition below 30 without them)."""
+    from fastfuncstuff_gb300.glm import engine
+
+    rng = np.random.default_rng(K)
+    mag = 10.0 ** np.linspace(low, high, K)
+    X = (rng.standard_normal((T, K)) * rng.permutation(mag)).astype(np.float32)
+    ax = G.get_default_arma_grids() if n is None else (torch.linspace(-0.8, 0.8, n),) * 2
+    g = G.make_grid(*ax, use_double=True)
+    f = engine.build_factors(torch.from_numpy(X).to(DEV), g, G.run_layout(T, [0]), with_tc=True)
+    torch.cuda.synchronize()
+    assert (f.info.cpu().numpy() == 0).all()
+    for p in range(0, g.P, max(1, g.P // 4)):
+        scaled = X.astype(np.float64) / np.linalg.norm(X.astype(np.float64), axis=0)
+        U = dense_factors(scaled, g.a[p], g.b[p], [0])[2]
+        assert np.abs(f.U[p, :, :T].cpu().numpy() - U).max() <= max(1e-5, K * 2.0**-24 * 30) * np.abs(U).max()
