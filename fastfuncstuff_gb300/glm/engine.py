@@ -669,7 +669,12 @@ def prep(Y: torch.Tensor, f: GridFactors, *, do_scale: bool = True, tensor_core:
 def _descent_plan(f: GridFactors, V: int):
     """The device arrays of the grid's descent plan when ``V`` voxels are
     better searched by it than over the full surface, else None."""
-    if f.U_hi is None or f.band_coef is not None or V * f.P * f.T < DESCENT_MIN_WORK:
+    if f.U_hi is None or f.band_coef is not None:
+        return None
+    work = V * f.P * f.T
+    if f.n_designs == 1:
+        work = work * (min(f.K, 100) + 10) // 67
+    if work < DESCENT_MIN_WORK:
         return None
     if f.P * f.n_designs >= DESCENT_MAX_KEYS:
         return None
@@ -686,12 +691,17 @@ def _descent_plan(f: GridFactors, V: int):
     return plan, cached[str(dev)]
 
 
-# The descent takes about twenty launches where the full surface takes three:
-# below this many voxels x pairs x samples the surface is no slower (search of
-# V voxels, us, descent / surface: 117 pairs, T = 400: V = 8,000 213 / 192,
-# 16,000 328 / 339; 561 pairs, T = 400: 2,000 267 / 208, 4,000 275 / 329,
-# 200,000 2656 / 12052; T = 200: 4,000 211 / 194, 8,000 220 / 317). A grid of
-# which the descent could read more than half takes the surface too.
+# The descent takes about twenty launches where the full surface takes three, 45 us
+# of host time: a small fit, which waits for the host, is slower by them although its
+# search on the device is faster. Fits of one design, us, descent / surface, by
+# W = voxels x pairs x samples (545 pairs, T = 400): K = 14: W = 6e8 831 / 788, 1.1e9
+# 824 / 787, 2.2e9 831 / 899; K = 20: 1.1e9 828 / 810, 1.5e9 841 / 905; K = 30: 4.5e8 831 /
+# 775, 8e8 840 / 886; T = 300, K = 100: 3e8 2381 / 2458, 8e8 2432 / 2881; 117 and 225 pairs
+# the same within 20% of W. The projection's share grows with K, and so does what
+# the device does beside: the line is W (K + 10) = 4e10, K up to 100. Grouped fits,
+# whose surface also needs a work list of the host's, are 10% faster by the descent
+# from W = 6e8 on (1,781 / 1,959 at K = 14, 4 designs). A grid of which the descent could
+# read more than half takes the surface too.
 DESCENT_MIN_WORK = 600_000_000
 DESCENT_SHARE = 2
 DESCENT_MAX_KEYS = 1 << 24  # (design, pair) keys that the lists' entries hold beside a slot

@@ -228,7 +228,24 @@ def test_builds_of_more_keys_than_the_descent_holds_keep_the_surface():
 
     ax = torch.linspace(-0.8, 0.8, 33)
     g = G.make_grid(ax, ax)
-    f = types.SimpleNamespace(U_hi=0, band_coef=None, P=g.P, T=100, grid=g, coef=torch.zeros(1))
+    f = types.SimpleNamespace(U_hi=0, band_coef=None, P=g.P, T=100, K=5, grid=g, coef=torch.zeros(1))
     for n, takes in (((1 << 24) // g.P, True), ((1 << 24) // g.P + 1, False)):
         f.n_designs = n
         assert (engine._descent_plan(f, 1_000_000) is not None) == takes
+
+
+@pytest.mark.parametrize("K,D,work", [(8, 1, 2.24e9), (14, 1, 1.68e9), (20, 1, 1.34e9), (30, 1, 1.01e9), (100, 1, 3.66e8),
+                                      (130, 1, 3.66e8), (14, 4, 6.0e8), (100, 4, 6.0e8)])
+def test_work_from_which_a_search_takes_the_descent(K, D, work):
+    """Voxels x pairs x samples from which the descent is chosen: by the columns
+    for one design, whose small fits wait for the host, and a fixed line for
+    grouped ones."""
+    import types
+
+    from fastfuncstuff_gb300.glm import engine
+
+    ax = torch.linspace(-0.8, 0.8, 33)
+    g = G.make_grid(ax, ax)
+    f = types.SimpleNamespace(U_hi=0, band_coef=None, P=g.P, T=400, K=K, grid=g, coef=torch.zeros(1), n_designs=D)
+    for share, takes in ((0.98, False), (1.02, True)):
+        assert (engine._descent_plan(f, int(share * work / (g.P * 400))) is not None) == takes
